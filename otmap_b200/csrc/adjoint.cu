@@ -9,11 +9,10 @@
 //   J^T lambda = G^T q,  J = dA/dpsi = (dA/dg) G      (mean-zero subspace: J 1 = 0, 1^T J = 0)
 //   dL/drho~  = e^2 lambda
 //   dL/drho   = (lambda - (lambda . rho) / S) / S,  S = sum(rho)   (ratio clamp inactive)
-// J^T is applied matrix-free: k_adj_vertex forms h_v = sum_c lambda_c dA_c/dg_v over the four
-// cells around each vertex (dA_c/dD1 = (D2y, -D2x)/2, dA_c/dD2 = (-D1y, D1x)/2 with the
-// cell diagonals D1 = g11 - g00 + (e,e), D2 = g01 - g10 + (-e,e)), and k_adj_cells gathers
-// (G^T h)_f over every vertex whose clamped gradient stencil touches cell f. Both are
-// deterministic gathers. lambda solves J^T lambda = b by restarted GMRES right-
+// J^T is applied matrix-free (jt_cell): h_v = sum_c lambda_c dA_c/dg_v over the four cells
+// around each vertex (dA_c/dD1 = (D2y, -D2x)/2, dA_c/dD2 = (-D1y, D1x)/2 with the cell
+// diagonals D1 = g11 - g00 + (e,e), D2 = g01 - g10 + (-e,e)), then (G^T h)_f over every vertex
+// whose clamped gradient stencil touches cell f. Both are deterministic gathers. lambda solves J^T lambda = b by restarted GMRES right-
 // preconditioned with the pseudo-inverse of M (the reference's pseudo-Laplacian; J = -M at
 // psi = 0), using the same cosine-transform Poisson solve as the forward loop; the
 // one-step mode stops at lambda = -M^+ b (one Poisson solve). For strongly deformed maps
@@ -34,74 +33,31 @@ __device__ __forceinline__ int clampv(int v, int n) { return v < 0 ? 0 : (v >= n
 // Device state of one restart cycle of the Krylov solve. The cycle's Arnoldi steps run on
 // the device (a CUDA graph with a WHILE node, or the same kernels launched one step at a
 // time): every step kernel reads the step index j here instead of taking it as a launch
-// argument, and the Givens kernel advances it and decides whether the cycle goes on.
+// argument; the last kernel of a step advances it and decides whether the cycle goes on.
 struct AdjCtl {
   int j;       // the step being taken: basis vectors 0..j are orthonormal
   int go;      // the cycle takes another step
   int m;       // restart length
   int budget;  // steps allowed in this cycle (the call's cap on Poisson solves)
   double bnorm, tol;
+  double rnorm;          // norm of the vector last formed by k_adj_resid
+  unsigned int counter;  // block ticket of the running kernel
+  int fault;             // the steps' transform gave up a bounded wait
 };
 
-// Displacement g of vertex (i, j) from the forward mesh.
-__device__ __forceinline__ double2 disp(const double* fwd, int n, int i, int j) {
-  const size_t v = (size_t)j + (size_t)i * (n + 1);
-  const double dx = 1.0 / (double)n;
-  return make_double2(fwd[2 * v] - (double)i * dx, fwd[2 * v + 1] - (double)j * dx);
-}
-
-// Diagonals of cell (ci, cj).
-__device__ __forceinline__ void cell_diags(const double* fwd, int n, int ci, int cj, double2& D1, double2& D2) {
-  const double e = 1.0 / (double)n;
-  double2 g00 = disp(fwd, n, ci, cj), g10 = disp(fwd, n, ci + 1, cj), g01 = disp(fwd, n, ci, cj + 1),
-          g11 = disp(fwd, n, ci + 1, cj + 1);
-  D1 = make_double2(g11.x - g00.x + e, g11.y - g00.y + e);
-  D2 = make_double2(g01.x - g10.x - e, g01.y - g10.y + e);
-}
-
-// h_v = sum over the cells c around vertex v of lambda_c dA_c / dg_v.
-__global__ void k_adj_vertex(int n, const double* fwd, const double* lambda, double* h) {
+// Displacements g of the vertices from the forward mesh.
+__global__ void k_adj_disp(int n, const double* fwd, double2* g) {
   const long v = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long V = (long)(n + 1) * (n + 1);
-  if (v >= V) return;
-  const int vi = (int)(v / (n + 1)), vj = (int)(v % (n + 1));
-  double hx = 0.0, hy = 0.0;
-  double2 D1, D2;
-  if (vi < n && vj < n) {  // v00 of cell (vi, vj): -dA/dD1
-    cell_diags(fwd, n, vi, vj, D1, D2);
-    const double l = 0.5 * lambda[(size_t)vi * n + vj];
-    hx += l * -D2.y;
-    hy += l * D2.x;
-  }
-  if (vi > 0 && vj < n) {  // v10 of cell (vi-1, vj): -dA/dD2
-    cell_diags(fwd, n, vi - 1, vj, D1, D2);
-    const double l = 0.5 * lambda[(size_t)(vi - 1) * n + vj];
-    hx += l * D1.y;
-    hy += l * -D1.x;
-  }
-  if (vi < n && vj > 0) {  // v01 of cell (vi, vj-1): dA/dD2
-    cell_diags(fwd, n, vi, vj - 1, D1, D2);
-    const double l = 0.5 * lambda[(size_t)vi * n + vj - 1];
-    hx += l * -D1.y;
-    hy += l * D1.x;
-  }
-  if (vi > 0 && vj > 0) {  // v11 of cell (vi-1, vj-1): dA/dD1
-    cell_diags(fwd, n, vi - 1, vj - 1, D1, D2);
-    const double l = 0.5 * lambda[(size_t)(vi - 1) * n + vj - 1];
-    hx += l * D2.y;
-    hy += l * -D2.x;
-  }
-  h[2 * v] = hx;
-  h[2 * v + 1] = hy;
+  if (v >= (long)(n + 1) * (n + 1)) return;
+  const double dx = 1.0 / (double)n;
+  g[v] = make_double2(fwd[2 * v] - (double)(v / (n + 1)) * dx, fwd[2 * v + 1] - (double)(v % (n + 1)) * dx);
 }
 
 // (G^T h)_f: vertex (vi, vj) reads cells (clamp(vi-1+a), clamp(vj-1+b)), a, b in {0, 1},
 // with gx coefficient (2a-1) n/2 and gy coefficient (2b-1) n/2
 // (otsolver_2dgrid.cpp:379-422 with clamped indices). Cell (i, j) collects every
-// (vertex, a, b) whose clamped position is (i, j); out = scale * G^T h (+ add).
-__global__ void k_adj_cells(int n, const double* h, double scale, const double* add, double* out,
-                            const AdjCtl* ctl, long ld) {
-  if (ctl) out += (size_t)(ctl->j + 1) * ld;  // the new basis vector of the step
+// (vertex, a, b) whose clamped position is (i, j).
+__global__ void k_adj_cells(int n, const double* h, double* out) {
   const long f = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= (long)n * n) return;
   const int i = (int)(f / n), j = (int)(f % n);
@@ -123,90 +79,290 @@ __global__ void k_adj_cells(int n, const double* h, double scale, const double* 
       const size_t v = (size_t)cj[q] + (size_t)ri[p] * (n + 1);
       acc += hw * ((2 * ra[p] - 1) * h[2 * v] + (2 * cb[q] - 1) * h[2 * v + 1]);
     }
-  out[f] = scale * acc + (add ? add[f] : 0.0);
+  out[f] = acc;
 }
 
-// partial[b * (m+1) + i] = sum over this block's cells of w . V_i, i < m (basis vectors
-// stored contiguously with stride `ld`), and partial[b * (m+1) + m] = w . w. The dot
-// products are formed DOT_CHUNK at a time in one pass over the cells (w read once per
-// chunk), each a per-thread FMA chain over the grid-stride cells, then reduced together.
-// With ctl: w is basis vector j + 1 and m = j + 1 (or 0: w . w alone, for norm_only).
-constexpr int DOT_CHUNK = 8;
-__global__ void k_adj_multidot(long N, const double* w, const double* V, long ld, int m, double* partial,
-                               const AdjCtl* ctl, int norm_only) {
-  __shared__ double red[32 * DOT_CHUNK];
-  if (ctl) {
-    w = V + (size_t)(ctl->j + 1) * ld;
-    m = norm_only ? 0 : ctl->j + 1;
+// ---- the Arnoldi step ----
+//
+// After z = M^+ v_j a step is four kernels: w = J^T z with its products with v_0..v_j
+// (k_adj_apply), the first Gram-Schmidt update with the products of the second
+// (k_adj_orth), the second update with the norm, the Givens rotation and the loop test
+// (k_adj_norm), and the normalisation (k_adj_scale_by). At 256^2 a step is bound by the
+// latency of launches and grid-wide reductions, not by the basis it reads from L2 (10 MB a
+// pass on average), so every reduction ends in the last block of the kernel that forms its
+// terms. Against one kernel per operation (source, vertices, cells, 3 x products, 3 x
+// one-block sums, 2 x update, scale, rotation) a step with its transform went from 96 to
+// 59 us at 256^2 (four concurrent ones: 147 to 83), from 159 to 92 us at 512^2.
+//
+// Cell f belongs to block (f / 256) mod 256 and thread f mod 256; a thread's cells (one for
+// N <= 65536) follow each other 65536 apart. A product is an FMA chain over a thread's cells,
+// a fixed tree over the block's threads and a sum over the blocks in block order: the order
+// is that of a grid of 256 blocks whatever the grid launched, so results do not depend on
+// the device.
+
+constexpr int AT = 256;         // threads per block
+constexpr int ANB = 256;        // blocks (fewer when the cells run out)
+constexpr int ADJ_MAX_M = 200;  // largest restart length
+constexpr int DOT_CHUNK = 8;    // products formed per pass over a thread's cells
+
+// (J^T lambda)_f of cell (i, j), gathered from the 3 x 3 cells and 4 x 4 vertices around it
+// (g: vertex displacements). h_v = sum over the cells c around vertex v of
+// lambda_c dA_c / dg_v: v00 of the cell at (vi, vj) takes -dA/dD1, v10 of (vi-1, vj) -dA/dD2,
+// v01 of (vi, vj-1) dA/dD2, v11 of (vi-1, vj-1) dA/dD1.
+__device__ __forceinline__ double jt_cell(int n, const double2* g, const double* lambda, int i, int j) {
+  const double e = 1.0 / (double)n, hw = 0.5 * (double)n;
+  double2 d1[3][3], d2[3][3];  // lambda/2 D1 and lambda/2 D2 of the cells around (i, j)
+  double2 p[2][4];             // vertex rows i-1+r, i+r
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const int vi = i - 1, vj = j - 1 + c;
+    p[0][c] = vi >= 0 && vj >= 0 && vj <= n ? g[(size_t)vi * (n + 1) + vj] : make_double2(0.0, 0.0);
   }
-  const int P = m + 1;
-  for (int i0 = 0; i0 < P; i0 += DOT_CHUNK) {
-    double s[DOT_CHUNK];
 #pragma unroll
-    for (int c = 0; c < DOT_CHUNK; ++c) s[c] = 0.0;
-    for (long f = (long)blockIdx.x * blockDim.x + threadIdx.x; f < N; f += (long)gridDim.x * blockDim.x) {
-      const double wf = w[f];
+  for (int r = 0; r < 3; ++r) {
 #pragma unroll
-      for (int c = 0; c < DOT_CHUNK; ++c) {
-        const int i = i0 + c;
-        if (i < P) s[c] = fma(wf, i < m ? V[(size_t)i * ld + f] : wf, s[c]);
-      }
+    for (int c = 0; c < 4; ++c) {
+      const int vi = i + r, vj = j - 1 + c;
+      p[(r + 1) & 1][c] = vi <= n && vj >= 0 && vj <= n ? g[(size_t)vi * (n + 1) + vj] : make_double2(0.0, 0.0);
     }
-    block_sum<DOT_CHUNK>(s, red);
-    if (threadIdx.x == 0)
 #pragma unroll
-      for (int c = 0; c < DOT_CHUNK; ++c)
-        if (i0 + c < P) partial[(size_t)blockIdx.x * P + i0 + c] = s[c];
+    for (int c = 0; c < 3; ++c) {
+      const int ci = i - 1 + r, cj = j - 1 + c;
+      const double l = ci >= 0 && cj >= 0 && ci < n && cj < n ? 0.5 * lambda[(size_t)ci * n + cj] : 0.0;
+      const double2 g00 = p[r & 1][c], g01 = p[r & 1][c + 1], g10 = p[(r + 1) & 1][c], g11 = p[(r + 1) & 1][c + 1];
+      d1[r][c] = make_double2(l * (g11.x - g00.x + e), l * (g11.y - g00.y + e));
+      d2[r][c] = make_double2(l * (g01.x - g10.x - e), l * (g01.y - g10.y + e));
+    }
+  }
+  double2 h[2][2];  // vertices (i, j) .. (i+1, j+1)
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+      h[a][b] = make_double2(((d1[a][b + 1].y - d2[a + 1][b + 1].y) - d1[a + 1][b].y) + d2[a][b].y,
+                             ((d2[a + 1][b + 1].x - d1[a][b + 1].x) + d1[a + 1][b].x) - d2[a][b].x);
+  // k_adj_cells' gather: vertex rows (i+1, a = 0), (i, a = 1) and, at the border, the clamped ones
+  double acc = 0.0;
+  auto add = [&](const double2& v, int a, int b) { acc += hw * ((a ? v.x : -v.x) + (b ? v.y : -v.y)); };
+  auto row = [&](const double2 (&v)[2], int a) {
+    add(v[1], a, 0);
+    add(v[0], a, 1);
+    if (j == 0) add(v[0], a, 0);
+    if (j == n - 1) add(v[1], a, 1);
+  };
+  row(h[1], 0);
+  row(h[0], 1);
+  if (i == 0) row(h[0], 0);
+  if (i == n - 1) row(h[1], 1);
+  return acc;
+}
+
+// Warp totals of s[0..7], each by the tree of warp_sum; afterwards s[0] on lane l is the
+// total of value 4 (l>>4 & 1) + 2 (l>>3 & 1) + (l>>2 & 1). Nine shuffles instead of the 40
+// of eight separate trees.
+__device__ __forceinline__ void warp_sum8(double (&s)[8], int lane) {
+#pragma unroll
+  for (int o = 16, h = 4; h >= 1; o >>= 1, h >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int q = 0; q < h; ++q) {
+      const double send = up ? s[q] : s[q + h], keep = up ? s[q + h] : s[q];
+      s[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  s[0] += __shfl_xor_sync(0xffffffffu, s[0], 2);
+  s[0] += __shfl_xor_sync(0xffffffffu, s[0], 1);
+}
+
+// block_sum's tree over the eight warps' values.
+__device__ __forceinline__ double sum_warps(const double* r, int stride) {
+  static_assert(AT / 32 == 8, "eight warps");
+  return ((r[0] + r[4 * stride]) + (r[2 * stride] + r[6 * stride])) +
+         ((r[stride] + r[5 * stride]) + (r[3 * stride] + r[7 * stride]));
+}
+
+// partial[i * ANB + block] = this block's part of w . V_i, i < P. The loads of a thread's
+// next chunk of vectors are issued before the current chunk is reduced.
+constexpr int RED_LD = ADJ_MAX_M + 8;
+__device__ __forceinline__ void block_dots(long N, const double* w, const double* V, long ld, int P, double* red,
+                                           double* partial) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long f0 = (long)blockIdx.x * AT + threadIdx.x;
+  if (N <= (long)ANB * AT) {  // one cell per thread
+    const bool in = f0 < N;
+    const double wf = in ? w[f0] : 0.0;
+    double v[DOT_CHUNK];
+    auto fetch = [&](int i0) {
+#pragma unroll
+      for (int c = 0; c < DOT_CHUNK; ++c) v[c] = in && i0 + c < P ? V[(size_t)(i0 + c) * ld + f0] : 0.0;
+    };
+    fetch(0);
+    for (int i0 = 0; i0 < P; i0 += DOT_CHUNK) {
+      double s[DOT_CHUNK];
+#pragma unroll
+      for (int c = 0; c < DOT_CHUNK; ++c) s[c] = fma(wf, v[c], 0.0);
+      fetch(i0 + DOT_CHUNK);
+      warp_sum8(s, lane);
+      const int i = i0 + ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+      if ((lane & 3) == 0 && i < P) red[warp * RED_LD + i] = s[0];
+    }
+  } else {
+    for (int i0 = 0; i0 < P; i0 += DOT_CHUNK) {
+      double s[DOT_CHUNK];
+#pragma unroll
+      for (int c = 0; c < DOT_CHUNK; ++c) s[c] = 0.0;
+#pragma unroll 2
+      for (long f = f0; f < N; f += (long)ANB * AT) {
+        const double wf = w[f];
+#pragma unroll
+        for (int c = 0; c < DOT_CHUNK; ++c)
+          if (i0 + c < P) s[c] = fma(wf, V[(size_t)(i0 + c) * ld + f], s[c]);
+      }
+      warp_sum8(s, lane);
+      const int i = i0 + ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+      if ((lane & 3) == 0 && i < P) red[warp * RED_LD + i] = s[0];
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < P; i += AT) partial[(size_t)i * ANB + blockIdx.x] = sum_warps(red + i, RED_LD);
+}
+
+// Last block: out(i, total) for the P totals of the blocks' partials, each summed in block
+// order by one thread from a staged copy (TOT_CHUNK values at a time).
+constexpr int TOT_CHUNK = 16, TOT_LD = ANB + 1;
+template <class F>
+__device__ __forceinline__ void totals(const double* partial, int P, double* stage, F out) {
+  const int nb = gridDim.x;
+  for (int i0 = 0; i0 < P; i0 += TOT_CHUNK) {
+    const int cnt = min(TOT_CHUNK, P - i0);
+    __syncthreads();
+    if (threadIdx.x < nb) {
+#pragma unroll
+      for (int c = 0; c < TOT_CHUNK; ++c)
+        if (c < cnt) stage[c * TOT_LD + threadIdx.x] = __ldcg(&partial[(size_t)(i0 + c) * ANB + threadIdx.x]);
+    }
+    __syncthreads();
+    if (threadIdx.x < cnt) {
+      double t = 0.0;
+#pragma unroll 16
+      for (int b = 0; b < nb; ++b) t += stage[threadIdx.x * TOT_LD + b];
+      out(i0 + threadIdx.x, t);
+    }
   }
 }
 
-// The block partials of k_adj_multidot summed in block order (thread i: entry i).
-__device__ __forceinline__ double sum_partials(const double* partial, int nblocks, int P, int i) {
-  double t = 0.0;
-  for (int b = 0; b < nblocks; ++b) t += partial[(size_t)b * P + i];
-  return t;
+// w = V_{j+1} = J^T z (z = M^+ v_j); Hessenberg column and combine coefficients c_i of the
+// first Gram-Schmidt pass.
+__global__ __launch_bounds__(AT) void k_adj_apply(int n, const double2* g, const double* z, double* V, long ld,
+                                                  AdjCtl* ctl, double* partial, double* hcol, double* c) {
+  __shared__ double red[AT / 32 * RED_LD], stage[TOT_CHUNK * TOT_LD];
+  if (!ctl->go) return;
+  const int j = ctl->j, P = j + 1;
+  const long N = (long)n * n;
+  double* w = V + (size_t)(j + 1) * ld;
+  for (long f = (long)blockIdx.x * AT + threadIdx.x; f < N; f += (long)ANB * AT)
+    w[f] = jt_cell(n, g, z, (int)(f / n), (int)(f % n));
+  block_dots(N, w, V, ld, P, red, partial);
+  if (!last_block(&ctl->counter, gridDim.x)) return;
+  totals(partial, P, stage, [&](int i, double d) {
+    c[i] = d;
+    hcol[i] = 0.0 + d;
+  });
 }
 
-// Gram-Schmidt pass over basis vectors 0..j: c_i = <w, v_i> (for the combine) and the
-// Hessenberg column entry H_ij accumulated over the two passes (pass 0 sets it).
-__global__ void k_adj_orth_reduce(const double* partial, int nblocks, int j, int pass, double* hcol, double* c,
-                                  const AdjCtl* ctl) {
-  if (ctl) j = ctl->j;
-  const int i = threadIdx.x;
-  if (i > j) return;
-  const double d = sum_partials(partial, nblocks, j + 2, i);
-  c[i] = d;
-  hcol[i] = (pass ? hcol[i] : 0.0) + d;
-}
-
-// |w| after the passes: H_{j+1,j} and the factor that normalises w (0 when |w| = 0).
-__global__ void k_adj_norm_reduce(const double* partial, int nblocks, int j, double* hcol, double* inv,
-                                  const AdjCtl* ctl) {
-  if (threadIdx.x != 0) return;
-  if (ctl) j = ctl->j;
-  const double hn = sqrt(sum_partials(partial, nblocks, 1, 0));
-  hcol[j + 1] = hn;
-  *inv = hn > 0 ? 1.0 / hn : 1.0;
-}
-
-__global__ void k_adj_scale_by(long N, double* v, const double* a, const AdjCtl* ctl, long ld) {
-  if (ctl) v += (size_t)(ctl->j + 1) * ld;
-  const long f = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (f < N) v[f] *= *a;
-}
-
-// w = a * w - sum_i c_i V_i (i < m); c in device memory; with ctl, w = V_{j+1} and m = j + 1
-__global__ void k_adj_combine(long N, double* w, double a, const double* V, long ld, int m, const double* c,
-                              const AdjCtl* ctl) {
-  if (ctl) {
-    w = const_cast<double*>(V) + (size_t)(ctl->j + 1) * ld;
-    m = ctl->j + 1;
+// w -= sum_i c_i V_i at this thread's cells; returns the chain of the new w^2 there.
+__device__ __forceinline__ double combine(long N, double* w, const double* V, long ld, int P, const double* c,
+                                          double* sc) {
+  for (int i = threadIdx.x; i < P; i += AT) sc[i] = c[i];
+  __syncthreads();
+  double ss = 0.0;
+  for (long f = (long)blockIdx.x * AT + threadIdx.x; f < N; f += (long)ANB * AT) {
+    double x = w[f];
+#pragma unroll 16
+    for (int i = 0; i < P; ++i) x = fma(-sc[i], V[(size_t)i * ld + f], x);
+    w[f] = x;
+    ss = fma(x, x, ss);
   }
+  return ss;
+}
+
+// First Gram-Schmidt update and the products of the second pass.
+__global__ __launch_bounds__(AT) void k_adj_orth(int n, double* V, long ld, AdjCtl* ctl, double* partial, double* hcol,
+                                                 double* c) {
+  __shared__ double sc[ADJ_MAX_M + 8], red[AT / 32 * RED_LD], stage[TOT_CHUNK * TOT_LD];
+  if (!ctl->go) return;
+  const int j = ctl->j, P = j + 1;
+  const long N = (long)n * n;
+  double* w = V + (size_t)(j + 1) * ld;
+  combine(N, w, V, ld, P, c, sc);
+  block_dots(N, w, V, ld, P, red, partial);
+  if (!last_block(&ctl->counter, gridDim.x)) return;
+  totals(partial, P, stage, [&](int i, double d) {
+    c[i] = d;
+    hcol[i] = hcol[i] + d;
+  });
+}
+
+// Second Gram-Schmidt update and H_{j+1,j} = |w|; then, on one thread, the end of step j: the
+// previous Givens rotations applied to the new Hessenberg column, the rotation that zeroes
+// H_{j+1,j}, the updated residual estimate |g_{j+1}|, and the loop test: go on while it is
+// above tol * |b|, the new basis vector is non-zero, the cycle has room, the call's budget
+// is not spent and the transform has not given up a wait. H is (m+1) x m, row-major. The
+// Poisson record of the next step gets its source.
+__global__ __launch_bounds__(AT) void k_adj_norm(int n, double* V, long ld, AdjCtl* ctl, double* inv, double* partial,
+                                                 const double* hcol, const double* c, double* H, double* cs, double* sn,
+                                                 double* gv, Inst* rec, cudaGraphConditionalHandle handle,
+                                                 int in_graph) {
+  __shared__ double sc[ADJ_MAX_M + 8], sh[ADJ_MAX_M + 8], ss[ADJ_MAX_M + 8], red[64], stage[TOT_CHUNK * TOT_LD];
+  if (!ctl->go) return;
+  const int j = ctl->j, P = j + 1;
+  const long N = (long)n * n;
+  double v[1] = {combine(N, V + (size_t)(j + 1) * ld, V, ld, P, c, sc)};
+  block_sum<1>(v, red);
+  if (threadIdx.x == 0) partial[blockIdx.x] = v[0];
+  if (!last_block(&ctl->counter, gridDim.x)) return;
+  for (int i = threadIdx.x; i < j; i += AT) {
+    sc[i] = cs[i];
+    ss[i] = sn[i];
+  }
+  for (int i = threadIdx.x; i <= j; i += AT) sh[i] = hcol[i];
+  const int m = ctl->m;
+  totals(partial, 1, stage, [&](int, double w2) {
+    const double hn = sqrt(w2);
+    double x = sh[0];
+    for (int i = 0; i < j; ++i) {
+      const double y = sh[i + 1];
+      sh[i] = sc[i] * x + ss[i] * y;
+      x = -ss[i] * x + sc[i] * y;
+    }
+    const double den = hypot(x, hn);
+    const double cj = den > 0 ? x / den : 1.0, sj = den > 0 ? hn / den : 0.0;
+    sh[j] = den;
+    cs[j] = cj;
+    sn[j] = sj;
+    const double gj = gv[j], gk = -sj * gj;
+    gv[j + 1] = gk;
+    gv[j] = cj * gj;
+    *inv = hn > 0 ? 1.0 / hn : 1.0;
+    const int k = j + 1;
+    const int go = (fabs(gk) / ctl->bnorm > ctl->tol) && hn != 0 && k < m && k < ctl->budget && !rec->fault;
+    ctl->j = k;
+    ctl->go = go;
+    rec->r[0] = V + (size_t)k * ld;
+    rec->active = go;
+    ctl->fault = rec->fault;
+    if (in_graph) cudaGraphSetConditional(handle, go ? 1u : 0u);
+  });
+  __syncthreads();
+  for (int i = threadIdx.x; i <= j; i += AT) H[(size_t)i * m + j] = sh[i];
+}
+
+// v_j = w / |w|, the vector k_adj_norm has just moved the cycle on to (the last one of a
+// cycle is not used).
+__global__ void k_adj_scale_by(long N, double* V, long ld, const double* a, const AdjCtl* ctl) {
+  if (!ctl->go) return;
   const long f = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= N) return;
-  double x = a * w[f];
-  for (int i = 0; i < m; ++i) x = fma(-c[i], V[(size_t)i * ld + f], x);
-  w[f] = x;
+  if (f < N) V[(size_t)ctl->j * ld + f] *= *a;
 }
 
 // Every Poisson record of the workspace ready for a new call: a bounded wait that gave up in
@@ -219,85 +375,79 @@ __global__ void k_adj_reset_recs(Inst* recs, int count) {
   }
 }
 
-// The Poisson record of the step reads basis vector j.
-__global__ void k_adj_set_src(Inst* rec, double* V, long ld, const AdjCtl* ctl) {
-  if (threadIdx.x == 0) rec->r[0] = V + (size_t)ctl->j * ld;
-}
-
-// Start of a restart cycle: residual norm rnorm in g_0.
-__global__ void k_adj_cycle_init(AdjCtl* ctl, double* gv, int m, double rnorm, double bnorm, double tol, int budget) {
-  if (threadIdx.x != 0) return;
+// Start of a restart cycle from the vector in V_0, whose norm k_adj_resid left in the state:
+// v_0, g and the cycle's state.
+__global__ void k_adj_cycle_init(long N, AdjCtl* ctl, double* gv, int m, double bnorm, double tol, int budget,
+                                 Inst* rec, double* V) {
+  const double rnorm = ctl->rnorm, a = 1.0 / rnorm;
+  const long f = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (f < N) V[f] *= a;
+  if (f <= m) gv[f] = f ? 0.0 : rnorm;
+  if (f != 0) return;
   ctl->j = 0;
   ctl->go = budget > 0 ? 1 : 0;
   ctl->m = m;
   ctl->budget = budget;
   ctl->bnorm = bnorm;
   ctl->tol = tol;
-  gv[0] = rnorm;
-  for (int i = 1; i <= m; ++i) gv[i] = 0.0;
+  ctl->fault = rec->fault;
+  rec->r[0] = V;
+  if (!rec->fault) rec->active = 1;
 }
 
-// End of Arnoldi step j (one thread): the new Hessenberg column, the previous Givens
-// rotations applied to it, the rotation that zeroes H_{j+1,j}, the updated residual
-// estimate |g_{j+1}|, and the loop test: go on while it is above tol * |b|, the new basis
-// vector is non-zero, the cycle has room and the call's budget is not spent. H is
-// (m+1) x m, row-major.
-__global__ void k_adj_givens(AdjCtl* ctl, const double* hcol, double* H, double* cs, double* sn, double* gv,
-                             cudaGraphConditionalHandle handle, int in_graph) {
-  if (threadIdx.x != 0) return;
-  const int j = ctl->j, m = ctl->m;
-  auto Hs = [&](int i, int c) -> double& { return H[(size_t)i * m + c]; };
-  for (int i = 0; i <= j + 1; ++i) Hs(i, j) = hcol[i];
-  const double hn = hcol[j + 1];
-  for (int i = 0; i < j; ++i) {
-    const double t = cs[i] * Hs(i, j) + sn[i] * Hs(i + 1, j);
-    Hs(i + 1, j) = -sn[i] * Hs(i, j) + cs[i] * Hs(i + 1, j);
-    Hs(i, j) = t;
-  }
-  const double den = hypot(Hs(j, j), Hs(j + 1, j));
-  cs[j] = den > 0 ? Hs(j, j) / den : 1.0;
-  sn[j] = den > 0 ? Hs(j + 1, j) / den : 0.0;
-  Hs(j, j) = den;
-  Hs(j + 1, j) = 0.0;
-  gv[j + 1] = -sn[j] * gv[j];
-  gv[j] = cs[j] * gv[j];
-  const int k = j + 1;
-  const int go = (fabs(gv[k]) / ctl->bnorm > ctl->tol) && hn != 0 && k < m && k < ctl->budget;
-  ctl->j = k;
-  ctl->go = go;
-  if (in_graph) cudaGraphSetConditional(handle, go ? 1u : 0u);
-}
-
-// H y = g for the k = j steps of the cycle (back substitution, one thread): y into c.
-__global__ void k_adj_trisolve(const AdjCtl* ctl, const double* H, const double* gv, double* y) {
-  if (threadIdx.x != 0) return;
+// H y = g for the k = j steps of the cycle: y into c (row-oriented back substitution by one
+// thread, on a shared copy of the triangle: read where it lies, each of its k^2 / 2 elements
+// was a wait on L2, 51 us at k = 40).
+__global__ __launch_bounds__(256) void k_adj_trisolve(const AdjCtl* ctl, const double* H, const double* gv, double* c) {
+  constexpr int KS = 64;  // triangles up to this order are staged; larger ones are read where they lie
+  __shared__ double sH[KS * KS], y[ADJ_MAX_M + 8];
   const int k = ctl->j, m = ctl->m;
-  for (int i = k - 1; i >= 0; --i) {
-    double t = gv[i];
-    for (int l = i + 1; l < k; ++l) t -= H[(size_t)i * m + l] * y[l];
-    y[i] = t / H[(size_t)i * m + i];
+  const bool staged = k <= KS;
+  if (staged)
+    for (int q = threadIdx.x; q < k * k; q += blockDim.x) sH[q] = H[(size_t)(q / k) * m + q % k];
+  for (int i = threadIdx.x; i < k; i += blockDim.x) y[i] = gv[i];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const double* R = staged ? sH : H;
+    const int ldr = staged ? k : m;
+    for (int i = k - 1; i >= 0; --i) {
+      double t = y[i];
+#pragma unroll 8
+      for (int l = i + 1; l < k; ++l) t -= R[(size_t)i * ldr + l] * y[l];
+      y[i] = t / R[(size_t)i * ldr + i];
+    }
   }
+  __syncthreads();
+  for (int i = threadIdx.x; i < k; i += blockDim.x) c[i] = y[i];
 }
 
-// out = sum_i c_i V_i (i < m; with ctl, the cycle's step count)
-__global__ void k_adj_span(long N, double* out, const double* V, long ld, int m, const double* c, const AdjCtl* ctl) {
-  if (ctl) m = ctl->j;
+// out = sum_i c_i v_i over the cycle's steps
+__global__ void k_adj_span(long N, double* out, const double* V, long ld, const double* c, const AdjCtl* ctl) {
+  const int m = ctl->j;
   const long f = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= N) return;
   double x = 0.0;
+#pragma unroll 8
   for (int i = 0; i < m; ++i) x = fma(c[i], V[(size_t)i * ld + f], x);
   out[f] = x;
 }
 
-// v = b - v
-__global__ void k_adj_resid(long N, const double* b, double* v) {
-  const long f = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (f < N) v[f] = b[f] - v[f];
-}
-
-__global__ void k_adj_scale(long N, double* v, double a) {
-  const long f = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (f < N) v[f] *= a;
+// v = b - J^T lambda (lambda null: v = b) and its norm into the state.
+__global__ __launch_bounds__(AT) void k_adj_resid(int n, const double2* g, const double* lambda, const double* b,
+                                                  double* v, AdjCtl* ctl, double* partial) {
+  __shared__ double red[64], stage[TOT_CHUNK * TOT_LD];
+  const long N = (long)n * n;
+  double s[1] = {0.0};
+  for (long f = (long)blockIdx.x * AT + threadIdx.x; f < N; f += (long)ANB * AT) {
+    double r = b[f];
+    if (lambda) r = r - jt_cell(n, g, lambda, (int)(f / n), (int)(f % n));
+    v[f] = r;
+    s[0] = fma(r, r, s[0]);
+  }
+  block_sum<1>(s, red);
+  if (threadIdx.x == 0) partial[blockIdx.x] = s[0];
+  if (!last_block(&ctl->counter, gridDim.x)) return;
+  totals(partial, 1, stage, [&](int, double t) { ctl->rnorm = sqrt(t); });
 }
 
 __global__ void k_adj_neg(long N, const double* z, double* lambda) {
@@ -310,24 +460,39 @@ __global__ void k_adj_add(long N, const double* z, double* lambda) {
   if (f < N) lambda[f] += z[f];
 }
 
-// lambda += -z
-__global__ void k_adj_axpy(long N, const double* z, double* lambda) {
-  const long f = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (f < N) lambda[f] -= z[f];
-}
-
-// sums[0] = lambda . rho, sums[1] = sum rho, reduced in a fixed order by one block
-__global__ void k_adj_rho_sums(long N, const double* lambda, const double* rho, double* sums) {
-  __shared__ double red[64];
+// sums[0] = lambda . rho, sums[1] = sum rho in the order of one block of 1024 threads (a chain
+// per thread, trees over its lanes and warps), each of its warps on an SM of its own: one SM
+// draws 4 MB at about 90 GB/s, 41 us at 512^2 where 32 take 8.
+constexpr int RHO_BLOCKS = 32;
+__global__ __launch_bounds__(32) void k_adj_rho_sums(long N, const double* lambda, const double* rho, AdjCtl* ctl,
+                                                     double* partial, double* sums) {
+  constexpr int B = 8, T = 32 * RHO_BLOCKS;
   double v[2] = {0.0, 0.0};
-  for (long f = threadIdx.x; f < N; f += blockDim.x) {
-    v[0] = fma(lambda[f], rho[f], v[0]);
-    v[1] += rho[f];
+  for (long f0 = (long)blockIdx.x * 32 + threadIdx.x; f0 < N; f0 += (long)B * T) {
+    double l[B], r[B];
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+      const long f = f0 + (long)k * T;
+      l[k] = f < N ? lambda[f] : 0.0;
+      r[k] = f < N ? rho[f] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+      v[0] = fma(l[k], r[k], v[0]);
+      v[1] += r[k];
+    }
   }
-  block_sum<2>(v, red);
+  v[0] = warp_sum(v[0]);
+  v[1] = warp_sum(v[1]);
   if (threadIdx.x == 0) {
-    sums[0] = v[0];
-    sums[1] = v[1];
+    partial[blockIdx.x] = v[0];
+    partial[RHO_BLOCKS + blockIdx.x] = v[1];
+  }
+  if (!last_block(&ctl->counter, RHO_BLOCKS)) return;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const double t = warp_sum(__ldcg(&partial[k * RHO_BLOCKS + threadIdx.x]));
+    if (threadIdx.x == 0) sums[k] = t;
   }
 }
 
@@ -351,8 +516,10 @@ struct AdjointWs : otm_context::Erased {
   size_t N = 0, V = 0, ld = 0;
   DevBuf buf, recs, lists;
   double *b, *lam, *z, *h, *t1, *t2, *Vb, *c, *part, *sums, *hcol, *inv;
-  double *fwdc, *H, *cs, *sn, *gv;  // the forward mesh of the call; the cycle's Hessenberg state
+  double2* g;               // the call's vertex displacements
+  double *H, *cs, *sn, *gv;  // the cycle's Hessenberg state
   AdjCtl* ctl = nullptr;
+  int nb = 0;  // blocks of the step kernels
   int G = 0, rows = 0, cols = 0, reg = 0, fft = 0;
   // the Arnoldi step as a graph with a WHILE node (built on first use) and its kernel count
   cudaGraphExec_t step_graph = nullptr;
@@ -361,7 +528,8 @@ struct AdjointWs : otm_context::Erased {
     if (step_graph) cudaGraphExecDestroy(step_graph);
   }
   // record k: src = basis vector k (k < m+1); record m+1: src = b; record m+2: src = h;
-  // record m+3: src = the basis vector of the current step (set on the device); dst = z
+  // record m+3: src = the basis vector of the current step (set on the device, as is its
+  // active flag); dst = z
   Inst* rec(int k) { return recs.as<Inst>() + k; }
 };
 
@@ -374,29 +542,37 @@ static AdjointWs* adjoint_ws(otm_context* ctx, int n, int m) {
   W->N = (size_t)n * n;
   W->V = (size_t)(n + 1) * (n + 1);
   W->ld = (W->N + 31) / 32 * 32;
-  const int nred = 256;
-  const size_t words = W->ld * 6 + 2 * W->V + (size_t)(m + 1) * W->ld + (m + 2) + (size_t)nred * (m + 2) + (m + 3) + 64 +
-                       16 + 2 * W->V + (size_t)(m + 1) * m + 3 * (size_t)m + 1;
+  W->nb = (int)std::min<size_t>(ANB, (W->N + AT - 1) / AT);
+  auto up = [](size_t w) { return (w + 31) / 32 * 32; };  // every array starts on 256 bytes
+  const size_t words = W->ld * 6 + up(2 * W->V) + (size_t)(m + 1) * W->ld + 3 * up(m + 2) + up((size_t)ANB * (m + 2)) +
+                       3 * up(8) + up((size_t)(m + 1) * m) + 2 * up(m);
   W->buf.reserve(sizeof(double) * words);
-  double* p = W->buf.as<double>();
-  W->b = p; p += W->ld;
-  W->lam = p; p += W->ld;
-  W->z = p; p += W->ld;
-  W->t1 = p; p += W->ld;
-  W->t2 = p; p += W->ld;
-  W->h = p; p += 2 * W->V + W->ld;
-  W->Vb = p; p += (size_t)(m + 1) * W->ld;
-  W->c = p; p += m + 2;
-  W->sums = p; p += 2;
-  W->part = p; p += (size_t)nred * (m + 2);
-  W->hcol = p; p += m + 2;  // the current Hessenberg column
-  W->inv = p; p += 8;
-  W->ctl = reinterpret_cast<AdjCtl*>(p); p += 8;
-  W->fwdc = p; p += 2 * W->V;
-  W->H = p; p += (size_t)(m + 1) * m;
-  W->cs = p; p += m;
-  W->sn = p; p += m;
-  W->gv = p;
+  double* q = W->buf.as<double>();
+  auto take = [&](size_t w) {
+    double* r = q;
+    q += up(w);
+    return r;
+  };
+  W->b = take(W->ld);
+  W->lam = take(W->ld);
+  W->z = take(W->ld);
+  W->t1 = take(W->ld);
+  W->t2 = take(W->ld);
+  W->h = take(W->ld);
+  W->g = reinterpret_cast<double2*>(take(2 * W->V));
+  W->Vb = take((size_t)(m + 1) * W->ld);
+  W->c = take(m + 2);
+  W->hcol = take(m + 2);
+  W->inv = take(8);
+  W->gv = take(m + 2);
+  W->part = take((size_t)ANB * (m + 2));
+  W->sums = take(8);
+  static_assert(sizeof(AdjCtl) <= 8 * sizeof(double), "the cycle state fits its slot");
+  W->ctl = reinterpret_cast<AdjCtl*>(take(8));
+  W->H = take((size_t)(m + 1) * m);
+  W->cs = take(m);
+  W->sn = take(m);
+  OTM_CUDA(cudaMemsetAsync(W->ctl, 0, sizeof(AdjCtl), ctx->stream));
   SizeTables* T = ctx->tables.at(n).get();
   Inst base;
   std::memset(&base, 0, sizeof(base));
@@ -457,36 +633,27 @@ static void poisson_rec(otm_context* ctx, AdjointWs* W, int k) {
   }
 }
 
-// One Arnoldi step j of the cycle (j read on the device): z = M^+ v_j, w = J^T z into
-// v_{j+1}, two classical Gram-Schmidt passes and the normalisation (reductions in block
-// order on the device), then the Givens kernel, which advances j and sets the loop test.
+// One Arnoldi step j of the cycle (j read on the device): z = M^+ v_j and the four step
+// kernels, which do nothing once the cycle has ended.
 static void arnoldi_step(otm_context* ctx, AdjointWs* W, int n, cudaGraphConditionalHandle handle, int in_graph) {
-  const long N = (long)W->N, ld = (long)W->ld;
-  const int RB = 256, nred = 256;
-  const unsigned gN = (unsigned)((W->N + RB - 1) / RB), gV = (unsigned)((W->V + RB - 1) / RB);
-  const AdjCtl* ctl = W->ctl;
-  launch(ctx, "adj_set_src", k_adj_set_src, 1, 32, W->rec(W->m + 3), W->Vb, ld, ctl);
+  const long ld = (long)W->ld;
+  Inst* rec = W->rec(W->m + 3);
   poisson_rec(ctx, W, W->m + 3);
-  launch(ctx, "adj_vertex", k_adj_vertex, gV, RB, n, (const double*)W->fwdc, (const double*)W->z, W->h);
-  launch(ctx, "adj_cells", k_adj_cells, gN, RB, n, (const double*)W->h, 1.0, (const double*)nullptr, W->Vb, ctl, ld);
-  const unsigned rt = (unsigned)((W->m + 1 + 31) / 32 * 32);
-  for (int pass = 0; pass < 2; ++pass) {
-    launch(ctx, "adj_dot", k_adj_multidot, nred, RB, N, (const double*)nullptr, (const double*)W->Vb, ld, 0, W->part,
-           ctl, 0);
-    launch(ctx, "adj_reduce", k_adj_orth_reduce, 1, rt, (const double*)W->part, nred, 0, pass, W->hcol, W->c, ctl);
-    launch(ctx, "adj_combine", k_adj_combine, gN, RB, N, W->Vb, 1.0, (const double*)W->Vb, ld, 0, (const double*)W->c,
-           ctl);
-  }
-  launch(ctx, "adj_dot", k_adj_multidot, nred, RB, N, (const double*)nullptr, (const double*)W->Vb, ld, 0, W->part, ctl,
-         1);
-  launch(ctx, "adj_reduce", k_adj_norm_reduce, 1, 32, (const double*)W->part, nred, 0, W->hcol, W->inv, ctl);
-  launch(ctx, "adj_scale", k_adj_scale_by, gN, RB, N, W->Vb, (const double*)W->inv, ctl, ld);
-  launch(ctx, "adj_givens", k_adj_givens, 1, 32, W->ctl, (const double*)W->hcol, W->H, W->cs, W->sn, W->gv, handle,
-         in_graph);
+  launch(ctx, "adj_apply", k_adj_apply, W->nb, AT, n, (const double2*)W->g, (const double*)W->z, W->Vb, ld, W->ctl,
+         W->part, W->hcol, W->c);
+  launch(ctx, "adj_orth", k_adj_orth, W->nb, AT, n, W->Vb, ld, W->ctl, W->part, W->hcol, W->c);
+  launch(ctx, "adj_norm", k_adj_norm, W->nb, AT, n, W->Vb, ld, W->ctl, W->inv, W->part, (const double*)W->hcol,
+         (const double*)W->c, W->H, W->cs, W->sn, W->gv, rec, handle, in_graph);
+  launch(ctx, "adj_scale", k_adj_scale_by, (unsigned)((W->N + 255) / 256), 256, (long)W->N, W->Vb, ld,
+         (const double*)W->inv, (const AdjCtl*)W->ctl);
 }
 
-// The cycle's steps as a graph: a WHILE node whose body is one Arnoldi step, its condition
-// set by the Givens kernel (at most m bodies per launch).
+// Steps per body of the cycle's WHILE node: a body costs 2.8 us beside its kernels (measured
+// with empty ones), a step after the cycle's end 7 launches that return at once (about 7 us).
+constexpr int STEPS_PER_BODY = 4;
+
+// The cycle's steps as a graph: a WHILE node whose body is STEPS_PER_BODY Arnoldi steps, its
+// condition set by the last kernel of a step (at most m steps per launch).
 static void build_step_graph(otm_context* ctx, AdjointWs* W, int n) {
   cudaStream_t st = ctx->stream;
   dct_reg_attrs(ctx->device);
@@ -507,7 +674,7 @@ static void build_step_graph(otm_context* ctx, AdjointWs* W, int n) {
     const long before = ctx->launches;
     OTM_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     try {
-      arnoldi_step(ctx, W, n, handle, 1);
+      for (int u = 0; u < STEPS_PER_BODY; ++u) arnoldi_step(ctx, W, n, handle, 1);
     } catch (...) {
       cudaGraph_t dummy;
       cudaStreamEndCapture(st, &dummy);
@@ -547,11 +714,11 @@ extern "C" int otm_adjoint(otm_context* ctx, int n, const double* density, const
     make_current(ctx);
     if (otm_init(ctx, n) != OTM_OK) throw BadArg{std::string("otm_adjoint: ") + otm_last_error()};
     cudaStream_t st = ctx->stream;
-    const int m = o.mode == OTM_ADJOINT_KRYLOV ? std::max(1, std::min(o.restart, 200)) : 1;
+    const int m = o.mode == OTM_ADJOINT_KRYLOV ? std::max(1, std::min(o.restart, ADJ_MAX_M)) : 1;
     AdjointWs* W = adjoint_ws(ctx, n, m);
     launch(ctx, "adj_reset", k_adj_reset_recs, 1, 256, W->rec(0), W->m + 4);
-    const size_t N = W->N, V = W->V, ld = W->ld;
-    const int RB = 256, nred = 256;
+    const size_t N = W->N, V = W->V;
+    const int RB = 256;
     // inputs: used in place when they are device memory, else staged into the workspace
     auto stage = [&](const double* src, double* tmp, size_t words) -> const double* {
       if (is_device_ptr(src)) return src;
@@ -570,27 +737,8 @@ extern "C" int otm_adjoint(otm_context* ctx, int n, const double* density, const
     double* d_lam = W->lam;
     double* d_z = W->z;
     double* d_h = W->h;
-    double* d_V = W->Vb;
-    double* d_c = W->c;
-    double* d_part = W->part;
     // b = G^T q
-    launch(ctx, "adj_cells", k_adj_cells, gN, RB, n, d_q, 1.0, (const double*)nullptr, d_b, (const AdjCtl*)nullptr, 0L);
-    std::vector<double> hp;
-    auto multidot = [&](const double* w, int k, std::vector<double>& out) {
-      launch(ctx, "adj_dot", k_adj_multidot, nred, RB, (long)N, w, (const double*)d_V, (long)ld, k, d_part,
-             (const AdjCtl*)nullptr, 0);
-      hp.resize((size_t)nred * (k + 1));
-      OTM_CUDA(cudaMemcpyAsync(hp.data(), d_part, sizeof(double) * hp.size(), cudaMemcpyDeviceToHost, st));
-      OTM_CUDA(cudaStreamSynchronize(st));
-      out.assign(k + 1, 0.0);
-      for (int blk = 0; blk < nred; ++blk)
-        for (int i = 0; i <= k; ++i) out[i] += hp[(size_t)blk * (k + 1) + i];
-    };
-    auto apply_jt = [&](const double* x, double* out) {
-      launch(ctx, "adj_vertex", k_adj_vertex, gV, RB, n, d_fwd, x, d_h);
-      launch(ctx, "adj_cells", k_adj_cells, gN, RB, n, (const double*)d_h, 1.0, (const double*)nullptr, out,
-             (const AdjCtl*)nullptr, 0L);
-    };
+    launch(ctx, "adj_cells", k_adj_cells, gN, RB, n, d_q, d_b);
     int solves = 0;
     double rel = -1.0;
     if (o.mode == OTM_ADJOINT_ONE_STEP) {
@@ -602,39 +750,31 @@ extern "C" int otm_adjoint(otm_context* ctx, int n, const double* density, const
       OTM_CUDA(cudaMemsetAsync(d_lam, 0, sizeof(double) * N, st));
       // Restarted GMRES(m) on J^T lambda = b, right-preconditioned: J^T M^+ y = b, lambda = M^+ y.
       // A cycle's Arnoldi steps run on the device (classical Gram-Schmidt applied twice,
-      // Givens rotations and the loop test in one-thread kernels) as one graph launch with a
-      // WHILE node -- or, in the host-driven loop mode and under the profiler, the same
-      // kernels one step at a time; the host reads the cycle's step count once per restart,
-      // forms the true residual and decides whether to restart.
-      std::vector<double> dots;
-      OTM_CUDA(cudaMemcpyAsync(d_V, d_b, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
-      OTM_CUDA(cudaMemcpyAsync(W->fwdc, d_fwd, sizeof(double) * 2 * V, cudaMemcpyDeviceToDevice, st));
-      multidot(d_V, 0, dots);
-      const double bnorm = std::sqrt(dots[0]);
+      // Givens rotations and the loop test) as one graph launch with a WHILE node -- or, in
+      // the host-driven loop mode and under the profiler, the same kernels one step at a
+      // time; the host reads the cycle's step count and the true residual's norm once per
+      // restart and decides whether to restart.
+      launch(ctx, "adj_disp", k_adj_disp, gV, RB, n, d_fwd, W->g);
       const bool graph = ctx->loop_mode == OTM_LOOP_GRAPH && !ctx->prof.on;
+      AdjCtl hc;
+      auto residual = [&](const double* lambda) {
+        launch(ctx, "adj_resid", k_adj_resid, W->nb, AT, n, (const double2*)W->g, lambda, (const double*)d_b, W->Vb,
+               W->ctl, W->part);
+        OTM_CUDA(cudaMemcpyAsync(&hc, W->ctl, sizeof(hc), cudaMemcpyDeviceToHost, st));
+        OTM_CUDA(cudaStreamSynchronize(st));
+      };
+      residual(nullptr);
+      const double bnorm = hc.rnorm;
       rel = bnorm > 0 ? 1.0 : 0.0;
-      bool first = true;
       while (bnorm > 0) {
-        double* v0 = d_V;
-        double rnorm;
-        if (first) {
-          rnorm = bnorm;
-          first = false;
-        } else {
-          apply_jt(d_lam, v0);
-          launch(ctx, "adj_resid", k_adj_resid, gN, RB, (long)N, (const double*)d_b, v0);
-          multidot(v0, 0, dots);
-          rnorm = std::sqrt(dots[0]);
-        }
-        rel = rnorm / bnorm;
+        rel = hc.rnorm / bnorm;
         if (!(rel > o.tol) || solves >= o.max_iter) break;
-        launch(ctx, "adj_scale", k_adj_scale, gN, RB, (long)N, v0, 1.0 / rnorm);
-        launch(ctx, "adj_cycle", k_adj_cycle_init, 1, 32, W->ctl, W->gv, m, rnorm, bnorm, o.tol, o.max_iter - solves);
+        launch(ctx, "adj_cycle", k_adj_cycle_init, std::max(gN, 1u), RB, (long)N, W->ctl, W->gv, m, bnorm, o.tol,
+               o.max_iter - solves, W->rec(W->m + 3), W->Vb);
         if (graph) {
           if (!W->step_graph) build_step_graph(ctx, W, n);
           OTM_CUDA(cudaGraphLaunch(W->step_graph, st));
         } else {
-          AdjCtl hc;
           do {
             arnoldi_step(ctx, W, n, (cudaGraphConditionalHandle)0, 0);
             OTM_CUDA(cudaMemcpyAsync(&hc, W->ctl, sizeof(hc), cudaMemcpyDeviceToHost, st));
@@ -643,22 +783,23 @@ extern "C" int otm_adjoint(otm_context* ctx, int n, const double* density, const
           } while (hc.go);
         }
         // lambda += M^+ (V y), H y = g solved on the device
-        launch(ctx, "adj_trisolve", k_adj_trisolve, 1, 32, (const AdjCtl*)W->ctl, (const double*)W->H,
-               (const double*)W->gv, d_c);
-        launch(ctx, "adj_span", k_adj_span, gN, RB, (long)N, d_h, (const double*)d_V, (long)ld, 0, (const double*)d_c,
-               (const AdjCtl*)W->ctl);
+        launch(ctx, "adj_trisolve", k_adj_trisolve, 1, 256, (const AdjCtl*)W->ctl, (const double*)W->H,
+               (const double*)W->gv, W->c);
+        launch(ctx, "adj_span", k_adj_span, gN, RB, (long)N, d_h, (const double*)W->Vb, (long)W->ld,
+               (const double*)W->c, (const AdjCtl*)W->ctl);
         poisson_rec(ctx, W, W->m + 2);  // z = M^+ h
         launch(ctx, "adj_add", k_adj_add, gN, RB, (long)N, (const double*)d_z, d_lam);
-        AdjCtl hc;
-        OTM_CUDA(cudaMemcpyAsync(&hc, W->ctl, sizeof(hc), cudaMemcpyDeviceToHost, st));
-        OTM_CUDA(cudaStreamSynchronize(st));
-        if (graph) ctx->launches += W->step_kernels * (long)hc.j;
+        residual(d_lam);
+        if (graph)
+          ctx->launches += W->step_kernels * (long)((hc.j + STEPS_PER_BODY - 1) / STEPS_PER_BODY);
         solves += hc.j + 1;
+        if (hc.fault) break;   // reported below
         if (hc.j == 0) break;  // no step was possible: nothing changes by restarting
       }
     }
     // chain through the density normalisation, reduced and applied on the device
-    launch(ctx, "adj_rho_sums", k_adj_rho_sums, 1, 1024, (long)N, (const double*)d_lam, d_rho, W->sums);
+    launch(ctx, "adj_rho_sums", k_adj_rho_sums, RHO_BLOCKS, 32, (long)N, (const double*)d_lam, d_rho, W->ctl,
+           W->part, W->sums);
     bool odev = is_device_ptr(grad_density);
     double* out = odev ? grad_density : d_z;
     launch(ctx, "adj_finish", k_adj_finish, gN, RB, (long)N, (const double*)d_lam, (const double*)W->sums, out);

@@ -178,3 +178,26 @@ def test_krylov_graph_and_host_loops_agree(n, restart):
     assert it0 == it1 and r0 == r1
     assert np.array_equal(g0, g1)
     assert r0 <= 1e-12
+
+
+# Sizes at the edges of the Arnoldi kernels' cell layout: fewer cells than a block, one block,
+# a partly filled last block, and more cells than 256 blocks hold (n > 256: chains of cells per
+# thread). The solve stops at a relative residual of 1e-12; on these smooth maps J^T M^+ is
+# well conditioned (GMRES takes about ten steps), so the gradient is within 1e-8.
+@pytest.mark.parametrize("n", [4, 15, 16, 17, 257, 300])
+def test_adjoint_cell_layout_edges(n):
+    from adjoint_ref import reference_gradient
+    from otmap_b200 import native as N
+    from otmap_b200 import workloads as W
+
+    ctx = N.Context(0)
+    _, img = W.softmax_logits(n, n, sigma_px=max(1.0, n / 64))
+    dens = W.to_cells(img)
+    fwd, st = _solve(N, ctx, n, dens)
+    assert st.residual < 1e-12
+    q = np.random.default_rng(n).standard_normal(((n + 1) ** 2, 2))
+    ref, _ = reference_gradient(fwd, dens, q, n)
+    g, ast = _adjoint(N, ctx, n, dens, fwd, q, N.ADJOINT_KRYLOV)
+    rel = np.linalg.norm(g - ref) / np.linalg.norm(ref)
+    assert rel <= 1e-8, (rel, ast.iterations, ast.relative_residual)
+    ctx.close()
