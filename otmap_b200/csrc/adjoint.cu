@@ -520,7 +520,7 @@ struct AdjointWs : otm_context::Erased {
   double *H, *cs, *sn, *gv;  // the cycle's Hessenberg state
   AdjCtl* ctl = nullptr;
   int nb = 0;  // blocks of the step kernels
-  int G = 0, rows = 0, cols = 0, reg = 0, fft = 0;
+  int G = 0, rows = 0, cols = 0, reg = 0, fft = 0, col_warps = 0;
   // the Arnoldi step as a graph with a WHILE node (built on first use) and its kernel count
   cudaGraphExec_t step_graph = nullptr;
   long step_kernels = 0;
@@ -593,7 +593,8 @@ static AdjointWs* adjoint_ws(otm_context* ctx, int n, int m) {
     base.logn = lg;
     W->reg = dct_reg_supported(n) ? 1 : 0;
     const int per = W->reg ? dct_reg_lines_per_block(n) : fft_lines(n);
-    const int cper = W->reg ? dct_reg_cols_per_block(n) : fft_lines(n);
+    W->col_warps = W->reg ? dct_reg_col_warps(n, 1, ctx->num_sms) : 0;
+    const int cper = W->reg ? dct_reg_cols_per_block(n, W->col_warps) : fft_lines(n);
     base.nrow = n / per;
     base.ncol = n / cper;
     W->rows = base.nrow;
@@ -625,7 +626,7 @@ static void poisson_rec(otm_context* ctx, AdjointWs* W, int k) {
   const int* L = W->lists.as<int>();
   if (W->fft) {
     if (W->reg)
-      dct_reg_run(ctx, W->n, false, d, L, 0, W->rows, L, 0, W->cols);
+      dct_reg_run(ctx, W->n, false, d, L, 0, W->rows, L, 0, W->cols, W->col_warps);
     else
       poisson_fft(ctx, d, L, 0, W->rows, L, 0, W->cols);
   } else {

@@ -100,6 +100,7 @@ struct Workspace {
   int split_strip0 = 0;  // strips of split-precision instances start here (FP64 ones before)
   struct Segment {  // instances of one size on one transform kernel family
     int n, reg, split, roff, rcnt, coff, ccnt;
+    int col_warps;  // warps per block of the column pass (register transforms)
   };
   std::vector<Segment> segments;
   // the iteration loop captured as a CUDA graph with a device-side WHILE node

@@ -211,24 +211,24 @@ __device__ __forceinline__ V pre3(int k, R a, R b, V pt) {
 template <class R, int N1, int N2>
 struct RowGeom {
   using V = typename RT<R>::V;
-  static constexpr int RW = RT<R>::RW;               // warps per block
+  static constexpr int RW = RT<R>::RW;               // most warps per block (RegDct::run picks the number)
   static constexpr int n = N1 * N2, LPW = 32 / N2;
   static constexpr int DATA = 2 * LPW * n;           // reals: the item's rows
   static constexpr int TRANS = LPW * N1 * (N2 + 1);  // reals: step-3 transpose buffers
   static constexpr int WARP = DATA + TRANS;          // reals per warp
   static_assert((WARP * sizeof(R)) % 16 == 0, "each warp's buffer starts 16-byte aligned");
   static constexpr int TABLES = 2 * n;               // complex: the step-2 twiddles, then pt
-  static constexpr size_t SMEM = sizeof(R) * RW * WARP + sizeof(V) * TABLES + 16 * RW;  // + mbarriers
+  static constexpr size_t smem(int warps) { return sizeof(R) * warps * WARP + sizeof(V) * TABLES + 16 * warps; }  // + mbarriers
 };
 
 // The block's copy of the size's step-2 twiddles (n entries) and post-twiddles pt (n entries),
 // read by every item of the persistent kernel: shared-memory latency instead of L1's.
 template <class R, int N1, int N2>
-__device__ __forceinline__ typename RT<R>::V* load_row_tables(R* sbuf, const Inst& I) {
+__device__ __forceinline__ typename RT<R>::V* load_row_tables(R* sbuf, int warps, const Inst& I) {
   using G = RowGeom<R, N1, N2>;
   using V = typename G::V;
   constexpr int n = G::n;
-  V* tab = reinterpret_cast<V*>(sbuf + G::RW * G::WARP);
+  V* tab = reinterpret_cast<V*>(sbuf + warps * G::WARP);
   const double2* tw2 = I.tw + (n >> 1);
   for (int e = threadIdx.x; e < n; e += blockDim.x) {
     const double2 a = __ldg(&tw2[e]), b = __ldg(&I.pt[e]);
@@ -297,7 +297,8 @@ __global__ __launch_bounds__(RT<R>::RW * 32, 1) void k_dct_rows_fwd(Inst* insts,
                                                                      int items, unsigned extra, long long limit) {
   using G = RowGeom<R, N1, N2>;
   using V = typename G::V;
-  constexpr int n = G::n, LPW = G::LPW, RW = G::RW;
+  constexpr int n = G::n, LPW = G::LPW;
+  const int RW = blockDim.x >> 5;
   const DctScale<R> ds(n);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R* sbuf = reinterpret_cast<R*>(smem_raw);
@@ -305,7 +306,7 @@ __global__ __launch_bounds__(RT<R>::RW * 32, 1) void k_dct_rows_fwd(Inst* insts,
   R* data = sbuf + warp * G::WARP;
   R* buf = data + G::DATA + sub * N1 * (N2 + 1);
   if (items <= 0) return;
-  const V* tab = load_row_tables<R, N1, N2>(sbuf, insts[row_inst[seg]]);
+  const V* tab = load_row_tables<R, N1, N2>(sbuf, RW, insts[row_inst[seg]]);
   const V* spt = tab + n;
   unsigned long long* bar =
       reinterpret_cast<unsigned long long*>(smem_raw + sizeof(R) * RW * G::WARP + sizeof(V) * G::TABLES) + warp;
@@ -389,7 +390,8 @@ __global__ __launch_bounds__(RT<R>::RW * 32, 1) void k_dct_rows_inv(Inst* insts,
                                                                      int items, unsigned extra, long long limit) {
   using G = RowGeom<R, N1, N2>;
   using V = typename G::V;
-  constexpr int n = G::n, LPW = G::LPW, RW = G::RW;
+  constexpr int n = G::n, LPW = G::LPW;
+  const int RW = blockDim.x >> 5;
   const DctScale<R> ds(n);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R* sbuf = reinterpret_cast<R*>(smem_raw);
@@ -397,7 +399,7 @@ __global__ __launch_bounds__(RT<R>::RW * 32, 1) void k_dct_rows_inv(Inst* insts,
   R* data = sbuf + warp * G::WARP;
   R* buf = data + G::DATA + sub * N1 * (N2 + 1);
   if (items <= 0) return;
-  const V* tab = load_row_tables<R, N1, N2>(sbuf, insts[row_inst[seg]]);
+  const V* tab = load_row_tables<R, N1, N2>(sbuf, RW, insts[row_inst[seg]]);
   const V* spt = tab + n;
   unsigned long long* bar =
       reinterpret_cast<unsigned long long*>(smem_raw + sizeof(R) * RW * G::WARP + sizeof(V) * G::TABLES) + warp;
@@ -472,7 +474,7 @@ __global__ __launch_bounds__(RT<R>::RW * 32, 1) void k_dct_rows_inv(Inst* insts,
 
 // Column pass, one warp per column pair (LPW pairs per warp when a line takes fewer than 32
 // lanes), so that the two FFTs and the exchanges between them stay inside the warp. A block
-// of 8 warps owns CPB = 8 LPW consecutive column pairs: it copies their tile of n rows into
+// of CT / 32 warps owns CPB = CT / 32 LPW consecutive column pairs: it copies their tile of n rows into
 // shared memory with coalesced 16-byte cp.async (rows stored in Makhoul order, row m holding
 // global row 2m for m < n/2 and 2(n-1-m)+1 above, so that the lanes of a line read
 // consecutive rows), each warp transforms its pairs -- DCT-II (split N1 x N2), division by
@@ -480,11 +482,15 @@ __global__ __launch_bounds__(RT<R>::RW * 32, 1) void k_dct_rows_inv(Inst* insts,
 // already lies) -- and the block writes the tile back in global row order. While the warps transform, the tile's
 // space holds, per line, a 2n-double region: the step-3 transpose buffer, and the line's
 // spectrum for the exchanges of X_k with X_{n-k}.
-template <class R, int N1, int N2>
+//
+// CT is 256 threads where that gives every SM a block. A lone small instance has too few
+// tiles for that (a 256^2 one 16, a 512^2 one 32), and then 128 or 64 threads (narrower tiles, the
+// same arithmetic per column) spread its columns over the chip: dct_reg_col_warps.
+template <class R, int N1, int N2, int CT_>
 struct ColGeom {
   using V = typename RT<R>::V;
   static constexpr int n = N1 * N2, LPW = 32 / N2;
-  static constexpr int CT = 256;                // threads per block
+  static constexpr int CT = CT_;                // threads per block
   static constexpr int CPB = (CT / 32) * LPW;   // column pairs per block
   static constexpr int CB = 2 * CPB;            // columns per block
   static constexpr int RS = CPB + 1;            // complex per tile row (odd: conflict-free line reads)
@@ -500,10 +506,10 @@ __device__ __forceinline__ int makhoul_inv(int i, int n) { return (i & 1) ? n - 
 
 // Persistent: each block copies the size's tables into shared memory once and then takes
 // the column tiles blockIdx.x, blockIdx.x + gridDim.x, ... of the segment.
-template <class R, int N1, int N2>
-__global__ __launch_bounds__(ColGeom<R, N1, N2>::CT, RT<R>::COL_BLOCKS) void k_dct_cols(const Inst* insts, const int* col_inst,
-                                                                        int seg, int items) {
-  using GG = ColGeom<R, N1, N2>;
+template <class R, int N1, int N2, int CT>
+__global__ __launch_bounds__(CT, RT<R>::COL_BLOCKS) void k_dct_cols(const Inst* insts, const int* col_inst, int seg,
+                                                                    int items) {
+  using GG = ColGeom<R, N1, N2, CT>;
   using V = typename GG::V;
   constexpr int n = GG::n, CPB = GG::CPB, CB = GG::CB, RS = GG::RS, LPW = GG::LPW;
   const DctScale<R> ds(n);
@@ -646,45 +652,66 @@ __global__ __launch_bounds__(ColGeom<R, N1, N2>::CT, RT<R>::COL_BLOCKS) void k_d
   }
 }
 
+constexpr int COL_VARIANTS = 3;  // 8, 4 and 2 warps per column block
+inline int col_variant(int warps) { return warps == 8 ? 0 : warps == 4 ? 1 : 2; }
+
 template <class R, int N1, int N2>
 struct RegDct {
   static constexpr int LPW = 32 / N2, RW = RT<R>::RW;
-  static size_t rows_smem() { return RowGeom<R, N1, N2>::SMEM; }
-  static size_t cols_smem() { return sizeof(R) * ColGeom<R, N1, N2>::SMEM; }
-  static constexpr int CB = ColGeom<R, N1, N2>::CB;
-  static int rows_blocks_per_sm;  // occupancy of the row kernels (set by attrs)
-  static int cols_blocks_per_sm;  // occupancy of the column kernel
+  static size_t rows_smem(int warps) { return RowGeom<R, N1, N2>::smem(warps); }
+  static int rows_blocks_per_sm;                 // occupancy of the row kernels (set by attrs)
+  static int cols_blocks_per_sm[COL_VARIANTS];  // occupancy of the column kernels
+  template <int CT>
+  static void col_attrs() {
+    const size_t smem = sizeof(R) * ColGeom<R, N1, N2, CT>::SMEM;
+    int a = 0;
+    OTM_CUDA(cudaFuncSetAttribute(k_dct_cols<R, N1, N2, CT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    OTM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_dct_cols<R, N1, N2, CT>, CT, smem));
+    cols_blocks_per_sm[col_variant(CT / 32)] = std::max(1, a);
+  }
   static void attrs() {
     OTM_CUDA(cudaFuncSetAttribute(k_dct_rows_fwd<R, N1, N2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)rows_smem()));
+                                  (int)rows_smem(RW)));
     OTM_CUDA(cudaFuncSetAttribute(k_dct_rows_inv<R, N1, N2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)rows_smem()));
-    OTM_CUDA(cudaFuncSetAttribute(k_dct_cols<R, N1, N2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)cols_smem()));
+                                  (int)rows_smem(RW)));
     int a = 0, b = 0;
-    OTM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_dct_rows_fwd<R, N1, N2>, RW * 32, rows_smem()));
-    OTM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_dct_rows_inv<R, N1, N2>, RW * 32, rows_smem()));
+    OTM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_dct_rows_fwd<R, N1, N2>, RW * 32, rows_smem(RW)));
+    OTM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_dct_rows_inv<R, N1, N2>, RW * 32, rows_smem(RW)));
     rows_blocks_per_sm = std::max(1, std::min(a, b));
-    OTM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_dct_cols<R, N1, N2>, 256, cols_smem()));
-    cols_blocks_per_sm = std::max(1, a);
+    col_attrs<256>();
+    col_attrs<128>();
+    col_attrs<64>();
   }
-  static void run(otm_context* ctx, Inst* d, const int* ri, int roff, int rcnt, const int* ci, int coff, int ccnt) {
-    const int grid = std::max(1, std::min((rcnt + RW - 1) / RW, rows_blocks_per_sm * ctx->num_sms));
+  template <int CT>
+  static void run_cols(otm_context* ctx, Inst* d, const int* ci, int coff, int ccnt) {
+    const int grid = std::max(1, std::min(ccnt, cols_blocks_per_sm[col_variant(CT / 32)] * ctx->num_sms));
+    launch_smem(ctx, sizeof(R) == 4 ? "dct32_cols" : "dct_cols", k_dct_cols<R, N1, N2, CT>, grid, CT,
+                sizeof(R) * ColGeom<R, N1, N2, CT>::SMEM, (const Inst*)d, ci, coff, ccnt);
+  }
+  static void run(otm_context* ctx, Inst* d, const int* ri, int roff, int rcnt, const int* ci, int coff, int ccnt,
+                  int col_warps) {
+    // a short list (a lone small instance) takes as many blocks as there are SMs and as few
+    // warps in each as that allows; the warps' work is the same either way
+    const int rw = std::max(1, std::min(RW, (rcnt + ctx->num_sms - 1) / ctx->num_sms));
+    const int grid = std::max(1, std::min((rcnt + rw - 1) / rw, rows_blocks_per_sm * ctx->num_sms));
     const unsigned extra = ctx->wait_test ? 16u : 0u;
     const long long limit = ctx->wait_test ? kTestWaitCycles : kWaitCycles;
     constexpr bool f = sizeof(R) == 4;
-    launch_smem(ctx, f ? "dct32_rows_fwd" : "dct_rows_fwd", k_dct_rows_fwd<R, N1, N2>, grid, RW * 32, rows_smem(), d, ri, roff, rcnt, extra,
-                limit);
-    const int cgrid = std::max(1, std::min(ccnt, cols_blocks_per_sm * ctx->num_sms));
-    launch_smem(ctx, f ? "dct32_cols" : "dct_cols", k_dct_cols<R, N1, N2>, cgrid, 256, cols_smem(), (const Inst*)d, ci, coff, ccnt);
-    launch_smem(ctx, f ? "dct32_rows_inv" : "dct_rows_inv", k_dct_rows_inv<R, N1, N2>, grid, RW * 32, rows_smem(), d, ri, roff, rcnt, extra,
-                limit);
+    launch_smem(ctx, f ? "dct32_rows_fwd" : "dct_rows_fwd", k_dct_rows_fwd<R, N1, N2>, grid, rw * 32, rows_smem(rw), d,
+                ri, roff, rcnt, extra, limit);
+    switch (col_warps) {
+      case 8: run_cols<256>(ctx, d, ci, coff, ccnt); break;
+      case 4: run_cols<128>(ctx, d, ci, coff, ccnt); break;
+      default: run_cols<64>(ctx, d, ci, coff, ccnt); break;
+    }
+    launch_smem(ctx, f ? "dct32_rows_inv" : "dct_rows_inv", k_dct_rows_inv<R, N1, N2>, grid, rw * 32, rows_smem(rw), d,
+                ri, roff, rcnt, extra, limit);
   }
 };
 template <class R, int N1, int N2>
 int RegDct<R, N1, N2>::rows_blocks_per_sm = 1;
 template <class R, int N1, int N2>
-int RegDct<R, N1, N2>::cols_blocks_per_sm = 1;
+int RegDct<R, N1, N2>::cols_blocks_per_sm[COL_VARIANTS] = {1, 1, 1};
 
 }  // namespace
 
@@ -729,14 +756,25 @@ int dct_reg_lines_per_block(int n) {  // rows per row-pass work item: two per FF
   }
 }
 
-int dct_reg_cols_per_block(int n) {
-  switch (n) {
-    case 64: return RegDct<double, 8, 8>::CB;
-    case 128: return RegDct<double, 8, 16>::CB;
-    case 256: return RegDct<double, 16, 16>::CB;
-    case 512: return RegDct<double, 16, 32>::CB;
-    default: return RegDct<double, 32, 32>::CB;
+// FFT lines (column pairs) of a warp of the column pass.
+static int lines_per_warp(int n) { return dct_reg_lines_per_block(n) / 2; }
+
+int dct_reg_cols_per_block(int n, int warps) { return 2 * warps * lines_per_warp(n); }
+
+int dct_reg_col_warps(int n, int instances, int num_sms) {
+  const long units = (long)instances * (n / (2 * lines_per_warp(n)));  // warps of work
+  int best = 8;
+  long least = 0;
+  for (int w : {8, 4, 2}) {
+    const long blocks = (units + w - 1) / w, load = (blocks + num_sms - 1) / num_sms * w;
+    if (w == 8 && blocks >= num_sms) return 8;
+    if (n / (2 * lines_per_warp(n)) % w != 0) continue;  // whole tiles only
+    if (least == 0 || load < least) {
+      least = load;
+      best = w;
+    }
   }
+  return best;
 }
 
 void dct_reg_attrs(int device) {
@@ -767,24 +805,24 @@ void dct_reg_attrs(int device) {
 
 template <class R>
 static void dct_reg_run_t(otm_context* ctx, int n, Inst* d, const int* ri, int roff, int rcnt, const int* ci, int coff,
-                          int ccnt) {
+                          int ccnt, int col_warps) {
   switch (n) {
-    case 64: RegDct<R, 8, 8>::run(ctx, d, ri, roff, rcnt, ci, coff, ccnt); break;
-    case 128: RegDct<R, 8, 16>::run(ctx, d, ri, roff, rcnt, ci, coff, ccnt); break;
-    case 256: RegDct<R, 16, 16>::run(ctx, d, ri, roff, rcnt, ci, coff, ccnt); break;
-    case 512: RegDct<R, 16, 32>::run(ctx, d, ri, roff, rcnt, ci, coff, ccnt); break;
-    case 1024: RegDct<R, 32, 32>::run(ctx, d, ri, roff, rcnt, ci, coff, ccnt); break;
+    case 64: RegDct<R, 8, 8>::run(ctx, d, ri, roff, rcnt, ci, coff, ccnt, col_warps); break;
+    case 128: RegDct<R, 8, 16>::run(ctx, d, ri, roff, rcnt, ci, coff, ccnt, col_warps); break;
+    case 256: RegDct<R, 16, 16>::run(ctx, d, ri, roff, rcnt, ci, coff, ccnt, col_warps); break;
+    case 512: RegDct<R, 16, 32>::run(ctx, d, ri, roff, rcnt, ci, coff, ccnt, col_warps); break;
+    case 1024: RegDct<R, 32, 32>::run(ctx, d, ri, roff, rcnt, ci, coff, ccnt, col_warps); break;
     default: throw BadArg{"dct_reg_run: unsupported size"};
   }
 }
 
 void dct_reg_run(otm_context* ctx, int n, bool fp32, Inst* d_insts, const int* row_inst, int roff, int rcnt,
-                 const int* col_inst, int coff, int ccnt) {
+                 const int* col_inst, int coff, int ccnt, int col_warps) {
   dct_reg_attrs(ctx->device);
   if (fp32)
-    dct_reg_run_t<float>(ctx, n, d_insts, row_inst, roff, rcnt, col_inst, coff, ccnt);
+    dct_reg_run_t<float>(ctx, n, d_insts, row_inst, roff, rcnt, col_inst, coff, ccnt, col_warps);
   else
-    dct_reg_run_t<double>(ctx, n, d_insts, row_inst, roff, rcnt, col_inst, coff, ccnt);
+    dct_reg_run_t<double>(ctx, n, d_insts, row_inst, roff, rcnt, col_inst, coff, ccnt, col_warps);
 }
 
 }  // namespace otm

@@ -141,10 +141,14 @@ bool dct_reg_supported(int n);
 // appended to the half table tw of the size.
 void dct_reg_step2_table(int n, const std::vector<double2>& tw, std::vector<double2>& out);
 int dct_reg_lines_per_block(int n);
-int dct_reg_cols_per_block(int n);
+// Columns per work item of the column pass with `warps` warps per block, and the number of
+// warps (8, 4 or 2) for `instances` instances of size n in one launch: 8 where that fills the
+// SMs, else the one that leaves the busiest SM the fewest warps of work.
+int dct_reg_cols_per_block(int n, int warps);
+int dct_reg_col_warps(int n, int instances, int num_sms);
 // fp32: the FP32 kernels (r_k, the transform temporary t1 and d_hat are FP32 arrays).
 void dct_reg_run(otm_context* ctx, int n, bool fp32, Inst* d_insts, const int* row_inst, int roff, int rcnt, const int* col_inst,
-                 int coff, int ccnt);
+                 int coff, int ccnt, int col_warps);
 // Tensor-core transform (dct_tc.cu) for split-precision instances of n in {128, ..., 1024}:
 // d_hat = C^T ((C r C^T) / lambda) C as four tcgen05 products, 3xTF32 in FP32.
 // The TF32 planes (hi then lo, n^2 floats each) of t1, t2 and rs hold every operand; the

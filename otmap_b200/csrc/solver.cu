@@ -645,9 +645,11 @@ static std::vector<Inst> layout_workspace(otm_context* ctx, const std::vector<in
       Inst& I = h[order[k]];
       const int reg = dct_reg_supported(I.n) ? 1 : 0;
       const int per = reg ? dct_reg_lines_per_block(I.n) : fft_lines(I.n);
-      const int cper = reg ? dct_reg_cols_per_block(I.n) : fft_lines(I.n);
-      if (segs.empty() || segs.back().n != I.n || segs.back().reg != reg)
-        segs.push_back({I.n, reg, I.split, rows, 0, cols, 0});
+      if (segs.empty() || segs.back().n != I.n || segs.back().reg != reg) {
+        const int same_size = (int)std::count_if(order.begin(), order.end(), [&](int q) { return h[q].n == I.n; });
+        segs.push_back({I.n, reg, I.split, rows, 0, cols, 0, reg ? dct_reg_col_warps(I.n, same_size, ctx->num_sms) : 0});
+      }
+      const int cper = reg ? dct_reg_cols_per_block(I.n, segs.back().col_warps) : fft_lines(I.n);
       I.row0 = rows;
       I.nrow = I.n / per;
       I.col0 = cols;
@@ -820,7 +822,7 @@ static void launch_iteration(otm_context* ctx, Inst* d_insts) {
   for (const auto& sg : ws.segments) {
     if (sg.reg)
       dct_reg_run(ctx, sg.n, sg.split != 0, d_insts, ws.row_inst.as<int>(), sg.roff, sg.rcnt, ws.col_inst.as<int>(), sg.coff,
-                  sg.ccnt);
+                  sg.ccnt, sg.col_warps);
     else
       poisson_fft(ctx, d_insts, ws.row_inst.as<int>(), sg.roff, sg.rcnt, ws.col_inst.as<int>(), sg.coff, sg.ccnt);
   }
