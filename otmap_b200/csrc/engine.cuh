@@ -67,59 +67,57 @@ __device__ __forceinline__ void stop_outcome(Inst& I) {
 __device__ __forceinline__ double cubic_eval(const double c[4], double t) { return ((c[3] * t + c[2]) * t + c[1]) * t + c[0]; }
 __device__ __forceinline__ double cubic_deriv(const double c[4], double t) { return (3.0 * c[3] * t + 2.0 * c[2]) * t + c[1]; }
 
-// Real roots of w3 t^3 + w2 t^2 + w1 t + w0: closed form of the depressed cubic
-// (Cardano for one real root, the trigonometric form for three) and two Newton
-// steps; replaces the companion-matrix eigensolver of otsolver_2dgrid.cpp:568-572.
-__device__ __forceinline__ int cubic_real_roots(const double w[4], double roots[3]) {
-  double a = w[2] / w[3], b = w[1] / w[3], c = w[0] / w[3];
-  if (!isfinite(a) || !isfinite(b) || !isfinite(c)) return 0;
-  double p = b - a * a / 3.0;
-  double q = 2.0 * a * a * a / 27.0 - a * b / 3.0 + c;
-  double disc = 0.25 * q * q + p * p * p / 27.0;
-  int m;
-  if (disc > 0.0) {
-    double sq = sqrt(disc);
-    double u = cbrt(-0.5 * q + (q <= 0.0 ? sq : -sq));
-    double y = (u != 0.0) ? u - p / (3.0 * u) : 0.0;
-    roots[0] = y - a / 3.0;
-    m = 1;
-  } else {
-    double r = sqrt(std_max(0.0, -p / 3.0));
-    if (r == 0.0) {
-      roots[0] = roots[1] = roots[2] = -a / 3.0;
-    } else {
-      double arg = std_max(-1.0, std_min(1.0, -0.5 * q / (r * r * r)));
-      double phi = acos(arg) / 3.0;
-      for (int k = 0; k < 3; ++k) roots[k] = 2.0 * r * cos(phi - 2.0943951023931954923 * k) - a / 3.0;
-    }
-    m = 3;
-  }
-  double cc[4] = {c, b, a, 1.0};
-  for (int k = 0; k < m; ++k)
-    for (int s = 0; s < 2; ++s) {
-      double f = cubic_eval(cc, roots[k]), df = cubic_deriv(cc, roots[k]);
-      if (df != 0.0 && isfinite(f / df)) roots[k] -= f / df;
-    }
-  return m;
-}
-
 // Among the real stationary points of e(t) = z0 + z1 t + ... + z4 t^4 in [-10, 10] the
-// one with least e(t); else t = 0.5 (otsolver_2dgrid.cpp:575-595).
+// one with least e(t); else t = 0.5 (otsolver_2dgrid.cpp:575-595). The roots of the cubic
+// e'(t) come in closed form (Cardano for one real root of the depressed cubic, the
+// trigonometric form for three) with two Newton steps each; that replaces the companion-
+// matrix eigensolver of otsolver_2dgrid.cpp:568-572. Called by a whole warp with the same z:
+// lane k takes root k, so that the cosines, divisions and Newton steps of three roots take
+// the time of one -- the step is a serial section of every iteration.
 __device__ __forceinline__ void pick_step(const double z[5], double* alpha, double* emin) {
-  double w[4] = {z[1], 2.0 * z[2], 3.0 * z[3], 4.0 * z[4]};
-  double roots[3];
-  int m = cubic_real_roots(w, roots);
+  const int lane = threadIdx.x & 31, root = lane < 2 ? lane : 2;
+  const double w0 = z[1], w1 = 2.0 * z[2], w2 = 3.0 * z[3], w3 = 4.0 * z[4];
+  const double a = w2 / w3, b = w1 / w3, c = w0 / w3;
+  int m = 0;
+  double t = 0.0;
+  if (isfinite(a) && isfinite(b) && isfinite(c)) {
+    const double p = b - a * a / 3.0;
+    const double q = 2.0 * a * a * a / 27.0 - a * b / 3.0 + c;
+    const double disc = 0.25 * q * q + p * p * p / 27.0;
+    if (disc > 0.0) {
+      const double sq = sqrt(disc);
+      const double u = cbrt(-0.5 * q + (q <= 0.0 ? sq : -sq));
+      const double y = (u != 0.0) ? u - p / (3.0 * u) : 0.0;
+      t = y - a / 3.0;
+      m = 1;
+    } else {
+      const double r = sqrt(std_max(0.0, -p / 3.0));
+      if (r == 0.0) {
+        t = -a / 3.0;
+      } else {
+        const double arg = std_max(-1.0, std_min(1.0, -0.5 * q / (r * r * r)));
+        const double phi = acos(arg) / 3.0;
+        t = 2.0 * r * cos(phi - 2.0943951023931954923 * root) - a / 3.0;
+      }
+      m = 3;
+    }
+    const double cc[4] = {c, b, a, 1.0};
+    for (int s = 0; s < 2; ++s) {
+      const double f = cubic_eval(cc, t), df = cubic_deriv(cc, t);
+      if (df != 0.0 && isfinite(f / df)) t -= f / df;
+    }
+  }
+  const double e = z[0] + t * (z[1] + t * (z[2] + t * (z[3] + t * z[4])));
+  const int ok = root < m && t >= -10.0 && t <= 10.0;
   bool found = false;
   double best = 0.0, rmin = 0.0;
-  for (int k = 0; k < m; ++k) {
-    double t = roots[k];
-    if (t >= -10.0 && t <= 10.0) {
-      double r = z[0] + t * (z[1] + t * (z[2] + t * (z[3] + t * z[4])));
-      if (!found || r < rmin) {
-        found = true;
-        best = t;
-        rmin = r;
-      }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const double tk = __shfl_sync(0xffffffffu, t, k), ek = __shfl_sync(0xffffffffu, e, k);
+    if (__shfl_sync(0xffffffffu, ok, k) && (!found || ek < rmin)) {
+      found = true;
+      best = tk;
+      rmin = ek;
     }
   }
   if (!found) {

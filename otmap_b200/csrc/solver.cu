@@ -203,6 +203,11 @@ __global__ __launch_bounds__(NT) void k_residual_init(Inst* insts, const int* ti
   double v[1] = {0.0};
   double mx = -INFINITY;
   if (t.inside) {
+    // the state the first iteration reads: potential, directions, the residual before r_0
+    I.psi[0][t.f] = 0.0;
+    I.d[0][t.f] = 0.0;
+    I.d[1][t.f] = 0.0;
+    I.r[2][t.f] = 0.0;
     double r = e * e - ea * I.rho[t.f];
     if (I.split) {
       // FP32 residual: the sums below start from the stored (rounded) values
@@ -437,14 +442,17 @@ __global__ __launch_bounds__(NT) void k_coeffs(Inst* insts, const int* tile_inst
   if (last_block(&I.counter, I.ntiles)) {
     double sum[6];
     reduce_partials<6>(partials, I.tile0, I.ntiles, sum, red);
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {  // block_sum's totals are on every lane of the first warp
       const double ea = elem_area(n);
       double z[5] = {I.residual * ea, 2.0 * sum[0], sum[1] + 2 * sum[2], 2.0 * sum[3], sum[4]};
       double alpha, rmin;
       pick_step(z, &alpha, &rmin);
-      I.alpha = alpha;
-      I.residual = rmin / ea;
-      I.dnorm = sqrt(sum[5]);
+      __syncwarp();
+      if (threadIdx.x == 0) {
+        I.alpha = alpha;
+        I.residual = rmin / ea;
+        I.dnorm = sqrt(sum[5]);
+      }
     }
   }
 }
@@ -593,16 +601,20 @@ static std::vector<Inst> layout_workspace(otm_context* ctx, const std::vector<in
   int tiles = 0, gemm = 0, rows = 0, cols = 0, tcitems = 0;
   // Taller sweep strips halve the per-strip overhead (ring prologue, block reduction) when
   // the batch has blocks to spare; a batch that does not fill the GPU twice over keeps
-  // 32-row strips for parallelism, and one with fewer 32-row blocks than SMs takes 16-row
-  // strips (a lone 512^2 solve: sums 28 -> 24.5 us, update 21 -> 16.4 us).
+  // 32-row strips for parallelism, and one with fewer 32-row blocks than SMs takes the
+  // tallest of 16, 8 and 4 rows that gives four SMs in five a block (a lone 512^2 solve 16:
+  // sums 28 -> 24.5 us, update 21 -> 16.4 us; a lone 256^2 one 4).
   int srows = 32;
   {
-    long blocks32 = 0;
-    for (int q = 0; q < count; ++q) blocks32 += strip_blocks(sizes[q], 32);
-    if (blocks32 >= 6L * ctx->num_sms)
+    auto blocks = [&](int rows) {
+      long b = 0;
+      for (int n : sizes) b += strip_blocks(n, rows);
+      return b;
+    };
+    if (blocks(32) >= 6L * ctx->num_sms)
       srows = 64;
-    else if (blocks32 < ctx->num_sms)
-      srows = 16;
+    else if (blocks(32) < ctx->num_sms)
+      for (srows = 16; srows > 4 && 5 * blocks(srows) < 4L * ctx->num_sms;) srows /= 2;
   }
   for (int q = 0; q < count; ++q) {
     int n = sizes[q];
@@ -836,6 +848,11 @@ static void launch_iteration(otm_context* ctx, Inst* d_insts) {
   sweep_update(ctx, d_insts, si, s64, s32, true, sp);
 }
 
+// Iterations per body of the loop's WHILE node: a body and its check kernel cost about 4 us
+// beside the iteration's kernels (measured with empty ones), an iteration after the last
+// instance stopped five launches that return at once (about 5 us).
+constexpr int ITERS_PER_BODY = 4;
+
 // Captures the iteration loop of the current workspace into a graph with a WHILE node.
 static void build_loop_graph(otm_context* ctx, int count) {
   Workspace& ws = ctx->ws();
@@ -861,7 +878,7 @@ static void build_loop_graph(otm_context* ctx, int count) {
     const long before = ctx->launches;
     OTM_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     try {
-      launch_iteration(ctx, ws.insts.as<Inst>());
+      for (int u = 0; u < ITERS_PER_BODY; ++u) launch_iteration(ctx, ws.insts.as<Inst>());
       launch(ctx, "loop_check", k_loop_check, 1, 256, (const Inst*)ws.insts.as<Inst>(), count,
              ws.loopctl.as<LoopCtl>(), handle);
     } catch (...) {
@@ -897,11 +914,6 @@ static std::vector<Inst> run_solver(otm_context* ctx, std::vector<Inst>& h, cons
     I.beta_cj = o.beta == OTM_BETA_CONJUGATE_JACOBIAN ? 1 : 0;
     I.threshold = o.threshold;
     I.max_ratio = o.max_ratio;
-    size_t N = (size_t)I.n * I.n;
-    OTM_CUDA(cudaMemsetAsync(I.psi[0], 0, N * sizeof(double), st));
-    OTM_CUDA(cudaMemsetAsync(I.d[0], 0, N * sizeof(double), st));
-    OTM_CUDA(cudaMemsetAsync(I.d[1], 0, N * sizeof(double), st));
-    OTM_CUDA(cudaMemsetAsync(I.r[2], 0, N * sizeof(double), st));
   }
   Inst* d_insts = ws.insts.as<Inst>();
   OTM_CUDA(cudaMemcpyAsync(d_insts, h.data(), sizeof(Inst) * count, cudaMemcpyHostToDevice, st));
@@ -1438,16 +1450,11 @@ extern "C" int otm_solve_noalloc(int n, const double* density, const otm_solver_
       g_noalloc_checked[dev][n] = 1;
     }
 
-    // state that must start at zero: the initial potential, the directions and the
-    // residual buffer read as r_{k-1} in the first iteration (the record is rewritten)
+    // the record is rewritten; the state that starts at zero is written by k_residual_init
     I.max_iter = o.max_iter;
     I.beta_cj = o.beta == OTM_BETA_CONJUGATE_JACOBIAN ? 1 : 0;
     I.threshold = o.threshold;
     I.max_ratio = o.max_ratio;
-    OTM_CUDA(cudaMemsetAsync(I.psi[0], 0, N * sizeof(double), st));
-    OTM_CUDA(cudaMemsetAsync(I.d[0], 0, N * sizeof(double), st));
-    OTM_CUDA(cudaMemsetAsync(I.d[1], 0, N * sizeof(double), st));
-    OTM_CUDA(cudaMemsetAsync(I.r[2], 0, N * sizeof(double), st));
     OTM_CUDA(cudaMemcpyAsync(d_inst, &I, sizeof(Inst), cudaMemcpyHostToDevice, st));
     OTM_CUDA(cudaMemcpyAsync(I.rho, density, N * sizeof(double),
                              is_device_ptr(density) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));

@@ -213,23 +213,46 @@ __device__ __forceinline__ StripCoord strip_coord(const Inst& I, int block) {
   return s;
 }
 
+// Warp totals of 16 < K <= 32 values per lane: afterwards v[0] on lane l is the total of value
+// l (l < K), formed by the tree of warp_sum. Each step hands half of the remaining values to
+// the partner lane: 31 exchanges instead of 5 K.
 template <int K>
-__device__ __forceinline__ void write_partials(double (&v)[K], double* red, double* partials, int block) {
-  block_sum<K>(v, red);
-  if (threadIdx.x == 0)
+__device__ __forceinline__ void warp_totals(double (&v)[K], int lane) {
+  static_assert(K > 16 && K <= 32, "one exchange of 16 halves the values");
 #pragma unroll
-    for (int k = 0; k < K; ++k) partials[(size_t)block * KA + k] = v[k];
+  for (int q = 0; q < 16; ++q) {
+    if (q + 16 < K) {
+      const bool up = lane & 16;
+      const double send = up ? v[q] : v[q + 16], keep = up ? v[q + 16] : v[q];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+    } else {
+      v[q] += __shfl_xor_sync(0xffffffffu, v[q], 16);
+    }
+  }
+#pragma unroll
+  for (int h = 8; h >= 1; h >>= 1) {
+    const bool up = lane & h;
+#pragma unroll
+    for (int q = 0; q < h; ++q) {
+      const double send = up ? v[q] : v[q + h], keep = up ? v[q + h] : v[q];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+    }
+  }
 }
 
+// Block totals of K values per thread: thread k < K returns value k's, formed by block_sum's
+// tree. red: SWARPS * 32 doubles. The reduction is on every block's way out and twice on the
+// last block's, where nothing else runs: with one tree per value it was half of a small
+// grid's sum sweep.
 template <int K>
-__device__ __forceinline__ void reduce_block_partials(const double* partials, int b0, int nb, double (&v)[K],
-                                                      double* red) {
-#pragma unroll
-  for (int k = 0; k < K; ++k) v[k] = 0.0;
-  for (int t = threadIdx.x; t < nb; t += blockDim.x)
-#pragma unroll
-    for (int k = 0; k < K; ++k) v[k] += __ldcg(&partials[(size_t)(b0 + t) * KA + k]);
-  block_sum<K>(v, red);
+__device__ __forceinline__ double block_totals(double (&v)[K], double* red) {
+  static_assert(SWARPS == 4, "the tree over the warps is written out");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = threadIdx.x;
+  warp_totals<K>(v, lane);
+  __syncthreads();
+  red[warp * 32 + lane] = v[0];
+  __syncthreads();
+  return k < K ? (red[k] + red[64 + k]) + (red[32 + k] + red[96 + k]) : 0.0;
 }
 
 // Sum slots of k_sweep_sums.
@@ -243,10 +266,12 @@ enum {
   S_COUNT
 };
 
-// Last block of an instance in the sum sweep (thread 0): restores the factor (n/2)^2 / 2
+// Last block of an instance in the sum sweep (one warp, every lane with the same sums; lane 0
+// writes): restores the factor (n/2)^2 / 2
 // of the line coefficients in the sums, then the early exit (otsolver_2dgrid.cpp:182),
 // beta (:248-261) and the step alpha of the quartic for d = d_hat + beta d_prev (:541-606).
 __device__ __forceinline__ void sums_step(Inst& I, double (&S)[S_COUNT], int n, int it) {
+  const bool writes = (threadIdx.x & 31) == 0;
   const double hw = 0.5 * (double)n;
   const double h2 = 0.5 * hw * hw, h4 = h2 * h2;
   S[S_JB] *= h2;
@@ -261,18 +286,20 @@ __device__ __forceinline__ void sums_step(Inst& I, double (&S)[S_COUNT], int n, 
 #pragma unroll
   for (int k = S_AB0; k < S_COUNT; ++k) S[k] *= h4;
   if (sqrt(S[S_HH]) <= 2.0 * DBL_MIN) {  // otsolver_2dgrid.cpp:182
-    I.active = 0;
-    I.outcome = OTM_SMALL_STEP;
+    if (writes) {
+      I.active = 0;
+      I.outcome = OTM_SMALL_STEP;
+    }
     return;
   }
   const bool use_beta = it >= 1 && I.beta_cj;
-  I.use_beta = use_beta ? 1 : 0;
+  double B = 0.0;
   if (use_beta) {
     const double alpha = I.alpha, eps = alpha / 2.0;
     const double num = -eps * S[S_JB] + eps * eps * S[S_JA];
-    I.beta = std_max(-1.0, num / S[S_JJ] / eps * alpha);
+    B = std_max(-1.0, num / S[S_JJ] / eps * alpha);
   }
-  const double B = use_beta ? I.beta : 0.0, B2 = B * B, B3 = B2 * B, B4 = B2 * B2;
+  const double B2 = B * B, B3 = B2 * B, B4 = B2 * B2;
   const double sbr = S[S_B1R] + B * S[S_B2R];
   const double sbb = S[S_B1B1] + 2.0 * B * S[S_B1B2] + B2 * S[S_B2B2];
   const double sar = S[S_A11R] + B * S[S_A12R] + B2 * S[S_A22R];
@@ -282,6 +309,10 @@ __device__ __forceinline__ void sums_step(Inst& I, double (&S)[S_COUNT], int n, 
   double z[5] = {I.residual * ea, 2.0 * sbr, sbb + 2 * sar, 2.0 * sab, saa};
   double alpha, rmin;
   pick_step(z, &alpha, &rmin);
+  __syncwarp();  // every lane has read the record
+  if (!writes) return;
+  I.use_beta = use_beta ? 1 : 0;
+  if (use_beta) I.beta = B;
   I.alpha = alpha;
   I.residual = rmin / ea;
   I.dnorm = sqrt(std_max(0.0, S[S_HH] + 2.0 * B * S[S_HQ] + B2 * S[S_QQ]));
@@ -416,7 +447,7 @@ struct RingS {
 template <class RT, bool SPLIT>
 __global__ __launch_bounds__(ST) void k_sweep_sums_t(Inst* insts, const int* strip_inst, int base, double* partials) {
   extern __shared__ __align__(16) unsigned char ring_raw[];
-  __shared__ double red[32 * S_COUNT];
+  __shared__ double red[32 * SWARPS];
   const int blk = base + blockIdx.x;
   Inst& I = insts[strip_inst[blk]];
   if (!I.active) return;
@@ -500,11 +531,28 @@ __global__ __launch_bounds__(ST) void k_sweep_sums_t(Inst* insts, const int* str
     }
     cp_async_wait<0>();
   }
-  write_partials<S_COUNT>(acc, red, partials, blk);
+  const double part = block_totals<S_COUNT>(acc, red);
+  if (threadIdx.x < S_COUNT) partials[(size_t)blk * KA + threadIdx.x] = part;
   if (last_block(&I.counter, I.nstrip)) {
     double S[S_COUNT];
-    reduce_block_partials<S_COUNT>(partials, I.strip0, I.nstrip, S, red);
-    if (threadIdx.x == 0) sums_step(I, S, n, it);
+#pragma unroll
+    for (int k = 0; k < S_COUNT; ++k) S[k] = 0.0;
+    for (int t = threadIdx.x; t < I.nstrip; t += ST) {
+      const double2* p = reinterpret_cast<const double2*>(partials + (size_t)(I.strip0 + t) * KA);
+      double2 x[(S_COUNT + 1) / 2];
+#pragma unroll
+      for (int k = 0; k < (S_COUNT + 1) / 2; ++k) x[k] = __ldcg(&p[k]);
+#pragma unroll
+      for (int k = 0; k < S_COUNT; ++k) S[k] += (k & 1) ? x[k >> 1].y : x[k >> 1].x;
+    }
+    const double total = block_totals<S_COUNT>(S, red);
+    if (threadIdx.x < S_COUNT) red[threadIdx.x] = total;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+#pragma unroll
+      for (int k = 0; k < S_COUNT; ++k) S[k] = red[k];
+      sums_step(I, S, n, it);
+    }
   }
 }
 
