@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <vector>
 
 #include "engine.cuh"
@@ -37,6 +38,7 @@ __device__ __forceinline__ int clampv(int v, int n) { return v < 0 ? 0 : (v >= n
 struct AdjCtl {
   int j;       // the step being taken: basis vectors 0..j are orthonormal
   int go;      // the cycle takes another step
+  int live;    // the map takes part in the cycle
   int m;       // restart length
   int budget;  // steps allowed in this cycle (the call's cap on Poisson solves)
   double bnorm, tol;
@@ -45,8 +47,25 @@ struct AdjCtl {
   int fault;             // the steps' transform gave up a bounded wait
 };
 
+// The adjoints of up to 8 maps of one size run together: block row y of every kernel works
+// for map y, on the map's own control block and its own slice of the workspace (the
+// pointers of map 0 plus y times the stride).
+constexpr int ADJ_MAPS = 8;
+struct AdjArgs {  // the call's buffers per map
+  const double* fwd[ADJ_MAPS];
+  const double* q[ADJ_MAPS];
+  const double* rho[ADJ_MAPS];
+  double* out[ADJ_MAPS];
+};
+struct AdjCycle {  // a restart cycle's parameters per map
+  double bnorm[ADJ_MAPS];
+  int budget[ADJ_MAPS], live[ADJ_MAPS];
+};
+
 // Displacements g of the vertices from the forward mesh.
-__global__ void k_adj_disp(int n, const double* fwd, double2* g) {
+__global__ void k_adj_disp(int n, AdjArgs args, double2* g, long stride) {
+  const double* fwd = args.fwd[blockIdx.y];
+  g += blockIdx.y * (stride / 2);
   const long v = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= (long)(n + 1) * (n + 1)) return;
   const double dx = 1.0 / (double)n;
@@ -57,7 +76,9 @@ __global__ void k_adj_disp(int n, const double* fwd, double2* g) {
 // with gx coefficient (2a-1) n/2 and gy coefficient (2b-1) n/2
 // (otsolver_2dgrid.cpp:379-422 with clamped indices). Cell (i, j) collects every
 // (vertex, a, b) whose clamped position is (i, j).
-__global__ void k_adj_cells(int n, const double* h, double* out) {
+__global__ void k_adj_cells(int n, AdjArgs args, double* out, long stride) {
+  const double* h = args.q[blockIdx.y];
+  out += blockIdx.y * stride;
   const long f = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= (long)n * n) return;
   const int i = (int)(f / n), j = (int)(f % n);
@@ -92,7 +113,7 @@ __global__ void k_adj_cells(int n, const double* h, double* out) {
 // pass on average), so every reduction ends in the last block of the kernel that forms its
 // terms. Against one kernel per operation (source, vertices, cells, 3 x products, 3 x
 // one-block sums, 2 x update, scale, rotation) a step with its transform went from 96 to
-// 59 us at 256^2 (four concurrent ones: 147 to 83), from 159 to 92 us at 512^2.
+// 51 us at 256^2 (four maps: 147 to 80), from 159 to 85 us at 512^2.
 //
 // Cell f belongs to block (f / 256) mod 256 and thread f mod 256; a thread's cells (one for
 // N <= 65536) follow each other 65536 apart. A product is an FMA chain over a thread's cells,
@@ -227,36 +248,61 @@ __device__ __forceinline__ void block_dots(long N, const double* w, const double
   for (int i = threadIdx.x; i < P; i += AT) partial[(size_t)i * ANB + blockIdx.x] = sum_warps(red + i, RED_LD);
 }
 
-// Last block: out(i, total) for the P totals of the blocks' partials, each summed in block
-// order by one thread from a staged copy (TOT_CHUNK values at a time).
-constexpr int TOT_CHUNK = 16, TOT_LD = ANB + 1;
+// Last block: out(i, total) for the P totals of the blocks' partials. Each is a chain of adds
+// in block order on one thread (the order that fixes the result), so all values' chains run
+// at once and the partials come through shared memory in tiles, the next tile's loads in
+// flight during a tile's adds.
+constexpr int TOT_V = 48, TOT_B = 64;  // values and blocks per tile
+constexpr int TOT_STAGE = TOT_V * (TOT_B + 1);
 template <class F>
 __device__ __forceinline__ void totals(const double* partial, int P, double* stage, F out) {
-  const int nb = gridDim.x;
-  for (int i0 = 0; i0 < P; i0 += TOT_CHUNK) {
-    const int cnt = min(TOT_CHUNK, P - i0);
-    __syncthreads();
-    if (threadIdx.x < nb) {
+  constexpr int PER = TOT_V * TOT_B / AT;
+  const int nb = gridDim.x, b = threadIdx.x % TOT_B, v0 = threadIdx.x / TOT_B;
+  for (int i0 = 0; i0 < P; i0 += TOT_V) {
+    const int cnt = min(TOT_V, P - i0);
+    double next[PER], t = 0.0;
+    auto fetch = [&](int b0) {
 #pragma unroll
-      for (int c = 0; c < TOT_CHUNK; ++c)
-        if (c < cnt) stage[c * TOT_LD + threadIdx.x] = __ldcg(&partial[(size_t)(i0 + c) * ANB + threadIdx.x]);
-    }
-    __syncthreads();
-    if (threadIdx.x < cnt) {
-      double t = 0.0;
+      for (int k = 0; k < PER; ++k) {
+        const int i = v0 + k * (AT / TOT_B);
+        next[k] = i < cnt && b0 + b < nb ? __ldcg(&partial[(size_t)(i0 + i) * ANB + b0 + b]) : 0.0;
+      }
+    };
+    fetch(0);
+    for (int b0 = 0; b0 < nb; b0 += TOT_B) {
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < PER; ++k) stage[(v0 + k * (AT / TOT_B)) * (TOT_B + 1) + b] = next[k];
+      __syncthreads();
+      fetch(b0 + TOT_B);
+      if (threadIdx.x < cnt) {
+        const double* s = stage + threadIdx.x * (TOT_B + 1);
+        if (b0 + TOT_B <= nb) {
 #pragma unroll 16
-      for (int b = 0; b < nb; ++b) t += stage[threadIdx.x * TOT_LD + b];
-      out(i0 + threadIdx.x, t);
+          for (int k = 0; k < TOT_B; ++k) t += s[k];
+        } else {
+          for (int k = 0; k < nb - b0; ++k) t += s[k];
+        }
+      }
     }
+    if (threadIdx.x < cnt) out(i0 + threadIdx.x, t);
   }
 }
 
 // w = V_{j+1} = J^T z (z = M^+ v_j); Hessenberg column and combine coefficients c_i of the
 // first Gram-Schmidt pass.
 __global__ __launch_bounds__(AT) void k_adj_apply(int n, const double2* g, const double* z, double* V, long ld,
-                                                  AdjCtl* ctl, double* partial, double* hcol, double* c) {
-  __shared__ double red[AT / 32 * RED_LD], stage[TOT_CHUNK * TOT_LD];
+                                                  AdjCtl* ctl, double* partial, double* hcol, double* c, long stride) {
+  __shared__ double red[AT / 32 * RED_LD], stage[TOT_STAGE];
+  const long off = blockIdx.y * stride;
+  ctl += blockIdx.y;
   if (!ctl->go) return;
+  g += off / 2;
+  z += off;
+  V += off;
+  partial += off;
+  hcol += off;
+  c += off;
   const int j = ctl->j, P = j + 1;
   const long N = (long)n * n;
   double* w = V + (size_t)(j + 1) * ld;
@@ -286,16 +332,60 @@ __device__ __forceinline__ double combine(long N, double* w, const double* V, lo
   return ss;
 }
 
-// First Gram-Schmidt update and the products of the second pass.
+// First Gram-Schmidt update and the products of the second pass. With one cell per thread and
+// a basis of at most ORTH_V vectors (a default cycle) the thread's basis values stay in
+// registers between the two, all their loads in flight together.
+constexpr int ORTH_V = 40;
 __global__ __launch_bounds__(AT) void k_adj_orth(int n, double* V, long ld, AdjCtl* ctl, double* partial, double* hcol,
-                                                 double* c) {
-  __shared__ double sc[ADJ_MAX_M + 8], red[AT / 32 * RED_LD], stage[TOT_CHUNK * TOT_LD];
+                                                 double* c, long stride) {
+  __shared__ double sc[ADJ_MAX_M + 8], red[AT / 32 * RED_LD], stage[TOT_STAGE];
+  const long off = blockIdx.y * stride;
+  ctl += blockIdx.y;
   if (!ctl->go) return;
+  V += off;
+  partial += off;
+  hcol += off;
+  c += off;
   const int j = ctl->j, P = j + 1;
   const long N = (long)n * n;
   double* w = V + (size_t)(j + 1) * ld;
-  combine(N, w, V, ld, P, c, sc);
-  block_dots(N, w, V, ld, P, red, partial);
+  if (N <= (long)ANB * AT && P <= ORTH_V) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long f = (long)blockIdx.x * AT + threadIdx.x;
+    const bool in = f < N;
+    double v[ORTH_V], x = in ? w[f] : 0.0;
+#pragma unroll
+    for (int i0 = 0; i0 < ORTH_V; i0 += DOT_CHUNK)
+      if (i0 < P) {
+#pragma unroll
+        for (int k = i0; k < i0 + DOT_CHUNK; ++k) v[k] = in && k < P ? V[(size_t)k * ld + f] : 0.0;
+      }
+    for (int i = threadIdx.x; i < P; i += AT) sc[i] = c[i];
+    __syncthreads();
+#pragma unroll
+    for (int i0 = 0; i0 < ORTH_V; i0 += DOT_CHUNK)
+      if (i0 < P) {
+#pragma unroll
+        for (int k = i0; k < i0 + DOT_CHUNK; ++k)
+          if (k < P) x = fma(-sc[k], v[k], x);
+      }
+    if (in) w[f] = x;
+#pragma unroll
+    for (int i0 = 0; i0 < ORTH_V; i0 += DOT_CHUNK)
+      if (i0 < P) {
+        double s[DOT_CHUNK];
+#pragma unroll
+        for (int k = 0; k < DOT_CHUNK; ++k) s[k] = fma(x, v[i0 + k], 0.0);
+        warp_sum8(s, lane);
+        const int i = i0 + ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+        if ((lane & 3) == 0 && i < P) red[warp * RED_LD + i] = s[0];
+      }
+    __syncthreads();
+    for (int i = threadIdx.x; i < P; i += AT) partial[(size_t)i * ANB + blockIdx.x] = sum_warps(red + i, RED_LD);
+  } else {
+    combine(N, w, V, ld, P, c, sc);
+    block_dots(N, w, V, ld, P, red, partial);
+  }
   if (!last_block(&ctl->counter, gridDim.x)) return;
   totals(partial, P, stage, [&](int i, double d) {
     c[i] = d;
@@ -311,10 +401,21 @@ __global__ __launch_bounds__(AT) void k_adj_orth(int n, double* V, long ld, AdjC
 // Poisson record of the next step gets its source.
 __global__ __launch_bounds__(AT) void k_adj_norm(int n, double* V, long ld, AdjCtl* ctl, double* inv, double* partial,
                                                  const double* hcol, const double* c, double* H, double* cs, double* sn,
-                                                 double* gv, Inst* rec, cudaGraphConditionalHandle handle,
-                                                 int in_graph) {
-  __shared__ double sc[ADJ_MAX_M + 8], sh[ADJ_MAX_M + 8], ss[ADJ_MAX_M + 8], red[64], stage[TOT_CHUNK * TOT_LD];
+                                                 double* gv, Inst* rec, long stride) {
+  __shared__ double sc[ADJ_MAX_M + 8], sh[ADJ_MAX_M + 8], ss[ADJ_MAX_M + 8], red[64], stage[TOT_STAGE];
+  const long off = blockIdx.y * stride;
+  ctl += blockIdx.y;
   if (!ctl->go) return;
+  V += off;
+  inv += off;
+  partial += off;
+  hcol += off;
+  c += off;
+  H += off;
+  cs += off;
+  sn += off;
+  gv += off;
+  rec += blockIdx.y;
   const int j = ctl->j, P = j + 1;
   const long N = (long)n * n;
   double v[1] = {combine(N, V + (size_t)(j + 1) * ld, V, ld, P, c, sc)};
@@ -351,18 +452,25 @@ __global__ __launch_bounds__(AT) void k_adj_norm(int n, double* V, long ld, AdjC
     rec->r[0] = V + (size_t)k * ld;
     rec->active = go;
     ctl->fault = rec->fault;
-    if (in_graph) cudaGraphSetConditional(handle, go ? 1u : 0u);
   });
   __syncthreads();
   for (int i = threadIdx.x; i <= j; i += AT) H[(size_t)i * m + j] = sh[i];
 }
 
 // v_j = w / |w|, the vector k_adj_norm has just moved the cycle on to (the last one of a
-// cycle is not used).
-__global__ void k_adj_scale_by(long N, double* V, long ld, const double* a, const AdjCtl* ctl) {
+// cycle is not used). The step's last kernel: in the graph it keeps the WHILE node going
+// while any map's cycle goes on.
+__global__ void k_adj_scale_by(long N, double* V, long ld, const double* a, const AdjCtl* ctl, long stride,
+                               cudaGraphConditionalHandle handle, int in_graph) {
+  if (in_graph && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+    int any = 0;
+    for (int y = 0; y < (int)gridDim.y; ++y) any |= ctl[y].go;
+    cudaGraphSetConditional(handle, any ? 1u : 0u);
+  }
+  ctl += blockIdx.y;
   if (!ctl->go) return;
   const long f = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (f < N) V[(size_t)ctl->j * ld + f] *= *a;
+  if (f < N) V[blockIdx.y * stride + (size_t)ctl->j * ld + f] *= a[blockIdx.y * stride];
 }
 
 // Every Poisson record of the workspace ready for a new call: a bounded wait that gave up in
@@ -376,31 +484,42 @@ __global__ void k_adj_reset_recs(Inst* recs, int count) {
 }
 
 // Start of a restart cycle from the vector in V_0, whose norm k_adj_resid left in the state:
-// v_0, g and the cycle's state.
-__global__ void k_adj_cycle_init(long N, AdjCtl* ctl, double* gv, int m, double bnorm, double tol, int budget,
-                                 Inst* rec, double* V) {
+// v_0, g, the cycle's state and the Poisson records of its steps (rec) and of its end (rec_h).
+__global__ void k_adj_cycle_init(long N, AdjCtl* ctl, double* gv, int m, AdjCycle cyc, double tol, Inst* rec,
+                                 Inst* rec_h, double* V, long stride) {
+  const int y = blockIdx.y;
+  ctl += y;
+  const int live = cyc.live[y];
   const double rnorm = ctl->rnorm, a = 1.0 / rnorm;
   const long f = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (f < N) V[f] *= a;
-  if (f <= m) gv[f] = f ? 0.0 : rnorm;
+  if (f < N && live) V[y * stride + f] *= a;
+  if (f <= m) gv[y * stride + f] = f ? 0.0 : rnorm;
   if (f != 0) return;
+  ctl->live = live;
   ctl->j = 0;
-  ctl->go = budget > 0 ? 1 : 0;
+  ctl->go = live && cyc.budget[y] > 0 ? 1 : 0;
   ctl->m = m;
-  ctl->budget = budget;
-  ctl->bnorm = bnorm;
+  ctl->budget = cyc.budget[y];
+  ctl->bnorm = cyc.bnorm[y];
   ctl->tol = tol;
-  ctl->fault = rec->fault;
-  rec->r[0] = V;
-  if (!rec->fault) rec->active = 1;
+  ctl->fault = rec[y].fault;
+  rec[y].r[0] = V + y * stride;
+  rec[y].active = live && !rec[y].fault;
+  rec_h[y].active = live && !rec_h[y].fault;
 }
 
 // H y = g for the k = j steps of the cycle: y into c (row-oriented back substitution by one
 // thread, on a shared copy of the triangle: read where it lies, each of its k^2 / 2 elements
 // was a wait on L2, 51 us at k = 40).
-__global__ __launch_bounds__(256) void k_adj_trisolve(const AdjCtl* ctl, const double* H, const double* gv, double* c) {
+__global__ __launch_bounds__(256) void k_adj_trisolve(const AdjCtl* ctl, const double* H, const double* gv, double* c,
+                                                      long stride) {
   constexpr int KS = 64;  // triangles up to this order are staged; larger ones are read where they lie
   __shared__ double sH[KS * KS], y[ADJ_MAX_M + 8];
+  ctl += blockIdx.y;
+  if (!ctl->live) return;
+  H += blockIdx.y * stride;
+  gv += blockIdx.y * stride;
+  c += blockIdx.y * stride;
   const int k = ctl->j, m = ctl->m;
   const bool staged = k <= KS;
   if (staged)
@@ -422,7 +541,13 @@ __global__ __launch_bounds__(256) void k_adj_trisolve(const AdjCtl* ctl, const d
 }
 
 // out = sum_i c_i v_i over the cycle's steps
-__global__ void k_adj_span(long N, double* out, const double* V, long ld, const double* c, const AdjCtl* ctl) {
+__global__ void k_adj_span(long N, double* out, const double* V, long ld, const double* c, const AdjCtl* ctl,
+                           long stride) {
+  ctl += blockIdx.y;
+  if (!ctl->live) return;
+  out += blockIdx.y * stride;
+  V += blockIdx.y * stride;
+  c += blockIdx.y * stride;
   const int m = ctl->j;
   const long f = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= N) return;
@@ -432,10 +557,20 @@ __global__ void k_adj_span(long N, double* out, const double* V, long ld, const 
   out[f] = x;
 }
 
-// v = b - J^T lambda (lambda null: v = b) and its norm into the state.
+// v = b - J^T lambda for the maps of the last cycle (lambda null: v = b, every map) and its
+// norm into the state.
 __global__ __launch_bounds__(AT) void k_adj_resid(int n, const double2* g, const double* lambda, const double* b,
-                                                  double* v, AdjCtl* ctl, double* partial) {
-  __shared__ double red[64], stage[TOT_CHUNK * TOT_LD];
+                                                  double* v, AdjCtl* ctl, double* partial, long stride) {
+  __shared__ double red[64], stage[TOT_STAGE];
+  ctl += blockIdx.y;
+  if (lambda) {
+    if (!ctl->live) return;
+    lambda += blockIdx.y * stride;
+  }
+  g += blockIdx.y * (stride / 2);
+  b += blockIdx.y * stride;
+  v += blockIdx.y * stride;
+  partial += blockIdx.y * stride;
   const long N = (long)n * n;
   double s[1] = {0.0};
   for (long f = (long)blockIdx.x * AT + threadIdx.x; f < N; f += (long)ANB * AT) {
@@ -450,12 +585,17 @@ __global__ __launch_bounds__(AT) void k_adj_resid(int n, const double2* g, const
   totals(partial, 1, stage, [&](int, double t) { ctl->rnorm = sqrt(t); });
 }
 
-__global__ void k_adj_neg(long N, const double* z, double* lambda) {
+__global__ void k_adj_neg(long N, const double* z, double* lambda, long stride) {
+  z += blockIdx.y * stride;
+  lambda += blockIdx.y * stride;
   const long f = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (f < N) lambda[f] = -z[f];
 }
 
-__global__ void k_adj_add(long N, const double* z, double* lambda) {
+__global__ void k_adj_add(long N, const double* z, double* lambda, const AdjCtl* ctl, long stride) {
+  if (!ctl[blockIdx.y].live) return;
+  z += blockIdx.y * stride;
+  lambda += blockIdx.y * stride;
   const long f = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (f < N) lambda[f] += z[f];
 }
@@ -464,8 +604,13 @@ __global__ void k_adj_add(long N, const double* z, double* lambda) {
 // per thread, trees over its lanes and warps), each of its warps on an SM of its own: one SM
 // draws 4 MB at about 90 GB/s, 41 us at 512^2 where 32 take 8.
 constexpr int RHO_BLOCKS = 32;
-__global__ __launch_bounds__(32) void k_adj_rho_sums(long N, const double* lambda, const double* rho, AdjCtl* ctl,
-                                                     double* partial, double* sums) {
+__global__ __launch_bounds__(32) void k_adj_rho_sums(long N, const double* lambda, AdjArgs args, AdjCtl* ctl,
+                                                     double* partial, double* sums, long stride) {
+  const double* rho = args.rho[blockIdx.y];
+  lambda += blockIdx.y * stride;
+  ctl += blockIdx.y;
+  partial += blockIdx.y * stride;
+  sums += blockIdx.y * stride;
   constexpr int B = 8, T = 32 * RHO_BLOCKS;
   double v[2] = {0.0, 0.0};
   for (long f0 = (long)blockIdx.x * 32 + threadIdx.x; f0 < N; f0 += (long)B * T) {
@@ -496,7 +641,10 @@ __global__ __launch_bounds__(32) void k_adj_rho_sums(long N, const double* lambd
   }
 }
 
-__global__ void k_adj_finish(long N, const double* lambda, const double* sums, double* out) {
+__global__ void k_adj_finish(long N, const double* lambda, const double* sums, AdjArgs args, long stride) {
+  double* out = args.out[blockIdx.y];
+  lambda += blockIdx.y * stride;
+  sums += blockIdx.y * stride;
   const long f = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (f < N) out[f] = (lambda[f] - sums[0] / sums[1]) / sums[1];
 }
@@ -508,46 +656,51 @@ using namespace otm;
 namespace otm {
 void dense_poisson(otm_context* ctx, Inst* d_inst, const int* gemm_inst, int G);
 
-// Adjoint workspace of one grid size, kept by the context: device vectors, the Krylov
-// basis and one Poisson record per (source, destination) pair the solver uses, so a call
-// allocates nothing and uploads nothing but its inputs' pointers.
+// Adjoint workspace of one grid size and number of maps, kept by the context: device vectors,
+// the Krylov bases and the Poisson records, so a call allocates nothing and uploads nothing
+// but its inputs' pointers.
 struct AdjointWs : otm_context::Erased {
-  int n = 0, m = 0;
+  int n = 0, m = 0, maps = 0;
   size_t N = 0, V = 0, ld = 0;
+  long stride = 0;  // doubles from one map's slice to the next one's
   DevBuf buf, recs, lists;
-  double *b, *lam, *z, *h, *t1, *t2, *Vb, *c, *part, *sums, *hcol, *inv;
-  double2* g;               // the call's vertex displacements
+  double *b, *lam, *z, *h, *t1, *t2, *Vb, *c, *part, *sums, *hcol, *inv;  // of map 0
+  double2* g;                // the call's vertex displacements
   double *H, *cs, *sn, *gv;  // the cycle's Hessenberg state
-  AdjCtl* ctl = nullptr;
-  int nb = 0;  // blocks of the step kernels
-  int G = 0, rows = 0, cols = 0, reg = 0, fft = 0, col_warps = 0;
+  AdjCtl* ctl = nullptr;     // one per map
+  int nb = 0;                // blocks of the step kernels per map
+  int G = 0, rows = 0, cols = 0, reg = 0, fft = 0, col_warps = 0;  // transform items over all maps
   // the Arnoldi step as a graph with a WHILE node (built on first use) and its kernel count
   cudaGraphExec_t step_graph = nullptr;
   long step_kernels = 0;
   ~AdjointWs() override {
     if (step_graph) cudaGraphExecDestroy(step_graph);
   }
-  // record k: src = basis vector k (k < m+1); record m+1: src = b; record m+2: src = h;
-  // record m+3: src = the basis vector of the current step (set on the device, as is its
-  // active flag); dst = z
-  Inst* rec(int k) { return recs.as<Inst>() + k; }
+  // Poisson records, one per map of each kind; destination z. Kind 0: source b; 1: source h;
+  // 2: source the basis vector of the current step (set on the device, as is the active flag)
+  Inst* rec(int kind) { return recs.as<Inst>() + kind * maps; }
 };
 
-static AdjointWs* adjoint_ws(otm_context* ctx, int n, int m) {
-  auto& slot = ctx->adjoint[n];
+static AdjointWs* adjoint_ws(otm_context* ctx, int n, int m, int maps) {
+  auto& slot = ctx->adjoint[n * ADJ_MAPS + maps - 1];
   if (slot && static_cast<AdjointWs*>(slot.get())->m >= m) return static_cast<AdjointWs*>(slot.get());
-  auto* W = new AdjointWs;
+  slot.reset();  // the smaller workspace's memory goes back first
+  auto own = std::make_unique<AdjointWs>();
+  AdjointWs* W = own.get();
   W->n = n;
   W->m = m;
+  W->maps = maps;
   W->N = (size_t)n * n;
   W->V = (size_t)(n + 1) * (n + 1);
   W->ld = (W->N + 31) / 32 * 32;
   W->nb = (int)std::min<size_t>(ANB, (W->N + AT - 1) / AT);
   auto up = [](size_t w) { return (w + 31) / 32 * 32; };  // every array starts on 256 bytes
-  const size_t words = W->ld * 6 + up(2 * W->V) + (size_t)(m + 1) * W->ld + 3 * up(m + 2) + up((size_t)ANB * (m + 2)) +
-                       3 * up(8) + up((size_t)(m + 1) * m) + 2 * up(m);
-  W->buf.reserve(sizeof(double) * words);
+  W->stride = (long)(W->ld * 6 + up(2 * W->V) + (size_t)(m + 1) * W->ld + 3 * up(m + 2) + up((size_t)ANB * (m + 2)) +
+                     2 * up(8) + up((size_t)(m + 1) * m) + 2 * up(m));
+  const size_t ctl_words = (sizeof(AdjCtl) * ADJ_MAPS + 7) / 8;
+  W->buf.reserve(sizeof(double) * ((size_t)W->stride * maps + up(ctl_words)));
   double* q = W->buf.as<double>();
+  W->ctl = reinterpret_cast<AdjCtl*>(q + (size_t)W->stride * maps);
   auto take = [&](size_t w) {
     double* r = q;
     q += up(w);
@@ -563,97 +716,104 @@ static AdjointWs* adjoint_ws(otm_context* ctx, int n, int m) {
   W->Vb = take((size_t)(m + 1) * W->ld);
   W->c = take(m + 2);
   W->hcol = take(m + 2);
-  W->inv = take(8);
   W->gv = take(m + 2);
   W->part = take((size_t)ANB * (m + 2));
+  W->inv = take(8);
   W->sums = take(8);
-  static_assert(sizeof(AdjCtl) <= 8 * sizeof(double), "the cycle state fits its slot");
-  W->ctl = reinterpret_cast<AdjCtl*>(take(8));
   W->H = take((size_t)(m + 1) * m);
   W->cs = take(m);
   W->sn = take(m);
-  OTM_CUDA(cudaMemsetAsync(W->ctl, 0, sizeof(AdjCtl), ctx->stream));
+  OTM_CUDA(cudaMemsetAsync(W->ctl, 0, sizeof(AdjCtl) * ADJ_MAPS, ctx->stream));
   SizeTables* T = ctx->tables.at(n).get();
   Inst base;
   std::memset(&base, 0, sizeof(base));
   base.n = n;
   base.active = 1;
-  base.t1 = W->t1;
-  base.t2 = W->t2;
   base.C = T->C.as<double>();
   base.cosk = T->cosk.as<double>();
   base.tw = T->tw.as<double2>();
   base.pt = T->pt.as<double2>();
   base.fft = (ctx->poisson_mode != OTM_POISSON_DENSE && fft_eligible(n)) ? 1 : 0;
   W->fft = base.fft;
-  int items;
   if (base.fft) {
     int lg = 0;
     while ((1 << lg) < n) ++lg;
     base.logn = lg;
     W->reg = dct_reg_supported(n) ? 1 : 0;
     const int per = W->reg ? dct_reg_lines_per_block(n) : fft_lines(n);
-    W->col_warps = W->reg ? dct_reg_col_warps(n, 1, ctx->num_sms) : 0;
+    W->col_warps = W->reg ? dct_reg_col_warps(n, maps, ctx->num_sms) : 0;
     const int cper = W->reg ? dct_reg_cols_per_block(n, W->col_warps) : fft_lines(n);
     base.nrow = n / per;
     base.ncol = n / cper;
-    W->rows = base.nrow;
-    W->cols = base.ncol;
-    items = std::max(W->rows, W->cols);
   } else {
     int t = (n + 63) / 64;
-    base.ngemm = W->G = items = t * t;
+    base.ngemm = t * t;
   }
-  std::vector<Inst> recs(m + 4, base);
-  for (int k = 0; k <= m; ++k) recs[k].r[0] = W->Vb + (size_t)k * W->ld;
-  recs[m + 1].r[0] = W->b;
-  recs[m + 2].r[0] = W->h;
-  recs[m + 3].r[0] = W->Vb;
-  for (auto& r : recs) r.dhat = W->z;
+  W->rows = base.nrow * maps;
+  W->cols = base.ncol * maps;
+  W->G = base.ngemm * maps;
+  std::vector<Inst> recs((size_t)3 * maps, base);
+  for (int y = 0; y < maps; ++y) {
+    const double* src[3] = {W->b, W->h, W->Vb};
+    for (int kind = 0; kind < 3; ++kind) {
+      Inst& r = recs[(size_t)kind * maps + y];
+      r.r[0] = const_cast<double*>(src[kind]) + y * W->stride;
+      r.dhat = W->z + y * W->stride;
+      r.t1 = W->t1 + y * W->stride;
+      r.t2 = W->t2 + y * W->stride;
+      r.row0 = y * base.nrow;
+      r.col0 = y * base.ncol;
+      r.gemm0 = y * base.ngemm;
+    }
+  }
   W->recs.reserve(sizeof(Inst) * recs.size());
-  W->lists.reserve(sizeof(int) * items);
-  std::vector<int> zeros(items, 0);
+  // work list: item -> map, for the rows, the columns and the product tiles
+  std::vector<int> items;
+  for (int per : {base.nrow, base.ncol, base.ngemm})
+    for (int y = 0; y < maps; ++y) items.insert(items.end(), per, y);
+  W->lists.reserve(sizeof(int) * items.size());
   OTM_CUDA(cudaMemcpyAsync(W->recs.p, recs.data(), sizeof(Inst) * recs.size(), cudaMemcpyHostToDevice, ctx->stream));
-  OTM_CUDA(cudaMemcpyAsync(W->lists.p, zeros.data(), sizeof(int) * items, cudaMemcpyHostToDevice, ctx->stream));
+  OTM_CUDA(cudaMemcpyAsync(W->lists.p, items.data(), sizeof(int) * items.size(), cudaMemcpyHostToDevice, ctx->stream));
   OTM_CUDA(cudaStreamSynchronize(ctx->stream));
-  slot.reset(W);
+  slot = std::move(own);
   return W;
 }
 
-// z = M^+ (source of record k)
-static void poisson_rec(otm_context* ctx, AdjointWs* W, int k) {
-  Inst* d = W->rec(k);
-  const int* L = W->lists.as<int>();
+// z = M^+ (source of the records of a kind), every map whose record is active
+static void poisson_rec(otm_context* ctx, AdjointWs* W, int kind) {
+  Inst* d = W->rec(kind);
+  const int *L = W->lists.as<int>(), *LC = L + W->rows, *LG = LC + W->cols;
   if (W->fft) {
     if (W->reg)
-      dct_reg_run(ctx, W->n, false, d, L, 0, W->rows, L, 0, W->cols, W->col_warps);
+      dct_reg_run(ctx, W->n, false, d, L, 0, W->rows, LC, 0, W->cols, W->col_warps);
     else
-      poisson_fft(ctx, d, L, 0, W->rows, L, 0, W->cols);
+      poisson_fft(ctx, d, L, 0, W->rows, LC, 0, W->cols);
   } else {
-    dense_poisson(ctx, d, L, W->G);
+    dense_poisson(ctx, d, LG, W->G);
   }
 }
 
-// One Arnoldi step j of the cycle (j read on the device): z = M^+ v_j and the four step
-// kernels, which do nothing once the cycle has ended.
+// One Arnoldi step j of every map's cycle (j read on the device): z = M^+ v_j and the four
+// step kernels, which do nothing for a map whose cycle has ended.
 static void arnoldi_step(otm_context* ctx, AdjointWs* W, int n, cudaGraphConditionalHandle handle, int in_graph) {
-  const long ld = (long)W->ld;
-  Inst* rec = W->rec(W->m + 3);
-  poisson_rec(ctx, W, W->m + 3);
-  launch(ctx, "adj_apply", k_adj_apply, W->nb, AT, n, (const double2*)W->g, (const double*)W->z, W->Vb, ld, W->ctl,
-         W->part, W->hcol, W->c);
-  launch(ctx, "adj_orth", k_adj_orth, W->nb, AT, n, W->Vb, ld, W->ctl, W->part, W->hcol, W->c);
-  launch(ctx, "adj_norm", k_adj_norm, W->nb, AT, n, W->Vb, ld, W->ctl, W->inv, W->part, (const double*)W->hcol,
-         (const double*)W->c, W->H, W->cs, W->sn, W->gv, rec, handle, in_graph);
-  launch(ctx, "adj_scale", k_adj_scale_by, (unsigned)((W->N + 255) / 256), 256, (long)W->N, W->Vb, ld,
-         (const double*)W->inv, (const AdjCtl*)W->ctl);
+  const long ld = (long)W->ld, sd = W->stride;
+  const dim3 grid(W->nb, W->maps);
+  Inst* rec = W->rec(2);
+  poisson_rec(ctx, W, 2);
+  launch(ctx, "adj_apply", k_adj_apply, grid, AT, n, (const double2*)W->g, (const double*)W->z, W->Vb, ld, W->ctl,
+         W->part, W->hcol, W->c, sd);
+  launch(ctx, "adj_orth", k_adj_orth, grid, AT, n, W->Vb, ld, W->ctl, W->part, W->hcol, W->c, sd);
+  launch(ctx, "adj_norm", k_adj_norm, grid, AT, n, W->Vb, ld, W->ctl, W->inv, W->part, (const double*)W->hcol,
+         (const double*)W->c, W->H, W->cs, W->sn, W->gv, rec, sd);
+  launch(ctx, "adj_scale", k_adj_scale_by, dim3((unsigned)((W->N + 255) / 256), W->maps), 256, (long)W->N, W->Vb, ld,
+         (const double*)W->inv, (const AdjCtl*)W->ctl, sd, handle, in_graph);
 }
 
-// Steps per body of the cycle's WHILE node: a body costs 2.8 us beside its kernels (measured
-// with empty ones), a step after the cycle's end 7 launches that return at once (about 7 us).
+// Steps per body of the cycles' WHILE node: a body costs 2.8 us beside its kernels (measured
+// with empty ones), a step after the last cycle's end 7 launches that return at once (about 7 us).
 constexpr int STEPS_PER_BODY = 4;
 
-// The cycle's steps as a graph: a WHILE node whose body is STEPS_PER_BODY Arnoldi steps, its
+// The cycles' steps as a graph: a WHILE node whose body is STEPS_PER_BODY Arnoldi steps, its
 // condition set by the last kernel of a step (at most m steps per launch).
 static void build_step_graph(otm_context* ctx, AdjointWs* W, int n) {
   cudaStream_t st = ctx->stream;
@@ -692,6 +852,158 @@ static void build_step_graph(otm_context* ctx, AdjointWs* W, int n) {
   cudaGraphDestroy(g);
 }
 
+// The adjoints of `count` (<= ADJ_MAPS) maps of size n side by side. One map's step is too
+// small to fill the GPU and bound by latency; run from a host thread and stream of its own each,
+// four took 83 us a step at 256^2 where one takes 51, and the time varied with the host. In
+// common launches four take 80 us, falling as maps finish (63 us a step over a call whose
+// longest map needs twice the steps of the others). Each map's arithmetic is that of a call
+// of its own.
+void adjoint_maps(otm_context* ctx, int n, int count, const double* const* density, const double* const* fwd_xy,
+                  const double* const* grad_fwd, const otm_adjoint_options& o, double* const* grad_density,
+                  otm_adjoint_stats* stats) {
+  cudaStream_t st = ctx->stream;
+  const int m = o.mode == OTM_ADJOINT_KRYLOV ? std::max(1, std::min(o.restart, ADJ_MAX_M)) : 1;
+  AdjointWs* W = adjoint_ws(ctx, n, m, count);
+  launch(ctx, "adj_reset", k_adj_reset_recs, 1, 32, W->rec(0), 3 * count);
+  const size_t N = W->N, V = W->V;
+  const long sd = W->stride;
+  const unsigned RB = 256;
+  const dim3 gN((unsigned)((N + RB - 1) / RB), count), gV((unsigned)((V + RB - 1) / RB), count), gT(W->nb, count);
+  // inputs: used in place when they are device memory, else staged
+  AdjArgs args = {};
+  {
+    size_t words = 0;
+    for (int y = 0; y < count; ++y)
+      words += (is_device_ptr(fwd_xy[y]) ? 0 : 2 * V) + (is_device_ptr(grad_fwd[y]) ? 0 : 2 * V) +
+               (is_device_ptr(density[y]) ? 0 : N);
+    if (words) ctx->staging.reserve(sizeof(double) * words);
+    double* next = ctx->staging.as<double>();
+    auto stage = [&](const double* src, size_t w) -> const double* {
+      if (is_device_ptr(src)) return src;
+      double* d = next;
+      next += w;
+      copy_in(ctx, d, src, sizeof(double) * w);
+      return d;
+    };
+    for (int y = 0; y < count; ++y) {
+      args.fwd[y] = stage(fwd_xy[y], 2 * V);
+      args.q[y] = stage(grad_fwd[y], 2 * V);
+      args.rho[y] = stage(density[y], N);
+      args.out[y] = is_device_ptr(grad_density[y]) ? grad_density[y] : W->z + y * sd;
+    }
+  }
+  // b = G^T q
+  launch(ctx, "adj_cells", k_adj_cells, gN, RB, n, args, W->b, sd);
+  std::vector<int> solves(count, 0);
+  std::vector<double> rel(count, -1.0);
+  if (o.mode == OTM_ADJOINT_ONE_STEP) {
+    // lambda = -M^+ b: the solve writes z, lambda = -z
+    poisson_rec(ctx, W, 0);
+    std::fill(solves.begin(), solves.end(), 1);
+    launch(ctx, "adj_scale", k_adj_neg, gN, RB, (long)N, (const double*)W->z, W->lam, sd);
+  } else {
+    for (int y = 0; y < count; ++y) OTM_CUDA(cudaMemsetAsync(W->lam + y * sd, 0, sizeof(double) * N, st));
+    // Restarted GMRES(m) on J^T lambda = b, right-preconditioned: J^T M^+ y = b, lambda = M^+ y.
+    // The cycles' Arnoldi steps run on the device (classical Gram-Schmidt applied twice,
+    // Givens rotations and the loop test) as one graph launch with a WHILE node -- or, in
+    // the host-driven loop mode and under the profiler, the same kernels one step at a
+    // time; the host reads the cycles' step counts and the true residuals' norms once per
+    // restart and decides which maps go on.
+    launch(ctx, "adj_disp", k_adj_disp, gV, RB, n, args, W->g, sd);
+    const bool graph = ctx->loop_mode == OTM_LOOP_GRAPH && !ctx->prof.on;
+    AdjCtl hc[ADJ_MAPS];
+    auto read = [&] {
+      OTM_CUDA(cudaMemcpyAsync(hc, W->ctl, sizeof(AdjCtl) * count, cudaMemcpyDeviceToHost, st));
+      OTM_CUDA(cudaStreamSynchronize(st));
+    };
+    auto residual = [&](const double* lambda) {
+      launch(ctx, "adj_resid", k_adj_resid, gT, AT, n, (const double2*)W->g, lambda, (const double*)W->b, W->Vb, W->ctl,
+             W->part, sd);
+      read();
+    };
+    residual(nullptr);
+    AdjCycle cyc = {};
+    std::vector<char> done(count, 0);
+    for (int y = 0; y < count; ++y) {
+      cyc.bnorm[y] = hc[y].rnorm;
+      if (!(cyc.bnorm[y] > 0)) {
+        rel[y] = 0.0;
+        done[y] = 1;
+      }
+    }
+    while (true) {
+      bool any = false;
+      for (int y = 0; y < count; ++y) {
+        if (!done[y]) {
+          rel[y] = hc[y].rnorm / cyc.bnorm[y];
+          if (!(rel[y] > o.tol) || solves[y] >= o.max_iter) done[y] = 1;
+        }
+        cyc.live[y] = !done[y];
+        cyc.budget[y] = o.max_iter - solves[y];
+        any |= !done[y];
+      }
+      if (!any) break;
+      launch(ctx, "adj_cycle", k_adj_cycle_init, gN, RB, (long)N, W->ctl, W->gv, m, cyc, o.tol, W->rec(2), W->rec(1),
+             W->Vb, sd);
+      if (graph) {
+        if (!W->step_graph) build_step_graph(ctx, W, n);
+        OTM_CUDA(cudaGraphLaunch(W->step_graph, st));
+      } else {
+        bool go = true;
+        while (go) {
+          arnoldi_step(ctx, W, n, (cudaGraphConditionalHandle)0, 0);
+          read();
+          ctx->prof.flush();
+          go = false;
+          for (int y = 0; y < count; ++y) go |= hc[y].go != 0;
+        }
+      }
+      // lambda += M^+ (V y), H y = g solved on the device
+      launch(ctx, "adj_trisolve", k_adj_trisolve, dim3(1, count), 256, (const AdjCtl*)W->ctl, (const double*)W->H,
+             (const double*)W->gv, W->c, sd);
+      launch(ctx, "adj_span", k_adj_span, gN, RB, (long)N, W->h, (const double*)W->Vb, (long)W->ld,
+             (const double*)W->c, (const AdjCtl*)W->ctl, sd);
+      poisson_rec(ctx, W, 1);  // z = M^+ h
+      launch(ctx, "adj_add", k_adj_add, gN, RB, (long)N, (const double*)W->z, W->lam, (const AdjCtl*)W->ctl, sd);
+      residual(W->lam);
+      int longest = 0;
+      bool fault = false;
+      for (int y = 0; y < count; ++y) {
+        if (!cyc.live[y]) continue;
+        longest = std::max(longest, hc[y].j);
+        solves[y] += hc[y].j + 1;
+        if (hc[y].j == 0) done[y] = 1;  // no step was possible: nothing changes by restarting
+        fault |= hc[y].fault != 0;
+      }
+      if (graph) ctx->launches += W->step_kernels * (long)((longest + STEPS_PER_BODY - 1) / STEPS_PER_BODY);
+      if (fault) break;  // reported below
+    }
+  }
+  // chain through the density normalisation, reduced and applied on the device
+  launch(ctx, "adj_rho_sums", k_adj_rho_sums, dim3(RHO_BLOCKS, count), 32, (long)N, (const double*)W->lam, args, W->ctl,
+         W->part, W->sums, sd);
+  launch(ctx, "adj_finish", k_adj_finish, gN, RB, (long)N, (const double*)W->lam, (const double*)W->sums, args, sd);
+  OTM_CUDA(cudaGetLastError());
+  for (int y = 0; y < count; ++y)
+    if (args.out[y] != grad_density[y]) copy_out(ctx, grad_density[y], args.out[y], sizeof(double) * N);
+  // a bounded wait inside a transform that gave up flags its record
+  std::vector<Inst> recs_h((size_t)3 * count);
+  OTM_CUDA(cudaMemcpyAsync(recs_h.data(), W->rec(0), sizeof(Inst) * recs_h.size(), cudaMemcpyDeviceToHost, st));
+  OTM_CUDA(cudaStreamSynchronize(st));
+  ctx->prof.flush();
+  for (const Inst& r : recs_h)
+    if (r.fault) throw DeviceTimeout{"otm_adjoint: a bounded device-side wait gave up"};
+  if (stats)
+    for (int y = 0; y < count; ++y) {
+      stats[y].iterations = solves[y];
+      stats[y].relative_residual = rel[y];
+    }
+}
+
+void check_adjoint_options(const otm_adjoint_options& o) {
+  if (o.mode != OTM_ADJOINT_ONE_STEP && o.mode != OTM_ADJOINT_KRYLOV) throw BadArg{"otm_adjoint: unknown mode"};
+}
+
 }  // namespace otm
 
 extern "C" void otm_default_adjoint_options(otm_adjoint_options* o) {
@@ -711,112 +1023,10 @@ extern "C" int otm_adjoint(otm_context* ctx, int n, const double* density, const
     otm_adjoint_options o;
     otm_default_adjoint_options(&o);
     if (opt) o = *opt;
-    if (o.mode != OTM_ADJOINT_ONE_STEP && o.mode != OTM_ADJOINT_KRYLOV) throw BadArg{"otm_adjoint: unknown mode"};
+    check_adjoint_options(o);
     make_current(ctx);
     if (otm_init(ctx, n) != OTM_OK) throw BadArg{std::string("otm_adjoint: ") + otm_last_error()};
-    cudaStream_t st = ctx->stream;
-    const int m = o.mode == OTM_ADJOINT_KRYLOV ? std::max(1, std::min(o.restart, ADJ_MAX_M)) : 1;
-    AdjointWs* W = adjoint_ws(ctx, n, m);
-    launch(ctx, "adj_reset", k_adj_reset_recs, 1, 256, W->rec(0), W->m + 4);
-    const size_t N = W->N, V = W->V;
-    const int RB = 256;
-    // inputs: used in place when they are device memory, else staged into the workspace
-    auto stage = [&](const double* src, double* tmp, size_t words) -> const double* {
-      if (is_device_ptr(src)) return src;
-      copy_in(ctx, tmp, src, sizeof(double) * words);
-      return tmp;
-    };
-    if (!is_device_ptr(fwd_xy) || !is_device_ptr(grad_fwd) || !is_device_ptr(density)) {
-      ctx->staging.reserve(sizeof(double) * (4 * V + N));
-    }
-    double* stg = ctx->staging.as<double>();
-    const double* d_fwd = stage(fwd_xy, stg, 2 * V);
-    const double* d_q = stage(grad_fwd, stg + 2 * V, 2 * V);
-    const double* d_rho = stage(density, stg + 4 * V, N);
-    const unsigned gN = (unsigned)((N + RB - 1) / RB), gV = (unsigned)((V + RB - 1) / RB);
-    double* d_b = W->b;
-    double* d_lam = W->lam;
-    double* d_z = W->z;
-    double* d_h = W->h;
-    // b = G^T q
-    launch(ctx, "adj_cells", k_adj_cells, gN, RB, n, d_q, d_b);
-    int solves = 0;
-    double rel = -1.0;
-    if (o.mode == OTM_ADJOINT_ONE_STEP) {
-      // lambda = -M^+ b: the solve writes z, lambda = -z
-      poisson_rec(ctx, W, W->m + 1);
-      ++solves;
-      launch(ctx, "adj_scale", k_adj_neg, gN, RB, (long)N, (const double*)d_z, d_lam);
-    } else {
-      OTM_CUDA(cudaMemsetAsync(d_lam, 0, sizeof(double) * N, st));
-      // Restarted GMRES(m) on J^T lambda = b, right-preconditioned: J^T M^+ y = b, lambda = M^+ y.
-      // A cycle's Arnoldi steps run on the device (classical Gram-Schmidt applied twice,
-      // Givens rotations and the loop test) as one graph launch with a WHILE node -- or, in
-      // the host-driven loop mode and under the profiler, the same kernels one step at a
-      // time; the host reads the cycle's step count and the true residual's norm once per
-      // restart and decides whether to restart.
-      launch(ctx, "adj_disp", k_adj_disp, gV, RB, n, d_fwd, W->g);
-      const bool graph = ctx->loop_mode == OTM_LOOP_GRAPH && !ctx->prof.on;
-      AdjCtl hc;
-      auto residual = [&](const double* lambda) {
-        launch(ctx, "adj_resid", k_adj_resid, W->nb, AT, n, (const double2*)W->g, lambda, (const double*)d_b, W->Vb,
-               W->ctl, W->part);
-        OTM_CUDA(cudaMemcpyAsync(&hc, W->ctl, sizeof(hc), cudaMemcpyDeviceToHost, st));
-        OTM_CUDA(cudaStreamSynchronize(st));
-      };
-      residual(nullptr);
-      const double bnorm = hc.rnorm;
-      rel = bnorm > 0 ? 1.0 : 0.0;
-      while (bnorm > 0) {
-        rel = hc.rnorm / bnorm;
-        if (!(rel > o.tol) || solves >= o.max_iter) break;
-        launch(ctx, "adj_cycle", k_adj_cycle_init, std::max(gN, 1u), RB, (long)N, W->ctl, W->gv, m, bnorm, o.tol,
-               o.max_iter - solves, W->rec(W->m + 3), W->Vb);
-        if (graph) {
-          if (!W->step_graph) build_step_graph(ctx, W, n);
-          OTM_CUDA(cudaGraphLaunch(W->step_graph, st));
-        } else {
-          do {
-            arnoldi_step(ctx, W, n, (cudaGraphConditionalHandle)0, 0);
-            OTM_CUDA(cudaMemcpyAsync(&hc, W->ctl, sizeof(hc), cudaMemcpyDeviceToHost, st));
-            OTM_CUDA(cudaStreamSynchronize(st));
-            ctx->prof.flush();
-          } while (hc.go);
-        }
-        // lambda += M^+ (V y), H y = g solved on the device
-        launch(ctx, "adj_trisolve", k_adj_trisolve, 1, 256, (const AdjCtl*)W->ctl, (const double*)W->H,
-               (const double*)W->gv, W->c);
-        launch(ctx, "adj_span", k_adj_span, gN, RB, (long)N, d_h, (const double*)W->Vb, (long)W->ld,
-               (const double*)W->c, (const AdjCtl*)W->ctl);
-        poisson_rec(ctx, W, W->m + 2);  // z = M^+ h
-        launch(ctx, "adj_add", k_adj_add, gN, RB, (long)N, (const double*)d_z, d_lam);
-        residual(d_lam);
-        if (graph)
-          ctx->launches += W->step_kernels * (long)((hc.j + STEPS_PER_BODY - 1) / STEPS_PER_BODY);
-        solves += hc.j + 1;
-        if (hc.fault) break;   // reported below
-        if (hc.j == 0) break;  // no step was possible: nothing changes by restarting
-      }
-    }
-    // chain through the density normalisation, reduced and applied on the device
-    launch(ctx, "adj_rho_sums", k_adj_rho_sums, RHO_BLOCKS, 32, (long)N, (const double*)d_lam, d_rho, W->ctl,
-           W->part, W->sums);
-    bool odev = is_device_ptr(grad_density);
-    double* out = odev ? grad_density : d_z;
-    launch(ctx, "adj_finish", k_adj_finish, gN, RB, (long)N, (const double*)d_lam, (const double*)W->sums, out);
-    OTM_CUDA(cudaGetLastError());
-    if (!odev) copy_out(ctx, grad_density, out, sizeof(double) * N);
-    // a bounded wait inside a transform that gave up flags its record
-    std::vector<Inst> recs_h((size_t)W->m + 4);
-    OTM_CUDA(cudaMemcpyAsync(recs_h.data(), W->rec(0), sizeof(Inst) * recs_h.size(), cudaMemcpyDeviceToHost, st));
-    OTM_CUDA(cudaStreamSynchronize(st));
-    ctx->prof.flush();
-    for (const Inst& r : recs_h)
-      if (r.fault) throw DeviceTimeout{"otm_adjoint: a bounded device-side wait gave up"};
-    if (stats) {
-      stats->iterations = solves;
-      stats->relative_residual = rel;
-    }
+    adjoint_maps(ctx, n, 1, &density, &fwd_xy, &grad_fwd, o, &grad_density, stats);
     return (int)OTM_OK;
   });
 }

@@ -186,14 +186,11 @@ struct otm_context {
     }
   };
   std::map<int, std::unique_ptr<GraphExec>> bvh_graphs;
-  // adjoint workspaces per grid size (adjoint.cu); type-erased to keep this header small
+  // adjoint workspaces per grid size and number of maps (adjoint.cu); type-erased to keep this header small
   struct Erased {
     virtual ~Erased() = default;
   };
   std::map<int, std::unique_ptr<Erased>> adjoint;
-  // contexts of the same device on which otm_barycenter_loss runs the adjoints of its maps
-  // concurrently, one host thread each (created on first use, destroyed by otm_destroy)
-  std::vector<otm_context*> helpers;
 };
 
 struct otm_map {
@@ -247,6 +244,13 @@ void raster_grid_backward(otm_context* ctx, int n, const double* xy, int rows, i
 // overwritten) from dL/dI (V x 2). Deterministic: per-face point lists in index order.
 void inverse_grid_backward(otm_context* ctx, int n, const double* fwd, const int* hit0, const double* dL_dI,
                            double* dL_dfwd);
+
+// Adjoints of `count` (<= 8) maps of size n (initialised) in common launches; otm_adjoint's
+// arguments per map (adjoint.cu). The options have been checked.
+void adjoint_maps(otm_context* ctx, int n, int count, const double* const* density, const double* const* fwd_xy,
+                  const double* const* grad_fwd, const otm_adjoint_options& o, double* const* grad_density,
+                  otm_adjoint_stats* stats);
+void check_adjoint_options(const otm_adjoint_options& o);
 
 // Launches `kernel` on the context stream, counting it and (when profiling) bracketing
 // it with CUDA events.

@@ -6,15 +6,11 @@
 #include <algorithm>
 #include <cstring>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "context.h"
 
 namespace otm {
-
-void dct_reg_attrs(int device);      // dct_reg.cu
-void poisson_fft_attrs(int device);  // poisson.cu
 
 // out = sum_k w_k mesh_k, left to right (bilerp / lerp of apps/barycenters.cpp:127-139).
 __global__ void k_blend(long V2, int count, const double* const* meshes, const double* w, double* out) {
@@ -523,52 +519,12 @@ extern "C" int otm_barycenter_loss(otm_context* ctx, int n, int count, const dou
         launch(ctx, "scale", k_scale, gv2, 256, (long)V2, weights[k], (const double*)dB, dI);
         inverse_grid_backward(ctx, n, fwd[k], hit0[k], dI, dF[k]);
       }
-      // the maps' adjoints are independent: each runs on its own context (this one for map
-      // 0, cached helpers of the same device for the others) from its own host thread, so
-      // their kernels -- a 512^2 Poisson solve fills a fraction of the GPU -- overlap
-      OTM_CUDA(cudaStreamSynchronize(st));
-      dct_reg_attrs(ctx->device);  // device-wide set-up done once, before the threads
-      poisson_fft_attrs(ctx->device);
-      while ((int)ctx->helpers.size() < count - 1) {
-        otm_context* h = nullptr;
-        const int hrc = otm_create(ctx->device, &h);
-        if (hrc != OTM_OK) return hrc;
-        ctx->helpers.push_back(h);
-      }
-      std::vector<int> rcs(count, OTM_OK);
+      // the maps' adjoints are independent and of one size: they run side by side
+      check_adjoint_options(ao);
       std::vector<otm_adjoint_stats> asts(count);
-      std::vector<std::string> errs(count);
-      std::vector<long> launches0(count, 0);
-      auto run = [&](int k) {
-        otm_context* c = k == 0 ? ctx : ctx->helpers[k - 1];
-        if (k > 0) {
-          c->poisson_mode = ctx->poisson_mode;
-          c->loop_mode = ctx->loop_mode;
-          c->wait_test = ctx->wait_test;
-          launches0[k] = c->launches;
-        }
-        rcs[k] = otm_adjoint(c, n, rho[k], fwd[k], dF[k], &ao, grad[k], &asts[k]);
-        if (rcs[k] != OTM_OK) errs[k] = otm_last_error();
-      };
-      {
-        std::vector<std::thread> threads;
-        try {
-          for (int k = 1; k < count; ++k) threads.emplace_back(run, k);
-        } catch (...) {  // a thread could not start: join those that did, then report
-          for (auto& t : threads) t.join();
-          throw;
-        }
-        run(0);
-        for (auto& t : threads) t.join();
-      }
-      make_current(ctx);
-      for (int k = 0; k < count; ++k)
-        if (rcs[k] != OTM_OK) {
-          set_error(errs[k]);
-          return rcs[k];
-        }
+      std::vector<const double*> cfwd(fwd.begin(), fwd.end()), cq(dF.begin(), dF.end());
+      adjoint_maps(ctx, n, count, rin.data(), cfwd.data(), cq.data(), ao, grad.data(), asts.data());
       for (int k = 0; k < count; ++k) {
-        if (k > 0) ctx->launches += ctx->helpers[k - 1]->launches - launches0[k];
         solves[k] = asts[k].iterations;
         ares[k] = asts[k].relative_residual;
         // expected = ... + w_k mean(density_k): d/ddensity_k = w_k / N per cell
