@@ -351,8 +351,8 @@ int otm_barycenter_loss(otm_context* ctx, int n, int count, const double* const*
 
 /* Context options (no counterpart in the reference).
  *   OTM_OPT_POISSON: how d_hat = M^+ r is computed.
- *     OTM_POISSON_AUTO  (default) fast cosine transform for power-of-two n in [8, 4096],
- *                       dense products otherwise
+ *     OTM_POISSON_AUTO  (default) fast cosine transform for n in [8, 4096], dense products
+ *                       otherwise
  *     OTM_POISSON_DENSE C.X.C^T products with the cosine basis, any n
  *     OTM_POISSON_FFT   fast transform where possible (same as AUTO)
  *     OTM_POISSON_TENSOR split-precision instances of n in {128, 256, 512, 1024}: the

@@ -736,15 +736,12 @@ static AdjointWs* adjoint_ws(otm_context* ctx, int n, int m, int maps) {
   base.fft = (ctx->poisson_mode != OTM_POISSON_DENSE && fft_eligible(n)) ? 1 : 0;
   W->fft = base.fft;
   if (base.fft) {
-    int lg = 0;
-    while ((1 << lg) < n) ++lg;
-    base.logn = lg;
     W->reg = dct_reg_supported(n) ? 1 : 0;
-    const int per = W->reg ? dct_reg_lines_per_block(n) : fft_lines(n);
+    const int per = W->reg ? dct_reg_lines_per_block(n) : fft_lines(n, false);
     W->col_warps = W->reg ? dct_reg_col_warps(n, maps, ctx->num_sms) : 0;
-    const int cper = W->reg ? dct_reg_cols_per_block(n, W->col_warps) : fft_lines(n);
-    base.nrow = n / per;
-    base.ncol = n / cper;
+    const int cper = W->reg ? dct_reg_cols_per_block(n, W->col_warps) : fft_lines(n, true);
+    base.nrow = (n + per - 1) / per;
+    base.ncol = (n + cper - 1) / cper;
   } else {
     int t = (n + 63) / 64;
     base.ngemm = t * t;
@@ -787,7 +784,7 @@ static void poisson_rec(otm_context* ctx, AdjointWs* W, int kind) {
     if (W->reg)
       dct_reg_run(ctx, W->n, false, d, L, 0, W->rows, LC, 0, W->cols, W->col_warps);
     else
-      poisson_fft(ctx, d, L, 0, W->rows, LC, 0, W->cols);
+      poisson_fft(ctx, W->n, d, L, 0, W->rows, LC, 0, W->cols);
   } else {
     dense_poisson(ctx, d, LG, W->G);
   }

@@ -30,9 +30,10 @@ struct Inst {
   double* t2;
   const double* C;
   const double* cosk;
-  const double2* tw;  // exp(-2 pi i k / n), k < n/2 (fast transform); then the step-2 table
+  const double2* tw;  // fast transform's tables: register sizes exp(-2 pi i k / n), k < n/2, then the
+                      // step-2 twiddles; other sizes fft_tables (poisson.cu)
   const double2* pt;  // (cos, sin)(pi k / (2n)), k < n (fast transform)
-  int fft, logn;      // fast transform used (n a power of two) / log2 n
+  int fft;            // fast transform used
   int split;          // split precision: r, d_hat, d, t1 hold FP32 values (psi, rho FP64)
   int tc0, ntc;       // tensor-core transform (dct_tc.cu): first item and item count of its work list
   int tcn;            // its output tile width (256, or 128 for n = 128)
@@ -129,10 +130,14 @@ __device__ __forceinline__ void pick_step(const double z[5], double* alpha, doub
 }
 
 
-// Host launcher of the fast cosine-transform Poisson solve (poisson.cu): d_hat = M^+ r_k
-// for every active instance with fft != 0.
-void poisson_fft(otm_context* ctx, Inst* d_insts, const int* row_inst, int roff, int nrow_items,
+// Fast cosine-transform Poisson solve for the sizes without a register transform (poisson.cu):
+// d_hat = M^+ r_k for the active instances, all of size n, of the row and column work lists.
+void poisson_fft(otm_context* ctx, int n, Inst* d_insts, const int* row_inst, int roff, int nrow_items,
                  const int* col_inst, int coff, int ncol_items);
+int fft_lines(int n, bool cols);  // rows or columns per work item
+void fft_tables(int n, std::vector<double2>& out);  // the contents of Inst::tw
+// Sizes with a fast transform; below 8 the dense products are as fast.
+inline bool fft_eligible(int n) { return n >= 8 && n <= 4096; }
 // Register-resident variant for n in {64, ..., 1024} (dct_reg.cu).
 bool dct_reg_supported(int n);
 // The register transforms' step-2 twiddles W_n^(t k1) in [register][lane] order (n entries),
@@ -175,10 +180,5 @@ void sweep_sums(otm_context* ctx, Inst* d_insts, const int* strip_inst, int base
 void sweep_update(otm_context* ctx, Inst* d_insts, const int* strip_inst, int base, int nblocks, bool split,
                   double* partials);
 constexpr int SWEEP_SLOTS = 32;  // partial-sum slots per sweep block
-
-// Elements staged in shared memory per block of the transform kernels.
-constexpr int FFT_ELEMS = 4096;
-inline int fft_lines(int n) { return n < FFT_ELEMS / n ? n : FFT_ELEMS / n; }
-inline bool fft_eligible(int n) { return n >= 8 && n <= FFT_ELEMS && (n & (n - 1)) == 0; }
 
 }  // namespace otm

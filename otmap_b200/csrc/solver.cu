@@ -8,9 +8,9 @@
 //
 // Per iteration (otsolver_2dgrid.cpp:160-220), for every active instance:
 //   d_hat = M^+ r_k    the cosine-transform Poisson solve (:175-179): register FFT
-//                      transforms (dct_reg.cu) for power-of-two n in 64..1024, shared-
-//                      memory FFTs (poisson.cu) for other powers of two, dense products
-//                      with the cosine basis (k_dct_gemm here) for any other n
+//                      transforms (dct_reg.cu) for power-of-two n in 64..1024, block FFTs
+//                      (poisson.cu) for any other n in 8..4096, dense products with the
+//                      cosine basis (k_dct_gemm here) beyond
 //   k_sweep_sums       |d_hat| (early exit, :182), beta (:248-261) and the quartic of the
 //                      line search; its last block solves the cubic (:541-595)
 //   k_sweep_update     d = d_hat + beta d_prev, psi += alpha d, r += alpha b + alpha^2 a
@@ -632,11 +632,7 @@ static std::vector<Inst> layout_workspace(otm_context* ctx, const std::vector<in
       I.ntc = dct_tc_tiles(n);
       I.tcn = dct_tc_tn(n);
       tcitems += I.ntc;
-    } else if (I.fft) {
-      int lg = 0;
-      while ((1 << lg) < n) ++lg;
-      I.logn = lg;
-    } else {
+    } else if (!I.fft) {
       I.gemm0 = gemm;
       I.ngemm = gemm_tiles_of(n);
       gemm += I.ngemm;
@@ -656,16 +652,16 @@ static std::vector<Inst> layout_workspace(otm_context* ctx, const std::vector<in
     for (size_t k = 0; k < order.size(); ++k) {
       Inst& I = h[order[k]];
       const int reg = dct_reg_supported(I.n) ? 1 : 0;
-      const int per = reg ? dct_reg_lines_per_block(I.n) : fft_lines(I.n);
+      const int per = reg ? dct_reg_lines_per_block(I.n) : fft_lines(I.n, false);
       if (segs.empty() || segs.back().n != I.n || segs.back().reg != reg) {
         const int same_size = (int)std::count_if(order.begin(), order.end(), [&](int q) { return h[q].n == I.n; });
         segs.push_back({I.n, reg, I.split, rows, 0, cols, 0, reg ? dct_reg_col_warps(I.n, same_size, ctx->num_sms) : 0});
       }
-      const int cper = reg ? dct_reg_cols_per_block(I.n, segs.back().col_warps) : fft_lines(I.n);
+      const int cper = reg ? dct_reg_cols_per_block(I.n, segs.back().col_warps) : fft_lines(I.n, true);
       I.row0 = rows;
-      I.nrow = I.n / per;
+      I.nrow = (I.n + per - 1) / per;
       I.col0 = cols;
-      I.ncol = I.n / cper;
+      I.ncol = (I.n + cper - 1) / cper;
       rows += I.nrow;
       cols += I.ncol;
       segs.back().rcnt += I.nrow;
@@ -836,7 +832,7 @@ static void launch_iteration(otm_context* ctx, Inst* d_insts) {
       dct_reg_run(ctx, sg.n, sg.split != 0, d_insts, ws.row_inst.as<int>(), sg.roff, sg.rcnt, ws.col_inst.as<int>(), sg.coff,
                   sg.ccnt, sg.col_warps);
     else
-      poisson_fft(ctx, d_insts, ws.row_inst.as<int>(), sg.roff, sg.rcnt, ws.col_inst.as<int>(), sg.coff, sg.ccnt);
+      poisson_fft(ctx, sg.n, d_insts, ws.row_inst.as<int>(), sg.roff, sg.rcnt, ws.col_inst.as<int>(), sg.coff, sg.ccnt);
   }
   if (ws.total_tc > 0) dct_tc_run(ctx, d_insts, ws.tc_inst.as<int>(), 0, ws.total_tc);
   const int* si = ws.strip_inst.as<int>();
@@ -1061,12 +1057,17 @@ static SizeTables* init_size(otm_context* ctx, int n) {
   T->cosk.reserve(sizeof(double) * n);
   cudaStream_t st = ctx->stream;
   if (fft_eligible(n)) {
-    std::vector<double2> tw(n / 2), pt(n);
-    for (int k = 0; k < n / 2; ++k) tw[k] = make_double2(std::cos(2.0 * M_PI * k / n), -std::sin(2.0 * M_PI * k / n));
+    std::vector<double2> tw, pt(n);
     for (int k = 0; k < n; ++k) pt[k] = make_double2(std::cos(M_PI * k / (2.0 * n)), std::sin(M_PI * k / (2.0 * n)));
-    std::vector<double2> tw2;
-    dct_reg_step2_table(n, tw, tw2);
-    tw.insert(tw.end(), tw2.begin(), tw2.end());
+    if (dct_reg_supported(n)) {
+      tw.resize(n / 2);
+      for (int k = 0; k < n / 2; ++k) tw[k] = make_double2(std::cos(2.0 * M_PI * k / n), -std::sin(2.0 * M_PI * k / n));
+      std::vector<double2> tw2;
+      dct_reg_step2_table(n, tw, tw2);
+      tw.insert(tw.end(), tw2.begin(), tw2.end());
+    } else {
+      fft_tables(n, tw);
+    }
     T->tw.reserve(sizeof(double2) * tw.size());
     T->pt.reserve(sizeof(double2) * n);
     OTM_CUDA(cudaMemcpyAsync(T->tw.p, tw.data(), sizeof(double2) * tw.size(), cudaMemcpyHostToDevice, st));

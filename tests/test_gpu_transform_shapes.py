@@ -31,3 +31,30 @@ def test_step_does_not_depend_on_block_shape(n, counts, precision):
             assert m.stats.iterations == 1
             assert np.abs(m.fwd_mesh() - ref[k % 2].fwd_mesh()).max() <= 1e-13
     ctx.close()
+
+
+# Sizes around the steps of the block transforms: the powers of two without a register
+# transform, the first and last n of each chirp length M (2n - 1 <= M), odd and even, primes and
+# composites. One iteration with the fast transform takes the dense products' step: both are
+# accurate to about 1e-14 of the potential, whose n/2-scaled differences (potential below 1e-2,
+# n <= 2049) are the displacements.
+@pytest.mark.parametrize("n", [8, 9, 16, 17, 31, 32, 33, 63, 65, 127, 129, 255, 257, 300, 499, 513, 1000, 1025, 2049])
+def test_fast_transform_takes_the_dense_step(n):
+    from otmap_b200 import native as N
+    from otmap_b200 import otmap as ot
+    from otmap_b200 import workloads as W
+
+    dens = W.to_cells(W.gaussian_mixture(n, n))
+    opt = ot.SolverOptions(max_iter=1)
+    out = []
+    for mode in (N.POISSON_AUTO, N.POISSON_DENSE):
+        ctx = N.Context(0)
+        ctx.set_poisson(mode)
+        out.append(ot.solve_batch([dens], opt, context=ctx)[0].fwd_mesh())
+        if mode == N.POISSON_AUTO:  # the same instance beside others of other sizes
+            more = ot.solve_batch([W.to_cells(W.gaussian_mixture(m, m)) for m in (40, 64, 100)] + [dens, dens], opt,
+                                  context=ctx)
+            assert np.abs(more[3].fwd_mesh() - out[0]).max() <= 1e-13
+            assert np.array_equal(more[3].fwd_mesh(), more[4].fwd_mesh())
+        ctx.close()
+    assert np.abs(out[0] - out[1]).max() <= 1e-11
