@@ -51,8 +51,15 @@ __device__ __forceinline__ bool inside_quad(double qx, double qy, const Quad& p)
          inside_tri(qx, qy, p.x[0], p.y[0], p.x[2], p.y[2], p.x[3], p.y[3]);
 }
 
-// bilinear_coordinates_in_quad, weights form (mesh_utils.cpp:18-59, 76-88).
-__device__ bool bilinear_weights(double qx, double qy, const Quad& p, double w[4]) {
+// bilinear_coordinates_in_quad, weights form (mesh_utils.cpp:18-59, 76-88), in two parts: the
+// terms of the two solution pairs (u, v) = (2 A3 / E3, 2 A0 / E0) and their conjugates
+// (false: no real solution), and the weights from them.
+struct Bilinear {
+  double A0, A3, E0, E3, E0p, E3p;
+};
+constexpr double kBilinearZero = 4 * DBL_MIN;
+
+__device__ __forceinline__ bool bilinear_terms(double qx, double qy, const Quad& p, Bilinear& t) {
   double A0 = signed_area3(qx, qy, p.x[0], p.y[0], p.x[1], p.y[1]);
   double A1 = signed_area3(qx, qy, p.x[1], p.y[1], p.x[2], p.y[2]);
   double A2 = signed_area3(qx, qy, p.x[2], p.y[2], p.x[3], p.y[3]);
@@ -63,15 +70,47 @@ __device__ bool bilinear_weights(double qx, double qy, const Quad& p, double w[4
   double D = B0 * B0 + B1 * B1 + 2 * A0 * A2 + 2 * A1 * A3;
   if (D < 0) return false;
   double sD = sqrt(D);
-  double E0 = 2 * A0 - B0 - B1 + sD;
-  double E3 = 2 * A3 - B3 - B0 + sD;
-  const double zero = 4 * DBL_MIN;
-  double v = fabs(A0) <= zero ? 0 : 2 * A0 / E0;
-  double u = fabs(A3) <= zero ? 0 : 2 * A3 / E3;
-  double E0p = 2 * A0 - B0 - B1 - sD;
-  double E3p = 2 * A3 - B3 - B0 - sD;
-  double v_alt = fabs(A0) <= zero ? 0 : 2 * A0 / E0p;
-  double u_alt = fabs(A3) <= zero ? 0 : 2 * A3 / E3p;
+  t.A0 = A0;
+  t.A3 = A3;
+  t.E0 = 2 * A0 - B0 - B1 + sD;
+  t.E3 = 2 * A3 - B3 - B0 + sD;
+  t.E0p = 2 * A0 - B0 - B1 - sD;
+  t.E3p = 2 * A3 - B3 - B0 - sD;
+  return true;
+}
+
+// What weights_inside will say of a point, where it is certain without the four divisions and
+// the snapping of bilinear_from_terms (half of a pixel test's instructions): 1 accepted, -1
+// rejected, 0 to be computed. The snapping tolerance is 1.5e-8 and a division rounds by 1e-16,
+// so a ratio beyond [0, 1] by 1e-7 stays outside and one 1e-7 within stays inside. A pair with u
+// or v outside leaves one of the four weights negative by at least 1e-8, or NaN; the second
+// pair only counts when the first is outside. NaN in any term compares false: computed.
+struct Verdict {
+  bool in, out;
+};
+__device__ __forceinline__ Verdict ratio_verdict(double num, double den) {
+  const double a = fabs(num), b = fabs(den), low = b * 1e-7;
+  const bool same = (__double2hiint(num) ^ __double2hiint(den)) >= 0;
+  const bool above = a > low;
+  return {same & above & (a < b * (1. - 1e-7)), (a > b * (1. + 1e-7)) | (!same & above)};
+}
+__device__ __forceinline__ int bilinear_verdict(const Bilinear& t) {
+  // |A| within `zero` makes the ratio an exact 0: on the border, computed
+  const bool v0 = fabs(t.A0) > kBilinearZero, u0 = fabs(t.A3) > kBilinearZero;
+  const double nv = 2 * t.A0, nu = 2 * t.A3;
+  const Verdict v = ratio_verdict(nv, t.E0), u = ratio_verdict(nu, t.E3);
+  if (v0 & u0 & v.in & u.in) return 1;
+  const Verdict va = ratio_verdict(nv, t.E0p), ua = ratio_verdict(nu, t.E3p);
+  return ((v0 & v.out) | (u0 & u.out)) & ((v0 & va.out) | (u0 & ua.out)) ? -1 : 0;
+}
+
+__device__ __forceinline__ void bilinear_from_terms(const Bilinear& t, double w[4]) {
+  const double A0 = t.A0, A3 = t.A3;
+  const double zero = kBilinearZero;
+  double v = fabs(A0) <= zero ? 0 : 2 * A0 / t.E0;
+  double u = fabs(A3) <= zero ? 0 : 2 * A3 / t.E3;
+  double v_alt = fabs(A0) <= zero ? 0 : 2 * A0 / t.E0p;
+  double u_alt = fabs(A3) <= zero ? 0 : 2 * A3 / t.E3p;
   const double eps = 1.4901161193847656e-08;  // sqrt(DBL_EPSILON), exact
   if (fabs(u) < eps) u = 0;
   if (fabs(v) < eps) v = 0;
@@ -97,6 +136,12 @@ __device__ bool bilinear_weights(double qx, double qy, const Quad& p, double w[4
     else if (fabs(w[k] - 1.) <= weps)
       w[k] = 1;
   }
+}
+
+__device__ bool bilinear_weights(double qx, double qy, const Quad& p, double w[4]) {
+  Bilinear t;
+  if (!bilinear_terms(qx, qy, p, t)) return false;
+  bilinear_from_terms(t, w);
   return true;
 }
 
@@ -753,19 +798,12 @@ __device__ __forceinline__ void tri_weights(double qx, double qy, const Quad& p,
   w[3] = 0.0;
 }
 
-struct FaceRaster {
+struct FaceBox {
   int x0, x1, y0, y1;  // pixel box [x0,x1) x [y0,y1), as rasterize_face computes it
-  double value;        // PerFace value: float(1/N) * density / |area|
+  __device__ __forceinline__ bool empty() const { return x0 >= x1 || y0 >= y1; }
 };
 
-__device__ __forceinline__ FaceRaster face_raster(const MeshRef& m, const double* density, float scale, int rows,
-                                                  int cols, int f) {
-  Quad p;
-  int vid[4];
-  const int c = load_face(m, f, p, vid);
-  FaceRaster r;
-  double in_mass = scale * (density ? density[f] : 1.0);
-  r.value = in_mass / face_abs_area(p, c);
+__device__ __forceinline__ FaceBox face_box(const Quad& p, int rows, int cols) {
   double ulx = fmin(fmin(fmin(p.x[0], p.x[1]), p.x[2]), p.x[3]);
   double uly = fmin(fmin(fmin(p.y[0], p.y[1]), p.y[2]), p.y[3]);
   double lrx = fmax(fmax(fmax(p.x[0], p.x[1]), p.x[2]), p.x[3]);
@@ -779,17 +817,12 @@ __device__ __forceinline__ FaceRaster face_raster(const MeshRef& m, const double
     if (v < -2.0e9) return -2000000000;
     return (int)v;
   };
+  FaceBox r;
   r.x0 = max(trunc_int(fx0), 0);
   r.y0 = max(trunc_int(fy0), 0);
   r.x1 = min(trunc_int(fx1) + 1, cols);
   r.y1 = min(trunc_int(fy1) + 1, rows);
   return r;
-}
-
-__global__ void k_face_boxes(MeshRef m, const double* density, float scale, int rows, int cols, FaceRaster* fr) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= m.nf) return;
-  fr[f] = face_raster(m, density, scale, rows, cols, f);
 }
 
 // Weights the reference's sequential loop would test at (f, x, y) when its bilinear
@@ -799,12 +832,14 @@ __global__ void k_face_boxes(MeshRef m, const double* density, float scale, int 
 // the most recent pixel whose solve succeeds. Bounded; gives zeros (the start state)
 // when it runs out, as the sequential emulation does before any solve. Triangles
 // never touch that Vector4d and are passed over.
-__device__ void stale_weights(const MeshRef& m, int rows, int cols, const FaceRaster* fr, int f, int x, int y,
-                              double w[4]) {
+__device__ __noinline__ void stale_weights(const MeshRef& m, int rows, int cols, int f, int x, int y, double w[4]) {
   int steps = 0;
   const int limit = 1 << 22;
+  Quad p;
+  int vid[4];
+  load_face(m, f, p, vid);
+  FaceBox r = face_box(p, rows, cols);
   while (steps < limit) {
-    FaceRaster r = fr[f];
     // previous pixel in face f's scan
     if (x > r.x0) {
       --x;
@@ -815,21 +850,18 @@ __device__ void stale_weights(const MeshRef& m, int rows, int cols, const FaceRa
       // last pixel of the previous quad with a non-empty box
       int g = f - 1;
       while (g >= 0 && steps < limit) {
-        const bool empty = fr[g].x0 >= fr[g].x1 || fr[g].y0 >= fr[g].y1;
-        const bool tri = m.start && (m.start[g + 1] - m.start[g] == 3);
-        if (!empty && !tri) break;
+        const int c = load_face(m, g, p, vid);
+        r = face_box(p, rows, cols);
+        if (!r.empty() && c != 3) break;
         --g;
         ++steps;
       }
       if (g < 0 || steps >= limit) break;
       f = g;
-      x = fr[g].x1 - 1;
-      y = fr[g].y1 - 1;
+      x = r.x1 - 1;
+      y = r.y1 - 1;
     }
     ++steps;
-    Quad p;
-    int vid[4];
-    load_face(m, f, p, vid);
     double qx = ((double)x + 0.5) / (double)cols, qy = ((double)y + 0.5) / (double)rows;
     if (bilinear_weights(qx, qy, p, w)) return;
   }
@@ -839,63 +871,205 @@ __device__ void stale_weights(const MeshRef& m, int rows, int cols, const FaceRa
 // Weights of face f at the centre of pixel (x, y) as the reference's loop forms them
 // (triangles: the barycentric transform; quads: bilinear coordinates, or the stale
 // weights where that solve fails). Returns the face's valence; vid gets its corners.
-__device__ __forceinline__ int pixel_weights(const MeshRef& m, int rows, int cols, const FaceRaster* fr, int f,
-                                             int x, int y, double w[4], int vid[4]) {
+__device__ __forceinline__ int pixel_weights(const MeshRef& m, int rows, int cols, int f, int x, int y, double w[4],
+                                             int vid[4]) {
   Quad p;
   const int c = load_face(m, f, p, vid);
   const double qx = ((double)x + 0.5) / (double)cols, qy = ((double)y + 0.5) / (double)rows;
   if (c == 3) {
     tri_weights(qx, qy, p, w);
   } else if (!bilinear_weights(qx, qy, p, w)) {
-    stale_weights(m, rows, cols, fr, f, x, y, w);
+    stale_weights(m, rows, cols, f, x, y, w);
   }
   return c;
 }
 
-// Box rows per face (0 for an empty box): the work list of k_raster_owner_rows.
-__global__ void k_box_rows(int nf, const FaceRaster* fr, int* rows_of) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= nf) return;
-  const FaceRaster r = fr[f];
-  rows_of[f] = (r.x0 < r.x1 && r.y0 < r.y1) ? r.y1 - r.y0 : 0;
+// Centres of pixels, (k + 0.5) / count; for a power of two the product with the exact
+// reciprocal is the same number.
+struct PixelAxis {
+  double count, inv;
+  bool pow2;
+  __device__ __forceinline__ explicit PixelAxis(int n) : count((double)n), inv(1.0 / (double)n), pow2((n & (n - 1)) == 0) {}
+  __device__ __forceinline__ double operator()(int k) const {
+    const double t = (double)k + 0.5;
+    return pow2 ? t * inv : t / count;
+  }
+};
+
+// Pixel tests whose bilinear solve fails (D < 0), to be decided by stale weights: a walk of any
+// length, which k_raster_stale makes with a thread each instead of holding up a warp of the
+// owner pass. Tests beyond the list's room are decided on the spot.
+struct StaleList {
+  int* count;
+  uint2* test;  // face, y << 16 | x
+  int room;
+};
+
+// The owner test: face f (corners p, valence c) records its index at pixel (x, y) when it
+// accepts the centre (the weights of pixel_weights lie in [0, 1]).
+__device__ __forceinline__ void test_pixel(const MeshRef& m, int rows, int cols, int f, const Quad& p, int c, int x,
+                                           int y, double qx, double qy, int* owner, const StaleList& stale) {
+  double w[4];
+  if (c == 3) {
+    tri_weights(qx, qy, p, w);
+  } else {
+    Bilinear t;
+    if (bilinear_terms(qx, qy, p, t)) {
+      const int verdict = bilinear_verdict(t);
+      if (verdict > 0) atomicMax(&owner[(size_t)y * cols + x], f);
+      if (verdict != 0) return;
+      bilinear_from_terms(t, w);
+    } else {
+      const int i = atomicAdd(stale.count, 1) + 1;  // the counter starts at -1
+      if (i < stale.room) {
+        stale.test[i] = make_uint2((unsigned)f, (unsigned)y << 16 | (unsigned)x);
+        return;
+      }
+      stale_weights(m, rows, cols, f, x, y, w);
+    }
+  }
+  if (weights_inside(w)) atomicMax(&owner[(size_t)y * cols + x], f);
+}
+
+__global__ __launch_bounds__(128) void k_raster_stale(MeshRef m, int rows, int cols, int* owner, StaleList stale) {
+  const int total = min(*stale.count + 1, stale.room);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const uint2 e = stale.test[i];
+    const int f = (int)e.x, x = (int)(e.y & 0xffffu), y = (int)(e.y >> 16);
+    double w[4];
+    stale_weights(m, rows, cols, f, x, y, w);
+    if (weights_inside(w)) atomicMax(&owner[(size_t)y * cols + x], f);
+  }
 }
 
 // The owner pass: every pixel centre of a face's box that the face accepts records the
 // face index with atomicMax, so each pixel ends with the highest accepting index -- the
-// face the reference's sequential loop writes last (rasterizer.cpp:162-236). One thread
-// per (face, box row) rather than per face: a stretched face
-// (the inverse maps of sharp densities have some that span much of the image) spreads over
-// as many threads as its box has rows, instead of holding one thread for its whole box
-// while the rest of the grid idles. Work item t belongs to the last face f with
-// row_start[f] <= t (row_start: exclusive prefix of the box rows, total at [nf]); grid-
-// stride over the total, which is read on the device. Same atomicMax of the face index,
-// so the owners are those of the per-face pass.
-__global__ void k_raster_owner_rows(MeshRef m, int rows, int cols, const FaceRaster* fr, const int* row_start,
-                                    int* owner) {
-  const int nf = m.nf;
-  const int total = row_start[nf];
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    int lo = 0, hi = nf;  // row_start[lo] <= t < row_start[hi]
+// face the reference's sequential loop writes last (rasterizer.cpp:162-236). One thread per
+// face forms its box and value. The tests of the boxes of at most SMALL_BOX pixels (a mesh
+// drawn near its own resolution has nothing else) are pooled over the warp, 32 at a time,
+// whatever the boxes' sizes; larger boxes go on a list whose pixels are spread over warps
+// (k_raster_big), so that a stretched face -- the inverse maps of sharp densities have some
+// that span much of the image -- does not hold one thread. Bound by instruction issue: about
+// 90 FP64 and 150 other instructions for each of 4.6 tests per face. With one thread per
+// (face, box row) for every face, found by a binary search over 2^20 row counts, and the
+// divisions of bilinear_from_terms in every test, the pass took 148 us at 1024^2 beside 30
+// of boxes, counting and scanning; now 67 us in all (a raster call 222 -> 114 us; the owner
+// part of a 512^2 barycenter image 83 -> 38 us).
+constexpr int SMALL_BOX = 32, RF_T = 128;
+constexpr int BIG_CHUNK = 128;  // pixels of a listed face per warp
+
+__global__ __launch_bounds__(RF_T) void k_raster_faces(MeshRef m, const double* density, float scale, int rows,
+                                                       int cols, double* value, int* owner, int* big_count, int* big,
+                                                       int* big_chunks, StaleList stale) {
+  __shared__ Quad s_quad[RF_T];
+  __shared__ int2 s_corner[RF_T];                        // first pixel of the lane's box
+  __shared__ unsigned short s_item[RF_T * SMALL_BOX];    // per test: lane, dx, dy
+  const int f = blockIdx.x * RF_T + threadIdx.x, lane = threadIdx.x & 31;
+  const PixelAxis px(cols), py(rows);
+  FaceBox b = {0, 0, 0, 0};
+  int c = 4, tests = 0;
+  if (f < m.nf) {
+    Quad p;
+    int vid[4];
+    c = load_face(m, f, p, vid);
+    const double in_mass = scale * (density ? density[f] : 1.0);
+    value[f] = in_mass / face_abs_area(p, c);  // PerFace value: float(1/N) * density / |area|
+    b = face_box(p, rows, cols);
+    s_corner[threadIdx.x] = make_int2(b.x0, b.y0);
+    s_quad[threadIdx.x] = p;
+    if (!b.empty()) {
+      const int wx = b.x1 - b.x0, wy = b.y1 - b.y0;
+      if (wx > SMALL_BOX || wy > SMALL_BOX || wx * wy > SMALL_BOX) {
+        const int i = atomicAdd(big_count, 1) + 1;  // counters start at -1
+        big[i] = f;
+        big_chunks[i] = (int)(((long long)wx * wy + BIG_CHUNK - 1) / BIG_CHUNK);
+      } else {
+        tests = wx * wy;
+      }
+    }
+  }
+  int upto = tests;  // inclusive prefix over the warp
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, upto, o);
+    if (lane >= o) upto += u;
+  }
+  const int total = __shfl_sync(0xffffffffu, upto, 31), warp0 = threadIdx.x & ~31;
+  unsigned short* items = s_item + warp0 * SMALL_BOX;
+  for (int k = 0, dx = 0, dy = 0, at = upto - tests; k < tests; ++k) {
+    items[at + k] = (unsigned short)(lane | dx << 5 | dy << 10);
+    if (++dx == b.x1 - b.x0) {
+      dx = 0;
+      ++dy;
+    }
+  }
+  const unsigned triangles = __ballot_sync(0xffffffffu, c == 3);
+  __syncwarp();
+  for (int item = lane; item < total; item += 32) {
+    const int e = items[item], l = e & 31;
+    const int2 at = s_corner[warp0 + l];
+    const int x = at.x + (e >> 5 & 31), y = at.y + (e >> 10);
+    test_pixel(m, rows, cols, f - lane + l, s_quad[warp0 + l], triangles >> l & 1 ? 3 : 4, x, y, px(x), py(y), owner,
+               stale);
+  }
+}
+
+// Exclusive prefix of the listed faces' chunks, total at [count] (one block; nothing but the
+// total when the list is empty).
+__global__ __launch_bounds__(1024) void k_big_scan(const int* big_count, const int* big_chunks, long long* start) {
+  __shared__ int warp_total[32];
+  const int count = *big_count + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  long long carry = 0;
+  for (int c0 = 0; c0 < count; c0 += 1024) {
+    const int i = c0 + threadIdx.x, v = i < count ? big_chunks[i] : 0;
+    int s = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += u;
+    }
+    if (lane == 31) warp_total[warp] = s;
+    __syncthreads();
+    long long before = 0, total = 0;
+    for (int w = 0; w < 32; ++w) {
+      const int t = warp_total[w];
+      if (w < warp) before += t;
+      total += t;
+    }
+    if (i < count) start[i] = carry + before + s - v;
+    carry += total;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) start[count] = carry;
+}
+
+// The listed faces: a warp per chunk of a box's pixels (row by row), lanes along it. Work item
+// t belongs to the last entry with start <= t.
+__global__ __launch_bounds__(256) void k_raster_big(MeshRef m, int rows, int cols, const int* big_count,
+                                                    const int* big, const long long* start, int* owner,
+                                                    StaleList stale) {
+  const int count = *big_count + 1, lane = threadIdx.x & 31;
+  const long long total = start[count];
+  const int warps = gridDim.x * (blockDim.x >> 5);
+  const PixelAxis px(cols), py(rows);
+  for (long long t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < total; t += warps) {
+    int lo = 0, hi = count;  // start[lo] <= t < start[hi]
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
-      if (row_start[mid] <= t) lo = mid; else hi = mid;
+      if (start[mid] <= t) lo = mid; else hi = mid;
     }
-    const int f = lo;
-    const FaceRaster r = fr[f];
-    const int y = r.y0 + (t - row_start[f]);
+    const int f = big[lo];
     Quad p;
     int vid[4];
     const int c = load_face(m, f, p, vid);
-    const double qy = ((double)y + 0.5) / (double)rows;
-    for (int x = r.x0; x < r.x1; ++x) {
-      const double qx = ((double)x + 0.5) / (double)cols;
-      double w[4];
-      if (c == 3) {
-        tri_weights(qx, qy, p, w);
-      } else if (!bilinear_weights(qx, qy, p, w)) {
-        stale_weights(m, rows, cols, fr, f, x, y, w);
-      }
-      if (weights_inside(w)) atomicMax(&owner[(size_t)y * cols + x], f);
+    const FaceBox b = face_box(p, rows, cols);
+    const long long wx = b.x1 - b.x0, area = wx * (b.y1 - b.y0), k0 = (t - start[lo]) * BIG_CHUNK;
+    const int left = (int)min((long long)BIG_CHUNK, area - k0);
+    const unsigned y0 = (unsigned)(k0 / wx), r0 = (unsigned)(k0 - y0 * wx), w = (unsigned)wx;
+    for (int k = lane; k < left; k += 32) {
+      const unsigned off = r0 + k, dy = off / w;
+      const int x = b.x0 + (int)(off - dy * w), y = b.y0 + (int)(y0 + dy);
+      test_pixel(m, rows, cols, f, p, c, x, y, px(x), py(y), owner, stale);
     }
   }
 }
@@ -903,7 +1077,7 @@ __global__ void k_raster_owner_rows(MeshRef m, int rows, int cols, const FaceRas
 // One thread per pixel: the owner's PerFace value, or for PerVertex (vval != nullptr)
 // the float interpolation of rasterize_face's loop, which scales vertex 0's value by
 // each weight (rasterizer.cpp:123-130, 174-181) and sums in float.
-__global__ void k_raster_resolve(MeshRef m, int rows, int cols, const FaceRaster* fr, const int* owner,
+__global__ void k_raster_resolve(MeshRef m, int rows, int cols, const double* value, const int* owner,
                                  const float* vval, double* img) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
@@ -914,13 +1088,13 @@ __global__ void k_raster_resolve(MeshRef m, int rows, int cols, const FaceRaster
     if (vval) {
       double w[4];
       int vid[4];
-      const int c = pixel_weights(m, rows, cols, fr, f, x, y, w, vid);
+      const int c = pixel_weights(m, rows, cols, f, x, y, w, vid);
       const float v0 = vval[vid[0]];
       float acc = 0.0f;
       for (int q = 0; q < c; ++q) acc = acc + v0 * (float)w[q];
       out = (double)acc;
     } else {
-      out = fr[f].value;
+      out = value[f];
     }
   }
   img[(size_t)y * cols + x] = out;
@@ -998,23 +1172,23 @@ __global__ void k_vertex_values_mesh(int nv, const int* vstart, int* vfaces, con
 // dL/dA_f per face of a grid mesh from the pixels it owns in the last raster: an owned
 // pixel's PerFace value is scale / |A_f| with A_f the signed fan area of face_abs_area,
 // so d value / d A_f = -value / A_f.
-__global__ void k_raster_area_grad(MeshRef m, int rows, int cols, const FaceRaster* fr, const int* owner,
+__global__ void k_raster_area_grad(MeshRef m, int rows, int cols, const double* value, const int* owner,
                                    const double* dL_dpix, double* dL_dA) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= m.nf) return;
-  const FaceRaster r = fr[f];
-  double acc = 0.0;
-  for (int y = r.y0; y < r.y1; ++y)
-    for (int x = r.x0; x < r.x1; ++x) {
-      const size_t q = (size_t)y * cols + x;
-      if (owner[q] == f) acc += dL_dpix[q];
-    }
   Quad p;
   int vid[4];
   load_face(m, f, p, vid);
+  const FaceBox b = face_box(p, rows, cols);
+  double acc = 0.0;
+  for (int y = b.y0; y < b.y1; ++y)
+    for (int x = b.x0; x < b.x1; ++x) {
+      const size_t q = (size_t)y * cols + x;
+      if (owner[q] == f) acc += dL_dpix[q];
+    }
   const double A = signed_area3(p.x[0], p.y[0], p.x[1], p.y[1], p.x[2], p.y[2]) +
                    signed_area3(p.x[0], p.y[0], p.x[2], p.y[2], p.x[3], p.y[3]);
-  dL_dA[f] = (acc != 0.0 && A != 0.0) ? -acc * r.value / A : 0.0;
+  dL_dA[f] = (acc != 0.0 && A != 0.0) ? -acc * value[f] / A : 0.0;
 }
 
 // Per vertex (i, j) of the grid mesh, in a fixed order over the faces around it (face
@@ -1193,14 +1367,14 @@ void raster_grid_backward(otm_context* ctx, int n, const double* xy, int rows, i
                           double* dL_dxy) {
   const int N = n * n;
   auto al = [](size_t b) { return (b + 255) / 256 * 256; };
-  // the layout raster_mesh leaves in the scratch: face boxes, then pixel owners
+  // the layout raster_mesh leaves in the scratch: face values, then pixel owners
   const char* base = ctx->raster_scratch.as<char>();
-  const FaceRaster* fr = reinterpret_cast<const FaceRaster*>(base);
-  const int* owner = reinterpret_cast<const int*>(base + al(sizeof(FaceRaster) * (size_t)(N > 0 ? N : 1)));
+  const double* value = reinterpret_cast<const double*>(base);
+  const int* owner = reinterpret_cast<const int*>(base + al(sizeof(double) * (size_t)(N > 0 ? N : 1)));
   DevBuf dA;
   dA.reserve(sizeof(double) * N);
   MeshRef m{xy, n, N, (n + 1) * (n + 1), nullptr, nullptr};
-  launch(ctx, "raster_area_grad", k_raster_area_grad, (N + 255) / 256, 256, m, rows, cols, fr, owner, dL_dpix,
+  launch(ctx, "raster_area_grad", k_raster_area_grad, (N + 255) / 256, 256, m, rows, cols, value, owner, dL_dpix,
          dA.as<double>());
   const long V = (long)(n + 1) * (n + 1);
   launch(ctx, "area_vertex_grad", k_grid_vertex_gather, (unsigned)((V + 255) / 256), 256, xy, n,
@@ -1388,28 +1562,37 @@ static void raster_mesh(otm_context* ctx, const MeshRef& m, const double* densit
   const int nf = m.nf;
   const size_t pix = (size_t)rows * cols;
   auto al = [](size_t b) { return (b + 255) / 256 * 256; };
-  const size_t b_fr = al(sizeof(FaceRaster) * (size_t)(nf > 0 ? nf : 1)), b_own = al(sizeof(int) * pix);
+  const size_t b_val = al(sizeof(double) * (size_t)(nf > 0 ? nf : 1)), b_own = al(sizeof(int) * (pix + 2));
   const size_t b_vv = al(sizeof(float) * (size_t)(m.nv > 0 ? m.nv : 1));
-  const size_t b_rows = al(sizeof(int) * (size_t)(nf + 1)), b_rs = al(sizeof(int) * ((nf + SCAN_B) / SCAN_B + 1));
-  ctx->raster_scratch.reserve(b_fr + b_own + b_vv + 2 * b_rows + b_rs);  // grows, kept for the next call
-  char* base = ctx->raster_scratch.as<char>();
-  FaceRaster* fr = reinterpret_cast<FaceRaster*>(base);
-  int* owner = reinterpret_cast<int*>(base + b_fr);
-  float* vval = reinterpret_cast<float*>(base + b_fr + b_own);
-  int* rows_of = reinterpret_cast<int*>(base + b_fr + b_own + b_vv);
-  int* row_start = reinterpret_cast<int*>(base + b_fr + b_own + b_vv + b_rows);
-  int* row_sums = reinterpret_cast<int*>(base + b_fr + b_own + b_vv + 2 * b_rows);
-  OTM_CUDA(cudaMemsetAsync(owner, 0xff, sizeof(int) * pix, st));  // -1: no face
+  const size_t b_list = al(sizeof(int) * (size_t)(nf + 1));
+  const size_t b_start = al(sizeof(long long) * (size_t)(nf + 1));
+  const size_t b_stale = al(sizeof(uint2) * (size_t)(nf + 1));
+  ctx->raster_scratch.reserve(b_val + b_own + b_vv + 2 * b_list + b_start + b_stale);  // grows, kept for the next call
+  char* next = ctx->raster_scratch.as<char>();
+  auto take = [&](size_t b) {
+    char* r = next;
+    next += b;
+    return r;
+  };
+  double* value = reinterpret_cast<double*>(take(b_val));
+  int* owner = reinterpret_cast<int*>(take(b_own));  // then the counters of the two lists
+  float* vval = reinterpret_cast<float*>(take(b_vv));
+  int* big = reinterpret_cast<int*>(take(b_list));
+  int* big_chunks = reinterpret_cast<int*>(take(b_list));
+  long long* big_start = reinterpret_cast<long long*>(take(b_start));
+  int* big_count = owner + pix;
+  StaleList stale{owner + pix + 1, reinterpret_cast<uint2*>(take(b_stale)), nf};
+  OTM_CUDA(cudaMemsetAsync(owner, 0xff, sizeof(int) * (pix + 2), st));  // -1: no face, empty lists
   // rasterizer.cpp:193 keeps 1/density.size() in a float
   const float scale = (float)(1. / (double)(density ? cells : nf));
   const int fblocks = nf > 0 ? (nf + 255) / 256 : 1;
-  launch(ctx, "face_boxes", k_face_boxes, fblocks, 256, m, density, scale, rows, cols, fr);
   if (nf > 0) {
-    launch(ctx, "box_rows", k_box_rows, fblocks, 256, nf, (const FaceRaster*)fr, rows_of);
-    exclusive_scan(st, rows_of, row_start, row_sums, nf);
-    ctx->launches += 3;
-    launch(ctx, "raster_owner", k_raster_owner_rows, ctx->num_sms * 8, 256, m, rows, cols, (const FaceRaster*)fr,
-           (const int*)row_start, owner);
+    launch(ctx, "raster_faces", k_raster_faces, (nf + RF_T - 1) / RF_T, RF_T, m, density, scale, rows, cols, value, owner,
+           big_count, big, big_chunks, stale);
+    launch(ctx, "big_scan", k_big_scan, 1, 1024, (const int*)big_count, (const int*)big_chunks, big_start);
+    launch(ctx, "raster_big", k_raster_big, ctx->num_sms * 8, 256, m, rows, cols, (const int*)big_count,
+           (const int*)big, (const long long*)big_start, owner, stale);
+    launch(ctx, "raster_stale", k_raster_stale, ctx->num_sms, 128, m, rows, cols, owner, stale);
   }
   const float* pv = nullptr;
   DevBuf vcount, vstart, vsums, vfaces, inv_area;  // indexed PerVertex temporaries
@@ -1438,7 +1621,7 @@ static void raster_mesh(otm_context* ctx, const MeshRef& m, const double* densit
     pv = vval;
   }
   dim3 blk(32, 8), grd((cols + 31) / 32, (rows + 7) / 8);
-  launch(ctx, "raster_resolve", k_raster_resolve, grd, blk, m, rows, cols, (const FaceRaster*)fr,
+  launch(ctx, "raster_resolve", k_raster_resolve, grd, blk, m, rows, cols, (const double*)value,
          (const int*)owner, pv, img);
   OTM_CUDA(cudaGetLastError());
   if (m.start && mode == OTM_RIO_PER_VERTEX) OTM_CUDA(cudaStreamSynchronize(st));  // temporaries freed on return
@@ -1523,7 +1706,7 @@ extern "C" int otm_rasterize_faces(otm_context* ctx, int n, const double* xy, in
     const int N = n * n;
     auto al = [](size_t b) { return (b + 255) / 256 * 256; };
     const int* owner =
-        reinterpret_cast<const int*>(ctx->raster_scratch.as<char>() + al(sizeof(FaceRaster) * (size_t)N));
+        reinterpret_cast<const int*>(ctx->raster_scratch.as<char>() + al(sizeof(double) * (size_t)N));
     OTM_CUDA(cudaMemcpyAsync(face, owner, sizeof(int) * pix, cudaMemcpyDefault, st));
     OTM_CUDA(cudaStreamSynchronize(st));
     ctx->prof.flush();
