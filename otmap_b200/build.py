@@ -23,7 +23,7 @@ INCLUDE = os.path.join(ROOT, "include")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 SOURCES = ["capi.cu", "solver.cu", "stencil.cu", "poisson.cu", "dct_reg.cu", "dct_tc.cu", "adjoint.cu", "locate.cu",
-           "pipeline.cu", "meshio.cu"]
+           "pipeline.cu", "meshio.cu", "hostcopy.cu"]
 
 
 def nvcc() -> str:

@@ -14,18 +14,6 @@ void set_error(const std::string& msg) { g_last_error = msg; }
 
 void make_current(otm_context* ctx) { OTM_CUDA(cudaSetDevice(ctx->device)); }
 
-void copy_in(otm_context* ctx, void* dst, const void* src, size_t bytes) {
-  if (!bytes) return;
-  OTM_CUDA(cudaMemcpyAsync(dst, src, bytes, is_device_ptr(src) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
-                           ctx->stream));
-}
-
-void copy_out(otm_context* ctx, void* dst, const void* src, size_t bytes) {
-  if (!bytes) return;
-  OTM_CUDA(cudaMemcpyAsync(dst, src, bytes, is_device_ptr(dst) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
-                           ctx->stream));
-}
-
 int Profiler::id(const char* name) {
   for (size_t k = 0; k < names.size(); ++k)
     if (std::strcmp(names[k], name) == 0) return (int)k;
@@ -109,15 +97,16 @@ extern "C" int otm_create(int device, otm_context** out) {
       OTM_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
       OTM_CUDA(cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device));
       // the per-map buffers come from this context's own memory pool (stream-ordered
-      // allocation), which keeps freed memory for the next map instead of returning it to
-      // the driver at every synchronisation; the device's default pool is left as it is
+      // allocation), as do the calls' temporaries; it keeps up to 4 GiB of freed memory for
+      // the next one instead of returning it to the driver at every synchronisation, and the
+      // device's default pool is left as it is
       cudaMemPoolProps props = {};
       props.allocType = cudaMemAllocationTypePinned;
       props.handleTypes = cudaMemHandleTypeNone;
       props.location.type = cudaMemLocationTypeDevice;
       props.location.id = device;
       OTM_CUDA(cudaMemPoolCreate(&ctx->pool, &props));
-      uint64_t keep = UINT64_MAX;
+      uint64_t keep = uint64_t(4) << 30;
       OTM_CUDA(cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
     } catch (...) {
       delete ctx;

@@ -36,7 +36,8 @@ struct DevBuf {
 // Device buffer from the stream-ordered allocator (cudaMallocFromPoolAsync / cudaFreeAsync
 // on the stream it was reserved on, from the context's memory pool): freeing it does not
 // synchronise the device, and the pool hands the memory to the next allocation. Used for
-// the per-map buffers, which live and die with each TransportMap.
+// the per-map buffers, which live and die with each TransportMap, and for the temporaries of
+// a call (a cudaMalloc and cudaFree of 25 MB cost a 512^2 barycenter image 0.4 ms).
 struct AsyncBuf {
   void* p = nullptr;
   size_t bytes = 0;
@@ -73,6 +74,11 @@ struct SizeTables {
 };
 
 struct Inst;  // device instance record (solver.cu)
+
+struct HostCopier;  // pinned ring and worker threads for pageable copies (hostcopy.cu)
+struct HostCopierDelete {
+  void operator()(HostCopier* c) const;
+};
 
 // Buffers of one batch configuration (the list of grid sizes), reused across calls.
 struct Workspace {
@@ -161,6 +167,8 @@ struct otm_context {
   otm::Workspace* wsp = nullptr;  // the workspace of the current call
   otm::Workspace& ws() { return *wsp; }
   otm::DevBuf staging;  // device staging for host inputs/outputs
+  std::unique_ptr<otm::HostCopier, otm::HostCopierDelete> copier;
+  bool copier_failed = false;
   // second stream of a batched solve: outputs of instances that stopped while the rest of
   // the batch iterates (created on first use), its staging and a pinned copy of the records
   cudaStream_t side = nullptr;
@@ -214,10 +222,13 @@ struct otm_map {
 namespace otm {
 // Makes the context's device current; defined in capi.cu.
 void make_current(otm_context* ctx);
-// Copies `bytes` from src (host or device) into dst (device), on the context stream.
+// Copies `bytes` from src (host or device) into dst (device), on the context stream; host
+// memory has been read when the call returns.
 void copy_in(otm_context* ctx, void* dst, const void* src, size_t bytes);
-// Copies `bytes` from src (device) into dst (host or device), on the context stream.
+// Copies `bytes` from src (device) into dst (host or device), on the context stream; complete
+// once the stream has been synchronised (pageable memory: possibly on return).
 void copy_out(otm_context* ctx, void* dst, const void* src, size_t bytes);
+void copy_out(otm_context* ctx, void* dst, const void* src, size_t bytes, cudaStream_t st);  // on another stream
 
 // Rasterizes the (n+1)^2 grid mesh xy (device) into img (device, rows*cols), in
 // OTM_RIO_PER_FACE or OTM_RIO_PER_VERTEX mode; density (device) NULL = unit density.

@@ -1371,8 +1371,8 @@ void raster_grid_backward(otm_context* ctx, int n, const double* xy, int rows, i
   const char* base = ctx->raster_scratch.as<char>();
   const double* value = reinterpret_cast<const double*>(base);
   const int* owner = reinterpret_cast<const int*>(base + al(sizeof(double) * (size_t)(N > 0 ? N : 1)));
-  DevBuf dA;
-  dA.reserve(sizeof(double) * N);
+  AsyncBuf dA;
+  dA.reserve(sizeof(double) * N, ctx->stream, ctx->pool);
   MeshRef m{xy, n, N, (n + 1) * (n + 1), nullptr, nullptr};
   launch(ctx, "raster_area_grad", k_raster_area_grad, (N + 255) / 256, 256, m, rows, cols, value, owner, dL_dpix,
          dA.as<double>());
@@ -1380,7 +1380,6 @@ void raster_grid_backward(otm_context* ctx, int n, const double* xy, int rows, i
   launch(ctx, "area_vertex_grad", k_grid_vertex_gather, (unsigned)((V + 255) / 256), 256, xy, n,
          (const double*)dA.as<double>(), (const double2*)nullptr, dL_dxy);
   OTM_CUDA(cudaGetLastError());
-  OTM_CUDA(cudaStreamSynchronize(ctx->stream));  // dA is released on return
 }
 
 void inverse_grid_backward(otm_context* ctx, int n, const double* fwd, const int* hit0, const double* dL_dI,
@@ -1391,8 +1390,8 @@ void inverse_grid_backward(otm_context* ctx, int n, const double* fwd, const int
   auto al = [](size_t b) { return (b + 255) / 256 * 256; };
   const size_t b_pg = al(sizeof(InvGrad) * V), b_cnt = al(sizeof(int) * (N + 1)), b_list = al(sizeof(int) * V);
   const size_t b_cs = al(sizeof(double2) * 4 * (size_t)N), b_sums = al(sizeof(int) * ((N + SCAN_B - 1) / SCAN_B + 1));
-  DevBuf buf;
-  buf.reserve(b_pg + 3 * b_cnt + b_list + b_cs + b_sums);
+  AsyncBuf buf;
+  buf.reserve(b_pg + 3 * b_cnt + b_list + b_cs + b_sums, st, ctx->pool);
   char* q = buf.as<char>();
   InvGrad* pg = reinterpret_cast<InvGrad*>(q);
   int* count = reinterpret_cast<int*>(q + b_pg);
@@ -1483,12 +1482,12 @@ extern "C" int otm_map_inverse_mode(otm_map* m, double* points, long count, int 
     int* df = face ? (fdev ? face : reinterpret_cast<int*>(base + al(bp))) : nullptr;
     int* dh = nhits ? (hdev ? nhits : reinterpret_cast<int*>(base + al(bp) + al(bf))) : nullptr;
     unsigned long long* dm = reinterpret_cast<unsigned long long*>(base + al(bp) + al(bf) + al(bh));
-    if (!pdev) OTM_CUDA(cudaMemcpyAsync(dp, points, bp, cudaMemcpyHostToDevice, st));
+    if (!pdev) copy_in(ctx, dp, points, bp);
     OTM_CUDA(cudaMemsetAsync(dm, 0, sizeof(unsigned long long), st));
     map_inverse_dev(m, dp, (long)count, mode, df, nullptr, dh, dm);
-    if (!pdev) OTM_CUDA(cudaMemcpyAsync(points, dp, bp, cudaMemcpyDeviceToHost, st));
-    if (face && !fdev) OTM_CUDA(cudaMemcpyAsync(face, df, bf, cudaMemcpyDeviceToHost, st));
-    if (nhits && !hdev) OTM_CUDA(cudaMemcpyAsync(nhits, dh, bh, cudaMemcpyDeviceToHost, st));
+    if (!pdev) copy_out(ctx, points, dp, bp);
+    if (face && !fdev) copy_out(ctx, face, df, bf);
+    if (nhits && !hdev) copy_out(ctx, nhits, dh, bh);
     unsigned long long miss = 0;
     OTM_CUDA(cudaMemcpyAsync(&miss, dm, sizeof(miss), cudaMemcpyDeviceToHost, st));
     OTM_CUDA(cudaStreamSynchronize(st));
@@ -1595,7 +1594,7 @@ static void raster_mesh(otm_context* ctx, const MeshRef& m, const double* densit
     launch(ctx, "raster_stale", k_raster_stale, ctx->num_sms, 128, m, rows, cols, owner, stale);
   }
   const float* pv = nullptr;
-  DevBuf vcount, vstart, vsums, vfaces, inv_area;  // indexed PerVertex temporaries
+  AsyncBuf vcount, vstart, vsums, vfaces, inv_area;  // indexed PerVertex temporaries
   if (mode == OTM_RIO_PER_VERTEX) {
     const unsigned vb = (unsigned)((m.nv + 255) / 256);
     if (!m.start) {
@@ -1603,15 +1602,15 @@ static void raster_mesh(otm_context* ctx, const MeshRef& m, const double* densit
     } else {
       int nref = 0;
       OTM_CUDA(cudaMemcpyAsync(&nref, m.start + nf, sizeof(int), cudaMemcpyDeviceToHost, st));
-      vcount.reserve(sizeof(int) * m.nv);
-      vstart.reserve(sizeof(int) * (m.nv + 1));
-      vsums.reserve(sizeof(int) * ((m.nv + SCAN_B - 1) / SCAN_B + 1));
-      inv_area.reserve(sizeof(double) * (size_t)(nf > 0 ? nf : 1));
+      vcount.reserve(sizeof(int) * m.nv, st, ctx->pool);
+      vstart.reserve(sizeof(int) * (m.nv + 1), st, ctx->pool);
+      vsums.reserve(sizeof(int) * ((m.nv + SCAN_B - 1) / SCAN_B + 1), st, ctx->pool);
+      inv_area.reserve(sizeof(double) * (size_t)(nf > 0 ? nf : 1), st, ctx->pool);
       OTM_CUDA(cudaMemsetAsync(vcount.p, 0, sizeof(int) * m.nv, st));
       launch(ctx, "vf_count", k_vf_count, fblocks, 256, m, vcount.as<int>());
       exclusive_scan(st, vcount.as<int>(), vstart.as<int>(), vsums.as<int>(), m.nv);
       OTM_CUDA(cudaStreamSynchronize(st));
-      vfaces.reserve(sizeof(int) * (size_t)(nref > 0 ? nref : 1));
+      vfaces.reserve(sizeof(int) * (size_t)(nref > 0 ? nref : 1), st, ctx->pool);
       OTM_CUDA(cudaMemsetAsync(vcount.p, 0, sizeof(int) * m.nv, st));
       launch(ctx, "vf_fill", k_vf_fill, fblocks, 256, m, (const int*)vstart.as<int>(), vcount.as<int>(),
              vfaces.as<int>(), inv_area.as<double>());
@@ -1624,7 +1623,6 @@ static void raster_mesh(otm_context* ctx, const MeshRef& m, const double* densit
   launch(ctx, "raster_resolve", k_raster_resolve, grd, blk, m, rows, cols, (const double*)value,
          (const int*)owner, pv, img);
   OTM_CUDA(cudaGetLastError());
-  if (m.start && mode == OTM_RIO_PER_VERTEX) OTM_CUDA(cudaStreamSynchronize(st));  // temporaries freed on return
 }
 
 void raster_grid(otm_context* ctx, int n, const double* xy, const double* density, int rows, int cols, int mode,
@@ -1659,27 +1657,27 @@ extern "C" int otm_rasterize_mode(otm_context* ctx, int n, const double* xy, con
     const int N = n * n;
     size_t V = (size_t)(n + 1) * (n + 1);
     size_t pix = (size_t)rows * cols;
-    DevBuf dxy, dden, dimg;
+    AsyncBuf dxy, dden, dimg;
     const double* pxy = xy;
     if (!is_device_ptr(xy)) {
-      dxy.reserve(sizeof(double) * 2 * V);
-      OTM_CUDA(cudaMemcpyAsync(dxy.p, xy, sizeof(double) * 2 * V, cudaMemcpyHostToDevice, st));
+      dxy.reserve(sizeof(double) * 2 * V, st, ctx->pool);
+      copy_in(ctx, dxy.p, xy, sizeof(double) * 2 * V);
       pxy = dxy.as<double>();
     }
     const double* pden = density;
     if (density && !is_device_ptr(density)) {
-      dden.reserve(sizeof(double) * N);
-      OTM_CUDA(cudaMemcpyAsync(dden.p, density, sizeof(double) * N, cudaMemcpyHostToDevice, st));
+      dden.reserve(sizeof(double) * N, st, ctx->pool);
+      copy_in(ctx, dden.p, density, sizeof(double) * N);
       pden = dden.as<double>();
     }
     bool idev = is_device_ptr(img);
     double* pimg = img;
     if (!idev) {
-      dimg.reserve(sizeof(double) * pix);
+      dimg.reserve(sizeof(double) * pix, st, ctx->pool);
       pimg = dimg.as<double>();
     }
     raster_grid(ctx, n, pxy, pden, rows, cols, mode, pimg);
-    if (!idev) OTM_CUDA(cudaMemcpyAsync(img, pimg, sizeof(double) * pix, cudaMemcpyDeviceToHost, st));
+    if (!idev) copy_out(ctx, img, pimg, sizeof(double) * pix);
     OTM_CUDA(cudaStreamSynchronize(st));
     ctx->prof.flush();
     return (int)OTM_OK;
@@ -1694,11 +1692,11 @@ extern "C" int otm_rasterize_faces(otm_context* ctx, int n, const double* xy, in
     make_current(ctx);
     cudaStream_t st = ctx->stream;
     const size_t V2 = 2 * (size_t)(n + 1) * (n + 1), pix = (size_t)rows * cols;
-    DevBuf buf;
-    buf.reserve(sizeof(double) * (V2 + pix) + 256);
+    AsyncBuf buf;
+    buf.reserve(sizeof(double) * (V2 + pix) + 256, st, ctx->pool);
     const double* pxy = xy;
     if (!is_device_ptr(xy)) {
-      OTM_CUDA(cudaMemcpyAsync(buf.p, xy, sizeof(double) * V2, cudaMemcpyHostToDevice, st));
+      copy_in(ctx, buf.p, xy, sizeof(double) * V2);
       pxy = buf.as<double>();
     }
     double* img = buf.as<double>() + V2;
@@ -1707,7 +1705,7 @@ extern "C" int otm_rasterize_faces(otm_context* ctx, int n, const double* xy, in
     auto al = [](size_t b) { return (b + 255) / 256 * 256; };
     const int* owner =
         reinterpret_cast<const int*>(ctx->raster_scratch.as<char>() + al(sizeof(double) * (size_t)N));
-    OTM_CUDA(cudaMemcpyAsync(face, owner, sizeof(int) * pix, cudaMemcpyDefault, st));
+    copy_out(ctx, face, owner, sizeof(int) * pix);
     OTM_CUDA(cudaStreamSynchronize(st));
     ctx->prof.flush();
     return (int)OTM_OK;
@@ -1748,36 +1746,36 @@ extern "C" int otm_rasterize_mesh(otm_context* ctx, int nv, const double* xy, in
     if (total > 0) to_host(hidx.data(), face_vertices, (size_t)total);
     if (nf > 0) check_faces(nv, nf, hstart.data(), hidx.data());
     const size_t pix = (size_t)rows * cols;
-    DevBuf dxy, dden, dimg, dstart, didx;
+    AsyncBuf dxy, dden, dimg, dstart, didx;
     const double* pxy = xy;
     if (nv > 0 && !is_device_ptr(xy)) {
-      dxy.reserve(sizeof(double) * 2 * (size_t)nv);
-      OTM_CUDA(cudaMemcpyAsync(dxy.p, xy, sizeof(double) * 2 * (size_t)nv, cudaMemcpyHostToDevice, st));
+      dxy.reserve(sizeof(double) * 2 * (size_t)nv, st, ctx->pool);
+      copy_in(ctx, dxy.p, xy, sizeof(double) * 2 * (size_t)nv);
       pxy = dxy.as<double>();
     }
     const double* pden = density;
     if (density && !is_device_ptr(density)) {
-      dden.reserve(sizeof(double) * (size_t)cells);
-      OTM_CUDA(cudaMemcpyAsync(dden.p, density, sizeof(double) * (size_t)cells, cudaMemcpyHostToDevice, st));
+      dden.reserve(sizeof(double) * (size_t)cells, st, ctx->pool);
+      copy_in(ctx, dden.p, density, sizeof(double) * (size_t)cells);
       pden = dden.as<double>();
     }
     bool idev = is_device_ptr(img);
     double* pimg = img;
     if (!idev) {
-      dimg.reserve(sizeof(double) * pix);
+      dimg.reserve(sizeof(double) * pix, st, ctx->pool);
       pimg = dimg.as<double>();
     }
     if (nf == 0) {
       OTM_CUDA(cudaMemsetAsync(pimg, 0, sizeof(double) * pix, st));
     } else {
-      dstart.reserve(sizeof(int) * ((size_t)nf + 1));
-      didx.reserve(sizeof(int) * (size_t)total);
-      OTM_CUDA(cudaMemcpyAsync(dstart.p, hstart.data(), sizeof(int) * ((size_t)nf + 1), cudaMemcpyHostToDevice, st));
-      OTM_CUDA(cudaMemcpyAsync(didx.p, hidx.data(), sizeof(int) * (size_t)total, cudaMemcpyHostToDevice, st));
+      dstart.reserve(sizeof(int) * ((size_t)nf + 1), st, ctx->pool);
+      didx.reserve(sizeof(int) * (size_t)total, st, ctx->pool);
+      copy_in(ctx, dstart.p, hstart.data(), sizeof(int) * ((size_t)nf + 1));
+      copy_in(ctx, didx.p, hidx.data(), sizeof(int) * (size_t)total);
       MeshRef m{pxy, 0, nf, nv, dstart.as<int>(), didx.as<int>()};
       raster_mesh(ctx, m, pden, cells, rows, cols, mode, pimg);
     }
-    if (!idev) OTM_CUDA(cudaMemcpyAsync(img, pimg, sizeof(double) * pix, cudaMemcpyDeviceToHost, st));
+    if (!idev) copy_out(ctx, img, pimg, sizeof(double) * pix);
     OTM_CUDA(cudaStreamSynchronize(st));
     ctx->prof.flush();
     return (int)OTM_OK;
@@ -1825,36 +1823,36 @@ extern "C" int otm_sample_image(otm_context* ctx, int nv, const double* xy, int 
       check_faces(nv, nf, hstart.data(), hidx.data());
     }
     const size_t pix = (size_t)rows * cols;
-    DevBuf dxy, dspf, dimg, dstart, didx;
+    AsyncBuf dxy, dspf, dimg, dstart, didx;
     const double* pxy = xy;
     if (nv > 0 && !is_device_ptr(xy)) {
-      dxy.reserve(sizeof(double) * 2 * (size_t)nv);
-      OTM_CUDA(cudaMemcpyAsync(dxy.p, xy, sizeof(double) * 2 * (size_t)nv, cudaMemcpyHostToDevice, st));
+      dxy.reserve(sizeof(double) * 2 * (size_t)nv, st, ctx->pool);
+      copy_in(ctx, dxy.p, xy, sizeof(double) * 2 * (size_t)nv);
       pxy = dxy.as<double>();
     }
     const int* pspf = samples_per_face;
     if (nf > 0 && !is_device_ptr(samples_per_face)) {
-      dspf.reserve(sizeof(int) * (size_t)nf);
-      OTM_CUDA(cudaMemcpyAsync(dspf.p, samples_per_face, sizeof(int) * (size_t)nf, cudaMemcpyHostToDevice, st));
+      dspf.reserve(sizeof(int) * (size_t)nf, st, ctx->pool);
+      copy_in(ctx, dspf.p, samples_per_face, sizeof(int) * (size_t)nf);
       pspf = dspf.as<int>();
     }
     const bool idev = is_device_ptr(img);
     double* pimg = img;
     if (!idev) {
-      dimg.reserve(sizeof(double) * pix);
+      dimg.reserve(sizeof(double) * pix, st, ctx->pool);
       pimg = dimg.as<double>();
     }
     MeshRef m{pxy, grid ? grid_n : 0, nf, nv, nullptr, nullptr};
     if (!grid && nf > 0) {
-      dstart.reserve(sizeof(int) * ((size_t)nf + 1));
-      didx.reserve(sizeof(int) * hidx.size());
-      OTM_CUDA(cudaMemcpyAsync(dstart.p, hstart.data(), sizeof(int) * hstart.size(), cudaMemcpyHostToDevice, st));
-      OTM_CUDA(cudaMemcpyAsync(didx.p, hidx.data(), sizeof(int) * hidx.size(), cudaMemcpyHostToDevice, st));
+      dstart.reserve(sizeof(int) * ((size_t)nf + 1), st, ctx->pool);
+      didx.reserve(sizeof(int) * hidx.size(), st, ctx->pool);
+      copy_in(ctx, dstart.p, hstart.data(), sizeof(int) * hstart.size());
+      copy_in(ctx, didx.p, hidx.data(), sizeof(int) * hidx.size());
       m.start = dstart.as<int>();
       m.idx = didx.as<int>();
     }
     splat(ctx, m, pspf, seed, rows, cols, pimg);
-    if (!idev) OTM_CUDA(cudaMemcpyAsync(img, pimg, sizeof(double) * pix, cudaMemcpyDeviceToHost, st));
+    if (!idev) copy_out(ctx, img, pimg, sizeof(double) * pix);
     OTM_CUDA(cudaStreamSynchronize(st));
     ctx->prof.flush();
     return (int)OTM_OK;

@@ -159,7 +159,7 @@ static std::vector<const double*> stage_meshes(otm_context* ctx, const double* c
       ptrs[k] = meshes[k];
     } else {
       double* d = stage + V2 * k;
-      OTM_CUDA(cudaMemcpyAsync(d, meshes[k], sizeof(double) * V2, cudaMemcpyHostToDevice, ctx->stream));
+      copy_in(ctx, d, meshes[k], sizeof(double) * V2);
       ptrs[k] = d;
     }
   }
@@ -178,8 +178,8 @@ extern "C" int otm_mesh_blend(otm_context* ctx, int n, int count, const double* 
     make_current(ctx);
     cudaStream_t st = ctx->stream;
     const size_t V2 = 2 * (size_t)(n + 1) * (n + 1);
-    DevBuf buf;
-    buf.reserve(sizeof(double) * (V2 * (count + 1) + count + 8) + sizeof(double*) * count);
+    AsyncBuf buf;
+    buf.reserve(sizeof(double) * (V2 * (count + 1) + count + 8) + sizeof(double*) * count, st, ctx->pool);
     double* base = buf.as<double>();
     std::vector<const double*> ptrs = stage_meshes(ctx, meshes, count, V2, base);
     double* d_out = base + V2 * count;
@@ -192,7 +192,7 @@ extern "C" int otm_mesh_blend(otm_context* ctx, int n, int count, const double* 
     launch(ctx, "blend", k_blend, (unsigned)((V2 + 255) / 256), 256, (long)V2, count, (const double* const*)d_ptrs,
            (const double*)d_w, dst);
     OTM_CUDA(cudaGetLastError());
-    if (!odev) OTM_CUDA(cudaMemcpyAsync(out, dst, sizeof(double) * V2, cudaMemcpyDeviceToHost, st));
+    if (!odev) copy_out(ctx, out, dst, sizeof(double) * V2);
     OTM_CUDA(cudaStreamSynchronize(st));
     ctx->prof.flush();
     return (int)OTM_OK;
@@ -208,12 +208,12 @@ extern "C" int otm_transport_cost(otm_context* ctx, int n, const double* src_xy,
     cudaStream_t st = ctx->stream;
     const size_t V2 = 2 * (size_t)(n + 1) * (n + 1), N = (size_t)n * n;
     const int nb = 512;
-    DevBuf buf;
-    buf.reserve(sizeof(double) * (2 * V2 + 2 * N + 2 * nb + 8));
+    AsyncBuf buf;
+    buf.reserve(sizeof(double) * (2 * V2 + 2 * N + 2 * nb + 8), st, ctx->pool);
     double* p = buf.as<double>();
     auto in = [&](const double* src, double* tmp, size_t words) -> const double* {
       if (is_device_ptr(src)) return src;
-      OTM_CUDA(cudaMemcpyAsync(tmp, src, sizeof(double) * words, cudaMemcpyHostToDevice, st));
+      copy_in(ctx, tmp, src, sizeof(double) * words);
       return tmp;
     };
     const double* d_src = in(src_xy, p, V2);
@@ -227,8 +227,7 @@ extern "C" int otm_transport_cost(otm_context* ctx, int n, const double* src_xy,
     OTM_CUDA(cudaGetLastError());
     double res[2];
     OTM_CUDA(cudaMemcpyAsync(res, d_res, sizeof(res), cudaMemcpyDeviceToHost, st));
-    if (per_face && !is_device_ptr(per_face))
-      OTM_CUDA(cudaMemcpyAsync(per_face, d_pf, sizeof(double) * N, cudaMemcpyDeviceToHost, st));
+    if (per_face && !is_device_ptr(per_face)) copy_out(ctx, per_face, d_pf, sizeof(double) * N);
     OTM_CUDA(cudaStreamSynchronize(st));
     ctx->prof.flush();
     *cost = res[0];
@@ -248,8 +247,8 @@ extern "C" int otm_barycenter(otm_context* ctx, int n, int count, const double* 
     cudaStream_t st = ctx->stream;
     const size_t V2 = 2 * (size_t)(n + 1) * (n + 1), pix = (size_t)rows * cols;
     const int nparts = 512;
-    DevBuf buf;
-    buf.reserve(sizeof(double) * (V2 * (count + 1) + count + pix + nparts + 16) + sizeof(double*) * count);
+    AsyncBuf buf;
+    buf.reserve(sizeof(double) * (V2 * (count + 1) + count + pix + nparts + 16) + sizeof(double*) * count, st, ctx->pool);
     double* base = buf.as<double>();
     std::vector<const double*> ptrs = stage_meshes(ctx, inv_meshes, count, V2, base);
     double* d_mesh = base + V2 * count;
@@ -272,8 +271,8 @@ extern "C" int otm_barycenter(otm_context* ctx, int n, int count, const double* 
     launch(ctx, "img_rescale", k_img_rescale, sb, 256, (long)pix, nparts, (const double*)d_part, expected_mean, pi,
            d_mean);
     OTM_CUDA(cudaGetLastError());
-    if (mesh_out && !mdev) OTM_CUDA(cudaMemcpyAsync(mesh_out, pm, sizeof(double) * V2, cudaMemcpyDeviceToHost, st));
-    if (!idev) OTM_CUDA(cudaMemcpyAsync(img, pi, sizeof(double) * pix, cudaMemcpyDeviceToHost, st));
+    if (mesh_out && !mdev) copy_out(ctx, mesh_out, pm, sizeof(double) * V2);
+    if (!idev) copy_out(ctx, img, pi, sizeof(double) * pix);
     double mean = 0;
     OTM_CUDA(cudaMemcpyAsync(&mean, d_mean, sizeof(double), cudaMemcpyDeviceToHost, st));
     OTM_CUDA(cudaStreamSynchronize(st));
@@ -292,17 +291,17 @@ extern "C" int otm_grid_transport_cost(otm_context* ctx, int n, const double* gr
     cudaStream_t st = ctx->stream;
     const size_t V2 = 2 * (size_t)(n + 1) * (n + 1), N = (size_t)n * n;
     const int nb = 512;
-    DevBuf buf;
-    buf.reserve(sizeof(double) * (V2 + 2 * N + nb + 8));
+    AsyncBuf buf;
+    buf.reserve(sizeof(double) * (V2 + 2 * N + nb + 8), st, ctx->pool);
     double* p = buf.as<double>();
     const double* d_g = grads_xy;
     if (!is_device_ptr(grads_xy)) {
-      OTM_CUDA(cudaMemcpyAsync(p, grads_xy, sizeof(double) * V2, cudaMemcpyHostToDevice, st));
+      copy_in(ctx, p, grads_xy, sizeof(double) * V2);
       d_g = p;
     }
     const double* d_den = density;
     if (!is_device_ptr(density)) {
-      OTM_CUDA(cudaMemcpyAsync(p + V2, density, sizeof(double) * N, cudaMemcpyHostToDevice, st));
+      copy_in(ctx, p + V2, density, sizeof(double) * N);
       d_den = p + V2;
     }
     double* d_pf = per_face ? (is_device_ptr(per_face) ? per_face : p + V2 + N) : nullptr;
@@ -314,8 +313,7 @@ extern "C" int otm_grid_transport_cost(otm_context* ctx, int n, const double* gr
     OTM_CUDA(cudaGetLastError());
     double res = 0;
     OTM_CUDA(cudaMemcpyAsync(&res, d_res, sizeof(double), cudaMemcpyDeviceToHost, st));
-    if (per_face && !is_device_ptr(per_face))
-      OTM_CUDA(cudaMemcpyAsync(per_face, d_pf, sizeof(double) * N, cudaMemcpyDeviceToHost, st));
+    if (per_face && !is_device_ptr(per_face)) copy_out(ctx, per_face, d_pf, sizeof(double) * N);
     OTM_CUDA(cudaStreamSynchronize(st));
     ctx->prof.flush();
     *total = res;
@@ -409,8 +407,8 @@ extern "C" int otm_barycenter_loss(otm_context* ctx, int n, int count, const dou
     // mesh (later dL/dI), dL/dF, first hits; then the blend, its gradient, image, target,
     // g, partials, scalars, blend pointers and weights
     const size_t per = al(N) * 3 + al(V2) * 3 + al((V + 1) / 2);
-    DevBuf buf;
-    buf.reserve(sizeof(double) * (per * count + al(V2) * 2 + al(pix) * 3 + al(2 * nparts) + al(64) + al(8) * 2));
+    AsyncBuf buf;
+    buf.reserve(sizeof(double) * (per * count + al(V2) * 2 + al(pix) * 3 + al(2 * nparts) + al(64) + al(8) * 2), st, ctx->pool);
     double* p = buf.as<double>();
     auto take = [&](size_t w) {
       double* r = p;

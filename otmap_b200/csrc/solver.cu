@@ -1204,10 +1204,8 @@ extern "C" int otm_solve_batch(otm_context* ctx, int count, const int* ns, const
       ctx->launches++;
       k_forward_mesh<<<(unsigned)((V + 255) / 256), 256, 0, ctx->side>>>((const Inst*)d_insts, q, dst);
       OTM_CUDA(cudaGetLastError());
-      if (!dev) OTM_CUDA(cudaMemcpyAsync(fwd_xy[q], dst, sizeof(double) * 2 * V, cudaMemcpyDefault, ctx->side));
-      if (adjusted && adjusted[q])
-        OTM_CUDA(cudaMemcpyAsync(adjusted[q], h[q].rho, sizeof(double) * (size_t)n * n, cudaMemcpyDefault,
-                                 ctx->side));
+      if (!dev) copy_out(ctx, fwd_xy[q], dst, sizeof(double) * 2 * V, ctx->side);
+      if (adjusted && adjusted[q]) copy_out(ctx, adjusted[q], h[q].rho, sizeof(double) * (size_t)n * n, ctx->side);
     };
     if (early) {
       if (!ctx->side) OTM_CUDA(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
