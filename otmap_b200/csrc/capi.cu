@@ -14,6 +14,11 @@ void set_error(const std::string& msg) { g_last_error = msg; }
 
 void make_current(otm_context* ctx) { OTM_CUDA(cudaSetDevice(ctx->device)); }
 
+void side_stream(otm_context* ctx) {
+  if (!ctx->side) OTM_CUDA(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+  if (!ctx->side_ready) OTM_CUDA(cudaEventCreateWithFlags(&ctx->side_ready, cudaEventDisableTiming));
+}
+
 int Profiler::id(const char* name) {
   for (size_t k = 0; k < names.size(); ++k)
     if (std::strcmp(names[k], name) == 0) return (int)k;

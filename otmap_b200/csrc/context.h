@@ -169,10 +169,11 @@ struct otm_context {
   otm::DevBuf staging;  // device staging for host inputs/outputs
   std::unique_ptr<otm::HostCopier, otm::HostCopierDelete> copier;
   bool copier_failed = false;
-  // second stream of a batched solve: outputs of instances that stopped while the rest of
-  // the batch iterates (created on first use), its staging and a pinned copy of the records
+  // second stream (created on first use): in a batched solve outputs of instances that stopped
+  // while the rest of the batch iterates, with its staging and a pinned copy of the records;
+  // in a locator build the bins
   cudaStream_t side = nullptr;
-  cudaEvent_t side_ready = nullptr;  // the batch's records are initialised (set-up kernels done)
+  cudaEvent_t side_ready = nullptr;  // order between the two streams
   otm::DevBuf staging_side;
   void* h_poll = nullptr;
   size_t h_poll_bytes = 0;
@@ -222,6 +223,8 @@ struct otm_map {
 namespace otm {
 // Makes the context's device current; defined in capi.cu.
 void make_current(otm_context* ctx);
+// Creates the context's second stream and its event, once; defined in capi.cu.
+void side_stream(otm_context* ctx);
 // Copies `bytes` from src (host or device) into dst (device), on the context stream; host
 // memory has been read when the call returns.
 void copy_in(otm_context* ctx, void* dst, const void* src, size_t bytes);

@@ -13,6 +13,7 @@
 
 #include <algorithm>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -92,7 +93,7 @@ __device__ __forceinline__ Verdict ratio_verdict(double num, double den) {
   const double a = fabs(num), b = fabs(den), low = b * 1e-7;
   const bool same = (__double2hiint(num) ^ __double2hiint(den)) >= 0;
   const bool above = a > low;
-  return {same & above & (a < b * (1. - 1e-7)), (a > b * (1. + 1e-7)) | (!same & above)};
+  return {bool(same & above & (a < b * (1. - 1e-7))), bool((a > b * (1. + 1e-7)) | (!same & above))};
 }
 __device__ __forceinline__ int bilinear_verdict(const Bilinear& t) {
   // |A| within `zero` makes the ratio an exact 0: on the border, computed
@@ -164,61 +165,101 @@ __device__ __forceinline__ void load_quad(const double* xy, int n, int f, Quad& 
   }
 }
 
-// ---- exclusive scan of int counts (three passes) ----
+// ---- exclusive scan of int counts ----
+//
+// Chunks of SCAN_B values: a block scans one (four values per thread, warp shuffles), one
+// block scans the chunks' sums, and a value's prefix is its chunk-local one plus its chunk's.
 
-constexpr int SCAN_B = 1024;
+constexpr int SCAN_B = 1024, SCAN_T = SCAN_B / 4;
 
-__global__ void k_scan_local(const int* in, int* out, int* block_sums, int count) {
-  __shared__ int s[SCAN_B];
-  int g = blockIdx.x * SCAN_B + threadIdx.x;
-  int v = g < count ? in[g] : 0;
-  s[threadIdx.x] = v;
+// Exclusive prefix of v over the block (a multiple of 32 threads, at most 1024); *total its sum.
+// warp_total: 32 ints of shared memory, free for reuse after the next barrier.
+__device__ __forceinline__ int block_prefix(int v, int* warp_total, int* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  int s = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, s, o);
+    if (lane >= o) s += u;
+  }
+  if (lane == 31) warp_total[warp] = s;
   __syncthreads();
-  for (int off = 1; off < SCAN_B; off <<= 1) {
-    int t = threadIdx.x >= off ? s[threadIdx.x - off] : 0;
-    __syncthreads();
-    s[threadIdx.x] += t;
-    __syncthreads();
+  int w = lane < nw ? warp_total[lane] : 0;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, w, o);
+    if (lane >= o) w += u;
   }
-  if (g < count) out[g] = s[threadIdx.x] - v;
-  if (threadIdx.x == SCAN_B - 1) block_sums[blockIdx.x] = s[threadIdx.x];
+  *total = __shfl_sync(0xffffffffu, w, 31);
+  const int before = __shfl_sync(0xffffffffu, w, (warp + 31) & 31);
+  return (warp ? before : 0) + s - v;
 }
 
-// Scans the block sums in place (one block of SCAN_B threads, chunks of SCAN_B values
-// with a running carry) and writes the grand total to out[count].
-__global__ void k_scan_sums(int* block_sums, int nblocks, int* out, int count) {
-  __shared__ int s[SCAN_B];
-  __shared__ int carry;
-  if (threadIdx.x == 0) carry = 0;
-  for (int c0 = 0; c0 < nblocks; c0 += SCAN_B) {
-    const int g = c0 + threadIdx.x;
-    const int v = g < nblocks ? block_sums[g] : 0;
-    s[threadIdx.x] = v;
-    __syncthreads();
-    for (int off = 1; off < SCAN_B; off <<= 1) {
-      int t = threadIdx.x >= off ? s[threadIdx.x - off] : 0;
-      __syncthreads();
-      s[threadIdx.x] += t;
-      __syncthreads();
+// Chunk-local prefixes of a chunk's values v[k] = value(4 t + k of the chunk).
+template <class F>
+__device__ __forceinline__ void scan_chunk(F value, int* out, int* sums, int count) {
+  __shared__ int warp_total[32];
+  const int g = blockIdx.x * SCAN_B + threadIdx.x * 4;
+  int v[4], t = 0, total;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    v[k] = g + k < count ? value(g + k) : 0;
+    t += v[k];
+  }
+  int p = block_prefix(t, warp_total, &total);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (g + k < count) out[g + k] = p;
+    p += v[k];
+  }
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+__global__ __launch_bounds__(SCAN_T) void k_scan_local(const int* in, int* out, int* sums, int count) {
+  scan_chunk([&](int i) { return in[i]; }, out, sums, count);
+}
+
+// The chunk sums' prefixes in place, one block of 1024 threads; returns the grand total.
+__device__ __forceinline__ int scan_sums(int* sums, int n) {
+  __shared__ int warp_total[32];
+  int carry = 0;
+  for (int c0 = 0; c0 < n; c0 += 4096) {
+    const int g = c0 + threadIdx.x * 4;
+    int v[4], t = 0, total;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[k] = g + k < n ? sums[g + k] : 0;
+      t += v[k];
     }
-    if (g < nblocks) block_sums[g] = carry + s[threadIdx.x] - v;
-    __syncthreads();
-    if (threadIdx.x == SCAN_B - 1) carry += s[threadIdx.x];
+    int p = carry + block_prefix(t, warp_total, &total);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (g + k < n) sums[g + k] = p;
+      p += v[k];
+    }
+    carry += total;
     __syncthreads();
   }
-  if (threadIdx.x == 0) out[count] = carry;
+  return carry;
 }
 
-__global__ void k_scan_add(int* out, const int* block_sums, int count) {
-  int g = blockIdx.x * SCAN_B + threadIdx.x;
-  if (g < count) out[g] += block_sums[blockIdx.x];
+__global__ __launch_bounds__(1024) void k_scan_sums(int* sums, int nblocks, int* out, int count) {
+  const int total = scan_sums(sums, nblocks);
+  if (threadIdx.x == 0) out[count] = total;
+}
+
+__global__ __launch_bounds__(SCAN_T) void k_scan_add(int* out, const int* sums, int count) {
+  const int g = blockIdx.x * SCAN_B + threadIdx.x * 4, add = sums[blockIdx.x];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (g + k < count) out[g + k] += add;
 }
 
 static void exclusive_scan(cudaStream_t st, const int* counts, int* starts, int* block_sums, int count) {
   int nb = (count + SCAN_B - 1) / SCAN_B;
-  k_scan_local<<<nb, SCAN_B, 0, st>>>(counts, starts, block_sums, count);
-  k_scan_sums<<<1, SCAN_B, 0, st>>>(block_sums, nb, starts, count);
-  k_scan_add<<<nb, SCAN_B, 0, st>>>(starts, block_sums, count);
+  k_scan_local<<<nb, SCAN_T, 0, st>>>(counts, starts, block_sums, count);
+  k_scan_sums<<<1, 1024, 0, st>>>(block_sums, nb, starts, count);
+  k_scan_add<<<nb, SCAN_T, 0, st>>>(starts, block_sums, count);
 }
 
 // ---- the reference's BVH face order (utils/bvh2d.cpp:29-64, 165-242) ----
@@ -242,17 +283,40 @@ static void exclusive_scan(cudaStream_t st, const int* counts, int* starts, int*
 //     loop exit that skips the final scan (last swap at start + S - 2 and start + S);
 //   * leaves: <= 4 faces, level >= 24, or a split that leaves one side empty.
 // Result per face: rank (position in the final face array) and the box of its leaf.
+//
+// The build runs in two phases. Nodes of more than BVH_SUB faces are split level by level
+// over the whole array, five kernels a level in the body of a WHILE node, windows of
+// positions without such a node passed over; a node of at most BVH_SUB faces is set aside
+// with its level. Only the face order moves (4 bytes a face); centroids and boxes are read
+// where they lie. Then each block takes the subtrees that start in its window of BVH_SUB
+// positions through all their remaining levels in shared memory. All 25 levels over the whole
+// array, nine kernels and two copies each and 52 bytes moved a face, took 1.73 ms for a
+// 1024^2 map, nearly all of it in passes over positions whose nodes were small. Now 0.74 ms go to the 20
+// levels of the first phase (bound by launches and by the dependent loads of each kernel: 37
+// us a level where the 20 MB it moves would take 4) and 0.25 ms to the second (bound by
+// its barriers; 512 threads on subtrees of up to 512 faces measured best among 128 .. 512 and
+// 128 .. 1024).
 
-constexpr int BVH_LEAF = 4, BVH_DEPTH = 24;
+constexpr int BVH_LEAF = 4, BVH_DEPTH = 24, BVH_SUB = 512;
 
-struct BvhNode {
+struct BvhNode {  // a node of more than BVH_SUB faces
   int start, end;
-  int leaf, dim;
-  float sv;
-  int mid, lo, hi;
+  int leaf, mid;
+  int lo, hi;  // children in the next level's list, or -1: set aside
   unsigned long long kmin[2], kmax[2];  // order-preserving keys of the box (atomics)
-  double box[4];                        // enlarged box: min x, min y, max x, max y
 };
+
+// State of a build: its buffers (set for each build) and the level being split.
+struct BvhCtl {
+  const double* xy;
+  int* rank;
+  double4* lbox;
+  int level;
+};
+
+// node_of of a position: the node's index in its level's list; ~start once its node has been
+// set aside; BVH_DONE when the face's leaf is recorded.
+constexpr int BVH_DONE = INT_MIN;
 
 __device__ __forceinline__ unsigned long long dkey(double x) {
   unsigned long long u = (unsigned long long)__double_as_longlong(x);
@@ -272,47 +336,59 @@ __device__ __forceinline__ void bvh_node_init(BvhNode& b, int start, int end) {
   b.kmax[0] = b.kmax[1] = 0ull;
 }
 
-// Face centroids (bvh2d.cpp:44-58: zero + the corners in circulator order, / 4), face
-// boxes, identity permutation, every position in the root node.
-__global__ void k_bvh_init(const double* xy, int n, int* fac, double2* cen, double4* fbox, int* node_of,
-                           BvhNode* root, int* counts) {
-  const int N = n * n;
-  int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f == 0) {
-    bvh_node_init(*root, 0, N);
-    counts[0] = 1;  // one node in the first level's list
-    counts[1] = 0;
-  }
-  if (f >= N) return;
-  Quad p;
-  int vid[4];
-  load_quad(xy, n, f, p, vid);
-  double cx = 0.0, cy = 0.0;
+// Enlarged box, split dimension and value of a node from the box of its faces (bvh2d.cpp:178-212).
+struct BvhSplit {
+  double4 box;  // min x, min y, max x, max y
+  int dim;
+  double sv;  // a float's value
+};
+__device__ __forceinline__ BvhSplit bvh_split(const double4& b) {
+  const double mn[2] = {b.x, b.y}, mx[2] = {b.z, b.w};
+  double diag[2], lo[2], hi[2];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    cx += p.x[k];
-    cy += p.y[k];
+  for (int c = 0; c < 2; ++c) {
+    diag[c] = mx[c] - mn[c];
+    const double en = diag[c] * (2. * DBL_EPSILON) + DBL_EPSILON;
+    lo[c] = mn[c] - en;
+    hi[c] = mx[c] + en;
   }
-  cen[f] = make_double2(cx / 4, cy / 4);
-  fbox[f] = make_double4(fmin(fmin(p.x[0], p.x[1]), fmin(p.x[2], p.x[3])),
-                         fmin(fmin(p.y[0], p.y[1]), fmin(p.y[2], p.y[3])),
-                         fmax(fmax(p.x[0], p.x[1]), fmax(p.x[2], p.x[3])),
-                         fmax(fmax(p.y[0], p.y[1]), fmax(p.y[2], p.y[3])));
-  fac[f] = f;
-  node_of[f] = 0;
+  BvhSplit r;
+  r.box = make_double4(lo[0], lo[1], hi[0], hi[1]);
+  r.dim = diag[1] > diag[0] ? 1 : 0;  // Eigen's maxCoeff: the first of equal maxima
+  r.sv = (double)(float)(0.5 * (r.dim ? hi[1] + lo[1] : hi[0] + lo[0]));
+  return r;
+}
+__device__ __forceinline__ BvhSplit bvh_split(const BvhNode& nd) {
+  return bvh_split(make_double4(dkey_inv(nd.kmin[0]), dkey_inv(nd.kmin[1]), dkey_inv(nd.kmax[0]), dkey_inv(nd.kmax[1])));
 }
 
-// Node boxes: per position its face box folded into its node's with 64-bit atomics on
-// order-preserving keys. A node's positions are contiguous, so a block whose 256
-// positions all belong to one node (the upper levels) reduces them first and issues one
-// set of atomics; otherwise every warp reduces each run of equal nodes with a segmented
-// shuffle scan and the last lane of a run issues its atomics.
+// split()'s return value (bvh2d.cpp:175) for a node [start, end) with S small centroids: q =
+// start + S, m swapped pairs, eq: the element now at q equals the split value, last: the last
+// pair's positions were q - 2 and q (the loop then exits right after its last swap without
+// the final scan: it tests the small element at q - 1 and returns q).
+__device__ __forceinline__ int bvh_mid(int q, int m, bool eq, bool last) { return q + (eq && !(m >= 1 && last) ? 1 : 0); }
+
+// Boxes hold no NaN (box_of_quad), so a comparison and a selection serve.
 __device__ __forceinline__ double4 box_join(double4 a, double4 b) {
-  return make_double4(fmin(a.x, b.x), fmin(a.y, b.y), fmax(a.z, b.z), fmax(a.w, b.w));
+  return make_double4(b.x < a.x ? b.x : a.x, b.y < a.y ? b.y : a.y, b.z > a.z ? b.z : a.z, b.w > a.w ? b.w : a.w);
+}
+__device__ __forceinline__ double4 box_shfl_xor(double4 b, int o, unsigned lanes = 0xffffffffu) {
+  return make_double4(__shfl_xor_sync(lanes, b.x, o), __shfl_xor_sync(lanes, b.y, o), __shfl_xor_sync(lanes, b.z, o),
+                      __shfl_xor_sync(lanes, b.w, o));
 }
 __device__ __forceinline__ double4 box_shfl_up(double4 b, int o) {
   return make_double4(__shfl_up_sync(0xffffffffu, b.x, o), __shfl_up_sync(0xffffffffu, b.y, o),
                       __shfl_up_sync(0xffffffffu, b.z, o), __shfl_up_sync(0xffffffffu, b.w, o));
+}
+__device__ __forceinline__ double4 box_none() { return make_double4(INFINITY, INFINITY, -INFINITY, -INFINITY); }
+// Box of a face's corners, NaN coordinates passed over (all of them: the empty box).
+__device__ __forceinline__ double4 box_of_quad(const Quad& p) {
+  const double4 b = make_double4(fmin(fmin(p.x[0], p.x[1]), fmin(p.x[2], p.x[3])),
+                                 fmin(fmin(p.y[0], p.y[1]), fmin(p.y[2], p.y[3])),
+                                 fmax(fmax(p.x[0], p.x[1]), fmax(p.x[2], p.x[3])),
+                                 fmax(fmax(p.y[0], p.y[1]), fmax(p.y[2], p.y[3])));
+  const bool x = b.x == b.x, y = b.y == b.y;
+  return make_double4(x ? b.x : INFINITY, y ? b.y : INFINITY, x ? b.z : -INFINITY, y ? b.w : -INFINITY);
 }
 __device__ __forceinline__ void box_atomic(BvhNode& nd, const double4& b) {
   atomicMin(&nd.kmin[0], dkey(b.x));
@@ -321,244 +397,576 @@ __device__ __forceinline__ void box_atomic(BvhNode& nd, const double4& b) {
   atomicMax(&nd.kmax[1], dkey(b.w));
 }
 
-constexpr int BBOX_T = 256;
+// A block's window of the array: BVH_PER positions per thread, BVH_BT apart.
+constexpr int BVH_BT = 256, BVH_PER = SCAN_B / BVH_BT;
 
-__global__ __launch_bounds__(BBOX_T) void k_bvh_bbox(int N, const int* node_of, const double4* fbox, BvhNode* nodes) {
+// Folds the boxes of the window's positions (id: their nodes, -1 for none) into the nodes with
+// 64-bit atomics on order-preserving keys. A node's positions are contiguous: a window that
+// lies in one node (the upper levels) is reduced first and issues one set of atomics;
+// otherwise every warp folds each run of equal nodes with a segmented shuffle scan and the
+// last lane of a run issues its atomics. Returns whether the window has any node. All threads
+// call it.
+__device__ __forceinline__ bool window_boxes(BvhNode* nodes, const int (&id)[BVH_PER], double4 (&box)[BVH_PER]) {
   __shared__ int s_first;
-  __shared__ double4 s_box[BBOX_T / 32];
-  const int p = blockIdx.x * BBOX_T + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int k = p < N ? node_of[p] : -1;
-  double4 b = k >= 0 ? fbox[p] : make_double4(0, 0, 0, 0);
-  if (threadIdx.x == 0) s_first = k;
-  __syncthreads();
-  const int first = s_first;
-  if (__syncthreads_and(k == first)) {  // one node (or only finished positions) in the block
-    if (first < 0) return;
+  __shared__ double4 s_box[BVH_BT / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  bool same = true, some = false;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      b.x = fmin(b.x, __shfl_xor_sync(0xffffffffu, b.x, o));
-      b.y = fmin(b.y, __shfl_xor_sync(0xffffffffu, b.y, o));
-      b.z = fmax(b.z, __shfl_xor_sync(0xffffffffu, b.z, o));
-      b.w = fmax(b.w, __shfl_xor_sync(0xffffffffu, b.w, o));
-    }
+  for (int j = 0; j < BVH_PER; ++j) {
+    same = same && id[j] == id[0];
+    some = some || id[j] >= 0;
+  }
+  if (threadIdx.x == 0) s_first = id[0];
+  if (!__syncthreads_or(some)) return false;
+  const int first = s_first;
+  if (__syncthreads_and(same && id[0] == first)) {
+    double4 b = box_join(box_join(box[0], box[1]), box_join(box[2], box[3]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) b = box_join(b, box_shfl_xor(b, o));
     if (lane == 0) s_box[warp] = b;
     __syncthreads();
     if (threadIdx.x == 0) {
       double4 t = s_box[0];
 #pragma unroll
-      for (int w = 1; w < BBOX_T / 32; ++w) t = box_join(t, s_box[w]);
+      for (int w = 1; w < BVH_BT / 32; ++w) t = box_join(t, s_box[w]);
       box_atomic(nodes[first], t);
     }
-    return;
+    return true;
   }
-  // runs of equal node ids are contiguous: inclusive segmented scan over each run
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const double4 u = box_shfl_up(b, o);
-    const int ku = __shfl_up_sync(0xffffffffu, k, o);
-    if (lane >= o && ku == k) b = box_join(b, u);
+  for (int j = 0; j < BVH_PER; ++j) {
+    const int k = id[j];
+    if (!__any_sync(0xffffffffu, k >= 0)) continue;
+    double4 b = box[j];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double4 u = box_shfl_up(b, o);
+      const int ku = __shfl_up_sync(0xffffffffu, k, o);
+      if (lane >= o && ku == k) b = box_join(b, u);
+    }
+    const int kn = __shfl_down_sync(0xffffffffu, k, 1);
+    if (k >= 0 && (lane == 31 || kn != k)) box_atomic(nodes[k], b);
   }
-  const int kn = __shfl_down_sync(0xffffffffu, k, 1);
-  if (k >= 0 && (lane == 31 || kn != k)) box_atomic(nodes[k], b);
+  return true;
 }
 
-// Enlarged box, leaf test by size and depth, split dimension and value (bvh2d.cpp:178-212).
-__global__ void k_bvh_decide(BvhNode* nodes, const int* count, int level) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= *count) return;
-  BvhNode& nd = nodes[k];
-  const double mn[2] = {dkey_inv(nd.kmin[0]), dkey_inv(nd.kmin[1])};
-  const double mx[2] = {dkey_inv(nd.kmax[0]), dkey_inv(nd.kmax[1])};
-  double diag[2];
-#pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    diag[c] = mx[c] - mn[c];
-    const double en = diag[c] * (2. * DBL_EPSILON) + DBL_EPSILON;
-    nd.box[c] = mn[c] - en;
-    nd.box[2 + c] = mx[c] + en;
-  }
-  if (nd.end - nd.start <= BVH_LEAF || level >= BVH_DEPTH) {
-    nd.leaf = 1;
-    return;
-  }
-  nd.dim = diag[1] > diag[0] ? 1 : 0;  // Eigen's maxCoeff: the first of equal maxima
-  nd.sv = (float)(0.5 * (nd.box[2 + nd.dim] + nd.box[nd.dim]));
+__global__ void k_bvh_root(BvhCtl* ctl, int N, BvhNode* root, int* sub_end, unsigned char* sub_level) {
+  bvh_node_init(*root, 0, N);
+  ctl->level = 0;
+  sub_end[0] = N;
+  sub_level[0] = 0;
 }
 
-// small[p] = 1 when position p's centroid lies below its (splitting) node's value.
-__global__ void k_bvh_classify(int N, const int* node_of, const double2* cen, const BvhNode* nodes, int* small) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= N) return;
-  const int k = node_of[p];
-  int s = 0;
-  if (k >= 0 && !nodes[k].leaf) {
-    const double2 c = cen[p];
-    s = (nodes[k].dim ? c.y : c.x) < (double)nodes[k].sv ? 1 : 0;
+// Face centroids (bvh2d.cpp:44-58: zero + the corners in circulator order, / 4), face
+// boxes, identity permutation, every position in the root node with its box -- or, for a
+// mesh of at most BVH_SUB faces, the root set aside.
+__global__ __launch_bounds__(BVH_BT) void k_bvh_init(const BvhCtl* ctl, int n, int* fac, int* final_fac, double2* cen,
+                                                     double4* fbox, int* node_of, BvhNode* root,
+                                                     unsigned char* window) {
+  const int N = n * n;
+  const double* xy = ctl->xy;
+  int id[BVH_PER];
+  double4 box[BVH_PER];
+#pragma unroll
+  for (int j = 0; j < BVH_PER; ++j) {
+    const int f = (blockIdx.x * BVH_PER + j) * BVH_BT + threadIdx.x;
+    id[j] = -1;
+    box[j] = box_none();
+    if (f >= N) continue;
+    Quad p;
+    int vid[4];
+    load_quad(xy, n, f, p, vid);
+    double cx = 0.0, cy = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      cx += p.x[k];
+      cy += p.y[k];
+    }
+    cen[f] = make_double2(cx / 4, cy / 4);
+    box[j] = box_of_quad(p);
+    fbox[f] = box[j];
+    if (N > BVH_SUB) {
+      fac[f] = f;
+      node_of[f] = id[j] = 0;
+    } else {
+      final_fac[f] = f;
+      node_of[f] = ~0;
+    }
   }
-  small[p] = s;
+  const bool some = window_boxes(root, id, box);
+  if (threadIdx.x == 0) window[blockIdx.x] = some ? 1 : 0;
 }
+
+// small[p] = 1 when position p's centroid lies below its node's split value, and the window-
+// local prefix counts lpre (N + 1 of them; a window's first is 0 from the first level on).
+__global__ __launch_bounds__(SCAN_T) void k_bvh_classify(int N, const BvhCtl* ctl, const int* node_of, const int* fac0,
+                                                         const int* fac1, const double2* cen, const BvhNode* even,
+                                                         const BvhNode* odd, const unsigned char* window0,
+                                                         const unsigned char* window1, unsigned char* small, int* lpre,
+                                                         int* sums) {
+  const int level = ctl->level;
+  const bool at_end = (long)blockIdx.x * SCAN_B >= N;  // the window of p = N alone
+  if (level > 0 && (at_end || !(level & 1 ? window1 : window0)[blockIdx.x])) {
+    if (threadIdx.x == 0) sums[blockIdx.x] = 0;
+    return;
+  }
+  const BvhNode* nodes = level & 1 ? odd : even;
+  const int* fac = level & 1 ? fac1 : fac0;
+  int last = -1;
+  BvhSplit sp;
+  scan_chunk(
+      [&](int p) {
+        const int k = p < N ? node_of[p] : -1;
+        if (k < 0) return 0;
+        if (k != last) {
+          sp = bvh_split(nodes[k]);
+          last = k;
+        }
+        const double2 c = cen[fac[p]];
+        const int s = (sp.dim ? c.y : c.x) < sp.sv ? 1 : 0;
+        small[p] = (unsigned char)s;
+        return s;
+      },
+      lpre, sums, N + 1);
+}
+
+__global__ __launch_bounds__(1024) void k_bvh_sums(int* sums, int nsums) { scan_sums(sums, nsums); }
+
+// Small positions before p.
+struct BvhPrefix {
+  const int *lpre, *sums;
+  __device__ __forceinline__ int operator()(int p) const { return lpre[p] + sums[p / SCAN_B]; }
+};
 
 // The partition's pairs: big elements among the first S positions (rank from the left)
 // and small elements after them (rank from the right) record their positions by rank.
-__global__ void k_bvh_slots(int N, const int* node_of, const BvhNode* nodes, const int* small, const int* spre,
-                            int* slot_big, int* slot_small) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= N) return;
-  const int k = node_of[p];
-  if (k < 0 || nodes[k].leaf) return;
-  const int start = nodes[k].start, end = nodes[k].end;
-  const int S = spre[end] - spre[start], q = start + S;
-  if (!small[p] && p < q) {
-    slot_big[start + (p - start) - (spre[p] - spre[start])] = p;
-  } else if (small[p] && p >= q) {
-    slot_small[start + spre[end] - spre[p + 1]] = p;
+__global__ __launch_bounds__(BVH_BT) void k_bvh_slots(int N, const BvhCtl* ctl, const int* node_of,
+                                                      const BvhNode* even, const BvhNode* odd,
+                                                      const unsigned char* window0, const unsigned char* window1,
+                                                      const unsigned char* small, BvhPrefix pre, int* slot_big,
+                                                      int* slot_small) {
+  const int level = ctl->level;
+  if (!(level & 1 ? window1 : window0)[blockIdx.x]) return;
+#pragma unroll
+  for (int j = 0; j < BVH_PER; ++j) {
+    const int p = (blockIdx.x * BVH_PER + j) * BVH_BT + threadIdx.x, k = p < N ? node_of[p] : -1;
+    if (k < 0) continue;
+    const BvhNode& nd = (level & 1 ? odd : even)[k];
+    const int start = nd.start, before = pre(start), upto = pre(nd.end), q = start + upto - before;
+    if (!small[p] && p < q) {
+      slot_big[start + (p - start) - (pre(p) - before)] = p;
+    } else if (small[p] && p >= q) {
+      slot_small[start + upto - pre(p) - 1] = p;
+    }
   }
 }
 
-// Each big element among the first S positions swaps with its partner (one thread per
-// pair, so the swap is race-free).
-__global__ void k_bvh_swap(int N, const int* node_of, const BvhNode* nodes, const int* small, const int* spre,
-                           const int* slot_small, int* fac, double2* cen, double4* fbox) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= N) return;
-  const int k = node_of[p];
-  if (k < 0 || nodes[k].leaf || small[p]) return;
-  const int start = nodes[k].start, end = nodes[k].end;
-  const int S = spre[end] - spre[start];
-  if (p >= start + S) return;
-  const int r = slot_small[start + (p - start) - (spre[p] - spre[start])];
-  const int tf = fac[p];
-  fac[p] = fac[r];
-  fac[r] = tf;
-  const double2 tc = cen[p];
-  cen[p] = cen[r];
-  cen[r] = tc;
-  const double4 tb = fbox[p];
-  fbox[p] = fbox[r];
-  fbox[r] = tb;
+// Position whose element stands at p once the pairs have traded places.
+__device__ __forceinline__ int bvh_source(int p, int start, int before, int upto, int pre_p, bool small,
+                                          const int* slot_big, const int* slot_small) {
+  const int q = start + upto - before;
+  if (!small && p < q) return slot_small[start + (p - start) - (pre_p - before)];
+  if (small && p >= q) return slot_big[start + upto - pre_p - 1];
+  return p;
 }
 
-// split()'s return value (bvh2d.cpp:175), the no-improvement leaf test (:214-221) and
-// the children, appended to the next level's list.
-__global__ void k_bvh_children(BvhNode* nodes, const int* count, const int* spre, const int* slot_big,
-                               const int* slot_small, const double2* cen, BvhNode* next, int* next_count) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= *count) return;
-  BvhNode& nd = nodes[k];
-  if (nd.leaf) return;
-  const int start = nd.start, end = nd.end, len = end - start;
-  const int S = spre[end] - spre[start];
-  int mid;
-  if (S == len) {
-    mid = end;  // no big element: the loop runs to `end` and both branches give end
-  } else {
-    const int q = start + S;
-    const int m = S - (spre[q] - spre[start]);  // swapped pairs
-    const double2 c = cen[q];
-    int eq = (nd.dim ? c.y : c.x) == (double)nd.sv ? 1 : 0;
-    // the loop exits right after its last swap (at q - 2 and q) without the final scan:
-    // it then tests the small element at q - 1 and returns q
-    if (eq && m >= 1 && slot_big[start + m - 1] == q - 2 && slot_small[start + m - 1] == q) eq = 0;
-    mid = q + eq;
+// The leaf tests by depth and no improvement (:214-221), the children -- listed for the next
+// level or set aside -- the level count and the loop test (one block).
+__global__ __launch_bounds__(1024) void k_bvh_children(BvhCtl* ctl, int* counts, BvhNode* even, BvhNode* odd,
+                                                       const int* fac0, const int* fac1, const unsigned char* small,
+                                                       BvhPrefix pre, const int* slot_big, const int* slot_small,
+                                                       const double2* cen, int* sub_end, unsigned char* sub_level,
+                                                       cudaGraphConditionalHandle handle, int in_graph) {
+  __shared__ int s_next;
+  const int level = ctl->level, count = level ? counts[level & 1] : 1;
+  BvhNode* nodes = level & 1 ? odd : even;
+  BvhNode* next = level & 1 ? even : odd;
+  const int* fac = level & 1 ? fac1 : fac0;
+  if (threadIdx.x == 0) s_next = 0;
+  __syncthreads();
+  for (int k = threadIdx.x; k < count; k += blockDim.x) {
+    BvhNode& nd = nodes[k];
+    const int start = nd.start, end = nd.end;
+    if (level >= BVH_DEPTH) {
+      nd.leaf = 1;
+      continue;
+    }
+    const int before = pre(start), upto = pre(end), S = upto - before;
+    int mid = end;  // no big element: the loop runs to `end` and both branches give end
+    if (S != end - start) {
+      const BvhSplit sp = bvh_split(nd);
+      const int q = start + S, pre_q = pre(q), m = S - (pre_q - before);
+      const double2 c = cen[fac[bvh_source(q, start, before, upto, pre_q, small[q] != 0, slot_big, slot_small)]];
+      const bool last = m >= 1 && slot_big[start + m - 1] == q - 2 && slot_small[start + m - 1] == q;
+      mid = bvh_mid(q, m, (sp.dim ? c.y : c.x) == sp.sv, last);
+    }
+    nd.mid = mid;
+    if (mid == start || mid == end) {
+      nd.leaf = 1;
+      continue;
+    }
+    auto child = [&](int s, int e) {
+      if (e - s > BVH_SUB) {
+        const int c = atomicAdd(&s_next, 1);
+        bvh_node_init(next[c], s, e);
+        return c;
+      }
+      sub_end[s] = e;
+      sub_level[s] = (unsigned char)(level + 1);
+      return -1;
+    };
+    nd.lo = child(start, mid);
+    nd.hi = child(mid, end);
   }
-  nd.mid = mid;
-  if (mid == start || mid == end) {
-    nd.leaf = 1;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    ctl->level = level + 1;
+    counts[(level + 1) & 1] = s_next;
+    if (in_graph) cudaGraphSetConditional(handle, s_next > 0 ? 1u : 0u);
+  }
+}
+
+// End of a level: the pairs trade places and every position moves to its child -- or, where the
+// node became a leaf, records its face's rank and leaf box -- with the boxes of the next
+// level's nodes.
+__global__ __launch_bounds__(BVH_BT) void k_bvh_move(int N, const BvhCtl* ctl, int* node_of, int* fac0, int* fac1,
+                                                     int* final_fac, const double4* fbox, BvhNode* even, BvhNode* odd,
+                                                     unsigned char* window0, unsigned char* window1,
+                                                     const unsigned char* small, BvhPrefix pre, const int* slot_big,
+                                                     const int* slot_small) {
+  const int level = ctl->level - 1;  // k_bvh_children has counted it
+  unsigned char* to = level & 1 ? window0 : window1;
+  if (!(level & 1 ? window1 : window0)[blockIdx.x]) {
+    if (threadIdx.x == 0) to[blockIdx.x] = 0;
     return;
   }
-  const int c0 = atomicAdd(next_count, 2);
-  bvh_node_init(next[c0], start, mid);
-  bvh_node_init(next[c0 + 1], mid, end);
-  nd.lo = c0;
-  nd.hi = c0 + 1;
+  const BvhNode* nodes = level & 1 ? odd : even;
+  const int* from = level & 1 ? fac1 : fac0;
+  int* into = level & 1 ? fac0 : fac1;
+  int id[BVH_PER];
+  double4 box[BVH_PER];
+#pragma unroll
+  for (int j = 0; j < BVH_PER; ++j) {
+    const int p = (blockIdx.x * BVH_PER + j) * BVH_BT + threadIdx.x, k = p < N ? node_of[p] : -1;
+    id[j] = -1;
+    box[j] = box_none();
+    if (k < 0) continue;
+    const BvhNode& nd = nodes[k];
+    const int start = nd.start;
+    const int src = level >= BVH_DEPTH ? p
+                                       : bvh_source(p, start, pre(start), pre(nd.end), pre(p), small[p] != 0, slot_big,
+                                                    slot_small);
+    const int f = from[src];
+    if (nd.leaf) {
+      ctl->rank[f] = p;
+      ctl->lbox[f] = bvh_split(nd).box;
+      node_of[p] = BVH_DONE;
+      continue;
+    }
+    const bool low = p < nd.mid;
+    const int child = low ? nd.lo : nd.hi;
+    if (child >= 0) {
+      into[p] = f;
+      node_of[p] = id[j] = child;
+      box[j] = fbox[f];
+    } else {
+      final_fac[p] = f;
+      node_of[p] = ~(low ? start : nd.mid);
+    }
+  }
+  const bool some = window_boxes(level & 1 ? even : odd, id, box);
+  if (threadIdx.x == 0) to[blockIdx.x] = some ? 1 : 0;
 }
 
-// Positions of leaves are final: record rank and leaf box per face; the others move to
-// their child node.
-__global__ void k_bvh_assign(int N, int* node_of, const BvhNode* nodes, const int* fac, int* rank, double4* lbox) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= N) return;
-  const int k = node_of[p];
-  if (k < 0) return;
-  const BvhNode& nd = nodes[k];
-  if (nd.leaf) {
-    const int f = fac[p];
-    rank[f] = p;
-    lbox[f] = make_double4(nd.box[0], nd.box[1], nd.box[2], nd.box[3]);
-    node_of[p] = -1;
-  } else {
-    node_of[p] = p < nd.mid ? nd.lo : nd.hi;
+// Second phase: block b takes the subtrees set aside that start in positions
+// [b BVH_SUB, (b+1) BVH_SUB) -- at most 2 BVH_SUB - 1 positions -- through their remaining
+// levels, all nodes of a level at once as in the first phase, on a permutation in shared
+// memory. Nodes of at most BVH_LEAF faces are recorded when they appear. A node's box is folded
+// by eight lanes when it has at most SMALL_NODE faces, else by a warp.
+constexpr int SMALL_NODE = 64;
+constexpr int BVH_WIN = 2 * BVH_SUB, BVH_T = 512, BVH_NODES = BVH_WIN / (BVH_LEAF + 1) + 1;
+
+struct BvhWindow {
+  double4 fbox[BVH_WIN];                   // by original position
+  double2 cen[BVH_WIN];
+  BvhSplit split[BVH_NODES];
+  int face[BVH_WIN];
+  unsigned short perm[BVH_WIN];            // original position of the element at a position
+  unsigned short node[BVH_WIN];            // the position's node, or NONE
+  unsigned short pre[BVH_WIN + 1];         // small positions before it
+  unsigned short slot_big[BVH_WIN], slot_small[BVH_WIN];
+  unsigned char small[BVH_WIN];
+  struct Node {
+    unsigned short start, end, mid, lo, hi;
+    unsigned char level, leaf;
+  } nodes[2][BVH_NODES];
+  int warp_total[32], count, lo, hi;
+};
+
+__global__ __launch_bounds__(BVH_T) void k_bvh_subtrees(int N, const BvhCtl* ctl, const int* node_of,
+                                                        const int* final_fac, const double2* cen, const double4* fbox,
+                                                        const int* sub_end, const unsigned char* sub_level) {
+  extern __shared__ __align__(16) unsigned char s_window[];
+  BvhWindow& W = *reinterpret_cast<BvhWindow*>(s_window);
+  constexpr unsigned short NONE = 0xffff;
+  constexpr int PER = BVH_WIN / BVH_T;
+  int* rank = ctl->rank;
+  double4* lbox = ctl->lbox;
+  const int w0 = blockIdx.x * BVH_SUB, w1 = min(w0 + BVH_SUB, N), lane = threadIdx.x & 31;
+  // the window's subtrees: the first starts at the first position that is its node's start,
+  // the last ends where the node of the last position starting in the window ends
+  if (threadIdx.x == 0) {
+    W.lo = N;
+    W.hi = 0;
+    W.count = 0;
+  }
+  __syncthreads();
+  for (int p = w0 + threadIdx.x; p < w1; p += BVH_T)
+    if (node_of[p] == ~p) {
+      atomicMin(&W.lo, p);
+      atomicMax(&W.hi, sub_end[p]);
+    }
+  __syncthreads();
+  const int base = W.lo, M = W.hi - W.lo;
+  if (M <= 0) return;
+  // a node of at most BVH_LEAF faces: its box over them, ranks and leaf boxes (one thread)
+  auto box_of = [&](int s, int e, int step) {
+    double4 b = W.fbox[W.perm[s]];
+    for (int p = s + step; p < e; p += step) b = box_join(b, W.fbox[W.perm[p]]);
+    return b;
+  };
+  auto record_leaf = [&](int s, int e) {
+    const double4 b = bvh_split(box_of(s, e, 1)).box;
+    for (int p = s; p < e; ++p) {
+      const int f = W.face[W.perm[p]];
+      rank[f] = base + p;
+      lbox[f] = b;
+    }
+  };
+  // load; every start makes its node, then every position finds it (slot_big: node of a start)
+  for (int p = threadIdx.x; p < M; p += BVH_T) {
+    W.perm[p] = (unsigned short)p;
+    if (node_of[base + p] == BVH_DONE) continue;  // of a leaf between subtrees
+    const int f = final_fac[base + p];
+    W.face[p] = f;
+    W.cen[p] = cen[f];
+    W.fbox[p] = fbox[f];
+  }
+  __syncthreads();
+  for (int p = threadIdx.x; p < M; p += BVH_T) {
+    if (node_of[base + p] != ~(base + p)) continue;
+    const int e = sub_end[base + p] - base;
+    unsigned short id = NONE;
+    if (e - p <= BVH_LEAF) {
+      record_leaf(p, e);
+    } else {
+      id = (unsigned short)atomicAdd(&W.count, 1);
+      W.nodes[0][id] = {(unsigned short)p, (unsigned short)e, 0, 0, 0, sub_level[base + p], 0};
+    }
+    W.slot_big[p] = id;
+  }
+  __syncthreads();
+  for (int p = threadIdx.x; p < M; p += BVH_T) {
+    const int k = node_of[base + p];
+    W.node[p] = k == BVH_DONE ? NONE : W.slot_big[~k - base];
+  }
+  int count = W.count;
+  for (int par = 0; count > 0; par ^= 1) {
+    auto* nodes = W.nodes[par];
+    auto* next = W.nodes[par ^ 1];
+    __syncthreads();
+    if (threadIdx.x == 0) W.count = 0;
+    for (int k = threadIdx.x >> 3; k < count; k += BVH_T / 8) {
+      const int s = nodes[k].start + (lane & 7), e = nodes[k].end;
+      if (e - nodes[k].start > SMALL_NODE) continue;
+      double4 b = s < e ? box_of(s, e, 8) : box_none();
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) b = box_join(b, box_shfl_xor(b, o, 0xffu << (lane & 24)));
+      if ((lane & 7) == 0) W.split[k] = bvh_split(b);
+    }
+    for (int k = threadIdx.x >> 5; k < count; k += BVH_T / 32) {
+      const int s = nodes[k].start + lane, e = nodes[k].end;
+      if (e - nodes[k].start <= SMALL_NODE) continue;
+      double4 b = s < e ? box_of(s, e, 32) : box_none();
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) b = box_join(b, box_shfl_xor(b, o));
+      if (lane == 0) W.split[k] = bvh_split(b);
+    }
+    __syncthreads();
+    // classify and count: thread t takes positions PER t .. PER t + PER - 1
+    {
+      int v[PER], t = 0, total;
+#pragma unroll
+      for (int j = 0; j < PER; ++j) {
+        const int p = threadIdx.x * PER + j, k = p < M ? W.node[p] : NONE;
+        v[j] = 0;
+        if (k != NONE) {
+          const double2 c = W.cen[W.perm[p]];
+          v[j] = (W.split[k].dim ? c.y : c.x) < W.split[k].sv ? 1 : 0;
+          W.small[p] = (unsigned char)v[j];
+        }
+        t += v[j];
+      }
+      int x = block_prefix(t, W.warp_total, &total);
+#pragma unroll
+      for (int j = 0; j < PER; ++j) {
+        const int p = threadIdx.x * PER + j;
+        if (p < M) W.pre[p] = (unsigned short)x;
+        x += v[j];
+      }
+      if (threadIdx.x == 0) W.pre[M] = (unsigned short)total;
+    }
+    __syncthreads();
+    for (int p = threadIdx.x; p < M; p += BVH_T) {
+      const int k = W.node[p];
+      if (k == NONE) continue;
+      const int s = nodes[k].start, before = W.pre[s], upto = W.pre[nodes[k].end], q = s + upto - before;
+      if (!W.small[p] && p < q)
+        W.slot_big[s + (p - s) - (W.pre[p] - before)] = (unsigned short)p;
+      else if (W.small[p] && p >= q)
+        W.slot_small[s + upto - W.pre[p] - 1] = (unsigned short)p;
+    }
+    __syncthreads();
+    for (int p = threadIdx.x; p < M; p += BVH_T) {
+      const int k = W.node[p];
+      if (k == NONE || W.small[p] || nodes[k].level >= BVH_DEPTH) continue;
+      const int s = nodes[k].start, before = W.pre[s];
+      if (p >= s + W.pre[nodes[k].end] - before) continue;
+      const int r = W.slot_small[s + (p - s) - (W.pre[p] - before)];
+      const unsigned short t = W.perm[p];
+      W.perm[p] = W.perm[r];
+      W.perm[r] = t;
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < count; k += BVH_T) {
+      auto& nd = nodes[k];
+      const int s = nd.start, e = nd.end;
+      nd.leaf = 1;
+      if (nd.level >= BVH_DEPTH) continue;
+      const int before = W.pre[s], S = W.pre[e] - before;
+      int mid = e;
+      if (S != e - s) {
+        const int q = s + S, m = S - (W.pre[q] - before);
+        const double2 c = W.cen[W.perm[q]];
+        const bool last = m >= 1 && W.slot_big[s + m - 1] == q - 2 && W.slot_small[s + m - 1] == q;
+        mid = bvh_mid(q, m, (W.split[k].dim ? c.y : c.x) == W.split[k].sv, last);
+      }
+      if (mid == s || mid == e) continue;
+      nd.leaf = 0;
+      nd.mid = (unsigned short)mid;
+      auto child = [&](int cs, int ce) -> unsigned short {
+        if (ce - cs <= BVH_LEAF) return NONE;
+        const int c = atomicAdd(&W.count, 1);
+        next[c] = {(unsigned short)cs, (unsigned short)ce, 0, 0, 0, (unsigned char)(nd.level + 1), 0};
+        return (unsigned short)c;
+      };
+      nd.lo = child(s, mid);
+      nd.hi = child(mid, e);
+    }
+    __syncthreads();
+    for (int p = threadIdx.x; p < M; p += BVH_T) {
+      const int k = W.node[p];
+      if (k == NONE) continue;
+      const auto& nd = nodes[k];
+      if (nd.leaf) {
+        const int f = W.face[W.perm[p]];
+        rank[f] = base + p;
+        lbox[f] = W.split[k].box;
+        W.node[p] = NONE;
+      } else {
+        const bool low = p < nd.mid;
+        const unsigned short c = low ? nd.lo : nd.hi;
+        W.node[p] = c;
+        if (c == NONE && p == (low ? nd.start : nd.mid)) record_leaf(p, low ? nd.mid : nd.end);
+      }
+    }
+    count = W.count;
   }
 }
 
-// rank[f] and the leaf box of f for the n^2 quads of the forward mesh xy (device). The
-// levels are a fixed sequence of ~250 small launches for a given n: they run as one CUDA
-// graph per size (captured on first use, kept in the context), on the context's grow-only
-// scratch, with the mesh copied in and the results copied out around it -- a host that
-// enqueues launches slowly then costs one launch instead of ~250. With profiling on, the
-// same launches are issued one by one so that each is timed.
+// rank[f] and the leaf box of f for the n^2 quads of the forward mesh xy (device). The launches
+// run as one CUDA graph per size (captured on first use, kept in the context) on the
+// context's grow-only scratch; a build's own buffers reach it through the control block.
+// With profiling on, the same launches are issued one by one so that each is timed.
 static void build_bvh_order(otm_context* ctx, const double* xy, int n, int* rank, double4* lbox) {
   cudaStream_t st = ctx->stream;
   const int N = n * n;
-  const int cap = std::min(1 << BVH_DEPTH, 2 * (N / (BVH_LEAF + 1)) + 2);
+  const int cap = N / (BVH_SUB + 1) + 2;  // nodes of a level in the first phase
   auto al = [](size_t b) { return (b + 255) / 256 * 256; };
-  const int nsums = (N + 1 + SCAN_B - 1) / SCAN_B + 1;
-  const size_t b_fac = al(sizeof(int) * N), b_cen = al(sizeof(double2) * N), b_box = al(sizeof(double4) * N);
-  const size_t b_int = al(sizeof(int) * (N + 1)), b_nodes = al(sizeof(BvhNode) * cap), b_sums = al(sizeof(int) * nsums);
-  const size_t b_xy = al(sizeof(double) * 2 * (size_t)(n + 1) * (n + 1));
+  const int windows = (N + SCAN_B - 1) / SCAN_B, nsums = N / SCAN_B + 1;
+  const size_t b_int = al(sizeof(int) * ((size_t)N + 1)), b_byte = al((size_t)N), b_nodes = al(sizeof(BvhNode) * cap);
+  const size_t b_cen = al(sizeof(double2) * N), b_box = al(sizeof(double4) * N), b_sums = al(sizeof(int) * nsums);
+  const size_t b_win = al((size_t)windows);
   DevBuf& buf = ctx->bvh_scratch;  // grow-only: no allocation once a size has been built
-  buf.reserve(b_fac + b_cen + 2 * b_box + 5 * b_int + 2 * b_nodes + b_sums + b_xy + b_fac + 256);
+  buf.reserve(8 * b_int + 2 * b_byte + b_cen + b_box + 2 * b_nodes + b_sums + 2 * b_win + 256);
   char* q = buf.as<char>();
   auto take = [&](size_t b) {
     char* r = q;
     q += b;
     return r;
   };
-  int* fac = reinterpret_cast<int*>(take(b_fac));
+  BvhCtl* ctl = reinterpret_cast<BvhCtl*>(take(256));
+  int* counts = reinterpret_cast<int*>(ctl + 1);  // nodes in the lists of even and odd levels
   double2* cen = reinterpret_cast<double2*>(take(b_cen));
   double4* fbox = reinterpret_cast<double4*>(take(b_box));
+  int* fac0 = reinterpret_cast<int*>(take(b_int));
+  int* fac1 = reinterpret_cast<int*>(take(b_int));
+  int* final_fac = reinterpret_cast<int*>(take(b_int));
   int* node_of = reinterpret_cast<int*>(take(b_int));
-  int* small = reinterpret_cast<int*>(take(b_int));
-  int* spre = reinterpret_cast<int*>(take(b_int));
+  int* lpre = reinterpret_cast<int*>(take(b_int));
   int* slot_big = reinterpret_cast<int*>(take(b_int));
   int* slot_small = reinterpret_cast<int*>(take(b_int));
-  BvhNode* lists[2] = {reinterpret_cast<BvhNode*>(take(b_nodes)), reinterpret_cast<BvhNode*>(take(b_nodes))};
+  int* sub_end = reinterpret_cast<int*>(take(b_int));
+  unsigned char* small = reinterpret_cast<unsigned char*>(take(b_byte));
+  unsigned char* sub_level = reinterpret_cast<unsigned char*>(take(b_byte));
+  BvhNode* even = reinterpret_cast<BvhNode*>(take(b_nodes));
+  BvhNode* odd = reinterpret_cast<BvhNode*>(take(b_nodes));
   int* sums = reinterpret_cast<int*>(take(b_sums));
-  int* counts = reinterpret_cast<int*>(take(256));  // node count of the current and next list
-  double* sxy = reinterpret_cast<double*>(take(b_xy));
-  int* srank = reinterpret_cast<int*>(take(b_fac));
-  double4* slbox = reinterpret_cast<double4*>(take(b_box));
-  auto levels = [&]() {
-    const unsigned ge = (unsigned)((N + 255) / 256);
-    launch(ctx, "bvh_init", k_bvh_init, ge, 256, (const double*)sxy, n, fac, cen, fbox, node_of, lists[0], counts);
-    for (int level = 0; level <= BVH_DEPTH; ++level) {
-      BvhNode* cur = lists[level & 1];
-      BvhNode* nxt = lists[(level + 1) & 1];
-      int* ccount = counts + (level & 1);
-      int* ncount = counts + ((level + 1) & 1);
-      const int ncap = std::min(level < 30 ? (1 << level) : cap, cap);
-      const unsigned gn = (unsigned)((ncap + 255) / 256);
-      OTM_CUDA(cudaMemsetAsync(ncount, 0, sizeof(int), st));
-      launch(ctx, "bvh_bbox", k_bvh_bbox, (unsigned)((N + BBOX_T - 1) / BBOX_T), BBOX_T, N, (const int*)node_of,
-             (const double4*)fbox, cur);
-      launch(ctx, "bvh_decide", k_bvh_decide, gn, 256, cur, (const int*)ccount, level);
-      launch(ctx, "bvh_classify", k_bvh_classify, ge, 256, N, (const int*)node_of, (const double2*)cen,
-             (const BvhNode*)cur, small);
-      exclusive_scan(st, small, spre, sums, N);
-      ctx->launches += 3;
-      launch(ctx, "bvh_slots", k_bvh_slots, ge, 256, N, (const int*)node_of, (const BvhNode*)cur, (const int*)small,
-             (const int*)spre, slot_big, slot_small);
-      launch(ctx, "bvh_swap", k_bvh_swap, ge, 256, N, (const int*)node_of, (const BvhNode*)cur, (const int*)small,
-             (const int*)spre, (const int*)slot_small, fac, cen, fbox);
-      launch(ctx, "bvh_children", k_bvh_children, gn, 256, cur, (const int*)ccount, (const int*)spre,
-             (const int*)slot_big, (const int*)slot_small, (const double2*)cen, nxt, ncount);
-      launch(ctx, "bvh_assign", k_bvh_assign, ge, 256, N, node_of, (const BvhNode*)cur, (const int*)fac, srank,
-             slbox);
-    }
+  unsigned char* win0 = reinterpret_cast<unsigned char*>(take(b_win));
+  unsigned char* win1 = reinterpret_cast<unsigned char*>(take(b_win));
+  const BvhPrefix pre{lpre, sums};
+  using CBytes = const unsigned char*;
+  auto level = [&](cudaGraphConditionalHandle handle, int in_graph) {
+    launch(ctx, "bvh_classify", k_bvh_classify, nsums, SCAN_T, N, (const BvhCtl*)ctl, (const int*)node_of,
+           (const int*)fac0, (const int*)fac1, (const double2*)cen, (const BvhNode*)even, (const BvhNode*)odd,
+           (CBytes)win0, (CBytes)win1, small, lpre, sums);
+    launch(ctx, "bvh_sums", k_bvh_sums, 1, 1024, sums, nsums);
+    launch(ctx, "bvh_slots", k_bvh_slots, windows, BVH_BT, N, (const BvhCtl*)ctl, (const int*)node_of,
+           (const BvhNode*)even, (const BvhNode*)odd, (CBytes)win0, (CBytes)win1, (CBytes)small, pre, slot_big,
+           slot_small);
+    launch(ctx, "bvh_children", k_bvh_children, 1, 1024, ctl, counts, even, odd, (const int*)fac0, (const int*)fac1,
+           (CBytes)small, pre, (const int*)slot_big, (const int*)slot_small, (const double2*)cen, sub_end, sub_level,
+           handle, in_graph);
+    launch(ctx, "bvh_move", k_bvh_move, windows, BVH_BT, N, (const BvhCtl*)ctl, node_of, fac0, fac1, final_fac,
+           (const double4*)fbox, even, odd, win0, win1, (CBytes)small, pre, (const int*)slot_big,
+           (const int*)slot_small);
   };
-  OTM_CUDA(cudaMemcpyAsync(sxy, xy, sizeof(double) * 2 * (size_t)(n + 1) * (n + 1), cudaMemcpyDeviceToDevice, st));
+  auto begin = [&] {
+    launch(ctx, "bvh_root", k_bvh_root, 1, 1, ctl, N, even, sub_end, sub_level);
+    launch(ctx, "bvh_init", k_bvh_init, windows, BVH_BT, (const BvhCtl*)ctl, n, fac0, final_fac, cen, fbox, node_of,
+           even, win0);
+  };
+  auto finish = [&] {
+    launch_smem(ctx, "bvh_subtrees", k_bvh_subtrees, (unsigned)((N + BVH_SUB - 1) / BVH_SUB), BVH_T, sizeof(BvhWindow),
+                N, (const BvhCtl*)ctl, (const int*)node_of, (const int*)final_fac, (const double2*)cen,
+                (const double4*)fbox, (const int*)sub_end, (CBytes)sub_level);
+  };
+  static bool attr[64] = {};  // per device ordinal
+  if (ctx->device >= 64 || !attr[ctx->device]) {
+    OTM_CUDA(cudaFuncSetAttribute(k_bvh_subtrees, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BvhWindow)));
+    if (ctx->device < 64) attr[ctx->device] = true;
+  }
+  BvhCtl h = {xy, rank, lbox, 0};
+  OTM_CUDA(cudaMemcpyAsync(ctl, &h, sizeof(h), cudaMemcpyHostToDevice, st));
   if (ctx->prof.on) {
-    levels();
+    begin();
+    int left[2] = {1, 1};
+    for (int l = 0; N > BVH_SUB && left[l & 1]; ++l) {
+      level((cudaGraphConditionalHandle)0, 0);
+      OTM_CUDA(cudaMemcpyAsync(left, counts, sizeof(left), cudaMemcpyDeviceToHost, st));
+      OTM_CUDA(cudaStreamSynchronize(st));
+    }
+    finish();
   } else {
     auto& slot = ctx->bvh_graphs[n];
     if (!slot || slot->base != buf.p) {
@@ -566,27 +974,64 @@ static void build_bvh_order(otm_context* ctx, const double* xy, int n, int* rank
       slot->base = buf.p;
       cudaGraph_t g = nullptr;
       const long before = ctx->launches;
-      OTM_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+      OTM_CUDA(cudaGraphCreate(&g, 0));
+      auto capture = [&](cudaGraph_t to, const cudaGraphNode_t* after, auto&& body) {
+        cudaGraph_t done = nullptr;
+        OTM_CUDA(cudaStreamBeginCaptureToGraph(st, to, after, nullptr, after ? 1 : 0, cudaStreamCaptureModeThreadLocal));
+        try {
+          body();
+        } catch (...) {
+          cudaStreamEndCapture(st, &done);
+          throw;
+        }
+        OTM_CUDA(cudaStreamEndCapture(st, &done));
+      };
       try {
-        levels();
+        // begin and finish around the loop: child graphs, so that each is one node
+        cudaGraph_t part = nullptr;
+        cudaGraphNode_t last;
+        auto add_part = [&](const cudaGraphNode_t* after, auto&& body) {
+          OTM_CUDA(cudaGraphCreate(&part, 0));
+          capture(part, nullptr, body);
+          OTM_CUDA(cudaGraphAddChildGraphNode(&last, g, after, after ? 1 : 0, part));
+          cudaGraphDestroy(part);
+          part = nullptr;
+        };
+        try {
+          add_part(nullptr, begin);
+          if (N > BVH_SUB) {
+            cudaGraphConditionalHandle handle;
+            OTM_CUDA(cudaGraphConditionalHandleCreate(&handle, g, 1, cudaGraphCondAssignDefault));
+            cudaGraphNodeParams params = {};
+            params.type = cudaGraphNodeTypeConditional;
+            params.conditional.handle = handle;
+            params.conditional.type = cudaGraphCondTypeWhile;
+            params.conditional.size = 1;
+            cudaGraphNode_t loop;
+            OTM_CUDA(cudaGraphAddNode(&loop, g, &last, 1, &params));
+            capture(params.conditional.phGraph_out[0], nullptr, [&] { level(handle, 1); });
+            last = loop;
+          }
+          const cudaGraphNode_t after = last;
+          add_part(&after, finish);
+        } catch (...) {
+          if (part) cudaGraphDestroy(part);
+          throw;
+        }
+        slot->kernels = ctx->launches - before;
+        ctx->launches = before;  // captured, not executed
+        OTM_CUDA(cudaGraphInstantiate(&slot->exec, g, 0));
       } catch (...) {
-        cudaGraph_t dummy;
-        cudaStreamEndCapture(st, &dummy);
-        if (dummy) cudaGraphDestroy(dummy);
+        ctx->launches = before;
+        slot.reset();
+        cudaGraphDestroy(g);
         throw;
       }
-      OTM_CUDA(cudaStreamEndCapture(st, &g));
-      slot->kernels = ctx->launches - before;
-      ctx->launches = before;  // captured, not executed
-      const cudaError_t e = cudaGraphInstantiate(&slot->exec, g, 0);
       cudaGraphDestroy(g);
-      OTM_CUDA(e);
     }
     OTM_CUDA(cudaGraphLaunch(slot->exec, st));
-    ctx->launches += slot->kernels;
+    ctx->launches += slot->kernels;  // with one level: how many were taken stays on the device
   }
-  OTM_CUDA(cudaMemcpyAsync(rank, srank, sizeof(int) * N, cudaMemcpyDeviceToDevice, st));
-  OTM_CUDA(cudaMemcpyAsync(lbox, slbox, sizeof(double4) * N, cudaMemcpyDeviceToDevice, st));
   OTM_CUDA(cudaGetLastError());
 }
 
@@ -644,98 +1089,245 @@ __global__ void k_bin_fill(const double* xy, int n, int B, const int* starts, in
 
 constexpr int MAXHITS = 8;
 
-// inv_impl (transport_map.cpp:50-102) per point. A face of the point's bin is a hit
-// when the point lies in the box of the face's BVH leaf (the reference only reaches
-// faces through their leaf, bvh2d.cpp:148-161) and passes the face tests of
-// bvh2d.cpp:117-142; hits are ordered by the face's position in the reference's BVH face
-// array, its traversal order. With several hits the reference keeps the weights of its
-// first hit and the face of the densest later one (transport_map.cpp:70-85); the
-// first-hit mode (inv_fast, bvh2d.cpp:66-81) keeps the first.
-__global__ void k_inverse(const double* xy, const double* density, int n, int B, const int* starts,
-                          const int* faces, const double4* boxes, const int* rank, const double4* lbox, double* pts,
-                          long P, int first_hit, int* face_out, int* hit0_out, int* nhits_out,
-                          unsigned long long* missing) {
-  long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= P) return;
-  double qx = fmin(fmax(pts[2 * i], 0.), 1.);
-  double qy = fmin(fmax(pts[2 * i + 1], 0.), 1.);
-  if (!(qx == qx)) qx = 0.;  // NaN input: clamp like Eigen's max/min would not; keep it finite
-  if (!(qy == qy)) qy = 0.;
-  int bx = (int)fmin(floor(qx * (double)B), (double)(B - 1));
-  int by = (int)fmin(floor(qy * (double)B), (double)(B - 1));
-  int b = by * B + bx;
-  int hf[MAXHITS], hr[MAXHITS];
-  double hw[MAXHITS][4];
-  int nh = 0;
-  for (int k = starts[b]; k < starts[b + 1]; ++k) {
-    int f = faces[k];
-    double4 bb = boxes[f];
+// inside_tri's answer where it is certain without its two divisions: 1 inside, -1 outside, 0 to
+// be computed. The test's tolerance is 1e-8; a term 1e-7 beyond it decides (NaN decides nothing).
+__device__ __forceinline__ int tri_verdict(double qx, double qy, double p0x, double p0y, double p1x, double p1y,
+                                           double p2x, double p2y) {
+  const double q2x = qx - p2x, q2y = qy - p2y;
+  const double eux = p1x - p2x, euy = p1y - p2y;
+  const double evx = p0x - p2x, evy = p0y - p2y;
+  double area2 = cross2(evx, evy, eux, euy);
+  double u = cross2(q2x, q2y, eux, euy), v = cross2(evx, evy, q2x, q2y);
+  if (area2 < 0) {
+    area2 = -area2;
+    u = -u;
+    v = -v;
+  }
+  const double m = area2 * 1e-7, s = u + v;
+  if ((u < -m) | (v < -m) | (s > area2 + m)) return -1;
+  return (u > m) & (v > m) & (s < area2 - m) ? 1 : 0;
+}
+
+// Whether point (qx, qy) hits face p: the face tests of bvh2d.cpp:117-142 (inside_quad, then
+// the bilinear weights in [0, 1]), by the certain verdicts where they decide.
+__device__ __forceinline__ bool hits_face(double qx, double qy, const Quad& p) {
+  const int t0 = tri_verdict(qx, qy, p.x[0], p.y[0], p.x[1], p.y[1], p.x[2], p.y[2]);
+  if (t0 <= 0) {
+    const int t1 = tri_verdict(qx, qy, p.x[0], p.y[0], p.x[2], p.y[2], p.x[3], p.y[3]);
+    if (t1 <= 0 && (t0 < 0) & (t1 < 0)) return false;
+    if (t1 <= 0 && !inside_quad(qx, qy, p)) return false;
+  }
+  Bilinear t;
+  if (!bilinear_terms(qx, qy, p, t)) return false;
+  const int verdict = bilinear_verdict(t);
+  if (verdict != 0) return verdict > 0;
+  double w[4];
+  bilinear_from_terms(t, w);
+  return weights_inside(w);
+}
+
+// The locator's arrays (build_locator, build_bvh_order).
+struct Locator {
+  const double* xy;
+  const double* density;
+  int n, B;
+  const int* starts;
+  const int* faces;
+  const double4* boxes;
+  const int* rank;
+  const double4* lbox;
+};
+
+// The first hit's face and the chosen one for a point with more hits than a warp's lists hold:
+// a walk of its bin that keeps the first MAXHITS in the reference's order.
+__device__ __noinline__ int many_hits(const Locator& L, int b, double qx, double qy, int densest, int* first) {
+  int hf[MAXHITS], hr[MAXHITS], nh = 0;
+  for (int k = L.starts[b]; k < L.starts[b + 1]; ++k) {
+    const int f = L.faces[k];
+    const double4 bb = L.boxes[f];
     if (qx < bb.x || qx > bb.z || qy < bb.y || qy > bb.w) continue;
-    const double4 lb = lbox[f];
-    if (!(lb.x <= qx && lb.y <= qy && qx <= lb.z && qy <= lb.w)) continue;  // AlignedBox::contains
     Quad p;
     int vid[4];
-    load_quad(xy, n, f, p, vid);
-    double w[4];
-    if (!inside_quad(qx, qy, p)) continue;
-    if (!bilinear_weights(qx, qy, p, w)) continue;
-    if (!weights_inside(w)) continue;
-    // insertion in increasing BVH position
-    const int rk = rank[f];
+    load_quad(L.xy, L.n, f, p, vid);
+    if (!hits_face(qx, qy, p)) continue;
+    const double4 lb = L.lbox[f];
+    if (!(lb.x <= qx && lb.y <= qy && qx <= lb.z && qy <= lb.w)) continue;
+    const int rk = L.rank[f];
+    if (nh >= MAXHITS && rk > hr[MAXHITS - 1]) continue;
     int pos = nh < MAXHITS ? nh : MAXHITS - 1;
-    if (nh >= MAXHITS && rk > hr[MAXHITS - 1]) {
-      ++nh;
-      continue;
-    }
     while (pos > 0 && hr[pos - 1] > rk) {
       hf[pos] = hf[pos - 1];
       hr[pos] = hr[pos - 1];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) hw[pos][c] = hw[pos - 1][c];
       --pos;
     }
     hf[pos] = f;
     hr[pos] = rk;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) hw[pos][c] = w[c];
-    ++nh;
+    if (nh < MAXHITS) ++nh;
   }
+  *first = hf[0];
+  int f = hf[0];
+  double best = L.density[f];
+  for (int k = 1; densest && k < nh; ++k) {
+    const double dk = L.density[hf[k]];
+    if (dk > best) {
+      f = hf[k];
+      best = dk > best;
+    }
+  }
+  return f;
+}
+
+// inv_impl (transport_map.cpp:50-102) per point. A face of the point's bin is a hit when the
+// point lies in the box of the face's BVH leaf (the reference only reaches faces through
+// their leaf, bvh2d.cpp:148-161) and passes the face tests; hits are ordered by the face's
+// position in the reference's BVH face array, its traversal order. With several hits the
+// reference keeps the weights of its first hit and the face of the densest later one
+// (transport_map.cpp:70-85); the first-hit mode (inv_fast, bvh2d.cpp:66-81) keeps the first.
+//
+// The lengths of the points' face lists differ widely (4.6 faces a bin on average, 200 where a
+// map squeezes its mesh), so a warp pools the lists of its 32 points: the box tests of all of
+// them 32 at a time, the faces that pass queued, and the face tests 32 at a time. Bound by
+// the latency of the chains bin, face, box and corners, leaf box from L2. With a thread walking its
+// own point's list, ten lanes in 32 worked and 2^20 points on a 1024^2 map took 428 us; now 168.
+constexpr int INV_T = 128;
+
+struct InverseWarp {
+  double2 q[32];                          // the points
+  unsigned long long hit[32][MAXHITS];    // per point: rank << 32 | face
+  int hits[32];
+  int queue_face[64];
+  unsigned char queue_lane[64];
+};
+
+__global__ __launch_bounds__(INV_T) void k_inverse(Locator L, double* pts, long P, int first_hit, int* face_out,
+                                                   int* hit0_out, int* nhits_out, unsigned long long* missing) {
+  __shared__ InverseWarp s_warp[INV_T / 32];
+  InverseWarp& W = s_warp[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const long i = (long)blockIdx.x * INV_T + threadIdx.x;
+  const int n = L.n, B = L.B;
+  double qx = 0., qy = 0.;
+  int b = 0, begin = 0, count = 0;
+  if (i < P) {
+    qx = fmin(fmax(pts[2 * i], 0.), 1.);
+    qy = fmin(fmax(pts[2 * i + 1], 0.), 1.);
+    if (!(qx == qx)) qx = 0.;  // NaN input: clamp like Eigen's max/min would not; keep it finite
+    if (!(qy == qy)) qy = 0.;
+    const int bx = (int)fmin(floor(qx * (double)B), (double)(B - 1));
+    const int by = (int)fmin(floor(qy * (double)B), (double)(B - 1));
+    b = by * B + bx;
+    begin = L.starts[b];
+    count = L.starts[b + 1] - begin;
+  }
+  W.q[lane] = make_double2(qx, qy);
+  W.hits[lane] = 0;
+  int upto = count;  // inclusive prefix over the warp
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, upto, o);
+    if (lane >= o) upto += u;
+  }
+  const int total = __shfl_sync(0xffffffffu, upto, 31), shift = begin - (upto - count);
+  __syncwarp();
+  auto test = [&](int e) {  // queue entry e
+    const int f = W.queue_face[e], l = W.queue_lane[e];
+    const double2 q = W.q[l];
+    Quad p;
+    int vid[4];
+    load_quad(L.xy, n, f, p, vid);
+    const double4 lb = L.lbox[f];
+    if (!(lb.x <= q.x && lb.y <= q.y && q.x <= lb.z && q.y <= lb.w)) return;  // AlignedBox::contains
+    if (!hits_face(q.x, q.y, p)) return;
+    const int k = atomicAdd(&W.hits[l], 1);
+    if (k < MAXHITS) W.hit[l][k] = (unsigned long long)(unsigned)L.rank[f] << 32 | (unsigned)f;
+  };
+  int queued = 0;
+  for (int base = 0; base < total; base += 32) {
+    const int item = base + lane;
+    int l = 0;  // the point the item belongs to: the first lane with upto > item
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      if (__shfl_sync(0xffffffffu, upto, l + o - 1) <= item) l += o;
+    l = min(l, 31);
+    const int k = item + __shfl_sync(0xffffffffu, shift, l);
+    bool pass = false;
+    int f = 0;
+    if (item < total) {
+      f = L.faces[k];
+      const double4 bb = L.boxes[f];
+      const double2 q = W.q[l];
+      pass = !(q.x < bb.x || q.x > bb.z || q.y < bb.y || q.y > bb.w);
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, pass);
+    if (pass) {
+      const int e = queued + __popc(m & ((1u << lane) - 1));
+      W.queue_face[e] = f;
+      W.queue_lane[e] = (unsigned char)l;
+    }
+    queued += __popc(m);
+    __syncwarp();
+    if (queued >= 32) {
+      queued -= 32;
+      test(queued + lane);
+      __syncwarp();
+    }
+  }
+  if (lane < queued) test(lane);
+  __syncwarp();
+  if (i >= P) return;
+  const int nh = W.hits[lane];
   if (nhits_out) nhits_out[i] = nh;
-  if (hit0_out) hit0_out[i] = nh > 0 ? hf[0] : -1;
   if (nh == 0) {
+    if (hit0_out) hit0_out[i] = -1;
     pts[2 * i] = NAN;
     pts[2 * i + 1] = NAN;
     if (face_out) face_out[i] = -1;
     atomicAdd(missing, 1ull);
     return;
   }
-  int f = hf[0];
-  int kmax = nh < MAXHITS ? nh : MAXHITS;
-  if (nh > 1 && !first_hit) {
-    double best = density[f];
-    for (int k = 1; k < kmax; ++k) {
-      double dk = density[hf[k]];
-      if (dk > best) {
-        f = hf[k];
-        best = dk > best;  // the reference stores the comparison's bool here (transport_map.cpp:82)
+  int first, f;
+  if (nh <= MAXHITS) {
+    for (int k = 1; k < nh; ++k) {  // by rank
+      const unsigned long long h = W.hit[lane][k];
+      int j = k;
+      for (; j > 0 && W.hit[lane][j - 1] > h; --j) W.hit[lane][j] = W.hit[lane][j - 1];
+      W.hit[lane][j] = h;
+    }
+    first = f = (int)(unsigned)W.hit[lane][0];
+    if (nh > 1 && !first_hit) {
+      double best = L.density[f];
+      for (int k = 1; k < nh; ++k) {
+        const int g = (int)(unsigned)W.hit[lane][k];
+        const double dk = L.density[g];
+        if (dk > best) {
+          f = g;
+          best = dk > best;  // the reference stores the comparison's bool here (transport_map.cpp:82)
+        }
       }
     }
+  } else {
+    f = many_hits(L, b, qx, qy, !first_hit, &first);
   }
+  if (hit0_out) hit0_out[i] = first;
   Quad p;
   int vid[4];
-  load_quad(xy, n, f, p, vid);
+  double w[4];
+  load_quad(L.xy, n, first, p, vid);
+  bilinear_weights(qx, qy, p, w);
   const double dx = 1.0 / (double)n;
+  // the corners of face f on the origin grid: (i, j), (i+1, j), (i+1, j+1), (i, j+1)
+  const int fi = f / n, fj = f - fi * n;
   double rx = 0, ry = 0;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    int vi = vid[k] / (n + 1), vj = vid[k] - (vid[k] / (n + 1)) * (n + 1);
+    const int vi = fi + (k == 1 || k == 2), vj = fj + (k >= 2);
     double ox = (double)vi * dx, oy = (double)vj * dx;
     if (k == 0) {
-      rx = hw[0][0] * ox;
-      ry = hw[0][0] * oy;
+      rx = w[0] * ox;
+      ry = w[0] * oy;
     } else {
-      rx += hw[0][k] * ox;
-      ry += hw[0][k] * oy;
+      rx += w[k] * ox;
+      ry += w[k] * oy;
     }
   }
   pts[2 * i] = rx;
@@ -1311,6 +1903,8 @@ __global__ void k_inv_face_sums(int N, const int* start, int* list, const InvGra
 
 // ---- host ----
 
+// The bins are built on the side stream while the BVH order, a chain of small launches that
+// leaves most of the GPU idle, runs on the context's (one after the other under the profiler).
 static void build_locator(otm_map* m) {
   otm_context* ctx = m->ctx;
   cudaStream_t st = ctx->stream;
@@ -1318,28 +1912,49 @@ static void build_locator(otm_map* m) {
   const int B = n;
   const int nb = B * B;
   m->bins = B;
-  m->bin_start.reserve(sizeof(int) * (nb + 1), ctx->stream, ctx->pool);
-  m->face_box.reserve(sizeof(double4) * N, ctx->stream, ctx->pool);
+  m->bin_start.reserve(sizeof(int) * (nb + 1), st, ctx->pool);
+  m->face_box.reserve(sizeof(double4) * N, st, ctx->pool);
+  m->bvh_rank.reserve(sizeof(int) * N, st, ctx->pool);
+  m->leaf_box.reserve(sizeof(double4) * N, st, ctx->pool);
   // bin counts and scan sums in the context's grow-only scratch
   const size_t b_counts = (sizeof(int) * nb + 255) / 256 * 256;
   ctx->locate_scratch.reserve(b_counts + sizeof(int) * ((nb + SCAN_B - 1) / SCAN_B + 1));
   int* counts = ctx->locate_scratch.as<int>();
   int* sums = reinterpret_cast<int*>(ctx->locate_scratch.as<char>() + b_counts);
-  OTM_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * nb, st));
   const double* xy = m->fwd.as<double>();
-  launch(ctx, "bin_count", k_bin_count, (N + 255) / 256, 256, xy, n, B, counts, m->face_box.as<double4>());
-  exclusive_scan(st, counts, m->bin_start.as<int>(), sums, nb);
-  int total = 0;
-  OTM_CUDA(cudaMemcpyAsync(&total, m->bin_start.as<int>() + nb, sizeof(int), cudaMemcpyDeviceToHost, st));
-  OTM_CUDA(cudaStreamSynchronize(st));
-  m->bin_faces.reserve(sizeof(int) * (size_t)(total > 0 ? total : 1), ctx->stream, ctx->pool);
-  OTM_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * nb, st));
-  launch(ctx, "bin_fill", k_bin_fill, (N + 255) / 256, 256, xy, n, B, (const int*)m->bin_start.as<int>(), counts,
-         m->bin_faces.as<int>());
-  OTM_CUDA(cudaGetLastError());
-  m->bvh_rank.reserve(sizeof(int) * N, ctx->stream, ctx->pool);
-  m->leaf_box.reserve(sizeof(double4) * N, ctx->stream, ctx->pool);
+  const bool beside = !ctx->prof.on;
+  cudaStream_t bs = st;
+  if (beside) {
+    side_stream(ctx);
+    bs = ctx->side;
+    OTM_CUDA(cudaEventRecord(ctx->side_ready, st));  // the mesh and the buffers above
+    OTM_CUDA(cudaStreamWaitEvent(bs, ctx->side_ready, 0));
+  }
   build_bvh_order(ctx, xy, n, m->bvh_rank.as<int>(), m->leaf_box.as<double4>());
+  try {
+    auto bin = [&](const char* name, auto kernel, auto... args) {
+      if (!beside) return launch(ctx, name, kernel, (N + 255) / 256, 256, args...);
+      ctx->launches++;
+      kernel<<<(N + 255) / 256, 256, 0, bs>>>(args...);
+    };
+    OTM_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * nb, bs));
+    bin("bin_count", k_bin_count, xy, n, B, counts, m->face_box.as<double4>());
+    exclusive_scan(bs, counts, m->bin_start.as<int>(), sums, nb);
+    int total = 0;
+    OTM_CUDA(cudaMemcpyAsync(&total, m->bin_start.as<int>() + nb, sizeof(int), cudaMemcpyDeviceToHost, bs));
+    OTM_CUDA(cudaStreamSynchronize(bs));
+    m->bin_faces.reserve(sizeof(int) * (size_t)(total > 0 ? total : 1), bs, ctx->pool);
+    OTM_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * nb, bs));
+    bin("bin_fill", k_bin_fill, xy, n, B, (const int*)m->bin_start.as<int>(), counts, m->bin_faces.as<int>());
+    OTM_CUDA(cudaGetLastError());
+    if (beside) {
+      OTM_CUDA(cudaEventRecord(ctx->side_ready, bs));
+      OTM_CUDA(cudaStreamWaitEvent(st, ctx->side_ready, 0));
+    }
+  } catch (...) {
+    cudaStreamSynchronize(bs);  // the map's buffers go back on the context's stream
+    throw;
+  }
   m->located = true;
 }
 
@@ -1354,12 +1969,10 @@ void map_inverse_dev(otm_map* m, double* pts, long count, int mode, int* face, i
   otm_context* ctx = m->ctx;
   if (!m->located) build_locator(m);
   if (count <= 0) return;
-  const unsigned grid = (unsigned)((count + 255) / 256);
-  launch(ctx, "inverse", k_inverse, grid, 256, (const double*)m->fwd.as<double>(),
-         (const double*)m->density.as<double>(), m->n, m->bins, (const int*)m->bin_start.as<int>(),
-         (const int*)m->bin_faces.as<int>(), (const double4*)m->face_box.as<double4>(),
-         (const int*)m->bvh_rank.as<int>(), (const double4*)m->leaf_box.as<double4>(), pts, count,
-         mode == OTM_INV_FIRST ? 1 : 0, face, hit0, nhits, missing);
+  const Locator L{m->fwd.as<double>(),      m->density.as<double>(),   m->n, m->bins, m->bin_start.as<int>(),
+                  m->bin_faces.as<int>(),   m->face_box.as<double4>(), m->bvh_rank.as<int>(), m->leaf_box.as<double4>()};
+  launch(ctx, "inverse", k_inverse, (unsigned)((count + INV_T - 1) / INV_T), INV_T, L, pts, count, mode == OTM_INV_FIRST ? 1 : 0, face, hit0, nhits,
+         missing);
   OTM_CUDA(cudaGetLastError());
 }
 

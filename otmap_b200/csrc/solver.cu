@@ -1208,8 +1208,7 @@ extern "C" int otm_solve_batch(otm_context* ctx, int count, const int* ns, const
       if (adjusted && adjusted[q]) copy_out(ctx, adjusted[q], h[q].rho, sizeof(double) * (size_t)n * n, ctx->side);
     };
     if (early) {
-      if (!ctx->side) OTM_CUDA(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
-      if (!ctx->side_ready) OTM_CUDA(cudaEventCreateWithFlags(&ctx->side_ready, cudaEventDisableTiming));
+      side_stream(ctx);
       ctx->staging_side.reserve(sizeof(double) * 2 * vmax);  // before the loop: no allocation inside it
       const size_t pb = sizeof(Inst) * (size_t)count;
       if (ctx->h_poll_bytes < pb) {
