@@ -295,6 +295,7 @@ __global__ __launch_bounds__(AT) void k_adj_apply(int n, const double2* g, const
                                                   AdjCtl* ctl, double* partial, double* hcol, double* c, long stride) {
   __shared__ double red[AT / 32 * RED_LD], stage[TOT_STAGE];
   const long off = blockIdx.y * stride;
+  overlap_wait();
   ctl += blockIdx.y;
   if (!ctl->go) return;
   g += off / 2;
@@ -309,6 +310,7 @@ __global__ __launch_bounds__(AT) void k_adj_apply(int n, const double2* g, const
   for (long f = (long)blockIdx.x * AT + threadIdx.x; f < N; f += (long)ANB * AT)
     w[f] = jt_cell(n, g, z, (int)(f / n), (int)(f % n));
   block_dots(N, w, V, ld, P, red, partial);
+  overlap_begin();
   if (!last_block(&ctl->counter, gridDim.x)) return;
   totals(partial, P, stage, [&](int i, double d) {
     c[i] = d;
@@ -340,6 +342,7 @@ __global__ __launch_bounds__(AT) void k_adj_orth(int n, double* V, long ld, AdjC
                                                  double* c, long stride) {
   __shared__ double sc[ADJ_MAX_M + 8], red[AT / 32 * RED_LD], stage[TOT_STAGE];
   const long off = blockIdx.y * stride;
+  overlap_wait();
   ctl += blockIdx.y;
   if (!ctl->go) return;
   V += off;
@@ -386,6 +389,7 @@ __global__ __launch_bounds__(AT) void k_adj_orth(int n, double* V, long ld, AdjC
     combine(N, w, V, ld, P, c, sc);
     block_dots(N, w, V, ld, P, red, partial);
   }
+  overlap_begin();
   if (!last_block(&ctl->counter, gridDim.x)) return;
   totals(partial, P, stage, [&](int i, double d) {
     c[i] = d;
@@ -404,6 +408,7 @@ __global__ __launch_bounds__(AT) void k_adj_norm(int n, double* V, long ld, AdjC
                                                  double* gv, Inst* rec, long stride) {
   __shared__ double sc[ADJ_MAX_M + 8], sh[ADJ_MAX_M + 8], ss[ADJ_MAX_M + 8], red[64], stage[TOT_STAGE];
   const long off = blockIdx.y * stride;
+  overlap_wait();
   ctl += blockIdx.y;
   if (!ctl->go) return;
   V += off;
@@ -419,6 +424,7 @@ __global__ __launch_bounds__(AT) void k_adj_norm(int n, double* V, long ld, AdjC
   const int j = ctl->j, P = j + 1;
   const long N = (long)n * n;
   double v[1] = {combine(N, V + (size_t)(j + 1) * ld, V, ld, P, c, sc)};
+  overlap_begin();
   block_sum<1>(v, red);
   if (threadIdx.x == 0) partial[blockIdx.x] = v[0];
   if (!last_block(&ctl->counter, gridDim.x)) return;
@@ -462,6 +468,7 @@ __global__ __launch_bounds__(AT) void k_adj_norm(int n, double* V, long ld, AdjC
 // while any map's cycle goes on.
 __global__ void k_adj_scale_by(long N, double* V, long ld, const double* a, const AdjCtl* ctl, long stride,
                                cudaGraphConditionalHandle handle, int in_graph) {
+  overlap_wait();
   if (in_graph && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
     int any = 0;
     for (int y = 0; y < (int)gridDim.y; ++y) any |= ctl[y].go;
@@ -791,11 +798,14 @@ static void poisson_rec(otm_context* ctx, AdjointWs* W, int kind) {
 }
 
 // One Arnoldi step j of every map's cycle (j read on the device): z = M^+ v_j and the four
-// step kernels, which do nothing for a map whose cycle has ended.
+// step kernels, which do nothing for a map whose cycle has ended. They overlap their
+// predecessor's end (common.cuh) except beside the product kernels, which do not wait for it:
+// the gradient at 512^2 takes 1.17 ms so, 1.21 launched plainly.
 static void arnoldi_step(otm_context* ctx, AdjointWs* W, int n, cudaGraphConditionalHandle handle, int in_graph) {
   const long ld = (long)W->ld, sd = W->stride;
   const dim3 grid(W->nb, W->maps);
   Inst* rec = W->rec(2);
+  const Overlap overlap(ctx, W->fft);
   poisson_rec(ctx, W, 2);
   launch(ctx, "adj_apply", k_adj_apply, grid, AT, n, (const double2*)W->g, (const double*)W->z, W->Vb, ld, W->ctl,
          W->part, W->hcol, W->c, sd);

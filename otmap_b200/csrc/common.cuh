@@ -92,6 +92,24 @@ __device__ __forceinline__ double block_max(double v, double* red) {
   return v;
 }
 
+// ---- programmatic dependent launch ----
+//
+// A kernel launched with ctx->overlap (context.h) may start while the one before it in the
+// stream still runs. It reads or writes nothing that another kernel changes before
+// overlap_wait, which returns when the kernel before it has completed with its writes visible;
+// no block leaves before that wait, so a kernel's end implies the end of all before it. Tables
+// and work lists may be read earlier, with loads that leave no copy in L1 of lines the wait
+// should see fresh. overlap_begin lets the successor's blocks take the places that this
+// kernel's have left: it stands behind the main loop, since blocks that only wait slow the ones
+// at work (at the kernels' entry nearly every size got slower than without). In a kernel
+// launched plainly both are no-ops.
+__device__ __forceinline__ void overlap_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class T>
+__device__ __forceinline__ const T* early_pointer(const T* const* p) {  // a pointer field, past L1
+  return reinterpret_cast<const T*>(__ldcg(reinterpret_cast<const unsigned long long*>(p)));
+}
+__device__ __forceinline__ void overlap_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // "Last block" election for a reduction spread over `total` blocks that share
 // `counter`: every block calls it once after thread 0 has written the block's
 // partials; it returns true (in all threads) in exactly one block, the last to

@@ -156,6 +156,7 @@ struct otm_context {
   int wait_test = 0;     // OTM_OPT_WAIT_TEST: bounded waits made to run out
   int precision = 0;     // OTM_PRECISION_FP64 / _SPLIT
   int autotune = 0;      // OTM_AUTOTUNE_OFF / _ON (sweep strip height per batch configuration)
+  bool overlap = false;  // launch() lets a kernel start before its predecessor's end (set around such launches)
   int last_srows = 0;    // strip height of the last solve call (OTM_INFO_STRIP_ROWS)
   otm::Profiler prof;
   std::map<int, std::unique_ptr<otm::SizeTables>> tables;
@@ -266,38 +267,50 @@ void adjoint_maps(otm_context* ctx, int n, int count, const double* const* densi
                   otm_adjoint_stats* stats);
 void check_adjoint_options(const otm_adjoint_options& o);
 
-// Launches `kernel` on the context stream, counting it and (when profiling) bracketing
-// it with CUDA events.
-template <class K, class... Args>
-void launch(otm_context* ctx, const char* name, K kernel, dim3 grid, dim3 block, Args... args) {
+// Launches `kernel` on the context stream with dynamic shared memory, counting it and (when
+// profiling) bracketing it with CUDA events. With ctx->overlap the launch is a programmatic
+// dependent one (common.cuh): only for kernels that wait before they touch shared state.
+template <class... KArgs, class... Args>
+void launch_smem(otm_context* ctx, const char* name, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                 Args... args) {
   ctx->launches++;
   if (ctx->prof.on) {
     int id = ctx->prof.id(name);
     cudaEvent_t a = ctx->prof.get(), b = ctx->prof.get();
     cudaEventRecord(a, ctx->stream);
-    kernel<<<grid, block, 0, ctx->stream>>>(args...);
+    kernel<<<grid, block, smem, ctx->stream>>>(args...);
     cudaEventRecord(b, ctx->stream);
     ctx->prof.pending.push_back({id, a, b});
+  } else if (ctx->overlap) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    OTM_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
   } else {
-    kernel<<<grid, block, 0, ctx->stream>>>(args...);
+    kernel<<<grid, block, smem, ctx->stream>>>(args...);
   }
+}
+template <class... KArgs, class... Args>
+void launch(otm_context* ctx, const char* name, void (*kernel)(KArgs...), dim3 grid, dim3 block, Args... args) {
+  launch_smem(ctx, name, kernel, grid, block, 0, args...);
 }
 
-// As launch(), with dynamic shared memory.
-template <class K, class... Args>
-void launch_smem(otm_context* ctx, const char* name, K kernel, dim3 grid, dim3 block, size_t smem, Args... args) {
-  ctx->launches++;
-  if (ctx->prof.on) {
-    int id = ctx->prof.id(name);
-    cudaEvent_t a = ctx->prof.get(), b = ctx->prof.get();
-    cudaEventRecord(a, ctx->stream);
-    kernel<<<grid, block, smem, ctx->stream>>>(args...);
-    cudaEventRecord(b, ctx->stream);
-    ctx->prof.pending.push_back({id, a, b});
-  } else {
-    kernel<<<grid, block, smem, ctx->stream>>>(args...);
-  }
-}
+// Sets ctx->overlap for a scope.
+struct Overlap {
+  otm_context* ctx;
+  bool was;
+  Overlap(otm_context* c, bool on) : ctx(c), was(c->overlap) { c->overlap = on; }
+  ~Overlap() { ctx->overlap = was; }
+  Overlap(const Overlap&) = delete;
+  Overlap& operator=(const Overlap&) = delete;
+};
 
 // Runs an entry point body, mapping exceptions to otm_status codes.
 template <class F>

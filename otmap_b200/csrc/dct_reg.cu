@@ -211,7 +211,6 @@ __device__ __forceinline__ V pre3(int k, R a, R b, V pt) {
 template <class R, int N1, int N2>
 struct RowGeom {
   using V = typename RT<R>::V;
-  static constexpr int RW = RT<R>::RW;               // most warps per block (RegDct::run picks the number)
   static constexpr int n = N1 * N2, LPW = 32 / N2;
   static constexpr int DATA = 2 * LPW * n;           // reals: the item's rows
   static constexpr int TRANS = LPW * N1 * (N2 + 1);  // reals: step-3 transpose buffers
@@ -229,9 +228,9 @@ __device__ __forceinline__ typename RT<R>::V* load_row_tables(R* sbuf, int warps
   using V = typename G::V;
   constexpr int n = G::n;
   V* tab = reinterpret_cast<V*>(sbuf + warps * G::WARP);
-  const double2* tw2 = I.tw + (n >> 1);
+  const double2 *tw2 = early_pointer(&I.tw) + (n >> 1), *pt = early_pointer(&I.pt);
   for (int e = threadIdx.x; e < n; e += blockDim.x) {
-    const double2 a = __ldg(&tw2[e]), b = __ldg(&I.pt[e]);
+    const double2 a = __ldg(&tw2[e]), b = __ldg(&pt[e]);
     tab[e] = mk2((R)a.x, (R)a.y);
     tab[n + e] = mk2((R)b.x, (R)b.y);
   }
@@ -313,6 +312,7 @@ __global__ __launch_bounds__(RT<R>::RW * 32, 1) void k_dct_rows_fwd(Inst* insts,
   const int stride = gridDim.x * RW;
   if (lane == 0) mbar_init(bar);
   __syncwarp();
+  overlap_wait();
   auto issue = [&](int it) -> bool {
     if (it >= items) return false;
     const Inst& J = insts[row_inst[seg + it]];
@@ -381,6 +381,7 @@ __global__ __launch_bounds__(RT<R>::RW * 32, 1) void k_dct_rows_fwd(Inst* insts,
     }
     item = next;
   }
+  overlap_begin();
 }
 
 // Inverse DCT-III of rows 2p and 2p+1 of T -> d_hat: the inputs W^a + i W^b of the two
@@ -406,6 +407,7 @@ __global__ __launch_bounds__(RT<R>::RW * 32, 1) void k_dct_rows_inv(Inst* insts,
   const int stride = gridDim.x * RW;
   if (lane == 0) mbar_init(bar);
   __syncwarp();
+  overlap_wait();
   auto issue = [&](int it) -> bool {
     if (it >= items) return false;
     const Inst& J = insts[row_inst[seg + it]];
@@ -470,6 +472,7 @@ __global__ __launch_bounds__(RT<R>::RW * 32, 1) void k_dct_rows_inv(Inst* insts,
     }
     item = next;
   }
+  overlap_begin();
 }
 
 // Column pass, one warp per column pair (LPW pairs per warp when a line takes fewer than 32
@@ -523,15 +526,17 @@ __global__ __launch_bounds__(CT, RT<R>::COL_BLOCKS) void k_dct_cols(const Inst* 
   R* scos = reinterpret_cast<R*>(spt + n);         // cos(pi k / n)
   {
     const Inst& I0 = insts[col_inst[seg]];
-    const double2* tw2 = I0.tw + (n >> 1);
+    const double2 *tw2 = early_pointer(&I0.tw) + (n >> 1), *pt = early_pointer(&I0.pt);
+    const double* cosk = early_pointer(&I0.cosk);
     for (int e = threadIdx.x; e < n; e += blockDim.x) {
-      const double2 a = __ldg(&tw2[e]), b = __ldg(&tw2[n + e]), c = __ldg(&I0.pt[e]);
+      const double2 a = __ldg(&tw2[e]), b = __ldg(&tw2[n + e]), c = __ldg(&pt[e]);
       stw[e] = mk2((R)a.x, (R)a.y);
       stw_sw[e] = mk2((R)b.x, (R)b.y);
       spt[e] = mk2((R)c.x, (R)c.y);
-      scos[e] = (R)__ldg(&I0.cosk[e]);
+      scos[e] = (R)__ldg(&cosk[e]);
     }
   }
+  overlap_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / N2, t = lane % N2;
   const int cp = warp * LPW + sub;  // this lane group's column pair within the block
   R* buf = sbuf + (warp * LPW + sub) * GG::LINE;  // this line's region of the tile space
@@ -645,6 +650,7 @@ __global__ __launch_bounds__(CT, RT<R>::COL_BLOCKS) void k_dct_cols(const Inst* 
 #pragma unroll
     for (int r = 0; r < N1; ++r) tile[(t + N2 * rbrev<N1>(r)) * RS + cp] = x2[r];
     __syncthreads();
+    if (b + gridDim.x >= items) overlap_begin();
     for (int e = threadIdx.x; e < n * CPB; e += GG::CT) {
       const int i = e / CPB, cc = e - i * CPB;
       *reinterpret_cast<V*>(T + (size_t)i * n + l0 + 2 * cc) = tile[makhoul_inv(i, n) * RS + cc];

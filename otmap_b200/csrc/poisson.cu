@@ -267,6 +267,7 @@ __global__ __launch_bounds__(Geom<M, false>::THREADS, Geom<M, false>::MIN_BLOCKS
   constexpr int T = G::T;
   extern __shared__ double2 smem[];
   const int item = seg + blockIdx.x;
+  overlap_wait();
   const Inst& I = insts[row_inst[item]];
   if (!I.active) return;
   const int n = I.n, line = threadIdx.x / T, t = threadIdx.x % T;
@@ -286,6 +287,7 @@ __global__ __launch_bounds__(Geom<M, false>::THREADS, Geom<M, false>::MIN_BLOCKS
     }
   }
   line_dft<M, CHIRP>(v, n, t, sm, Tables<M>(I.tw));
+  overlap_begin();
   const double s0 = sqrt(1.0 / n), s1 = sqrt(2.0 / n);
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
@@ -305,6 +307,7 @@ __global__ __launch_bounds__(Geom<M, true>::THREADS, Geom<M, true>::MIN_BLOCKS) 
   constexpr int T = G::T, LB = G::LB;
   extern __shared__ double2 smem[];
   const int item = seg + blockIdx.x;
+  overlap_wait();
   const Inst& I = insts[col_inst[item]];
   if (!I.active) return;
   const int n = I.n, line = threadIdx.x % LB, t = threadIdx.x / LB;
@@ -352,6 +355,7 @@ __global__ __launch_bounds__(Geom<M, true>::THREADS, Geom<M, true>::MIN_BLOCKS) 
     if (k < n) v[q] = dct3_pre(k, u[q], sm[slot(k ? n - k : 0)], __ldg(&I.pt[k]));
   }
   line_dft<M, CHIRP>(v, n, t, sm, tab);
+  overlap_begin();
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const int m = t + q * T;
@@ -369,6 +373,7 @@ __global__ __launch_bounds__(Geom<M, false>::THREADS, Geom<M, false>::MIN_BLOCKS
   constexpr int T = G::T;
   extern __shared__ double2 smem[];
   const int item = seg + blockIdx.x;
+  overlap_wait();
   const Inst& I = insts[row_inst[item]];
   if (!I.active) return;
   const int n = I.n, line = threadIdx.x / T, t = threadIdx.x % T;
@@ -396,6 +401,7 @@ __global__ __launch_bounds__(Geom<M, false>::THREADS, Geom<M, false>::MIN_BLOCKS
     v[q] = dct3_pre(k, y, ym, __ldg(&I.pt[k]));
   }
   line_dft<M, CHIRP>(v, n, t, sm, Tables<M>(I.tw));
+  overlap_begin();
   // sample j of a row is element j/2 or n-1-j/2 of the reordered sequence
 #pragma unroll
   for (int q = 0; q < 8; ++q) {

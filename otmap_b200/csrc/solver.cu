@@ -820,9 +820,14 @@ __global__ void k_loop_check(const Inst* insts, int count, LoopCtl* ctl, cudaGra
   }
 }
 
-// Launches one iteration of every active instance (Poisson solve + the two sweeps).
+// Launches one iteration of every active instance (Poisson solve + the two sweeps). The kernels
+// overlap their predecessor's end (common.cuh) where all of them wait for it: the product
+// kernels and the tensor-core transform do not. Microseconds per iteration, plain and so:
+// 64^2 29.9 and 27.7, 256^2 38.5 and 35.4, 512^2 57.0 and 54.1, 1024^2 79.4 and 75.8, eight 1024^2
+// 337.9 and 335.2; split 1024^2 76.3 and 73.3, eight 272.3 and 265.5.
 static void launch_iteration(otm_context* ctx, Inst* d_insts) {
   Workspace& ws = ctx->ws();
+  const Overlap overlap(ctx, ws.total_gemm == 0 && ws.total_tc == 0);
   const int G = ws.total_gemm;
   if (G > 0)
     for (int s = 0; s < 4; ++s)
