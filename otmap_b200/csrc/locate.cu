@@ -504,6 +504,7 @@ __global__ __launch_bounds__(SCAN_T) void k_bvh_classify(int N, const BvhCtl* ct
                                                          const BvhNode* odd, const unsigned char* window0,
                                                          const unsigned char* window1, unsigned char* small, int* lpre,
                                                          int* sums) {
+  overlap_wait();
   const int level = ctl->level;
   const bool at_end = (long)blockIdx.x * SCAN_B >= N;  // the window of p = N alone
   if (level > 0 && (at_end || !(level & 1 ? window1 : window0)[blockIdx.x])) {
@@ -530,7 +531,10 @@ __global__ __launch_bounds__(SCAN_T) void k_bvh_classify(int N, const BvhCtl* ct
       lpre, sums, N + 1);
 }
 
-__global__ __launch_bounds__(1024) void k_bvh_sums(int* sums, int nsums) { scan_sums(sums, nsums); }
+__global__ __launch_bounds__(1024) void k_bvh_sums(int* sums, int nsums) {
+  overlap_wait();
+  scan_sums(sums, nsums);
+}
 
 // Small positions before p.
 struct BvhPrefix {
@@ -545,6 +549,7 @@ __global__ __launch_bounds__(BVH_BT) void k_bvh_slots(int N, const BvhCtl* ctl, 
                                                       const unsigned char* window0, const unsigned char* window1,
                                                       const unsigned char* small, BvhPrefix pre, int* slot_big,
                                                       int* slot_small) {
+  overlap_wait();
   const int level = ctl->level;
   if (!(level & 1 ? window1 : window0)[blockIdx.x]) return;
 #pragma unroll
@@ -578,6 +583,7 @@ __global__ __launch_bounds__(1024) void k_bvh_children(BvhCtl* ctl, int* counts,
                                                        const double2* cen, int* sub_end, unsigned char* sub_level,
                                                        cudaGraphConditionalHandle handle, int in_graph) {
   __shared__ int s_next;
+  overlap_wait();
   const int level = ctl->level, count = level ? counts[level & 1] : 1;
   BvhNode* nodes = level & 1 ? odd : even;
   BvhNode* next = level & 1 ? even : odd;
@@ -634,6 +640,7 @@ __global__ __launch_bounds__(BVH_BT) void k_bvh_move(int N, const BvhCtl* ctl, i
                                                      unsigned char* window0, unsigned char* window1,
                                                      const unsigned char* small, BvhPrefix pre, const int* slot_big,
                                                      const int* slot_small) {
+  overlap_wait();
   const int level = ctl->level - 1;  // k_bvh_children has counted it
   unsigned char* to = level & 1 ? window0 : window1;
   if (!(level & 1 ? window1 : window0)[blockIdx.x]) {
@@ -884,6 +891,13 @@ __global__ __launch_bounds__(BVH_T) void k_bvh_subtrees(int N, const BvhCtl* ctl
   }
 }
 
+// Levels per body of the first phase's WHILE node. A body costs about 3 us beside its kernels, a
+// level after the last one five launches that return at once; the kernels overlap their
+// predecessor's end (common.cuh). A query of 2^20 points on a new mesh of 64^2, 256^2 and 1024^2
+// faces: one level per body with plain launches 455, 704 and 1477 us, overlapped 442, 674 and
+// 1446, two levels 422, 670 and 1408, three 418, 648 and 1408, four 432, 668 and 1399.
+constexpr int LEVELS_PER_BODY = 3;
+
 // rank[f] and the leaf box of f for the n^2 quads of the forward mesh xy (device). The launches
 // run as one CUDA graph per size (captured on first use, kept in the context) on the
 // context's grow-only scratch; a build's own buffers reach it through the control block.
@@ -1009,7 +1023,10 @@ static void build_bvh_order(otm_context* ctx, const double* xy, int n, int* rank
             params.conditional.size = 1;
             cudaGraphNode_t loop;
             OTM_CUDA(cudaGraphAddNode(&loop, g, &last, 1, &params));
-            capture(params.conditional.phGraph_out[0], nullptr, [&] { level(handle, 1); });
+            capture(params.conditional.phGraph_out[0], nullptr, [&] {
+              const Overlap overlap(ctx, true);
+              for (int l = 0; l < LEVELS_PER_BODY; ++l) level(handle, 1);
+            });
             last = loop;
           }
           const cudaGraphNode_t after = last;
@@ -1030,7 +1047,7 @@ static void build_bvh_order(otm_context* ctx, const double* xy, int n, int* rank
       cudaGraphDestroy(g);
     }
     OTM_CUDA(cudaGraphLaunch(slot->exec, st));
-    ctx->launches += slot->kernels;  // with one level: how many were taken stays on the device
+    ctx->launches += slot->kernels;  // one body of levels: how many ran stays on the device
   }
   OTM_CUDA(cudaGetLastError());
 }
