@@ -470,7 +470,10 @@ __global__ __launch_bounds__(ST) void k_sweep_sums_t(Inst* insts, const int* str
     const int last = min(sc.i0 + I.srows, n);  // cell rows i0 .. last-1; grid rows i0-1 .. last
     R.rows_end = last;
     R.setup();
-#pragma unroll
+    // not unrolled: the seven copies of issue() cost more in instruction fetches, once per launch,
+    // than the loop (64^2 alone 29.3 -> 28.4 us per iteration, 256^2 35.5 -> 34.7, 1024^2 unchanged
+    // within 1%, split 1024^2 75.3 -> 73.7)
+#pragma unroll 1
     for (int k = 0; k < RD - 1; ++k) R.issue(sc.i0 - 1 + k);
     VG gp, gh, gq;
 #pragma unroll 2
@@ -586,7 +589,7 @@ __global__ __launch_bounds__(ST) void k_sweep_update_t(Inst* insts, const int* s
     const int last = min(sc.i0 + I.srows, n);
     R.rows_end = last;
     R.setup();
-#pragma unroll
+#pragma unroll 1
     for (int k = 0; k < RD - 1; ++k) R.issue(sc.i0 - 1 + k);
     // d = d_hat + beta d_prev, formed from the staged rows exactly as the reference
     // forms the vector d before its gradients (otsolver_2dgrid.cpp:199)
