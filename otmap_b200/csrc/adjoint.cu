@@ -805,7 +805,7 @@ static void arnoldi_step(otm_context* ctx, AdjointWs* W, int n, cudaGraphConditi
   const long ld = (long)W->ld, sd = W->stride;
   const dim3 grid(W->nb, W->maps);
   Inst* rec = W->rec(2);
-  const Overlap overlap(ctx, W->fft);
+  const Overlap overlap(ctx, W->fft, (long)W->N * W->maps);
   poisson_rec(ctx, W, 2);
   launch(ctx, "adj_apply", k_adj_apply, grid, AT, n, (const double2*)W->g, (const double*)W->z, W->Vb, ld, W->ctl,
          W->part, W->hcol, W->c, sd);

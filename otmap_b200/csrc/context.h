@@ -101,6 +101,7 @@ struct Workspace {
   int total_tiles = 0, total_gemm = 0, total_rows = 0, total_cols = 0, total_strips = 0, total_tc = 0;
   int mode = -1;       // poisson mode the layout was built for
   int precision = -1;  // precision the layout was built for
+  long cells = 0;      // of all instances
   int srows = 0;       // strip height of the sweeps (rule or autotuned)
   bool tuned = false;  // srows was chosen by timing (OTM_OPT_AUTOTUNE)
   int split_strip0 = 0;  // strips of split-precision instances start here (FP64 ones before)
@@ -157,6 +158,7 @@ struct otm_context {
   int precision = 0;     // OTM_PRECISION_FP64 / _SPLIT
   int autotune = 0;      // OTM_AUTOTUNE_OFF / _ON (sweep strip height per batch configuration)
   bool overlap = false;  // launch() lets a kernel start before its predecessor's end (set around such launches)
+  int early = 0;         // ... and its successor at once (OVERLAP_EARLY_CELLS)
   int last_srows = 0;    // strip height of the last solve call (OTM_INFO_STRIP_ROWS)
   otm::Profiler prof;
   std::map<int, std::unique_ptr<otm::SizeTables>> tables;
@@ -302,12 +304,27 @@ void launch(otm_context* ctx, const char* name, void (*kernel)(KArgs...), dim3 g
   launch_smem(ctx, name, kernel, grid, block, 0, args...);
 }
 
-// Sets ctx->overlap for a scope.
+// Sets ctx->overlap for a scope; cells: of all the instances in the launches. Up to
+// OVERLAP_EARLY_CELLS a register transform's kernel (ctx->early) lets its successor's blocks in
+// as soon as it runs, so that they are resident when it ends: it leaves most of the chip free.
+// Behind the main loop the trigger comes too late for them. From more cells on the blocks let
+// in early gather on the few SMs with room and the successor runs unevenly. Microseconds per
+// iteration late and early: 64^2 27.7 and 26.3, 128^2 33.0 and 31.6, 256^2 34.7 and 33.8, sixteen
+// 64^2 33.9 and 32.6; but 512^2 54.5 and 61.6, four 256^2 43.6 and 45.6. (The block transforms of
+// other sizes lose 1.3 us at 50^2 to 200^2 when they trigger early, the sum sweep 0.7 us at 256^2.)
+constexpr long OVERLAP_EARLY_CELLS = 256L * 256;
 struct Overlap {
   otm_context* ctx;
-  bool was;
-  Overlap(otm_context* c, bool on) : ctx(c), was(c->overlap) { c->overlap = on; }
-  ~Overlap() { ctx->overlap = was; }
+  const bool overlap;
+  const int early;
+  Overlap(otm_context* c, bool on, long cells) : ctx(c), overlap(c->overlap), early(c->early) {
+    c->overlap = on;
+    c->early = on && cells <= OVERLAP_EARLY_CELLS;
+  }
+  ~Overlap() {
+    ctx->overlap = overlap;
+    ctx->early = early;
+  }
   Overlap(const Overlap&) = delete;
   Overlap& operator=(const Overlap&) = delete;
 };

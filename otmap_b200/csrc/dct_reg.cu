@@ -293,7 +293,7 @@ __device__ __forceinline__ void wait_fault(Inst& I, unsigned long long* bar, uns
 // Forward DCT-II of rows 2p and 2p+1 of r_k (one complex FFT per row pair) -> T.
 template <class R, int N1, int N2>
 __global__ __launch_bounds__(RT<R>::RW * 32, 1) void k_dct_rows_fwd(Inst* insts, const int* row_inst, int seg,
-                                                                     int items, unsigned extra, long long limit) {
+                                                                     int items, unsigned extra, long long limit, int early) {
   using G = RowGeom<R, N1, N2>;
   using V = typename G::V;
   constexpr int n = G::n, LPW = G::LPW;
@@ -313,6 +313,7 @@ __global__ __launch_bounds__(RT<R>::RW * 32, 1) void k_dct_rows_fwd(Inst* insts,
   if (lane == 0) mbar_init(bar);
   __syncwarp();
   overlap_wait();
+  if (early) overlap_begin();
   auto issue = [&](int it) -> bool {
     if (it >= items) return false;
     const Inst& J = insts[row_inst[seg + it]];
@@ -388,7 +389,7 @@ __global__ __launch_bounds__(RT<R>::RW * 32, 1) void k_dct_rows_fwd(Inst* insts,
 // rows go through one inverse FFT; its real and imaginary parts are the two rows.
 template <class R, int N1, int N2>
 __global__ __launch_bounds__(RT<R>::RW * 32, 1) void k_dct_rows_inv(Inst* insts, const int* row_inst, int seg,
-                                                                     int items, unsigned extra, long long limit) {
+                                                                     int items, unsigned extra, long long limit, int early) {
   using G = RowGeom<R, N1, N2>;
   using V = typename G::V;
   constexpr int n = G::n, LPW = G::LPW;
@@ -408,6 +409,7 @@ __global__ __launch_bounds__(RT<R>::RW * 32, 1) void k_dct_rows_inv(Inst* insts,
   if (lane == 0) mbar_init(bar);
   __syncwarp();
   overlap_wait();
+  if (early) overlap_begin();
   auto issue = [&](int it) -> bool {
     if (it >= items) return false;
     const Inst& J = insts[row_inst[seg + it]];
@@ -511,7 +513,7 @@ __device__ __forceinline__ int makhoul_inv(int i, int n) { return (i & 1) ? n - 
 // the column tiles blockIdx.x, blockIdx.x + gridDim.x, ... of the segment.
 template <class R, int N1, int N2, int CT>
 __global__ __launch_bounds__(CT, RT<R>::COL_BLOCKS) void k_dct_cols(const Inst* insts, const int* col_inst, int seg,
-                                                                    int items) {
+                                                                    int items, int early) {
   using GG = ColGeom<R, N1, N2, CT>;
   using V = typename GG::V;
   constexpr int n = GG::n, CPB = GG::CPB, CB = GG::CB, RS = GG::RS, LPW = GG::LPW;
@@ -537,6 +539,7 @@ __global__ __launch_bounds__(CT, RT<R>::COL_BLOCKS) void k_dct_cols(const Inst* 
     }
   }
   overlap_wait();
+  if (early) overlap_begin();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / N2, t = lane % N2;
   const int cp = warp * LPW + sub;  // this lane group's column pair within the block
   R* buf = sbuf + (warp * LPW + sub) * GG::LINE;  // this line's region of the tile space
@@ -692,7 +695,7 @@ struct RegDct {
   static void run_cols(otm_context* ctx, Inst* d, const int* ci, int coff, int ccnt) {
     const int grid = std::max(1, std::min(ccnt, cols_blocks_per_sm[col_variant(CT / 32)] * ctx->num_sms));
     launch_smem(ctx, sizeof(R) == 4 ? "dct32_cols" : "dct_cols", k_dct_cols<R, N1, N2, CT>, grid, CT,
-                sizeof(R) * ColGeom<R, N1, N2, CT>::SMEM, (const Inst*)d, ci, coff, ccnt);
+                sizeof(R) * ColGeom<R, N1, N2, CT>::SMEM, (const Inst*)d, ci, coff, ccnt, ctx->early);
   }
   static void run(otm_context* ctx, Inst* d, const int* ri, int roff, int rcnt, const int* ci, int coff, int ccnt,
                   int col_warps) {
@@ -704,14 +707,14 @@ struct RegDct {
     const long long limit = ctx->wait_test ? kTestWaitCycles : kWaitCycles;
     constexpr bool f = sizeof(R) == 4;
     launch_smem(ctx, f ? "dct32_rows_fwd" : "dct_rows_fwd", k_dct_rows_fwd<R, N1, N2>, grid, rw * 32, rows_smem(rw), d,
-                ri, roff, rcnt, extra, limit);
+                ri, roff, rcnt, extra, limit, ctx->early);
     switch (col_warps) {
       case 8: run_cols<256>(ctx, d, ci, coff, ccnt); break;
       case 4: run_cols<128>(ctx, d, ci, coff, ccnt); break;
       default: run_cols<64>(ctx, d, ci, coff, ccnt); break;
     }
     launch_smem(ctx, f ? "dct32_rows_inv" : "dct_rows_inv", k_dct_rows_inv<R, N1, N2>, grid, rw * 32, rows_smem(rw), d,
-                ri, roff, rcnt, extra, limit);
+                ri, roff, rcnt, extra, limit, ctx->early);
   }
 };
 template <class R, int N1, int N2>

@@ -1024,7 +1024,7 @@ static void build_bvh_order(otm_context* ctx, const double* xy, int n, int* rank
             cudaGraphNode_t loop;
             OTM_CUDA(cudaGraphAddNode(&loop, g, &last, 1, &params));
             capture(params.conditional.phGraph_out[0], nullptr, [&] {
-              const Overlap overlap(ctx, true);
+              const Overlap overlap(ctx, true, N);
               for (int l = 0; l < LEVELS_PER_BODY; ++l) level(handle, 1);
             });
             last = loop;

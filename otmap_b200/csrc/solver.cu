@@ -589,6 +589,8 @@ static void set_strips(otm_context* ctx, Workspace& ws, std::vector<Inst>& h, in
   OTM_CUDA(cudaStreamSynchronize(ctx->stream));  // the host list is released on return
   ws.split_strip0 = split0;
   ws.total_strips = strips;
+  ws.cells = 0;
+  for (const Inst& I : h) ws.cells += (long)I.n * I.n;
   ws.srows = srows;
 }
 
@@ -827,7 +829,7 @@ __global__ void k_loop_check(const Inst* insts, int count, LoopCtl* ctl, cudaGra
 // 337.9 and 335.2; split 1024^2 76.3 and 73.3, eight 272.3 and 265.5.
 static void launch_iteration(otm_context* ctx, Inst* d_insts) {
   Workspace& ws = ctx->ws();
-  const Overlap overlap(ctx, ws.total_gemm == 0 && ws.total_tc == 0);
+  const Overlap overlap(ctx, ws.total_gemm == 0 && ws.total_tc == 0, ws.cells);
   const int G = ws.total_gemm;
   if (G > 0)
     for (int s = 0; s < 4; ++s)
