@@ -605,7 +605,12 @@ static std::vector<Inst> layout_workspace(otm_context* ctx, const std::vector<in
   // the batch has blocks to spare; a batch that does not fill the GPU twice over keeps
   // 32-row strips for parallelism, and one with fewer 32-row blocks than SMs takes the
   // tallest of 16, 8 and 4 rows that gives four SMs in five a block (a lone 512^2 solve 16:
-  // sums 28 -> 24.5 us, update 21 -> 16.4 us; a lone 256^2 one 4).
+  // sums 28 -> 24.5 us, update 21 -> 16.4 us; a lone 256^2 one 4). Several instances of one
+  // register-transform size (the maps of a barycenter loss) stay at 16 rows: the height is the
+  // order of the sums, and the gradient of a map whose adjoint ends at its limit of solves turns on
+  // the last bit of the mesh (four 64^2 take 22 us per iteration so, 18 with 4 rows). So does split
+  // precision, whose FP32 fields turn any change of rounding into one of theirs (256^2 alone 37 us
+  // per iteration with 16 rows, 33 with 4).
   int srows = 32;
   {
     auto blocks = [&](int rows) {
@@ -613,10 +618,13 @@ static std::vector<Inst> layout_workspace(otm_context* ctx, const std::vector<in
       for (int n : sizes) b += strip_blocks(n, rows);
       return b;
     };
+    const bool alike = count > 1 && dct_reg_supported(sizes[0]) &&
+                       std::all_of(sizes.begin(), sizes.end(), [&](int n) { return n == sizes[0]; });
+    const int least = alike || ctx->precision == OTM_PRECISION_SPLIT ? 16 : 4;
     if (blocks(32) >= 6L * ctx->num_sms)
       srows = 64;
     else if (blocks(32) < ctx->num_sms)
-      for (srows = 16; srows > 4 && 5 * blocks(srows) < 4L * ctx->num_sms;) srows /= 2;
+      for (srows = 16; srows > least && 5 * blocks(srows) < 4L * ctx->num_sms;) srows /= 2;
   }
   for (int q = 0; q < count; ++q) {
     int n = sizes[q];
