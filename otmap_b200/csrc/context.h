@@ -102,6 +102,7 @@ struct Workspace {
   int mode = -1;       // poisson mode the layout was built for
   int precision = -1;  // precision the layout was built for
   long cells = 0;      // of all instances
+  int cluster_blocks = 0;  // blocks per instance of the one-kernel loop (0: the loop of kernels)
   int srows = 0;       // strip height of the sweeps (rule or autotuned)
   bool tuned = false;  // srows was chosen by timing (OTM_OPT_AUTOTUNE)
   int split_strip0 = 0;  // strips of split-precision instances start here (FP64 ones before)

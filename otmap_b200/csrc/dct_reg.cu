@@ -31,7 +31,7 @@
 #include <cmath>
 #include <vector>
 
-#include "engine.cuh"
+#include "cluster.cuh"
 
 namespace otm {
 namespace {
@@ -196,6 +196,166 @@ __device__ __forceinline__ V pre3(int k, R a, R b, V pt) {
   return mk2((R)0.5 * rfma(a, pt.x, b * pt.y), (R)0.5 * rfma(a, pt.y, -b * pt.x));
 }
 
+// ---- a line pair's passages between the grid's rows or columns and the registers ----
+
+// Makhoul order: sample m < n/2 is x[2m], sample m >= n/2 is x[2(n-1-m)+1]. Lane t reads the
+// pairs x[2(N2 m1 + t)], x[2(N2 m1 + t) + 1] (m1 < N1/2): the first is its own sample
+// m = N2 m1 + t, the second is sample n-1-m, which belongs to lane N2-1-t (`mirror`) at
+// m1' = N1-1-m1 and is passed there by a shuffle.
+template <class R, int N1, int N2, class V>
+__device__ __forceinline__ void rows_fwd_in(const R* xa, const R* xb, int t, int mirror, V (&v)[N1]) {
+#pragma unroll
+  for (int m1 = 0; m1 < N1 / 2; ++m1) {
+    const V pa = *reinterpret_cast<const V*>(xa + 2 * (N2 * m1 + t));
+    const V pb = *reinterpret_cast<const V*>(xb + 2 * (N2 * m1 + t));
+    v[m1] = mk2(pa.x, pb.x);
+    v[N1 - 1 - m1] = mk2(__shfl_sync(0xffffffffu, pa.y, mirror), __shfl_sync(0xffffffffu, pb.y, mirror));
+  }
+}
+
+// Coefficients of both rows from the line's spectrum (X_{n-k} is held by src_lane).
+template <class R, int N1, int N2, class V>
+__device__ __forceinline__ void rows_fwd_out(const V (&u)[N2], int t, int src_lane, const V* spt, const DctScale<R>& ds,
+                                             R* ya, R* yb) {
+#pragma unroll
+  for (int r = 0; r < N2; ++r) {
+    const V send = (t == 0) ? u[partner_reg<N2>(r, true)] : u[partner_reg<N2>(r, false)];
+    const R px = __shfl_sync(0xffffffffu, send.x, src_lane);
+    const R py = __shfl_sync(0xffffffffu, send.y, src_lane);
+    if (t < N1) {
+      const int k = t + N1 * rbrev<N2>(r);
+      const V Z = u[r];
+      const V A = mk2((R)0.5 * (Z.x + px), (R)0.5 * (Z.y - py));
+      const V B = mk2((R)0.5 * (Z.y + py), (R)0.5 * (px - Z.x));
+      const V w = spt[k];
+      const R sk = ds(k);
+      ya[k] = post2(A, w, sk);
+      yb[k] = post2(B, w, sk);
+    }
+  }
+}
+
+// The inverse line's samples from both rows' coefficients.
+template <class R, int N1, int N2, class V>
+__device__ __forceinline__ void rows_inv_in(const R* Xa, const R* Xb, int t, const V* spt, const DctScale<R>& ds,
+                                            V (&v)[N1]) {
+  constexpr int n = N1 * N2;
+#pragma unroll
+  for (int m1 = 0; m1 < N1; ++m1) {
+    const int k = N2 * m1 + t;
+    const V w = spt[k];
+    const R sk = ds(k), snk = k == 0 ? (R)0 : ds(n - k);
+    const V Wa = pre3(k, sk * Xa[k], k == 0 ? (R)0 : snk * Xa[n - k], w);
+    const V Wb = pre3(k, sk * Xb[k], k == 0 ? (R)0 : snk * Xb[n - k], w);
+    v[m1] = mk2(Wa.x - Wb.y, Wa.y + Wb.x);
+  }
+}
+
+template <class R, int N1, int N2, class V>
+__device__ __forceinline__ void rows_inv_out(const V (&u)[N2], int t, int mirror, R* xa, R* xb) {
+  // Output m = t + N1 k2 goes to x[2m] for m < n/2; its neighbour x[2m+1] is output
+  // n-1-m, held by lane N1-1-t in the register of k2' = N2-1-k2: one shuffle and a
+  // 16-byte store per pair.
+#pragma unroll
+  for (int r = 0; r < N2; ++r) {
+    if (rbrev<N2>(r) >= N2 / 2) continue;
+    const V other = u[rbrev<N2>(N2 - 1 - rbrev<N2>(r))];
+    const R qa = __shfl_sync(0xffffffffu, other.x, mirror);
+    const R qb = __shfl_sync(0xffffffffu, other.y, mirror);
+    if (t < N1) {
+      const int m = t + N1 * rbrev<N2>(r);
+      *reinterpret_cast<V*>(xa + 2 * m) = mk2(u[r].x, qa);
+      *reinterpret_cast<V*>(xb + 2 * m) = mk2(u[r].y, qb);
+    }
+  }
+}
+
+// A column pair's samples v (Makhoul order) to those of its solution x2: DCT-II (split N1 x N2),
+// division by lambda, DCT-III (split N2 x N1). buf: the line's region of 2n reals.
+template <class R, int N1, int N2, class V>
+__device__ __forceinline__ void column_solve(int t, int la, R* buf, const V* stw, const V* stw_sw, const V* spt,
+                                             const R* scos, const DctScale<R>& ds, V (&v)[N1], V (&x2)[N1]) {
+  constexpr int n = N1 * N2;
+  V* zl = reinterpret_cast<V*>(buf);
+  V u[N2];
+  fft_line<N1, N2>(t, buf, stw, false, v, u);
+  // Z_k (k = t + N1 rbrev(r)) into the line's region, then each lane separates the two
+  // spectra with Z_{n-k}, divides by lambda_kl (the (0,0) mode is dropped) and keeps
+  // s_k U_k, which goes back to the region for the partner's DCT-III input
+  __syncwarp();
+  if (t < N1) {
+#pragma unroll
+    for (int r = 0; r < N2; ++r) zl[t + N1 * rbrev<N2>(r)] = u[r];
+  }
+  __syncwarp();
+  if (t < N1) {
+    // U = X / lambda for the 2 LG values of a group of LG coefficients with one division:
+    // each lambda's reciprocal is the product of the other lambdas over the product of all
+    // (every lambda lies in (0, 4], so the products neither overflow nor underflow; the
+    // result is within about ten ulps of separate divisions, which cost several times the
+    // time and instruction footprint: 95 -> 74 us per column pass at 8 x 1024^2)
+    constexpr int LG = RT<R>::DIV_GROUP;
+    const R cla = scos[la], clb = scos[la + 1];
+#pragma unroll
+    for (int r0 = 0; r0 < N2; r0 += LG) {
+      R Xa[LG], Xb[LG], lam[2 * LG], sk[LG];
+      bool zero[LG];
+#pragma unroll
+      for (int g = 0; g < LG; ++g) {
+        const int r = r0 + g;
+        const int k = t + N1 * rbrev<N2>(r);
+        const V Z = u[r], P = zl[(n - k) & (n - 1)];
+        const V A = mk2((R)0.5 * (Z.x + P.x), (R)0.5 * (Z.y - P.y));
+        const V B = mk2((R)0.5 * (Z.y + P.y), (R)0.5 * (P.x - Z.x));
+        const V w = spt[k];
+        sk[g] = ds(k);
+        Xa[g] = post2(A, w, sk[g]);
+        Xb[g] = post2(B, w, sk[g]);
+        const R ck = scos[k];
+        zero[g] = (k == 0 && la == 0);  // the (0,0) mode is dropped
+        lam[2 * g] = zero[g] ? (R)1 : (R)2 - (R)2 * ck * cla;
+        lam[2 * g + 1] = (R)2 - (R)2 * ck * clb;
+      }
+      R pre[2 * LG + 1], suf[2 * LG + 1];
+      pre[0] = (R)1;
+      suf[2 * LG] = (R)1;
+#pragma unroll
+      for (int j = 0; j < 2 * LG; ++j) pre[j + 1] = pre[j] * lam[j];
+#pragma unroll
+      for (int j = 2 * LG - 1; j >= 0; --j) suf[j] = suf[j + 1] * lam[j];
+      const R inv = (R)1 / pre[2 * LG];
+#pragma unroll
+      for (int g = 0; g < LG; ++g) {
+        const R ia = (pre[2 * g] * suf[2 * g + 1]) * inv;
+        const R ib = (pre[2 * g + 1] * suf[2 * g + 2]) * inv;
+        const R Ua = zero[g] ? (R)0 : Xa[g] * ia;
+        const R Ub = Xb[g] * ib;
+        u[r0 + g] = mk2(sk[g] * Ua, sk[g] * Ub);
+      }
+    }
+  }
+  __syncwarp();
+  if (t < N1) {
+#pragma unroll
+    for (int r = 0; r < N2; ++r) zl[t + N1 * rbrev<N2>(r)] = u[r];
+  }
+  __syncwarp();
+  // inverse DCT-III of the two columns, split N2 x N1: lane t (< N1) takes the samples
+  // k = t + N1 m1 it holds; U_{n-k} comes from the region
+  V w2[N2];
+#pragma unroll
+  for (int m1 = 0; m1 < N2; ++m1) {
+    const int k = t < N1 ? t + N1 * m1 : 0;
+    const V a = u[rbrev<N2>(m1)];
+    const V bb = zl[(n - k) & (n - 1)];
+    const V w = spt[k];
+    const V Wa = pre3(k, a.x, bb.x, w), Wb = pre3(k, a.y, bb.y, w);
+    w2[m1] = mk2(Wa.x - Wb.y, Wa.y + Wb.x);
+  }
+  __syncwarp();  // the region's spectrum is read: it becomes the transpose buffer
+  fft_line<N2, N1>(t, buf, stw_sw, true, w2, x2);
+}
+
 // ---- row passes: software-pipelined over the warp's work items ----
 //
 // A work item is LPW consecutive row pairs (one per FFT line of the warp), 2*LPW whole
@@ -343,43 +503,17 @@ __global__ __launch_bounds__(RT<R>::RW * 32, 1) void k_dct_rows_fwd(Inst* insts,
       return;
     }
     phase ^= 1;
-    // Makhoul order: sample m < n/2 is x[2m], sample m >= n/2 is x[2(n-1-m)+1]. Lane t
-    // reads the pairs x[2(N2 m1 + t)], x[2(N2 m1 + t) + 1] (m1 < N1/2): the first is its
-    // own sample m = N2 m1 + t, the second is sample n-1-m, which belongs to lane
-    // N2-1-t at m1' = N1-1-m1 and is passed there by a shuffle.
     const R* xa = data + sub * 2 * n;
-    const R* xb = xa + n;
     V v[N1];
     V u[N2];
-#pragma unroll
-    for (int m1 = 0; m1 < N1 / 2; ++m1) {
-      const V pa = *reinterpret_cast<const V*>(xa + 2 * (N2 * m1 + t));
-      const V pb = *reinterpret_cast<const V*>(xb + 2 * (N2 * m1 + t));
-      v[m1] = mk2(pa.x, pb.x);
-      v[N1 - 1 - m1] = mk2(__shfl_sync(0xffffffffu, pa.y, mirror), __shfl_sync(0xffffffffu, pb.y, mirror));
-    }
+    rows_fwd_in<R, N1, N2>(xa, xa + n, t, mirror, v);
     __syncwarp();
     pending = issue(next);  // the next item's rows arrive while this one is transformed
     const int row = (seg + item - I.row0) * 2 * LPW + 2 * sub;
     R* ya = reinterpret_cast<R*>(I.t1) + (size_t)row * n;
     R* yb = ya + n;
     fft_line<N1, N2>(t, buf, tab, false, v, u);
-#pragma unroll
-    for (int r = 0; r < N2; ++r) {
-      const V send = (t == 0) ? u[partner_reg<N2>(r, true)] : u[partner_reg<N2>(r, false)];
-      const R px = __shfl_sync(0xffffffffu, send.x, src_lane);
-      const R py = __shfl_sync(0xffffffffu, send.y, src_lane);
-      if (t < N1) {
-        const int k = t + N1 * rbrev<N2>(r);
-        const V Z = u[r];
-        const V A = mk2((R)0.5 * (Z.x + px), (R)0.5 * (Z.y - py));
-        const V B = mk2((R)0.5 * (Z.y + py), (R)0.5 * (px - Z.x));
-        const V w = spt[k];
-        const R sk = ds(k);
-        ya[k] = post2(A, w, sk);
-        yb[k] = post2(B, w, sk);
-      }
-    }
+    rows_fwd_out<R, N1, N2>(u, t, src_lane, spt, ds, ya, yb);
     item = next;
   }
   overlap_begin();
@@ -439,39 +573,16 @@ __global__ __launch_bounds__(RT<R>::RW * 32, 1) void k_dct_rows_inv(Inst* insts,
     }
     phase ^= 1;
     const R* Xa = data + sub * 2 * n;
-    const R* Xb = Xa + n;
     V v[N1];
     V u[N2];
-#pragma unroll
-    for (int m1 = 0; m1 < N1; ++m1) {
-      const int k = N2 * m1 + t;
-      const V w = spt[k];
-      const R sk = ds(k), snk = k == 0 ? (R)0 : ds(n - k);
-      const V Wa = pre3(k, sk * Xa[k], k == 0 ? (R)0 : snk * Xa[n - k], w);
-      const V Wb = pre3(k, sk * Xb[k], k == 0 ? (R)0 : snk * Xb[n - k], w);
-      v[m1] = mk2(Wa.x - Wb.y, Wa.y + Wb.x);
-    }
+    rows_inv_in<R, N1, N2>(Xa, Xa + n, t, spt, ds, v);
     __syncwarp();
     pending = issue(next);
     const int row = (seg + item - I.row0) * 2 * LPW + 2 * sub;
     R* xa = reinterpret_cast<R*>(I.dhat) + (size_t)row * n;
     R* xb = xa + n;
     fft_line<N1, N2>(t, buf, tab, true, v, u);
-    // Output m = t + N1 k2 goes to x[2m] for m < n/2; its neighbour x[2m+1] is output
-    // n-1-m, held by lane N1-1-t in the register of k2' = N2-1-k2: one shuffle and a
-    // 16-byte store per pair.
-#pragma unroll
-    for (int r = 0; r < N2; ++r) {
-      if (rbrev<N2>(r) >= N2 / 2) continue;
-      const V other = u[rbrev<N2>(N2 - 1 - rbrev<N2>(r))];
-      const R qa = __shfl_sync(0xffffffffu, other.x, mirror);
-      const R qb = __shfl_sync(0xffffffffu, other.y, mirror);
-      if (t < N1) {
-        const int m = t + N1 * rbrev<N2>(r);
-        *reinterpret_cast<V*>(xa + 2 * m) = mk2(u[r].x, qa);
-        *reinterpret_cast<V*>(xb + 2 * m) = mk2(u[r].y, qb);
-      }
-    }
+    rows_inv_out<R, N1, N2>(u, t, mirror, xa, xb);
     item = next;
   }
   overlap_begin();
@@ -543,7 +654,6 @@ __global__ __launch_bounds__(CT, RT<R>::COL_BLOCKS) void k_dct_cols(const Inst* 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / N2, t = lane % N2;
   const int cp = warp * LPW + sub;  // this lane group's column pair within the block
   R* buf = sbuf + (warp * LPW + sub) * GG::LINE;  // this line's region of the tile space
-  V* zl = reinterpret_cast<V*>(buf);
   for (int b = blockIdx.x; b < items; b += gridDim.x) {
     const int item = seg + b;
     const Inst& I = insts[col_inst[item]];
@@ -566,88 +676,12 @@ __global__ __launch_bounds__(CT, RT<R>::COL_BLOCKS) void k_dct_cols(const Inst* 
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
     V v[N1];
-    V u[N2];
-    // forward DCT-II of the two columns (one complex line; samples in Makhoul order)
+    // the two columns (one complex line; samples in Makhoul order)
 #pragma unroll
     for (int m1 = 0; m1 < N1; ++m1) v[m1] = tile[(N2 * m1 + t) * RS + cp];
     __syncthreads();  // the tile's space now holds the lines' regions
-    fft_line<N1, N2>(t, buf, stw, false, v, u);
-    // Z_k (k = t + N1 rbrev(r)) into the line's region, then each lane separates the two
-    // spectra with Z_{n-k}, divides by lambda_kl (the (0,0) mode is dropped) and keeps
-    // s_k U_k, which goes back to the region for the partner's DCT-III input
-    __syncwarp();
-    if (t < N1) {
-#pragma unroll
-      for (int r = 0; r < N2; ++r) zl[t + N1 * rbrev<N2>(r)] = u[r];
-    }
-    __syncwarp();
-    if (t < N1) {
-      // U = X / lambda for the 2 LG values of a group of LG coefficients with one division:
-      // each lambda's reciprocal is the product of the other lambdas over the product of all
-      // (every lambda lies in (0, 4], so the products neither overflow nor underflow; the
-      // result is within about ten ulps of separate divisions, which cost several times the
-      // time and instruction footprint: 95 -> 74 us per column pass at 8 x 1024^2)
-      constexpr int LG = RT<R>::DIV_GROUP;
-      const R cla = scos[la], clb = scos[la + 1];
-#pragma unroll
-      for (int r0 = 0; r0 < N2; r0 += LG) {
-        R Xa[LG], Xb[LG], lam[2 * LG], sk[LG];
-        bool zero[LG];
-#pragma unroll
-        for (int g = 0; g < LG; ++g) {
-          const int r = r0 + g;
-          const int k = t + N1 * rbrev<N2>(r);
-          const V Z = u[r], P = zl[(n - k) & (n - 1)];
-          const V A = mk2((R)0.5 * (Z.x + P.x), (R)0.5 * (Z.y - P.y));
-          const V B = mk2((R)0.5 * (Z.y + P.y), (R)0.5 * (P.x - Z.x));
-          const V w = spt[k];
-          sk[g] = ds(k);
-          Xa[g] = post2(A, w, sk[g]);
-          Xb[g] = post2(B, w, sk[g]);
-          const R ck = scos[k];
-          zero[g] = (k == 0 && la == 0);  // the (0,0) mode is dropped
-          lam[2 * g] = zero[g] ? (R)1 : (R)2 - (R)2 * ck * cla;
-          lam[2 * g + 1] = (R)2 - (R)2 * ck * clb;
-        }
-        R pre[2 * LG + 1], suf[2 * LG + 1];
-        pre[0] = (R)1;
-        suf[2 * LG] = (R)1;
-#pragma unroll
-        for (int j = 0; j < 2 * LG; ++j) pre[j + 1] = pre[j] * lam[j];
-#pragma unroll
-        for (int j = 2 * LG - 1; j >= 0; --j) suf[j] = suf[j + 1] * lam[j];
-        const R inv = (R)1 / pre[2 * LG];
-#pragma unroll
-        for (int g = 0; g < LG; ++g) {
-          const R ia = (pre[2 * g] * suf[2 * g + 1]) * inv;
-          const R ib = (pre[2 * g + 1] * suf[2 * g + 2]) * inv;
-          const R Ua = zero[g] ? (R)0 : Xa[g] * ia;
-          const R Ub = Xb[g] * ib;
-          u[r0 + g] = mk2(sk[g] * Ua, sk[g] * Ub);
-        }
-      }
-    }
-    __syncwarp();
-    if (t < N1) {
-#pragma unroll
-      for (int r = 0; r < N2; ++r) zl[t + N1 * rbrev<N2>(r)] = u[r];
-    }
-    __syncwarp();
-    // inverse DCT-III of the two columns, split N2 x N1: lane t (< N1) takes the samples
-    // k = t + N1 m1 it holds; U_{n-k} comes from the region
-    V w2[N2];
     V x2[N1];
-#pragma unroll
-    for (int m1 = 0; m1 < N2; ++m1) {
-      const int k = t < N1 ? t + N1 * m1 : 0;
-      const V a = u[rbrev<N2>(m1)];
-      const V bb = zl[(n - k) & (n - 1)];
-      const V w = spt[k];
-      const V Wa = pre3(k, a.x, bb.x, w), Wb = pre3(k, a.y, bb.y, w);
-      w2[m1] = mk2(Wa.x - Wb.y, Wa.y + Wb.x);
-    }
-    __syncwarp();  // the region's spectrum is read: it becomes the transpose buffer
-    fft_line<N2, N1>(t, buf, stw_sw, true, w2, x2);
+    column_solve<R, N1, N2>(t, la, buf, stw, stw_sw, spt, scos, ds, v, x2);
     __syncthreads();  // every warp is done with its transpose buffer: the space is the tile again
     // output sample m = t + N2 rbrev<N1>(r) (Makhoul order) of both columns
 #pragma unroll
@@ -721,6 +755,74 @@ template <class R, int N1, int N2>
 int RegDct<R, N1, N2>::rows_blocks_per_sm = 1;
 template <class R, int N1, int N2>
 int RegDct<R, N1, N2>::cols_blocks_per_sm[COL_VARIANTS] = {1, 1, 1};
+
+// ---- the passes for the one-cluster solve (cluster.cuh), on the tables of k_dct_cols ----
+
+template <int N1, int N2>
+struct ClusterRegDct {
+  static constexpr int n = N1 * N2, LPW = 32 / N2, ITEMS = n / (2 * LPW);  // row or column pairs by warps
+  static_assert(LPW * 2 * n * sizeof(double) <= CL_WARP_BYTES, "a warp's lines fit in its region");
+  static int table_bytes(int) { return sizeof(double) * 7 * n; }
+  double2 *stw, *stw_sw, *spt;
+  double* scos;
+  const int sub = (threadIdx.x & 31) / N2, t = (threadIdx.x & 31) % N2, first = sub * N2;
+  const DctScale<double> ds{n};
+  __device__ __forceinline__ ClusterRegDct(const Inst& I, unsigned char* smem) {
+    stw = reinterpret_cast<double2*>(smem);
+    stw_sw = stw + n;
+    spt = stw_sw + n;
+    scos = reinterpret_cast<double*>(spt + n);
+    for (int e = threadIdx.x; e < n; e += CL_T) {
+      stw[e] = I.tw[(n >> 1) + e];
+      stw_sw[e] = I.tw[(n >> 1) + n + e];
+      spt[e] = I.pt[e];
+      scos[e] = I.cosk[e];
+    }
+  }
+  __device__ __forceinline__ double* line(const ClusterBlock& B) const {
+    return reinterpret_cast<double*>(B.region()) + sub * 2 * n;
+  }
+  __device__ __forceinline__ void rows_fwd(const ClusterBlock& B, int it) const {
+    const double* r = B.I.r[it % 3];
+    double* T = B.I.t1;
+    B.items(ITEMS, [&](int item) {
+      const size_t row = (size_t)(2 * (item * LPW + sub)) * n;
+      double2 v[N1], u[N2];
+      rows_fwd_in<double, N1, N2>(r + row, r + row + n, t, first + (N2 - 1 - t), v);
+      fft_line<N1, N2>(t, line(B), stw, false, v, u);
+      rows_fwd_out<double, N1, N2>(u, t, first + (t < N1 ? (N1 - t) % N1 : 0), spt, ds, T + row, T + row + n);
+    });
+  }
+  __device__ __forceinline__ void cols(const ClusterBlock& B) const {
+    B.items(ITEMS, [&](int item) {
+      const int la = 2 * (item * LPW + sub);
+      double* T = B.I.t1 + la;
+      // sample m of a column is row 2m, or 2(n-1-m)+1 in the upper half
+      auto at = [&](int m) {
+        return reinterpret_cast<double2*>(T + (size_t)(m < n / 2 ? 2 * m : 2 * (n - 1 - m) + 1) * n);
+      };
+      double2 v[N1], x[N1];
+#pragma unroll
+      for (int m1 = 0; m1 < N1; ++m1) v[m1] = *at(N2 * m1 + t);
+      column_solve<double, N1, N2>(t, la, line(B), stw, stw_sw, spt, scos, ds, v, x);
+#pragma unroll
+      for (int r = 0; r < N1; ++r) *at(t + N2 * rbrev<N1>(r)) = x[r];
+      __syncwarp();
+    });
+  }
+  __device__ __forceinline__ void rows_inv(const ClusterBlock& B) const {
+    const double* T = B.I.t1;
+    double* d = B.I.dhat;
+    B.items(ITEMS, [&](int item) {
+      const size_t row = (size_t)(2 * (item * LPW + sub)) * n;
+      double2 v[N1], u[N2];
+      rows_inv_in<double, N1, N2>(T + row, T + row + n, t, spt, ds, v);
+      fft_line<N1, N2>(t, line(B), stw, true, v, u);
+      rows_inv_out<double, N1, N2>(u, t, first + (t < N1 ? N1 - 1 - t : 0), d + row, d + row + n);
+    });
+  }
+};
+using ClusterDct64 = ClusterRegDct<8, 8>;
 
 }  // namespace
 
@@ -832,6 +934,15 @@ void dct_reg_run(otm_context* ctx, int n, bool fp32, Inst* d_insts, const int* r
     dct_reg_run_t<float>(ctx, n, d_insts, row_inst, roff, rcnt, col_inst, coff, ccnt, col_warps);
   else
     dct_reg_run_t<double>(ctx, n, d_insts, row_inst, roff, rcnt, col_inst, coff, ccnt, col_warps);
+}
+
+int dct_reg_cluster_blocks(otm_context* ctx, int n, int count) {
+  return n == ClusterDct64::n ? cluster_blocks<ClusterDct64>(ctx, n, count) : 0;
+}
+
+void dct_reg_cluster(otm_context* ctx, int n, int count, int blocks, Inst* d_insts, double* partials) {
+  dct_reg_attrs(ctx->device);
+  cluster_launch<ClusterDct64>(ctx, n, count, blocks, d_insts, partials);
 }
 
 }  // namespace otm

@@ -169,6 +169,12 @@ void dct_tc_run(otm_context* ctx, Inst* d_insts, const int* tc_inst, int base, i
 // before any stream capture).
 void sweep_attrs(int device);
 void dct_reg_attrs(int device);
+// The whole loop of `count` small instances of size n in FP64, one cluster of `blocks` blocks each
+// (cluster.cuh); blocks 0: not for this size or batch.
+int dct_reg_cluster_blocks(otm_context* ctx, int n, int count);
+void dct_reg_cluster(otm_context* ctx, int n, int count, int blocks, Inst* d_insts, double* partials);
+int poisson_cluster_blocks(otm_context* ctx, int n, int count);
+void poisson_cluster(otm_context* ctx, int n, int count, int blocks, Inst* d_insts, double* partials);
 void poisson_fft_attrs(int device);
 
 // Two-pass stencil sweep of an iteration (stencil.cu).

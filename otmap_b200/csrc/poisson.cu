@@ -41,7 +41,7 @@
 #include <cmath>
 #include <vector>
 
-#include "engine.cuh"
+#include "cluster.cuh"
 
 namespace otm {
 namespace {
@@ -150,45 +150,57 @@ __device__ __forceinline__ int place(int t, int q) {
   constexpr int S = L > 8 ? L / 8 : 1;
   return L > 8 ? (t / S) * L + t % S + q * S : 8 * t + q;
 }
+// Where a line's threads live and its tables lie.
+struct BlockLine {  // in the block of one of the kernels below; tables in global memory
+  static __device__ __forceinline__ void sync() { __syncthreads(); }
+  static __device__ __forceinline__ double2 table(const double2* p) { return __ldg(p); }
+  static __device__ __forceinline__ void computed() { overlap_begin(); }
+};
+struct WarpLine {  // in a warp of the one-cluster solve; tables in shared memory
+  static __device__ __forceinline__ void sync() { __syncwarp(); }
+  static __device__ __forceinline__ double2 table(const double2* p) { return *p; }
+  static __device__ __forceinline__ void computed() {}
+};
+
 // Moves the elements from the places of pass A to those of pass B.
-template <int A, int B>
+template <int A, int B, class Line>
 __device__ __forceinline__ void exchange(double2 (&v)[8], int t, double2* sm) {
-  __syncthreads();
+  Line::sync();
 #pragma unroll
   for (int q = 0; q < 8; ++q) sm[slot(place<A>(t, q))] = v[q];
-  __syncthreads();
+  Line::sync();
 #pragma unroll
   for (int q = 0; q < 8; ++q) v[q] = sm[slot(place<B>(t, q))];
 }
 
 // Forward transform: element q of thread t is x[t + q M/8] on entry and at position 8 t + q
 // of the digit-reversed order on return.
-template <int L>
+template <int L, class Line>
 __device__ __forceinline__ void fft_fwd(double2 (&v)[8], int t, double2* sm, const double2* __restrict__ tw) {
   if constexpr (L > 8) {
     constexpr int S = L / 8;
     double2 w[7];
 #pragma unroll
-    for (int r = 1; r < 8; ++r) w[r - 1] = __ldg(&tw[(r - 1) * S + t % S]);
+    for (int r = 1; r < 8; ++r) w[r - 1] = Line::table(&tw[(r - 1) * S + t % S]);
     dft8<false>(v);
 #pragma unroll
     for (int r = 1; r < 8; ++r) v[r] = cmul(v[r], w[r - 1]);
-    exchange<L, S>(v, t, sm);
-    fft_fwd<S>(v, t, sm, tw + 7 * S);
+    exchange<L, S, Line>(v, t, sm);
+    fft_fwd<S, Line>(v, t, sm, tw + 7 * S);
   } else {
     last_pass<L, false>(v);
   }
 }
 // Its inverse (unnormalised), from the digit-reversed order back to x[t + q M/8].
-template <int L>
+template <int L, class Line>
 __device__ __forceinline__ void fft_inv(double2 (&v)[8], int t, double2* sm, const double2* __restrict__ tw) {
   if constexpr (L > 8) {
     constexpr int S = L / 8;
-    fft_inv<S>(v, t, sm, tw + 7 * S);
+    fft_inv<S, Line>(v, t, sm, tw + 7 * S);
     double2 w[7];
 #pragma unroll
-    for (int r = 1; r < 8; ++r) w[r - 1] = __ldg(&tw[(r - 1) * S + t % S]);
-    exchange<S, L>(v, t, sm);
+    for (int r = 1; r < 8; ++r) w[r - 1] = Line::table(&tw[(r - 1) * S + t % S]);
+    exchange<S, L, Line>(v, t, sm);
 #pragma unroll
     for (int r = 1; r < 8; ++r) v[r] = cmulc(v[r], w[r - 1]);
     dft8<true>(v);
@@ -216,32 +228,32 @@ struct Tables {
 
 // n-point DFT of the line pair: v[q] = x[t + q T] (zero from n on) on entry; Z_k, k < n, in
 // sm[slot(k)] on return (after the closing barrier).
-template <int M, bool CHIRP>
+template <int M, bool CHIRP, class Line>
 __device__ __forceinline__ void line_dft(double2 (&v)[8], int n, int t, double2* sm, const Tables<M>& tab) {
   constexpr int T = M / 8;
   if (CHIRP) {
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int m = t + q * T;
-      v[q] = m < n ? cmul(v[q], __ldg(&tab.chirp[m])) : make_double2(0.0, 0.0);
+      v[q] = m < n ? cmul(v[q], Line::table(&tab.chirp[m])) : make_double2(0.0, 0.0);
     }
-    fft_fwd<M>(v, t, sm, tab.tw);
+    fft_fwd<M, Line>(v, t, sm, tab.tw);
 #pragma unroll
-    for (int q = 0; q < 8; ++q) v[q] = cmul(v[q], __ldg(&tab.kernel[q * T + t]));
-    fft_inv<M>(v, t, sm, tab.tw);
-    __syncthreads();
+    for (int q = 0; q < 8; ++q) v[q] = cmul(v[q], Line::table(&tab.kernel[q * T + t]));
+    fft_inv<M, Line>(v, t, sm, tab.tw);
+    Line::sync();
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int k = t + q * T;
-      if (k < n) sm[slot(k)] = cmul(v[q], __ldg(&tab.chirp[k]));
+      if (k < n) sm[slot(k)] = cmul(v[q], Line::table(&tab.chirp[k]));
     }
   } else {
-    fft_fwd<M>(v, t, sm, tab.tw);
-    __syncthreads();
+    fft_fwd<M, Line>(v, t, sm, tab.tw);
+    Line::sync();
 #pragma unroll
     for (int q = 0; q < 8; ++q) sm[slot(frequency<M>(8 * t + q))] = v[q];
   }
-  __syncthreads();
+  Line::sync();
 }
 
 // Source of sample m of the reordered sequence.
@@ -261,6 +273,135 @@ __device__ __forceinline__ double2 dct3_pre(int k, double2 y, double2 ym, double
   return make_double2(ax - by, -(ay + bx));
 }
 
+// ---- the passes for one line pair ----
+
+// Rows i and i + 1 of src (n x n) -> their coefficients in T.
+template <int M, bool CHIRP, class Line>
+__device__ __forceinline__ void row_pair_fwd(const double* src, double* T, int n, int i, int t, double2* sm,
+                                             const Tables<M>& tab, const double2* pt) {
+  constexpr int LT = M / 8;
+  const bool a = i < n, b = i + 1 < n;
+  double2 v[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int m = t + q * LT;
+    v[q] = make_double2(0.0, 0.0);
+    if (m < n) {
+      const double* p = src + (size_t)i * n + makhoul(m, n);
+      if (a) v[q].x = p[0];
+      if (b) v[q].y = p[n];
+    }
+  }
+  line_dft<M, CHIRP, Line>(v, n, t, sm, tab);
+  Line::computed();
+  const double s0 = sqrt(1.0 / n), s1 = sqrt(2.0 / n);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int k = t + q * LT;
+    if (k >= n) continue;
+    const double2 X = dct2_post(sm[slot(k)], sm[slot(k ? n - k : 0)], Line::table(&pt[k]), k ? s1 : s0);
+    if (a) T[(size_t)i * n + k] = X.x;
+    if (b) T[(size_t)(i + 1) * n + k] = X.y;
+  }
+}
+
+// Columns l and l + 1 of T, in place: coefficients, division by lambda, and back.
+template <int M, bool CHIRP, class Line>
+__device__ __forceinline__ void column_pair(double* T, int n, int l, int t, double2* sm, const Tables<M>& tab,
+                                            const double2* pt, const double* cosk) {
+  constexpr int LT = M / 8;
+  const bool a = l < n, b = l + 1 < n;
+  double2 v[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int m = t + q * LT;
+    v[q] = make_double2(0.0, 0.0);
+    if (m < n) {
+      const double* p = T + (size_t)makhoul(m, n) * n + l;
+      if (a) v[q].x = p[0];
+      if (b) v[q].y = p[1];
+    }
+  }
+  line_dft<M, CHIRP, Line>(v, n, t, sm, tab);
+  // the coefficients over lambda, times s_k for the way back
+  const double s0 = sqrt(1.0 / n), s1 = sqrt(2.0 / n);
+  const double ca = a ? cosk[l] : 0.0, cb = b ? cosk[l + 1] : 0.0;
+  double2 u[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int k = t + q * LT;
+    u[q] = make_double2(0.0, 0.0);
+    if (k >= n) continue;
+    const double sk = k ? s1 : s0, ck = cosk[k];
+    const double2 X = dct2_post(sm[slot(k)], sm[slot(k ? n - k : 0)], Line::table(&pt[k]), sk);
+    const double la = 2.0 - 2.0 * ck * ca, lb = 2.0 - 2.0 * ck * cb;
+    u[q] = make_double2(k == 0 && l == 0 ? 0.0 : sk * (X.x / la), sk * (X.y / lb));
+  }
+  Line::sync();
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int k = t + q * LT;
+    if (k < n) sm[slot(k)] = u[q];
+  }
+  Line::sync();
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int k = t + q * LT;
+    v[q] = make_double2(0.0, 0.0);
+    if (k < n) v[q] = dct3_pre(k, u[q], sm[slot(k ? n - k : 0)], Line::table(&pt[k]));
+  }
+  line_dft<M, CHIRP, Line>(v, n, t, sm, tab);
+  Line::computed();
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int m = t + q * LT;
+    if (m >= n) continue;
+    const double2 z = sm[slot(m)];
+    double* p = T + (size_t)makhoul(m, n) * n + l;
+    if (a) p[0] = z.x;
+    if (b) p[1] = -z.y;
+  }
+}
+
+// Rows i and i + 1 of T -> their samples in out.
+template <int M, bool CHIRP, class Line>
+__device__ __forceinline__ void row_pair_inv(const double* T, double* out, int n, int i, int t, double2* sm,
+                                             const Tables<M>& tab, const double2* pt) {
+  constexpr int LT = M / 8;
+  const bool a = i < n, b = i + 1 < n;
+  const double s0 = sqrt(1.0 / n), s1 = sqrt(2.0 / n);
+  double2 v[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int k = t + q * LT;
+    v[q] = make_double2(0.0, 0.0);
+    if (k >= n) continue;
+    const double* p = T + (size_t)i * n;
+    const double sk = k ? s1 : s0;
+    double2 y = make_double2(0.0, 0.0), ym = y;
+    if (a) {
+      y.x = sk * p[k];
+      if (k) ym.x = s1 * p[n - k];
+    }
+    if (b) {
+      y.y = sk * p[n + k];
+      if (k) ym.y = s1 * p[n + n - k];
+    }
+    v[q] = dct3_pre(k, y, ym, Line::table(&pt[k]));
+  }
+  line_dft<M, CHIRP, Line>(v, n, t, sm, tab);
+  Line::computed();
+  // sample j of a row is element j/2 or n-1-j/2 of the reordered sequence
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int j = t + q * LT;
+    if (j >= n) continue;
+    const double2 z = sm[slot((j & 1) ? n - 1 - (j >> 1) : (j >> 1))];
+    if (a) out[(size_t)i * n + j] = z.x;
+    if (b) out[(size_t)(i + 1) * n + j] = -z.y;
+  }
+}
+
 template <int M, bool CHIRP>
 __global__ __launch_bounds__(Geom<M, false>::THREADS, Geom<M, false>::MIN_BLOCKS) void k_fft_rows_fwd(const Inst* insts, const int* row_inst, int seg) {
   using G = Geom<M, false>;
@@ -273,30 +414,7 @@ __global__ __launch_bounds__(Geom<M, false>::THREADS, Geom<M, false>::MIN_BLOCKS
   const int n = I.n, line = threadIdx.x / T, t = threadIdx.x % T;
   const int i = 2 * ((item - I.row0) * G::LB + line);  // rows i and i + 1
   double2* sm = smem + line * G::SLOTS;
-  const double* src = I.r[I.it % 3];
-  const bool a = i < n, b = i + 1 < n;
-  double2 v[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int m = t + q * T;
-    v[q] = make_double2(0.0, 0.0);
-    if (m < n) {
-      const double* p = src + (size_t)i * n + makhoul(m, n);
-      if (a) v[q].x = p[0];
-      if (b) v[q].y = p[n];
-    }
-  }
-  line_dft<M, CHIRP>(v, n, t, sm, Tables<M>(I.tw));
-  overlap_begin();
-  const double s0 = sqrt(1.0 / n), s1 = sqrt(2.0 / n);
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int k = t + q * T;
-    if (k >= n) continue;
-    const double2 X = dct2_post(sm[slot(k)], sm[slot(k ? n - k : 0)], __ldg(&I.pt[k]), k ? s1 : s0);
-    if (a) I.t1[(size_t)i * n + k] = X.x;
-    if (b) I.t1[(size_t)(i + 1) * n + k] = X.y;
-  }
+  row_pair_fwd<M, CHIRP, BlockLine>(I.r[I.it % 3], I.t1, n, i, t, sm, Tables<M>(I.tw), I.pt);
 }
 
 // In place on t1, two adjacent columns per line; consecutive threads take the block's lines
@@ -313,58 +431,7 @@ __global__ __launch_bounds__(Geom<M, true>::THREADS, Geom<M, true>::MIN_BLOCKS) 
   const int n = I.n, line = threadIdx.x % LB, t = threadIdx.x / LB;
   const int l = 2 * ((item - I.col0) * LB + line);  // columns l and l + 1
   double2* sm = smem + line * G::SLOTS;
-  const bool a = l < n, b = l + 1 < n;
-  const Tables<M> tab(I.tw);
-  double2 v[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int m = t + q * T;
-    v[q] = make_double2(0.0, 0.0);
-    if (m < n) {
-      const double* p = I.t1 + (size_t)makhoul(m, n) * n + l;
-      if (a) v[q].x = p[0];
-      if (b) v[q].y = p[1];
-    }
-  }
-  line_dft<M, CHIRP>(v, n, t, sm, tab);
-  // the coefficients over lambda, times s_k for the way back
-  const double s0 = sqrt(1.0 / n), s1 = sqrt(2.0 / n);
-  const double ca = a ? I.cosk[l] : 0.0, cb = b ? I.cosk[l + 1] : 0.0;
-  double2 u[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int k = t + q * T;
-    u[q] = make_double2(0.0, 0.0);
-    if (k >= n) continue;
-    const double sk = k ? s1 : s0, ck = I.cosk[k];
-    const double2 X = dct2_post(sm[slot(k)], sm[slot(k ? n - k : 0)], __ldg(&I.pt[k]), sk);
-    const double la = 2.0 - 2.0 * ck * ca, lb = 2.0 - 2.0 * ck * cb;
-    u[q] = make_double2(k == 0 && l == 0 ? 0.0 : sk * (X.x / la), sk * (X.y / lb));
-  }
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int k = t + q * T;
-    if (k < n) sm[slot(k)] = u[q];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int k = t + q * T;
-    v[q] = make_double2(0.0, 0.0);
-    if (k < n) v[q] = dct3_pre(k, u[q], sm[slot(k ? n - k : 0)], __ldg(&I.pt[k]));
-  }
-  line_dft<M, CHIRP>(v, n, t, sm, tab);
-  overlap_begin();
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int m = t + q * T;
-    if (m >= n) continue;
-    const double2 z = sm[slot(m)];
-    double* p = I.t1 + (size_t)makhoul(m, n) * n + l;
-    if (a) p[0] = z.x;
-    if (b) p[1] = -z.y;
-  }
+  column_pair<M, CHIRP, BlockLine>(I.t1, n, l, t, sm, Tables<M>(I.tw), I.pt, I.cosk);
 }
 
 template <int M, bool CHIRP>
@@ -379,39 +446,49 @@ __global__ __launch_bounds__(Geom<M, false>::THREADS, Geom<M, false>::MIN_BLOCKS
   const int n = I.n, line = threadIdx.x / T, t = threadIdx.x % T;
   const int i = 2 * ((item - I.row0) * G::LB + line);
   double2* sm = smem + line * G::SLOTS;
-  const bool a = i < n, b = i + 1 < n;
-  const double s0 = sqrt(1.0 / n), s1 = sqrt(2.0 / n);
-  double2 v[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int k = t + q * T;
-    v[q] = make_double2(0.0, 0.0);
-    if (k >= n) continue;
-    const double* p = I.t1 + (size_t)i * n;
-    const double sk = k ? s1 : s0;
-    double2 y = make_double2(0.0, 0.0), ym = y;
-    if (a) {
-      y.x = sk * p[k];
-      if (k) ym.x = s1 * p[n - k];
-    }
-    if (b) {
-      y.y = sk * p[n + k];
-      if (k) ym.y = s1 * p[n + n - k];
-    }
-    v[q] = dct3_pre(k, y, ym, __ldg(&I.pt[k]));
-  }
-  line_dft<M, CHIRP>(v, n, t, sm, Tables<M>(I.tw));
-  overlap_begin();
-  // sample j of a row is element j/2 or n-1-j/2 of the reordered sequence
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int j = t + q * T;
-    if (j >= n) continue;
-    const double2 z = sm[slot((j & 1) ? n - 1 - (j >> 1) : (j >> 1))];
-    if (a) I.dhat[(size_t)i * n + j] = z.x;
-    if (b) I.dhat[(size_t)(i + 1) * n + j] = -z.y;
-  }
+  row_pair_inv<M, CHIRP, BlockLine>(I.t1, I.dhat, n, i, t, sm, Tables<M>(I.tw), I.pt);
 }
+
+// ---- the passes for the one-cluster solve (cluster.cuh): lines of at most a warp ----
+
+template <int M, bool CHIRP>
+struct ClusterFft {
+  static constexpr int T = M / 8, LPW = 32 / T, SLOTS = Geom<M, false>::SLOTS;
+  static_assert(T <= 32 && LPW * SLOTS * sizeof(double2) <= CL_WARP_BYTES, "a warp's lines fit in its region");
+  static __host__ __device__ int entries(int n) { return Passes<M>::twiddles() + (CHIRP ? M + n : 0); }
+  static int table_bytes(int n) { return (int)(sizeof(double2) * (entries(n) + n) + (sizeof(double) * n + 15) / 16 * 16); }
+  const int n, sub = (threadIdx.x & 31) / T, t = (threadIdx.x & 31) % T, items;
+  double2 *tab, *pt;
+  double* cosk;
+  __device__ __forceinline__ ClusterFft(const Inst& I, unsigned char* smem)
+      : n(I.n), items(((I.n + 1) / 2 + LPW - 1) / LPW), tab(reinterpret_cast<double2*>(smem)) {
+    pt = tab + entries(n);
+    cosk = reinterpret_cast<double*>(pt + n);
+    for (int e = threadIdx.x; e < entries(n); e += CL_T) tab[e] = I.tw[e];
+    for (int e = threadIdx.x; e < n; e += CL_T) {
+      pt[e] = I.pt[e];
+      cosk[e] = I.cosk[e];
+    }
+  }
+  __device__ __forceinline__ double2* line(const ClusterBlock& B) const {
+    return reinterpret_cast<double2*>(B.region()) + sub * SLOTS;
+  }
+  __device__ __forceinline__ void rows_fwd(const ClusterBlock& B, int it) const {
+    B.items(items, [&](int item) {
+      row_pair_fwd<M, CHIRP, WarpLine>(B.I.r[it % 3], B.I.t1, n, 2 * (item * LPW + sub), t, line(B), Tables<M>(tab), pt);
+    });
+  }
+  __device__ __forceinline__ void cols(const ClusterBlock& B) const {
+    B.items(items, [&](int item) {
+      column_pair<M, CHIRP, WarpLine>(B.I.t1, n, 2 * (item * LPW + sub), t, line(B), Tables<M>(tab), pt, cosk);
+    });
+  }
+  __device__ __forceinline__ void rows_inv(const ClusterBlock& B) const {
+    B.items(items, [&](int item) {
+      row_pair_inv<M, CHIRP, WarpLine>(B.I.t1, B.I.dhat, n, 2 * (item * LPW + sub), t, line(B), Tables<M>(tab), pt);
+    });
+  }
+};
 
 // ---- host ----
 
@@ -551,6 +628,28 @@ void poisson_fft(otm_context* ctx, int n, Inst* d_insts, const int* row_inst, in
                 coff);
     launch_smem(ctx, "fft_rows_inv", k_fft_rows_inv<M, C>, nrow_items, GR::THREADS, GR::SMEM, (const Inst*)d_insts,
                 row_inst, roff);
+  });
+}
+
+// Largest size solved by a cluster: above it a line takes more threads than a warp has (at 127^2
+// the cluster is 1.15 times as fast as the kernels: cluster.cuh).
+constexpr int CLUSTER_MAX = 128;
+
+int poisson_cluster_blocks(otm_context* ctx, int n, int count) {
+  int blocks = 0;
+  if (n <= CLUSTER_MAX)
+    dispatch(n, [&](auto Mc, auto ch) {
+      constexpr int M = decltype(Mc)::value;
+      if constexpr (M <= 256) blocks = cluster_blocks<ClusterFft<M, decltype(ch)::value>>(ctx, n, count);
+    });
+  return blocks;
+}
+
+void poisson_cluster(otm_context* ctx, int n, int count, int blocks, Inst* d_insts, double* partials) {
+  dispatch(n, [&](auto Mc, auto ch) {
+    constexpr int M = decltype(Mc)::value;
+    if constexpr (M <= 256)
+      cluster_launch<ClusterFft<M, decltype(ch)::value>>(ctx, n, count, blocks, d_insts, partials);
   });
 }
 

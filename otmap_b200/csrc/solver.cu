@@ -740,11 +740,18 @@ static std::vector<Inst> layout_workspace(otm_context* ctx, const std::vector<in
     }
   }
   // sweep strips: a new layout takes the rule's height, a cached one keeps its own
-  // (possibly autotuned) height and work list
-  if (!same)
+  // (possibly autotuned) height and work list. In the one-kernel loop of a small instance the
+  // cluster's warps take a strip each where 16 rows or fewer allow that.
+  if (!same) {
+    ws.cluster_blocks = 0;
+    if (segs.size() == 1 && !segs[0].split && gemm == 0 && tcitems == 0)
+      ws.cluster_blocks = (segs[0].reg ? dct_reg_cluster_blocks : poisson_cluster_blocks)(ctx, segs[0].n, count);
+    if (ws.cluster_blocks > 0)
+      while (srows < 16 && strip_blocks(segs[0].n, srows) > 2 * ws.cluster_blocks) srows *= 2;
     set_strips(ctx, ws, h, srows);
-  else
+  } else {
     assign_strips(h, ws.srows);
+  }
   double* base = ws.arena.as<double>();
   for (int q = 0; q < count; ++q) {
     Inst& I = h[q];
@@ -941,10 +948,16 @@ static std::vector<Inst> run_solver(otm_context* ctx, std::vector<Inst>& h, cons
 
   Inst* hp = static_cast<Inst*>(ws.h_pinned);
   if (ctx->loop_mode == OTM_LOOP_GRAPH && !ctx->prof.on) {
-    if (!ws.graph_exec) build_loop_graph(ctx, count);
+    const bool one_kernel = ws.cluster_blocks > 0 && !ctx->wait_test;
     LoopCtl c = {0u, (unsigned int)o.max_iter + 2u, 0, 0};
-    OTM_CUDA(cudaMemcpyAsync(ws.loopctl.p, &c, sizeof(c), cudaMemcpyHostToDevice, st));
-    OTM_CUDA(cudaGraphLaunch(ws.graph_exec, st));
+    if (one_kernel) {
+      (ws.segments[0].reg ? dct_reg_cluster : poisson_cluster)(ctx, h[0].n, count, ws.cluster_blocks, d_insts,
+                                                               ws.sweep_partials.as<double>());
+    } else {
+      if (!ws.graph_exec) build_loop_graph(ctx, count);
+      OTM_CUDA(cudaMemcpyAsync(ws.loopctl.p, &c, sizeof(c), cudaMemcpyHostToDevice, st));
+      OTM_CUDA(cudaGraphLaunch(ws.graph_exec, st));
+    }
     if (stopped && done) {
       Inst* poll = static_cast<Inst*>(ctx->h_poll);
       // the records start inactive on the host side: watch them only once the set-up
@@ -968,7 +981,7 @@ static std::vector<Inst> run_solver(otm_context* ctx, std::vector<Inst>& h, cons
       OTM_CUDA(cudaStreamSynchronize(ctx->side));
     }
     OTM_CUDA(cudaMemcpyAsync(hp, d_insts, sizeof(Inst) * count, cudaMemcpyDeviceToHost, st));
-    OTM_CUDA(cudaMemcpyAsync(&c, ws.loopctl.p, sizeof(c), cudaMemcpyDeviceToHost, st));
+    if (!one_kernel) OTM_CUDA(cudaMemcpyAsync(&c, ws.loopctl.p, sizeof(c), cudaMemcpyDeviceToHost, st));
     OTM_CUDA(cudaStreamSynchronize(st));
     ctx->launches += ws.graph_body_kernels * (long)c.count;
     if (c.error) throw CudaError{cudaErrorLaunchTimeout, "device loop exceeded its iteration bound"};
