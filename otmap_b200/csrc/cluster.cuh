@@ -5,15 +5,16 @@
 // cluster of up to 16 blocks keeps an instance from its first iteration to its last: the kernels'
 // line and strip functions on the same arrays (L2-resident), a hardware cluster barrier between
 // the stages (0.6 us with its release and acquire), the size's tables and the instance's record in
-// every block's shared memory: each block forms the totals and the step from the partial sums itself, all alike, so
-// nothing is handed round. The sums are formed by the kernels' trees over the same strips.
+// every block's shared memory: each block forms the totals and the step from the partial sums
+// itself, all alike, so nothing is handed round. The sums are formed by the kernels' trees over
+// the same strips.
 //
-// Bound by latency up to the size at which 16 SMs' FP64 and shared-memory rates are (64^2: an
-// iteration is 30000 cycles, 6500 of them barriers, 5000 the step). Microseconds per iteration by the
-// kernels and so: 20^2 32.7 and 20.7, 32^2 34.4 and 19.8, 50^2 34.5 and 24.4, 64^2 25.6 and 15.9, 100^2
-// 35.8 and 30.6, 127^2 35.9 and 31.3; eight 64^2 29.9 and 18.3, eight 100^2 41.0 and 38.5. With the
-// register transforms 128^2 took 33.3 against 31.6 and 256^2 37.6 against 33.8: those keep the kernels, as
-// do batches of more instances than clusters run at once.
+// Bound by latency (64^2: an iteration is 30000 cycles, 6500 of them barriers, 5000 the step) up to
+// the size at which the FP64 and shared-memory rates of 16 SMs bound it. Microseconds per
+// iteration by the kernels and so: 20^2 32.7 and 23.2, 32^2 34.4 and 21.1, 50^2 34.5 and 28.3, 64^2
+// 25.6 and 16.9, 100^2 35.8 and 30.8, 127^2 35.9 and 31.4; eight 50^2 38.9 and 30.0, eight 100^2 41.0
+// and 38.5. With the register transforms 128^2 took 33.3 against 31.6 and 256^2 37.6 against 33.8:
+// those keep the kernels, as do batches of more instances than clusters run at once.
 #pragma once
 
 #include <type_traits>
