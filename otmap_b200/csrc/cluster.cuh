@@ -101,7 +101,7 @@ __device__ __forceinline__ void cluster_update(const ClusterBlock& B, int it) {
 }
 
 // Transform: the three passes of M^+ over the instance's lines, tables in shared memory:
-// table_bytes(n) of it, Transform(I, smem) (fills them), rows_fwd(B, it), cols(B), rows_inv(B).
+// table_bytes(n) of it (n <= MAX_N), Transform(I, smem) (fills them), rows_fwd(B, it), cols(B), rows_inv(B).
 template <class Transform>
 __global__ __launch_bounds__(CL_T, 1) void k_cluster_loop(Inst* insts, double* partials, int table_bytes) {
   extern __shared__ __align__(16) unsigned char cluster_smem[];
@@ -169,17 +169,24 @@ cudaLaunchConfig_t cluster_config(otm_context* ctx, int n, int count, int blocks
   return cfg;
 }
 
+// The kernel's limits, the same for every size it takes: another thread may be launching it.
+template <class Transform>
+void cluster_attrs() {
+  const auto kernel = k_cluster_loop<Transform>;
+  OTM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                Transform::table_bytes(Transform::MAX_N) + CL_WARPS * CL_WARP_BYTES));
+  OTM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+}
+
 // Blocks per cluster (16, else 8) with which `count` clusters run at once, or 0.
 template <class Transform>
 int cluster_blocks(otm_context* ctx, int n, int count) {
+  cluster_attrs<Transform>();
   for (int c : {16, 8}) {
     cudaLaunchAttribute attr = {};
     const cudaLaunchConfig_t cfg = cluster_config<Transform>(ctx, n, count, c, &attr);
-    const auto kernel = k_cluster_loop<Transform>;
-    OTM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
-    OTM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     int fit = 0;
-    if (cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&fit, k_cluster_loop<Transform>, &cfg) != cudaSuccess) {
       cudaGetLastError();
       fit = 0;
     }
@@ -191,11 +198,8 @@ template <class Transform>
 void cluster_launch(otm_context* ctx, int n, int count, int blocks, Inst* d_insts, double* partials) {
   cudaLaunchAttribute attr = {};
   const cudaLaunchConfig_t cfg = cluster_config<Transform>(ctx, n, count, blocks, &attr);
-  const auto kernel = k_cluster_loop<Transform>;
-  // the limit may have been set for a smaller size of the same kernel since
-  OTM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
   ctx->launches++;
-  OTM_CUDA(cudaLaunchKernelEx(&cfg, kernel, d_insts, partials, Transform::table_bytes(n)));
+  OTM_CUDA(cudaLaunchKernelEx(&cfg, k_cluster_loop<Transform>, d_insts, partials, Transform::table_bytes(n)));
 }
 
 }  // namespace otm

@@ -760,7 +760,7 @@ int RegDct<R, N1, N2>::cols_blocks_per_sm[COL_VARIANTS] = {1, 1, 1};
 
 template <int N1, int N2>
 struct ClusterRegDct {
-  static constexpr int n = N1 * N2, LPW = 32 / N2, ITEMS = n / (2 * LPW);  // row or column pairs by warps
+  static constexpr int n = N1 * N2, MAX_N = n, LPW = 32 / N2, ITEMS = n / (2 * LPW);  // row or column pairs by warps
   static_assert(LPW * 2 * n * sizeof(double) <= CL_WARP_BYTES, "a warp's lines fit in its region");
   static int table_bytes(int) { return sizeof(double) * 7 * n; }
   double2 *stw, *stw_sw, *spt;

@@ -453,7 +453,7 @@ __global__ __launch_bounds__(Geom<M, false>::THREADS, Geom<M, false>::MIN_BLOCKS
 
 template <int M, bool CHIRP>
 struct ClusterFft {
-  static constexpr int T = M / 8, LPW = 32 / T, SLOTS = Geom<M, false>::SLOTS;
+  static constexpr int T = M / 8, LPW = 32 / T, SLOTS = Geom<M, false>::SLOTS, MAX_N = M;
   static_assert(T <= 32 && LPW * SLOTS * sizeof(double2) <= CL_WARP_BYTES, "a warp's lines fit in its region");
   static __host__ __device__ int entries(int n) { return Passes<M>::twiddles() + (CHIRP ? M + n : 0); }
   static int table_bytes(int n) { return (int)(sizeof(double2) * (entries(n) + n) + (sizeof(double) * n + 15) / 16 * 16); }

@@ -56,3 +56,35 @@ def test_loop_ends(n):
     flat = np.ones_like(mix)
     for max_iter, threshold in ((0, 1e-7), (1, 1e-7), (3, 1e-7), (400, 0.0)):
         _both([mix, flat, mix], ot.SolverOptions(max_iter=max_iter, threshold=threshold))
+
+
+def test_threads_on_sizes_of_one_kernel():
+    """Contexts of their own on host threads, sizes that share a kernel with different shared-memory needs."""
+    import threading
+
+    from otmap_b200 import native as N
+    from otmap_b200 import otmap as ot
+    from otmap_b200 import workloads as W
+
+    sizes = [66, 100, 127, 66]
+    dens = [W.to_cells(W.gaussian_mixture(n, 40 + n)) for n in sizes]
+    want = [ot.solve_batch([d])[0].fwd_mesh() for d in dens]
+    wrong = []
+
+    def work(k):
+        try:
+            for _ in range(15):
+                ctx = N.Context(0)  # a new layout each time
+                got = ot.solve_batch([dens[k]], context=ctx)[0].fwd_mesh()
+                ctx.close()
+                if not np.array_equal(got, want[k]):
+                    wrong.append(k)
+        except Exception as e:  # noqa: BLE001
+            wrong.append((k, e))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(sizes))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
