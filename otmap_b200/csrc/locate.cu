@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "context.h"
+#include "place_list.cuh"
 
 namespace otm {
 
@@ -1509,9 +1510,13 @@ struct PixelAxis {
 // length, which k_raster_stale makes with a thread each instead of holding up a warp of the
 // owner pass. Tests beyond the list's room are decided on the spot.
 struct StaleList {
-  int* count;
-  uint2* test;  // face, y << 16 | x
+  PlaceCount* count;  // of the tests that asked for a place, less one: it starts at -1
+  uint2* test;        // face, y << 16 | x
   int room;
+  // A place of the list for this thread, or one at or beyond `room`.
+  __device__ __forceinline__ int place() const {
+    return take_place(room, [&] { return atomicAdd(count, 1ull) + 1; });
+  }
 };
 
 // The owner test: face f (corners p, valence c) records its index at pixel (x, y) when it
@@ -1529,7 +1534,7 @@ __device__ __forceinline__ void test_pixel(const MeshRef& m, int rows, int cols,
       if (verdict != 0) return;
       bilinear_from_terms(t, w);
     } else {
-      const int i = atomicAdd(stale.count, 1) + 1;  // the counter starts at -1
+      const int i = stale.place();
       if (i < stale.room) {
         stale.test[i] = make_uint2((unsigned)f, (unsigned)y << 16 | (unsigned)x);
         return;
@@ -1541,7 +1546,7 @@ __device__ __forceinline__ void test_pixel(const MeshRef& m, int rows, int cols,
 }
 
 __global__ __launch_bounds__(128) void k_raster_stale(MeshRef m, int rows, int cols, int* owner, StaleList stale) {
-  const int total = min(*stale.count + 1, stale.room);
+  const int total = (int)min(*stale.count + 1, (PlaceCount)stale.room);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const uint2 e = stale.test[i];
     const int f = (int)e.x, x = (int)(e.y & 0xffffu), y = (int)(e.y >> 16);
@@ -2191,7 +2196,7 @@ static void raster_mesh(otm_context* ctx, const MeshRef& m, const double* densit
   const int nf = m.nf;
   const size_t pix = (size_t)rows * cols;
   auto al = [](size_t b) { return (b + 255) / 256 * 256; };
-  const size_t b_val = al(sizeof(double) * (size_t)(nf > 0 ? nf : 1)), b_own = al(sizeof(int) * (pix + 2));
+  const size_t b_val = al(sizeof(double) * (size_t)(nf > 0 ? nf : 1)), b_own = al(sizeof(int) * (pix + 6));
   const size_t b_vv = al(sizeof(float) * (size_t)(m.nv > 0 ? m.nv : 1));
   const size_t b_list = al(sizeof(int) * (size_t)(nf + 1));
   const size_t b_start = al(sizeof(long long) * (size_t)(nf + 1));
@@ -2209,9 +2214,10 @@ static void raster_mesh(otm_context* ctx, const MeshRef& m, const double* densit
   int* big = reinterpret_cast<int*>(take(b_list));
   int* big_chunks = reinterpret_cast<int*>(take(b_list));
   long long* big_start = reinterpret_cast<long long*>(take(b_start));
-  int* big_count = owner + pix;
-  StaleList stale{owner + pix + 1, reinterpret_cast<uint2*>(take(b_stale)), nf};
-  OTM_CUDA(cudaMemsetAsync(owner, 0xff, sizeof(int) * (pix + 2), st));  // -1: no face, empty lists
+  int* counters = owner + (pix + 1) / 2 * 2;  // 8-byte aligned
+  int* big_count = counters;
+  StaleList stale{reinterpret_cast<PlaceCount*>(counters + 2), reinterpret_cast<uint2*>(take(b_stale)), nf};
+  OTM_CUDA(cudaMemsetAsync(owner, 0xff, sizeof(int) * (pix + 6), st));  // -1: no face, empty lists
   // rasterizer.cpp:193 keeps 1/density.size() in a float
   const float scale = (float)(1. / (double)(density ? cells : nf));
   const int fblocks = nf > 0 ? (nf + 255) / 256 : 1;
