@@ -1239,13 +1239,6 @@ __global__ __launch_bounds__(INV_T) void k_inverse(Locator L, double* pts, long 
   }
   W.q[lane] = make_double2(qx, qy);
   W.hits[lane] = 0;
-  int upto = count;  // inclusive prefix over the warp
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int u = __shfl_up_sync(0xffffffffu, upto, o);
-    if (lane >= o) upto += u;
-  }
-  const int total = __shfl_sync(0xffffffffu, upto, 31), shift = begin - (upto - count);
   __syncwarp();
   auto test = [&](int e) {  // queue entry e
     const int f = W.queue_face[e], l = W.queue_lane[e];
@@ -1260,34 +1253,45 @@ __global__ __launch_bounds__(INV_T) void k_inverse(Locator L, double* pts, long 
     if (k < MAXHITS) W.hit[l][k] = (unsigned long long)(unsigned)L.rank[f] << 32 | (unsigned)f;
   };
   int queued = 0;
-  for (int base = 0; base < total; base += 32) {
-    const int item = base + lane;
-    int l = 0;  // the point the item belongs to: the first lane with upto > item
+  for (int left = count; __any_sync(0xffffffffu, left > 0);) {  // once but for lists of 2^26 faces
+    const int part = pool_part(left);
+    int upto = part;  // inclusive prefix over the warp
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-      if (__shfl_sync(0xffffffffu, upto, l + o - 1) <= item) l += o;
-    l = min(l, 31);
-    const int k = item + __shfl_sync(0xffffffffu, shift, l);
-    bool pass = false;
-    int f = 0;
-    if (item < total) {
-      f = L.faces[k];
-      const double4 bb = L.boxes[f];
-      const double2 q = W.q[l];
-      pass = !(q.x < bb.x || q.x > bb.z || q.y < bb.y || q.y > bb.w);
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += u;
     }
-    const unsigned m = __ballot_sync(0xffffffffu, pass);
-    if (pass) {
-      const int e = queued + __popc(m & ((1u << lane) - 1));
-      W.queue_face[e] = f;
-      W.queue_lane[e] = (unsigned char)l;
-    }
-    queued += __popc(m);
-    __syncwarp();
-    if (queued >= 32) {
-      queued -= 32;
-      test(queued + lane);
+    const int total = __shfl_sync(0xffffffffu, upto, 31), shift = begin + (count - left) - (upto - part);
+    left -= part;
+    for (int base = 0; base < total; base += 32) {
+      const int item = base + lane;
+      int l = 0;  // the point the item belongs to: the first lane with upto > item
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        if (__shfl_sync(0xffffffffu, upto, l + o - 1) <= item) l += o;
+      l = min(l, 31);
+      const int k = item + __shfl_sync(0xffffffffu, shift, l);
+      bool pass = false;
+      int f = 0;
+      if (item < total) {
+        f = L.faces[k];
+        const double4 bb = L.boxes[f];
+        const double2 q = W.q[l];
+        pass = !(q.x < bb.x || q.x > bb.z || q.y < bb.y || q.y > bb.w);
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, pass);
+      if (pass) {
+        const int e = queued + __popc(m & ((1u << lane) - 1));
+        W.queue_face[e] = f;
+        W.queue_lane[e] = (unsigned char)l;
+      }
+      queued += __popc(m);
       __syncwarp();
+      if (queued >= 32) {
+        queued -= 32;
+        test(queued + lane);
+        __syncwarp();
+      }
     }
   }
   if (lane < queued) test(lane);
