@@ -690,8 +690,9 @@ struct AdjointWs : otm_context::Erased {
 
 static AdjointWs* adjoint_ws(otm_context* ctx, int n, int m, int maps) {
   auto& slot = ctx->adjoint[n * ADJ_MAPS + maps - 1];
-  if (slot && static_cast<AdjointWs*>(slot.get())->m >= m) return static_cast<AdjointWs*>(slot.get());
-  slot.reset();  // the smaller workspace's memory goes back first
+  const int fft = (ctx->poisson_mode != OTM_POISSON_DENSE && fft_eligible(n)) ? 1 : 0;
+  if (auto* W = static_cast<AdjointWs*>(slot.get()); W && W->m >= m && W->fft == fft) return W;
+  slot.reset();  // the former workspace's memory goes back first
   auto own = std::make_unique<AdjointWs>();
   AdjointWs* W = own.get();
   W->n = n;
@@ -740,8 +741,7 @@ static AdjointWs* adjoint_ws(otm_context* ctx, int n, int m, int maps) {
   base.cosk = T->cosk.as<double>();
   base.tw = T->tw.as<double2>();
   base.pt = T->pt.as<double2>();
-  base.fft = (ctx->poisson_mode != OTM_POISSON_DENSE && fft_eligible(n)) ? 1 : 0;
-  W->fft = base.fft;
+  base.fft = W->fft = fft;
   if (base.fft) {
     W->reg = dct_reg_supported(n) ? 1 : 0;
     const int per = W->reg ? dct_reg_lines_per_block(n) : fft_lines(n, false);
