@@ -680,9 +680,11 @@ struct AdjointWs : otm_context::Erased {
   // the Arnoldi step as a graph with a WHILE node (built on first use) and its kernel count
   cudaGraphExec_t step_graph = nullptr;
   long step_kernels = 0;
-  ~AdjointWs() override {
+  void drop_graph() override {
     if (step_graph) cudaGraphExecDestroy(step_graph);
+    step_graph = nullptr;
   }
+  ~AdjointWs() override { drop_graph(); }
   // Poisson records, one per map of each kind; destination z. Kind 0: source b; 1: source h;
   // 2: source the basis vector of the current step (set on the device, as is the active flag)
   Inst* rec(int kind) { return recs.as<Inst>() + kind * maps; }

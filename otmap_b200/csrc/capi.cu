@@ -210,7 +210,10 @@ extern "C" int otm_set_option(otm_context* ctx, int key, int value) {
     if (ctx->wait_test != value) {
       cudaSetDevice(ctx->device);
       cudaStreamSynchronize(ctx->stream);
-      for (auto& w : ctx->workspaces) w->drop_graph();  // the captured launches carry the wait parameters
+      // the captured launches carry the wait parameters
+      for (auto& w : ctx->workspaces) w->drop_graph();
+      for (auto& a : ctx->adjoint)
+        if (a.second) a.second->drop_graph();
     }
     ctx->wait_test = value;
     return OTM_OK;

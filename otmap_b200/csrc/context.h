@@ -202,6 +202,7 @@ struct otm_context {
   // adjoint workspaces per grid size and number of maps (adjoint.cu); type-erased to keep this header small
   struct Erased {
     virtual ~Erased() = default;
+    virtual void drop_graph() = 0;  // captured launches carry the wait parameters
   };
   std::map<int, std::unique_ptr<Erased>> adjoint;
 };

@@ -53,3 +53,25 @@ def test_poisson_option(n, mode):
         ctx.set_poisson(poisson)
         assert np.array_equal(_adjoint(ctx, n, mode, inputs), alone[poisson])
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [64, 128])
+def test_wait_test_option(n):
+    """Adjoints first computed while the bounded waits are made to run out (an error, and the
+    steps' launches captured with it) are right once the option is off; and the option takes
+    effect after launches captured without it."""
+    from otmap_b200 import native as N
+
+    inputs = _inputs(n)
+    clean = N.Context(0)
+    good = _adjoint(clean, n, N.ADJOINT_KRYLOV, inputs)
+    clean.close()
+    ctx = N.Context(0)
+    for _ in range(2):
+        N.check(N.lib().otm_set_option(ctx.handle, N.OPT_WAIT_TEST, 1))
+        with pytest.raises(N.OtmError) as e:
+            _adjoint(ctx, n, N.ADJOINT_KRYLOV, inputs)
+        assert e.value.code == N.ERR_TIMEOUT
+        N.check(N.lib().otm_set_option(ctx.handle, N.OPT_WAIT_TEST, 0))
+        assert np.array_equal(_adjoint(ctx, n, N.ADJOINT_KRYLOV, inputs), good)
+    ctx.close()
