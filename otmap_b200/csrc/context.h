@@ -106,7 +106,7 @@ struct Workspace {
   int srows = 0;       // strip height of the sweeps (rule or autotuned)
   bool tuned = false;  // srows was chosen by timing (OTM_OPT_AUTOTUNE)
   int split_strip0 = 0;  // strips of split-precision instances start here (FP64 ones before)
-  struct Segment {  // instances of one size on one transform kernel family
+  struct Segment {  // instances of one register-transform size or of one family of others
     int n, reg, split, roff, rcnt, coff, ccnt;
     int col_warps;  // warps per block of the column pass (register transforms)
   };

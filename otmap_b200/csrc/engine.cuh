@@ -131,10 +131,11 @@ __device__ __forceinline__ void pick_step(const double z[5], double* alpha, doub
 
 
 // Fast cosine-transform Poisson solve for the sizes without a register transform (poisson.cu):
-// d_hat = M^+ r_k for the active instances, all of size n, of the row and column work lists.
+// d_hat = M^+ r_k for the active instances, all of n's family, of the row and column work lists.
 void poisson_fft(otm_context* ctx, int n, Inst* d_insts, const int* row_inst, int roff, int nrow_items,
                  const int* col_inst, int coff, int ncol_items);
-int fft_lines(int n, bool cols);  // rows or columns per work item
+int fft_family(int n);  // sizes of one family (transform length and kind) share launches
+int fft_lines(int n, bool cols);  // rows or columns per work item, the same for a family
 void fft_tables(int n, std::vector<double2>& out);  // the contents of Inst::tw
 // Sizes with a fast transform; below 8 the dense products are as fast.
 inline bool fft_eligible(int n) { return n >= 8 && n <= 4096; }

@@ -567,6 +567,8 @@ void dft_host(std::vector<Cld>& x) {
 
 }  // namespace
 
+int fft_family(int n) { return 2 * length_of(n) + (pow2(n) ? 0 : 1); }
+
 int fft_lines(int n, bool cols) {
   int lines = 0;
   dispatch(n, [&](auto Mc, auto) {

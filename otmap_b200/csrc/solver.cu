@@ -651,19 +651,25 @@ static std::vector<Inst> layout_workspace(otm_context* ctx, const std::vector<in
     // planes), each padded to 32 doubles (256 bytes)
     cells += (11 + (I.ntc > 0 ? 1 : 0)) * (((size_t)n * n + 31) / 32 * 32);
   }
-  // fast-transform work lists, grouped into one segment per (kernel family, size)
+  // fast-transform work lists, grouped into segments that share launches: one per register-transform
+  // size, and one per family of other sizes -- their kernels take n from the record. (With a segment
+  // per size 24 instances of 40^2 .. 63^2 took 74 launches and 404 us per iteration, 43 so; 136 with
+  // the dense products, which take all sizes in four launches.)
   std::vector<Workspace::Segment> segs;
   {
     std::vector<int> order;
     for (int q = 0; q < count; ++q)
       if (h[q].fft) order.push_back(q);
-    auto key = [&](int q) { return std::make_pair(dct_reg_supported(h[q].n) ? 1 : 0, h[q].n); };
+    auto key = [&](int q) {
+      const int n = h[q].n;
+      return dct_reg_supported(n) ? std::make_pair(1, n) : std::make_pair(0, fft_family(n));
+    };
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return key(a) < key(b); });
     for (size_t k = 0; k < order.size(); ++k) {
       Inst& I = h[order[k]];
       const int reg = dct_reg_supported(I.n) ? 1 : 0;
       const int per = reg ? dct_reg_lines_per_block(I.n) : fft_lines(I.n, false);
-      if (segs.empty() || segs.back().n != I.n || segs.back().reg != reg) {
+      if (k == 0 || key(order[k]) != key(order[k - 1])) {
         const int same_size = (int)std::count_if(order.begin(), order.end(), [&](int q) { return h[q].n == I.n; });
         segs.push_back({I.n, reg, I.split, rows, 0, cols, 0, reg ? dct_reg_col_warps(I.n, same_size, ctx->num_sms) : 0});
       }
@@ -744,7 +750,8 @@ static std::vector<Inst> layout_workspace(otm_context* ctx, const std::vector<in
   // cluster's warps take a strip each where 16 rows or fewer allow that.
   if (!same) {
     ws.cluster_blocks = 0;
-    if (segs.size() == 1 && !segs[0].split && gemm == 0 && tcitems == 0)
+    const bool one_size = std::all_of(sizes.begin(), sizes.end(), [&](int n) { return n == sizes[0]; });
+    if (one_size && segs.size() == 1 && !segs[0].split && gemm == 0 && tcitems == 0)
       ws.cluster_blocks = (segs[0].reg ? dct_reg_cluster_blocks : poisson_cluster_blocks)(ctx, segs[0].n, count);
     if (ws.cluster_blocks > 0)
       while (srows < 16 && strip_blocks(segs[0].n, srows) > 2 * ws.cluster_blocks) srows *= 2;
