@@ -396,10 +396,13 @@ int otm_barycenter_loss(otm_context* ctx, int n, int count, const double* const*
 #define OTM_PRECISION_SPLIT 1
 /* Strip height of the two stencil sweeps of a batch configuration (its list of sizes,
  * Poisson mode and precision): OTM_AUTOTUNE_OFF (default) takes it from a fixed rule (64
- * rows when the batch has many 32-row blocks per SM, 16 when it has fewer than the SMs,
- * else 32); OTM_AUTOTUNE_ON times a few iterations of the first call's own densities at
- * each of 16, 32 and 64 rows (host-driven loop, CUDA events) and keeps the fastest for
- * that configuration (the real solve then starts from the same initial state). The strip
+ * rows when the batch has many 32-row blocks per SM, 32 when it has one for every SM, else
+ * 16, 8 or 4: the tallest with blocks for most SMs, 8 and 4 in FP64 only and not for
+ * several instances of one size in {64, 128, 256, 512, 1024}); OTM_AUTOTUNE_ON times a few
+ * iterations of the first call's own densities at each of 16, 32 and 64 rows -- 4 and 8
+ * too where the rule's height is below 16 -- (host-driven loop, CUDA events) and keeps the
+ * fastest for that configuration (the real solve then starts from the same initial state).
+ * Instances that one kernel solves (OTM_LOOP_GRAPH above) keep the rule's height. The strip
  * height changes the order of the partial sums, so results can differ from the untuned
  * configuration's at the last bits. */
 #define OTM_OPT_AUTOTUNE 5

@@ -1016,13 +1016,16 @@ static std::vector<Inst> run_solver(otm_context* ctx, std::vector<Inst>& h, cons
 // densities at each candidate strip height (host-driven loop, CUDA events on the context
 // stream, the second of two runs), the fastest kept for the configuration. Every run
 // starts from the raw densities (the set-up normalises them in place), and so does the
-// real solve afterwards.
+// real solve afterwards. Heights below 16 are tried where the rule has gone below 16 (a lone
+// 256^2 solve takes 39 us per iteration with 16 rows, 33 with the rule's 4). The one-kernel
+// loop keeps the rule's height, which fits its cluster: the kernels timed here are not the
+// ones that it would run.
 static void tune_strips(otm_context* ctx, std::vector<Inst>& h, const otm_solver_options& o,
                         const double* const* density) {
   Workspace& ws = ctx->ws();
   const int K = 4;
   ws.tuned = true;
-  if (o.max_iter < K) return;  // nothing worth timing
+  if (o.max_iter < K || ws.cluster_blocks > 0) return;  // nothing worth timing
   auto reload = [&] {
     for (size_t q = 0; q < h.size(); ++q)
       copy_in(ctx, h[q].rho, density[q], sizeof(double) * (size_t)h[q].n * h[q].n);
@@ -1037,7 +1040,8 @@ static void tune_strips(otm_context* ctx, std::vector<Inst>& h, const otm_solver
     ctx->loop_mode = OTM_LOOP_HOST;
     OTM_CUDA(cudaEventCreate(&a));
     OTM_CUDA(cudaEventCreate(&b));
-    for (int c : {16, 32, 64}) {
+    for (int c : {4, 8, 16, 32, 64}) {
+      if (c < std::min(rule, 16)) continue;
       set_strips(ctx, ws, h, c);
       float ms = 0.f;
       for (int rep = 0; rep < 2; ++rep) {

@@ -219,7 +219,8 @@ class Context:
 
     def set_autotune(self, on: bool):
         """AUTOTUNE_ON: the sweeps' strip height of a batch configuration is timed on its
-        first call (16, 32, 64 rows) and the fastest kept; AUTOTUNE_OFF (default): a fixed rule."""
+        first call (16, 32, 64 rows; 4 and 8 where the rule goes below 16) and the fastest
+        kept; AUTOTUNE_OFF (default): a fixed rule."""
         check(lib().otm_set_option(self._h, OPT_AUTOTUNE, AUTOTUNE_ON if on else AUTOTUNE_OFF))
 
     def get_option(self, key: int) -> int:
