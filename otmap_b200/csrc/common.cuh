@@ -6,23 +6,12 @@
 #include <cstdio>
 #include <string>
 
+#include "async_buf.h"
+
 namespace otm {
 
 // Thread-local message behind otm_last_error().
 void set_error(const std::string& msg);
-
-struct CudaError {
-  cudaError_t code;
-  std::string where;
-};
-
-#define OTM_CUDA(call)                                                                  \
-  do {                                                                                  \
-    cudaError_t _e = (call);                                                            \
-    if (_e != cudaSuccess)                                                              \
-      throw ::otm::CudaError{_e, std::string(#call) + " at " + __FILE__ + ":" +         \
-                                     std::to_string(__LINE__)};                         \
-  } while (0)
 
 struct BadArg {
   std::string what;

@@ -33,33 +33,6 @@ struct DevBuf {
   }
 };
 
-// Device buffer from the stream-ordered allocator (cudaMallocFromPoolAsync / cudaFreeAsync
-// on the stream it was reserved on, from the context's memory pool): freeing it does not
-// synchronise the device, and the pool hands the memory to the next allocation. Used for
-// the per-map buffers, which live and die with each TransportMap, and for the temporaries of
-// a call (a cudaMalloc and cudaFree of 25 MB cost a 512^2 barycenter image 0.4 ms).
-struct AsyncBuf {
-  void* p = nullptr;
-  size_t bytes = 0;
-  cudaStream_t st = nullptr;
-  AsyncBuf() = default;
-  AsyncBuf(const AsyncBuf&) = delete;
-  AsyncBuf& operator=(const AsyncBuf&) = delete;
-  ~AsyncBuf() { release(); }
-  void release() {
-    if (p) cudaFreeAsync(p, st);
-    p = nullptr;
-    bytes = 0;
-  }
-  // Grows (never shrinks) to at least `b` bytes on stream s from `pool`; contents are not
-  // preserved.
-  void reserve(size_t b, cudaStream_t s, cudaMemPool_t pool);
-  template <class T>
-  T* as() const {
-    return static_cast<T*>(p);
-  }
-};
-
 // Per grid size: the orthonormal DCT-II basis and cos(pi k / n), built by otm_init.
 struct SizeTables {
   int n = 0;

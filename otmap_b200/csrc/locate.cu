@@ -1974,7 +1974,8 @@ static void build_locator(otm_map* m) {
     int total = 0;
     OTM_CUDA(cudaMemcpyAsync(&total, m->bin_start.as<int>() + nb, sizeof(int), cudaMemcpyDeviceToHost, bs));
     OTM_CUDA(cudaStreamSynchronize(bs));
-    m->bin_faces.reserve(sizeof(int) * (size_t)(total > 0 ? total : 1), bs, ctx->pool);
+    // filled on bs, read and freed on the context's stream (the two are joined below)
+    m->bin_faces.reserve(sizeof(int) * (size_t)(total > 0 ? total : 1), bs, ctx->pool, st);
     OTM_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * nb, bs));
     bin("bin_fill", k_bin_fill, xy, n, B, (const int*)m->bin_start.as<int>(), counts, m->bin_faces.as<int>());
     OTM_CUDA(cudaGetLastError());
