@@ -21,7 +21,7 @@ struct CudaError {
   } while (0)
 
 // Device buffer from the stream-ordered allocator (cudaMallocFromPoolAsync / cudaFreeAsync
-// from the context's memory pool): freeing it does not synchronise the device, and the pool
+// from one of the context's memory pools): freeing it does not synchronise the device, and the pool
 // hands the memory to the next allocation. It is freed on its home stream, after the work
 // queued there: the stream of its last users, which need not be the one it is reserved on. Used for
 // the per-map buffers, which live and die with each TransportMap, and for the temporaries of

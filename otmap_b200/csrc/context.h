@@ -123,7 +123,8 @@ struct Profiler {
 struct otm_context {
   int device = 0;
   cudaStream_t stream = nullptr;
-  cudaMemPool_t pool = nullptr;  // stream-ordered allocations of the per-map buffers
+  cudaMemPool_t pool = nullptr;   // stream-ordered allocations of the per-map buffers
+  cudaMemPool_t temps = nullptr;  // and of the calls' temporaries
   int num_sms = 0;
   long launches = 0;  // kernels launched by this context since creation
   int poisson_mode = 0;  // OTM_POISSON_AUTO / _DENSE / _FFT
