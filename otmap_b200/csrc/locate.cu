@@ -1549,11 +1549,11 @@ __device__ __forceinline__ void test_pixel(const MeshRef& m, int rows, int cols,
   if (weights_inside(w)) atomicMax(&owner[(size_t)y * cols + x], f);
 }
 
-// Bound by the latency of the walks' divisions and loads, so it takes eight blocks per SM: with one
+// Bound by the latency of the walks' divisions and loads, so it takes four blocks per SM: with one
 // block it was 31 us for 256^2 jittered quads drawn at 512^2 and 168 for 1024^2 ones at 1024^2, now 18
 // and 62 (the calls 148 -> 134 and 365 -> 259 us; a thread per face, walking inside the owner pass,
 // 130 and 494). An empty list takes 6.5 us either way.
-constexpr int STALE_BLOCKS = 8;
+constexpr int STALE_BLOCKS = 4;
 __global__ __launch_bounds__(128) void k_raster_stale(MeshRef m, int rows, int cols, int* owner, StaleList stale) {
   const int total = (int)min(*stale.count + 1, (PlaceCount)stale.room);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
