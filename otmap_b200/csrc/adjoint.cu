@@ -663,14 +663,17 @@ using namespace otm;
 namespace otm {
 void dense_poisson(otm_context* ctx, Inst* d_inst, const int* gemm_inst, int G);
 
-// Adjoint workspace of one grid size and number of maps, kept by the context: device vectors,
-// the Krylov bases and the Poisson records, so a call allocates nothing and uploads nothing
-// but its inputs' pointers.
+// Adjoint workspace of one grid size, number of maps and kind of transform, kept by the context:
+// the layout of its device vectors and Krylov bases and its Poisson records, so a call
+// allocates nothing and uploads nothing but its inputs' pointers. The vectors hold nothing from
+// one call to the next: all workspaces lie in one allocation of the context, as large as the
+// largest needs (a slice per map: 1.6 GB at 2048^2, so losses of 8 maps, then 7, 6, ... would
+// keep 36 of them if each had its own).
 struct AdjointWs : otm_context::Erased {
   int n = 0, m = 0, maps = 0;
   size_t N = 0, V = 0, ld = 0;
   long stride = 0;  // doubles from one map's slice to the next one's
-  DevBuf buf, recs, lists;
+  DevBuf recs, lists, ctls;
   double *b, *lam, *z, *h, *t1, *t2, *Vb, *c, *part, *sums, *hcol, *inv;  // of map 0
   double2* g;                // the call's vertex displacements
   double *H, *cs, *sn, *gv;  // the cycle's Hessenberg state
@@ -691,10 +694,13 @@ struct AdjointWs : otm_context::Erased {
 };
 
 static AdjointWs* adjoint_ws(otm_context* ctx, int n, int m, int maps) {
-  auto& slot = ctx->adjoint[n * ADJ_MAPS + maps - 1];
   const int fft = (ctx->poisson_mode != OTM_POISSON_DENSE && fft_eligible(n)) ? 1 : 0;
-  if (auto* W = static_cast<AdjointWs*>(slot.get()); W && W->m >= m && W->fft == fft) return W;
-  slot.reset();  // the former workspace's memory goes back first
+  const int key = (n * ADJ_MAPS + maps - 1) * 2 + fft;
+  if (const auto it = ctx->adjoint.find(key); it != ctx->adjoint.end()) {
+    auto* W = static_cast<AdjointWs*>(it->second.get());
+    if (W->m >= m) return W;
+    ctx->adjoint.erase(it);
+  }
   auto own = std::make_unique<AdjointWs>();
   AdjointWs* W = own.get();
   W->n = n;
@@ -707,10 +713,14 @@ static AdjointWs* adjoint_ws(otm_context* ctx, int n, int m, int maps) {
   auto up = [](size_t w) { return (w + 31) / 32 * 32; };  // every array starts on 256 bytes
   W->stride = (long)(W->ld * 6 + up(2 * W->V) + (size_t)(m + 1) * W->ld + 3 * up(m + 2) + up((size_t)ANB * (m + 2)) +
                      2 * up(8) + up((size_t)(m + 1) * m) + 2 * up(m));
-  const size_t ctl_words = (sizeof(AdjCtl) * ADJ_MAPS + 7) / 8;
-  W->buf.reserve(sizeof(double) * ((size_t)W->stride * maps + up(ctl_words)));
-  double* q = W->buf.as<double>();
-  W->ctl = reinterpret_cast<AdjCtl*>(q + (size_t)W->stride * maps);
+  const size_t bytes = sizeof(double) * (size_t)W->stride * maps;
+  if (bytes > ctx->adjoint_buf.bytes) {
+    ctx->adjoint.clear();  // their pointers and graphs go with the allocation
+    ctx->adjoint_buf.reserve(bytes);
+  }
+  double* q = ctx->adjoint_buf.as<double>();
+  W->ctls.reserve(sizeof(AdjCtl) * maps);
+  W->ctl = W->ctls.as<AdjCtl>();
   auto take = [&](size_t w) {
     double* r = q;
     q += up(w);
@@ -733,7 +743,7 @@ static AdjointWs* adjoint_ws(otm_context* ctx, int n, int m, int maps) {
   W->H = take((size_t)(m + 1) * m);
   W->cs = take(m);
   W->sn = take(m);
-  OTM_CUDA(cudaMemsetAsync(W->ctl, 0, sizeof(AdjCtl) * ADJ_MAPS, ctx->stream));
+  OTM_CUDA(cudaMemsetAsync(W->ctl, 0, sizeof(AdjCtl) * maps, ctx->stream));
   SizeTables* T = ctx->tables.at(n).get();
   Inst base;
   std::memset(&base, 0, sizeof(base));
@@ -781,7 +791,7 @@ static AdjointWs* adjoint_ws(otm_context* ctx, int n, int m, int maps) {
   OTM_CUDA(cudaMemcpyAsync(W->recs.p, recs.data(), sizeof(Inst) * recs.size(), cudaMemcpyHostToDevice, ctx->stream));
   OTM_CUDA(cudaMemcpyAsync(W->lists.p, items.data(), sizeof(int) * items.size(), cudaMemcpyHostToDevice, ctx->stream));
   OTM_CUDA(cudaStreamSynchronize(ctx->stream));
-  slot = std::move(own);
+  ctx->adjoint[key] = std::move(own);
   return W;
 }
 

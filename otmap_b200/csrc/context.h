@@ -173,12 +173,14 @@ struct otm_context {
     }
   };
   std::map<int, std::unique_ptr<GraphExec>> bvh_graphs;
-  // adjoint workspaces per grid size and number of maps (adjoint.cu); type-erased to keep this header small
+  // adjoint workspaces per grid size, number of maps and kind of transform (adjoint.cu), and the
+  // memory they share; type-erased to keep this header small
   struct Erased {
     virtual ~Erased() = default;
     virtual void drop_graph() = 0;  // captured launches carry the wait parameters
   };
   std::map<int, std::unique_ptr<Erased>> adjoint;
+  otm::DevBuf adjoint_buf;
 };
 
 struct otm_map {
