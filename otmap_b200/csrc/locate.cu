@@ -1567,45 +1567,62 @@ __global__ __launch_bounds__(128) void k_raster_stale(MeshRef m, int rows, int c
 
 // The owner pass: every pixel centre of a face's box that the face accepts records the
 // face index with atomicMax, so each pixel ends with the highest accepting index -- the
-// face the reference's sequential loop writes last (rasterizer.cpp:162-236). One thread per
-// face forms its box and value. The tests of the boxes of at most SMALL_BOX pixels (a mesh
-// drawn near its own resolution has nothing else) are pooled over the warp, 32 at a time,
-// whatever the boxes' sizes; larger boxes go on a list whose pixels are spread over warps
-// (k_raster_big), so that a stretched face -- the inverse maps of sharp densities have some
-// that span much of the image -- does not hold one thread. Bound by instruction issue: about
+// face the reference's sequential loop writes last (rasterizer.cpp:162-236). A lane per
+// face, FACES of a warp, forms its box and value. The tests of the boxes of at most SMALL_BOX
+// pixels (a mesh drawn near its own resolution has nothing else) are pooled over the warp, 32
+// at a time, whatever the boxes' sizes; larger boxes go on two lists (k_raster_listed), so that
+// a stretched face -- the inverse maps of sharp densities have some that span much of the
+// image -- does not hold one warp. Bound by instruction issue: about
 // 90 FP64 and 150 other instructions for each of 4.6 tests per face. With one thread per
 // (face, box row) for every face, found by a binary search over 2^20 row counts, and the
 // divisions of bilinear_from_terms in every test, the pass took 148 us at 1024^2 beside 30
 // of boxes, counting and scanning; now 67 us in all (a raster call 222 -> 114 us; the owner
 // part of a 512^2 barycenter image 83 -> 38 us).
 constexpr int SMALL_BOX = 32, RF_T = 128;
-constexpr int BIG_CHUNK = 128;  // pixels of a listed face per warp
+// Largest box on the first list: a smooth 100^2 mesh drawn at 1400^2 (boxes of 210 to 260 pixels) takes
+// 111 us with 256, 95 with 512, 95 with 1024; a folded 40^2 one at 240^2 98, 107 and 106.
+constexpr int MID_BOX = 512;
+constexpr int BIG_CHUNK = 128;  // pixels of a face of the second list per warp
 
+// Faces with larger boxes: those of up to MID_BOX pixels from the end of `face` backwards, larger
+// ones from its start with their numbers of chunks. Counters start at -1.
+struct FaceLists {
+  int *mid_count, *big_count;
+  int* face;
+  int* big_chunks;
+};
+
+template <int FACES>
 __global__ __launch_bounds__(RF_T) void k_raster_faces(MeshRef m, const double* density, float scale, int rows,
-                                                       int cols, double* value, int* owner, int* big_count, int* big,
-                                                       int* big_chunks, StaleList stale) {
-  __shared__ Quad s_quad[RF_T];
-  __shared__ int2 s_corner[RF_T];                        // first pixel of the lane's box
-  __shared__ unsigned short s_item[RF_T * SMALL_BOX];    // per test: lane, dx, dy
-  const int f = blockIdx.x * RF_T + threadIdx.x, lane = threadIdx.x & 31;
+                                                       int cols, double* value, int* owner, FaceLists lists,
+                                                       StaleList stale) {
+  constexpr int SLOTS = RF_T / 32 * FACES;  // faces of the block
+  __shared__ Quad s_quad[SLOTS];
+  __shared__ int2 s_corner[SLOTS];                      // first pixel of the face's box
+  __shared__ unsigned short s_item[SLOTS * SMALL_BOX];  // per test: lane, dx, dy
+  const int lane = threadIdx.x & 31, slot0 = (threadIdx.x >> 5) * FACES, f0 = blockIdx.x * SLOTS + slot0, f = f0 + lane;
   const PixelAxis px(cols), py(rows);
   FaceBox b = {0, 0, 0, 0};
   int c = 4, tests = 0;
-  if (f < m.nf) {
+  if (lane < FACES && f < m.nf) {
     Quad p;
     int vid[4];
     c = load_face(m, f, p, vid);
     const double in_mass = scale * (density ? density[f] : 1.0);
     value[f] = in_mass / face_abs_area(p, c);  // PerFace value: float(1/N) * density / |area|
     b = face_box(p, rows, cols);
-    s_corner[threadIdx.x] = make_int2(b.x0, b.y0);
-    s_quad[threadIdx.x] = p;
+    s_corner[slot0 + lane] = make_int2(b.x0, b.y0);
+    s_quad[slot0 + lane] = p;
     if (!b.empty()) {
       const int wx = b.x1 - b.x0, wy = b.y1 - b.y0;
       if (wx > SMALL_BOX || wy > SMALL_BOX || wx * wy > SMALL_BOX) {
-        const int i = atomicAdd(big_count, 1) + 1;  // counters start at -1
-        big[i] = f;
-        big_chunks[i] = (int)(((long long)wx * wy + BIG_CHUNK - 1) / BIG_CHUNK);
+        if (wx > MID_BOX || wy > MID_BOX || wx * wy > MID_BOX) {
+          const int i = atomicAdd(lists.big_count, 1) + 1;
+          lists.face[i] = f;
+          lists.big_chunks[i] = (int)(((long long)wx * wy + BIG_CHUNK - 1) / BIG_CHUNK);
+        } else {
+          lists.face[m.nf - 1 - (atomicAdd(lists.mid_count, 1) + 1)] = f;
+        }
       } else {
         tests = wx * wy;
       }
@@ -1617,8 +1634,8 @@ __global__ __launch_bounds__(RF_T) void k_raster_faces(MeshRef m, const double* 
     const int u = __shfl_up_sync(0xffffffffu, upto, o);
     if (lane >= o) upto += u;
   }
-  const int total = __shfl_sync(0xffffffffu, upto, 31), warp0 = threadIdx.x & ~31;
-  unsigned short* items = s_item + warp0 * SMALL_BOX;
+  const int total = __shfl_sync(0xffffffffu, upto, 31);
+  unsigned short* items = s_item + slot0 * SMALL_BOX;
   for (int k = 0, dx = 0, dy = 0, at = upto - tests; k < tests; ++k) {
     items[at + k] = (unsigned short)(lane | dx << 5 | dy << 10);
     if (++dx == b.x1 - b.x0) {
@@ -1630,10 +1647,9 @@ __global__ __launch_bounds__(RF_T) void k_raster_faces(MeshRef m, const double* 
   __syncwarp();
   for (int item = lane; item < total; item += 32) {
     const int e = items[item], l = e & 31;
-    const int2 at = s_corner[warp0 + l];
+    const int2 at = s_corner[slot0 + l];
     const int x = at.x + (e >> 5 & 31), y = at.y + (e >> 10);
-    test_pixel(m, rows, cols, f - lane + l, s_quad[warp0 + l], triangles >> l & 1 ? 3 : 4, x, y, px(x), py(y), owner,
-               stale);
+    test_pixel(m, rows, cols, f0 + l, s_quad[slot0 + l], triangles >> l & 1 ? 3 : 4, x, y, px(x), py(y), owner, stale);
   }
 }
 
@@ -1666,34 +1682,75 @@ __global__ __launch_bounds__(1024) void k_big_scan(const int* big_count, const i
   if (threadIdx.x == 0) start[count] = carry;
 }
 
-// The listed faces: a warp per chunk of a box's pixels (row by row), lanes along it. Work item
-// t belongs to the last entry with start <= t.
-__global__ __launch_bounds__(256) void k_raster_big(MeshRef m, int rows, int cols, const int* big_count,
-                                                    const int* big, const long long* start, int* owner,
-                                                    StaleList stale) {
-  const int count = *big_count + 1, lane = threadIdx.x & 31;
-  const long long total = start[count];
-  const int warps = gridDim.x * (blockDim.x >> 5);
+// The listed faces, in units of work: some boxes of the first list -- as many as give every warp a unit,
+// at most 32 -- or a chunk of a box of the second (row by row; chunk t belongs to the last entry with
+// start <= t). A warp pools a unit's tests, each found in the prefix of the boxes' sizes. With all
+// listed boxes in chunks a smooth 200^2 mesh drawn at 1200^2 (boxes of 49 pixels) took 228 us: 84 in
+// one block's scan of 40000 entries, 94 in warps that searched them all and had half their lanes
+// idle; now 88, 41 of them here (a thread per box row, the form before that, 89). Three blocks
+// of 84 registers per SM: four of 64 took 44 us there, two of 106 registers 48.
+constexpr int RL_T = 256, RL_BLOCKS = 3;
+
+__global__ __launch_bounds__(RL_T, RL_BLOCKS) void k_raster_listed(MeshRef m, int rows, int cols, FaceLists lists,
+                                                        const long long* start, int* owner, StaleList stale) {
+  __shared__ Quad s_quad[RL_T];
+  __shared__ int4 s_box[RL_T];  // first row's first pixel and width of a face's box, first test in that row
+  __shared__ int s_upto[RL_T];  // inclusive prefix of the tests over the warp
+  const int lane = threadIdx.x & 31, warp0 = threadIdx.x & ~31;
+  const int warps = gridDim.x * (RL_T / 32), warp = blockIdx.x * (RL_T / 32) + (threadIdx.x >> 5);
   const PixelAxis px(cols), py(rows);
-  for (long long t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < total; t += warps) {
-    int lo = 0, hi = count;  // start[lo] <= t < start[hi]
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (start[mid] <= t) lo = mid; else hi = mid;
+  const int mids = *lists.mid_count + 1, bigs = *lists.big_count + 1;
+  const int per = max(1, min((mids + warps - 1) / warps, 32)), groups = (mids + per - 1) / per;
+  const long long units = groups + start[bigs];
+  for (long long t = warp; t < units; t += warps) {
+    int f = 0, c = 4, upto = 0;
+    auto take = [&](int face, long long k0, int limit) {
+      f = face;
+      Quad p;
+      int vid[4];
+      c = load_face(m, f, p, vid);
+      const FaceBox b = face_box(p, rows, cols);
+      const long long wx = b.x1 - b.x0, left = wx * (b.y1 - b.y0) - k0;
+      const int y0 = (int)(k0 / wx);
+      s_box[threadIdx.x] = make_int4(b.x0, b.y0 + y0, (int)wx, (int)(k0 - y0 * wx));
+      s_quad[threadIdx.x] = p;
+      upto = (int)min(left, (long long)limit);
+    };
+    if (t < groups) {
+      const long long e = t * per + lane;
+      if (lane < per && e < mids) take(lists.face[m.nf - 1 - e], 0, MID_BOX);
+    } else if (lane == 0) {
+      int lo = 0, hi = bigs;  // start[lo] <= chunk < start[hi]
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (start[mid] <= t - groups) lo = mid; else hi = mid;
+      }
+      take(lists.face[lo], (t - groups - start[lo]) * BIG_CHUNK, BIG_CHUNK);
     }
-    const int f = big[lo];
-    Quad p;
-    int vid[4];
-    const int c = load_face(m, f, p, vid);
-    const FaceBox b = face_box(p, rows, cols);
-    const long long wx = b.x1 - b.x0, area = wx * (b.y1 - b.y0), k0 = (t - start[lo]) * BIG_CHUNK;
-    const int left = (int)min((long long)BIG_CHUNK, area - k0);
-    const unsigned y0 = (unsigned)(k0 / wx), r0 = (unsigned)(k0 - y0 * wx), w = (unsigned)wx;
-    for (int k = lane; k < left; k += 32) {
-      const unsigned off = r0 + k, dy = off / w;
-      const int x = b.x0 + (int)(off - dy * w), y = b.y0 + (int)(y0 + dy);
-      test_pixel(m, rows, cols, f, p, c, x, y, px(x), py(y), owner, stale);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += u;
     }
+    s_upto[threadIdx.x] = upto;
+    const int tests = __shfl_sync(0xffffffffu, upto, 31);
+    const unsigned triangles = __ballot_sync(0xffffffffu, c == 3);
+    __syncwarp();
+    for (int item0 = 0; item0 < tests; item0 += 32) {
+      const int item = item0 + lane;
+      int l = 0;  // the box the test belongs to: the first lane with a prefix above the item
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        if (s_upto[warp0 + l + o - 1] <= item) l += o;
+      l = min(l, 31);
+      const int face = __shfl_sync(0xffffffffu, f, l);
+      if (item >= tests) continue;
+      const int4 box = s_box[warp0 + l];
+      const unsigned k = box.w + item - (l ? s_upto[warp0 + l - 1] : 0), w = box.z, dy = k / w;
+      const int x = box.x + (int)(k - dy * w), y = box.y + (int)dy;
+      test_pixel(m, rows, cols, face, s_quad[warp0 + l], triangles >> l & 1 ? 3 : 4, x, y, px(x), py(y), owner, stale);
+    }
+    __syncwarp();
   }
 }
 
@@ -2221,22 +2278,35 @@ static void raster_mesh(otm_context* ctx, const MeshRef& m, const double* densit
   double* value = reinterpret_cast<double*>(take(b_val));
   int* owner = reinterpret_cast<int*>(take(b_own));  // then the counters of the two lists
   float* vval = reinterpret_cast<float*>(take(b_vv));
-  int* big = reinterpret_cast<int*>(take(b_list));
-  int* big_chunks = reinterpret_cast<int*>(take(b_list));
-  long long* big_start = reinterpret_cast<long long*>(take(b_start));
   int* counters = owner + (pix + 1) / 2 * 2;  // 8-byte aligned
-  int* big_count = counters;
+  FaceLists lists{counters, counters + 1, reinterpret_cast<int*>(take(b_list)), reinterpret_cast<int*>(take(b_list))};
+  long long* big_start = reinterpret_cast<long long*>(take(b_start));
   StaleList stale{reinterpret_cast<PlaceCount*>(counters + 2), reinterpret_cast<uint2*>(take(b_stale)), nf};
   OTM_CUDA(cudaMemsetAsync(owner, 0xff, sizeof(int) * (pix + 6), st));  // -1: no face, empty lists
   // rasterizer.cpp:193 keeps 1/density.size() in a float
   const float scale = (float)(1. / (double)(density ? cells : nf));
   const int fblocks = nf > 0 ? (nf + 255) / 256 : 1;
   if (nf > 0) {
-    launch(ctx, "raster_faces", k_raster_faces, (nf + RF_T - 1) / RF_T, RF_T, m, density, scale, rows, cols, value, owner,
-           big_count, big, big_chunks, stale);
-    launch(ctx, "big_scan", k_big_scan, 1, 1024, (const int*)big_count, (const int*)big_chunks, big_start);
-    launch(ctx, "raster_big", k_raster_big, ctx->num_sms * 8, 256, m, rows, cols, (const int*)big_count,
-           (const int*)big, (const long long*)big_start, owner, stale);
+    auto faces = [&](auto kernel, int per_warp) {
+      const int slots = RF_T / 32 * per_warp;
+      launch(ctx, "raster_faces", kernel, (nf + slots - 1) / slots, RF_T, m, density, scale, rows, cols, value, owner,
+             lists, stale);
+    };
+    // 32 faces a warp where that gives an SM 16 warps, else fewer: a mesh of few faces has its tests on
+    // few warps. Calls with 32, 8, 4 and 1 faces a warp: 40^2 faces folded at 64^2 79, 53, 50 and 47 us,
+    // 96^2 smooth at 288^2 47, 36, 34 and 39, 128^2 at 128^2 35, 33, 34 and 42; with 32, 8 and 2 200^2
+    // at 600^2 52, 46 and 57, 512^2 at 512^2 49, 66 and 133.
+    if (nf >= 512 * ctx->num_sms)
+      faces(k_raster_faces<32>, 32);
+    else if (nf >= 64 * ctx->num_sms)
+      faces(k_raster_faces<8>, 8);
+    else if (nf >= 16 * ctx->num_sms)
+      faces(k_raster_faces<4>, 4);
+    else
+      faces(k_raster_faces<1>, 1);
+    launch(ctx, "big_scan", k_big_scan, 1, 1024, (const int*)lists.big_count, (const int*)lists.big_chunks, big_start);
+    launch(ctx, "raster_listed", k_raster_listed, ctx->num_sms * RL_BLOCKS, RL_T, m, rows, cols, lists,
+           (const long long*)big_start, owner, stale);
     launch(ctx, "raster_stale", k_raster_stale, ctx->num_sms * STALE_BLOCKS, 128, m, rows, cols, owner, stale);
   }
   const float* pv = nullptr;
