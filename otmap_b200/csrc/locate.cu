@@ -1067,7 +1067,7 @@ __device__ __forceinline__ void face_bins(const Quad& p, int B, int& bx0, int& b
   box = make_double4(mnx - m, mny - m, mxx + m, mxy + m);
   auto cl = [B](double v) {
     double t = floor(v * (double)B);
-    return t < 0 ? 0 : (t >= B ? B - 1 : (int)t);
+    return t >= B ? B - 1 : (t > 0 ? (int)t : 0);  // 0 for NaN
   };
   bx0 = cl(box.x);
   bx1 = cl(box.z);
