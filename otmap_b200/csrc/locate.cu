@@ -1075,18 +1075,30 @@ __device__ __forceinline__ void face_bins(const Quad& p, int B, int& bx0, int& b
   by1 = cl(box.w);
 }
 
-__global__ void k_bin_count(const double* xy, int n, int B, int* counts, double4* boxes) {
-  int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= n * n) return;
-  Quad p;
-  int vid[4];
-  load_quad(xy, n, f, p, vid);
-  int bx0, bx1, by0, by1;
-  double4 box;
-  face_bins(p, B, bx0, bx1, by0, by1, box);
-  boxes[f] = box;
-  for (int by = by0; by <= by1; ++by)
+// The bins' counts, and their sum in 64 bits. Once that is beyond an int the bins are too many
+// (build_locator) and faces of many bins leave theirs out.
+__global__ void k_bin_count(const double* xy, int n, int B, int* counts, double4* boxes, unsigned long long* sum) {
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned long long bins = 0;
+  int bx0 = 0, bx1 = -1, by0 = 0, by1 = -1;
+  if (f < n * n) {
+    Quad p;
+    int vid[4];
+    load_quad(xy, n, f, p, vid);
+    double4 box;
+    face_bins(p, B, bx0, bx1, by0, by1, box);
+    boxes[f] = box;
+    bins = (unsigned long long)(bx1 - bx0 + 1) * (by1 - by0 + 1);
+  }
+  unsigned long long all = bins;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
+  if ((threadIdx.x & 31) == 0) atomicAdd(sum, all);
+  __syncwarp();
+  for (int by = by0; by <= by1; ++by) {
+    if (bins > 64 && __ldcg(sum) > (unsigned long long)INT_MAX) return;
     for (int bx = bx0; bx <= bx1; ++bx) atomicAdd(&counts[by * B + bx], 1);
+  }
 }
 
 __global__ void k_bin_fill(const double* xy, int n, int B, const int* starts, int* cursor, int* faces) {
@@ -1999,18 +2011,17 @@ static void build_locator(otm_map* m) {
   otm_context* ctx = m->ctx;
   cudaStream_t st = ctx->stream;
   const int n = m->n, N = n * n;
-  const int B = n;
-  const int nb = B * B;
-  m->bins = B;
-  m->bin_start.reserve(sizeof(int) * (nb + 1), st, ctx->pool);
+  m->bin_start.reserve(sizeof(int) * (N + 1), st, ctx->pool);
   m->face_box.reserve(sizeof(double4) * N, st, ctx->pool);
   m->bvh_rank.reserve(sizeof(int) * N, st, ctx->pool);
   m->leaf_box.reserve(sizeof(double4) * N, st, ctx->pool);
-  // bin counts and scan sums in the context's grow-only scratch
-  const size_t b_counts = (sizeof(int) * nb + 255) / 256 * 256;
-  ctx->locate_scratch.reserve(b_counts + sizeof(int) * ((nb + SCAN_B - 1) / SCAN_B + 1));
+  // bin counts, scan sums and the lists' length in the context's grow-only scratch
+  auto al = [](size_t b) { return (b + 255) / 256 * 256; };
+  const size_t b_counts = al(sizeof(int) * N), b_sums = al(sizeof(int) * ((N + SCAN_B - 1) / SCAN_B + 1));
+  ctx->locate_scratch.reserve(b_counts + b_sums + sizeof(unsigned long long));
   int* counts = ctx->locate_scratch.as<int>();
   int* sums = reinterpret_cast<int*>(ctx->locate_scratch.as<char>() + b_counts);
+  unsigned long long* length = reinterpret_cast<unsigned long long*>(ctx->locate_scratch.as<char>() + b_counts + b_sums);
   const double* xy = m->fwd.as<double>();
   const bool beside = !ctx->prof.on;
   cudaStream_t bs = st;
@@ -2027,15 +2038,23 @@ static void build_locator(otm_map* m) {
       ctx->launches++;
       kernel<<<(N + 255) / 256, 256, 0, bs>>>(args...);
     };
-    OTM_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * nb, bs));
-    bin("bin_count", k_bin_count, xy, n, B, counts, m->face_box.as<double4>());
-    exclusive_scan(bs, counts, m->bin_start.as<int>(), sums, nb);
-    int total = 0;
-    OTM_CUDA(cudaMemcpyAsync(&total, m->bin_start.as<int>() + nb, sizeof(int), cudaMemcpyDeviceToHost, bs));
-    OTM_CUDA(cudaStreamSynchronize(bs));
+    // n x n bins; fewer while the lists' length is beyond an int (a 512^2 mesh whose faces each cover a
+    // sixth of the square has 10^10 entries). The bins only narrow a query's faces down.
+    int B = n;
+    unsigned long long total = 0;
+    for (;; B = (B + 1) / 2) {
+      OTM_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * B * B, bs));
+      OTM_CUDA(cudaMemsetAsync(length, 0, sizeof(*length), bs));
+      bin("bin_count", k_bin_count, xy, n, B, counts, m->face_box.as<double4>(), length);
+      exclusive_scan(bs, counts, m->bin_start.as<int>(), sums, B * B);
+      OTM_CUDA(cudaMemcpyAsync(&total, length, sizeof(total), cudaMemcpyDeviceToHost, bs));
+      OTM_CUDA(cudaStreamSynchronize(bs));
+      if (total <= (unsigned long long)INT_MAX) break;
+    }
+    m->bins = B;
     // filled on bs, read and freed on the context's stream (the two are joined below)
     m->bin_faces.reserve(sizeof(int) * (size_t)(total > 0 ? total : 1), bs, ctx->pool, st);
-    OTM_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * nb, bs));
+    OTM_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * B * B, bs));
     bin("bin_fill", k_bin_fill, xy, n, B, (const int*)m->bin_start.as<int>(), counts, m->bin_faces.as<int>());
     OTM_CUDA(cudaGetLastError());
     if (beside) {

@@ -1,5 +1,6 @@
-"""The point locator on a mesh with vertices that are not numbers: its other faces are located as
-without them."""
+"""The point locator on meshes far from any map: faces that each cover a third of the square (their
+lists over n^2 bins would be longer than an int can index: fewer bins are taken), against the
+oracle; and a mesh with vertices that are not numbers, whose other faces are located as without them."""
 
 import numpy as np
 import pytest
@@ -16,6 +17,20 @@ def _inverse(n, xy, density, pts):
     missing = m.apply_inverse(p, face, hits)
     m.release()
     return p, face, hits, missing
+
+
+@pytest.mark.parametrize("n", [40, 288])  # 288: 82944 faces of 0.36 * 82944 bins, 2.5e9 entries
+def test_random_vertices(oracle_port, n):
+    rng = np.random.default_rng(n)
+    xy = np.ascontiguousarray(rng.uniform(size=((n + 1) ** 2, 2)))
+    density = rng.uniform(0.5, 2.0, n * n)
+    pts = np.concatenate([rng.uniform(size=(30, 2)), rng.uniform(0.0, 0.004, size=(20, 2))])
+    q, faces, hits, _ = oracle_port.apply_inverse(xy, density, n, pts)
+    p, face, nh, _ = _inverse(n, xy, density, pts)
+    assert np.array_equal(nh, hits)
+    few = hits <= 8  # the hits kept in order per point
+    assert np.array_equal(face[few], faces[few])
+    assert np.array_equal(p[few], q[few], equal_nan=True)
 
 
 def test_vertices_that_are_not_numbers():
