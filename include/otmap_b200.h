@@ -366,7 +366,6 @@ int otm_barycenter_loss(otm_context* ctx, int n, int count, const double* const*
 /*   OTM_OPT_LOOP: how the iteration loop is driven.
  *     OTM_LOOP_GRAPH (default) one CUDA graph launch per solve: the iteration kernels sit
  *                    in the body of a device-side WHILE node that stops when no instance
- *                    is active (no host round trip between iterations)
  *                    is active (no host round trip between iterations); small FP64 instances
  *                    of one size take one kernel, a thread-block cluster each, instead
  *     OTM_LOOP_HOST  kernels launched from the host, loop test read back every 4

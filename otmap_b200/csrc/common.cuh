@@ -90,8 +90,8 @@ __device__ __forceinline__ double block_max(double v, double* red) {
 // and work lists may be read earlier, with loads that leave no copy in L1 of lines the wait
 // should see fresh. overlap_begin lets the successor's blocks take the places that this
 // kernel's have left: it stands behind the main loop, since blocks that only wait slow the ones
-// at work (at the kernels' entry nearly every size got slower than without). In a kernel
-// launched plainly both are no-ops.
+// at work -- but on entry in the register transforms of small batches, which leave most of the
+// chip free (OVERLAP_EARLY_CELLS). In a kernel launched plainly both are no-ops.
 __device__ __forceinline__ void overlap_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <class T>
 __device__ __forceinline__ const T* early_pointer(const T* const* p) {  // a pointer field, past L1

@@ -206,8 +206,9 @@ namespace otm {
 void make_current(otm_context* ctx);
 // Creates the context's second stream and its event, once; defined in capi.cu.
 void side_stream(otm_context* ctx);
-// Copies `bytes` from src (host or device) into dst (device), on the context stream; host
-// memory has been read when the call returns.
+// Copies `bytes` from src (host or device) into dst (device), on the context stream; pageable
+// host memory has been read when the call returns, pinned memory once the stream has been
+// synchronised.
 void copy_in(otm_context* ctx, void* dst, const void* src, size_t bytes);
 // Copies `bytes` from src (device) into dst (host or device), on the context stream; complete
 // once the stream has been synchronised (pageable memory: possibly on return).

@@ -292,10 +292,10 @@ static void exclusive_scan(cudaStream_t st, const int* counts, int* starts, int*
 // where they lie. Then each block takes the subtrees that start in its window of BVH_SUB
 // positions through all their remaining levels in shared memory. All 25 levels over the whole
 // array, nine kernels and two copies each and 52 bytes moved a face, took 1.73 ms for a
-// 1024^2 map, nearly all of it in passes over positions whose nodes were small. Now 0.74 ms go to the 20
-// levels of the first phase (bound by launches and by the dependent loads of each kernel: 37
-// us a level where the 20 MB it moves would take 4) and 0.25 ms to the second (bound by
-// its barriers; 512 threads on subtrees of up to 512 faces measured best among 128 .. 512 and
+// 1024^2 map, nearly all of it in passes over positions whose nodes were small. Now 0.56 ms go to the 20
+// levels of the first phase (bound by launches and by the dependent loads of each kernel: 28
+// us a level, 37 launched plainly, where the 20 MB it moves would take 4) and 0.25 ms to the
+// second (bound by its barriers; 512 threads on subtrees of up to 512 faces measured best among 128 .. 512 and
 // 128 .. 1024).
 
 constexpr int BVH_LEAF = 4, BVH_DEPTH = 24, BVH_SUB = 512;

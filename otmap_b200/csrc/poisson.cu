@@ -27,7 +27,8 @@
 // registers, 8 per thread on M/8 threads, as radix-8 passes (decimation in frequency; the
 // last radix is 2, 4 or 8) that trade elements through shared memory; the inverse runs
 // the passes backwards, so the digit-reversed order between the two is never undone.
-// Tables come from the host in extended precision, rounded once.
+// The passes' and the chirp's tables come from the host in extended precision, rounded once; the
+// quarter-wave twiddles and the cosines (pt, cosk) are formed in double, as for the other sizes.
 //
 // What it replaces: n not a power of two took four dense products with the cosine basis
 // (8 n^3 flops; 4 x 145 us at n = 500, 4 x 404 at 1000), 2048 and 4096 radix-4 passes over

@@ -600,7 +600,8 @@ static std::vector<Inst> layout_workspace(otm_context* ctx, const std::vector<in
   // sums 28 -> 24.5 us, update 21 -> 16.4 us; a lone 256^2 one 4). Several instances of one
   // register-transform size (the maps of a barycenter loss) stay at 16 rows: the height is the
   // order of the sums, and the gradient of a map whose adjoint ends at its limit of solves turns on
-  // the last bit of the mesh (four 64^2 take 24 us per iteration so, 19 with 4 rows). So does split
+  // the last bit of the mesh (four 64^2 take 24 us per iteration so, 19 with 4 rows; maps of other
+  // sizes and lone ones, whose heights have no such rule, are as sensitive). So does split
   // precision, whose FP32 fields turn any change of rounding into one of theirs (256^2 alone 39 us
   // per iteration with 16 rows, 33 with 4).
   int srows = 32;

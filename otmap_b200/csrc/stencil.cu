@@ -14,8 +14,8 @@
 //                  block advances the iteration and tests the loop condition (:160).
 //
 // Geometry: one warp owns a strip of 32 consecutive columns (j, contiguous in memory) and
-// Inst::srows rows (32; 64 when the batch has strips to spare, 16 when it has too few to
-// fill the SMs) and walks down it. Grid rows are prefetched asynchronously (cp.async) into
+// Inst::srows rows (32; 64 when the batch has strips to spare, 16, 8 or 4 when it has too few
+// to fill the SMs) and walks down it. Grid rows are prefetched asynchronously (cp.async) into
 // a per-warp ring of RD rows in shared memory, so RD-2 rows per warp are in flight while
 // it computes; the previous vertex-gradient row is kept in registers. The strip's two halo
 // columns are staged with the row; neighbours come from the ring. A block is SWARPS strips

@@ -7,7 +7,7 @@
 namespace otm {
 
 constexpr int SW = 32;        // strip width (one warp)
-// strip height (rows per warp): Inst::srows, 16, 32 or 64 per batch (layout_workspace)
+// strip height (rows per warp): Inst::srows, 4 to 64 per batch (layout_workspace)
 constexpr int SWARPS = 4;     // strips per block
 constexpr int ST = SW * SWARPS;
 constexpr int KA = SWEEP_SLOTS;  // partial-sum slots per block
