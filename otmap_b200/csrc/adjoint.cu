@@ -673,7 +673,8 @@ struct AdjointWs : otm_context::Erased {
   int n = 0, m = 0, maps = 0;
   size_t N = 0, V = 0, ld = 0;
   long stride = 0;  // doubles from one map's slice to the next one's
-  DevBuf recs, lists, ctls;
+  DevBuf recs;  // the Poisson records, then ctl and the work lists
+  int* lists = nullptr;
   double *b, *lam, *z, *h, *t1, *t2, *Vb, *c, *part, *sums, *hcol, *inv;  // of map 0
   double2* g;                // the call's vertex displacements
   double *H, *cs, *sn, *gv;  // the cycle's Hessenberg state
@@ -719,8 +720,6 @@ static AdjointWs* adjoint_ws(otm_context* ctx, int n, int m, int maps) {
     ctx->adjoint_buf.reserve(bytes);
   }
   double* q = ctx->adjoint_buf.as<double>();
-  W->ctls.reserve(sizeof(AdjCtl) * maps);
-  W->ctl = W->ctls.as<AdjCtl>();
   auto take = [&](size_t w) {
     double* r = q;
     q += up(w);
@@ -743,7 +742,6 @@ static AdjointWs* adjoint_ws(otm_context* ctx, int n, int m, int maps) {
   W->H = take((size_t)(m + 1) * m);
   W->cs = take(m);
   W->sn = take(m);
-  OTM_CUDA(cudaMemsetAsync(W->ctl, 0, sizeof(AdjCtl) * maps, ctx->stream));
   SizeTables* T = ctx->tables.at(n).get();
   Inst base;
   std::memset(&base, 0, sizeof(base));
@@ -782,14 +780,17 @@ static AdjointWs* adjoint_ws(otm_context* ctx, int n, int m, int maps) {
       r.gemm0 = y * base.ngemm;
     }
   }
-  W->recs.reserve(sizeof(Inst) * recs.size());
   // work list: item -> map, for the rows, the columns and the product tiles
   std::vector<int> items;
   for (int per : {base.nrow, base.ncol, base.ngemm})
     for (int y = 0; y < maps; ++y) items.insert(items.end(), per, y);
-  W->lists.reserve(sizeof(int) * items.size());
+  static_assert(sizeof(Inst) % alignof(AdjCtl) == 0 && sizeof(AdjCtl) % alignof(int) == 0, "one buffer for the three");
+  W->recs.reserve(sizeof(Inst) * recs.size() + sizeof(AdjCtl) * maps + sizeof(int) * items.size());
+  W->ctl = reinterpret_cast<AdjCtl*>(W->recs.as<Inst>() + recs.size());
+  W->lists = reinterpret_cast<int*>(W->ctl + maps);
+  OTM_CUDA(cudaMemsetAsync(W->ctl, 0, sizeof(AdjCtl) * maps, ctx->stream));
   OTM_CUDA(cudaMemcpyAsync(W->recs.p, recs.data(), sizeof(Inst) * recs.size(), cudaMemcpyHostToDevice, ctx->stream));
-  OTM_CUDA(cudaMemcpyAsync(W->lists.p, items.data(), sizeof(int) * items.size(), cudaMemcpyHostToDevice, ctx->stream));
+  OTM_CUDA(cudaMemcpyAsync(W->lists, items.data(), sizeof(int) * items.size(), cudaMemcpyHostToDevice, ctx->stream));
   OTM_CUDA(cudaStreamSynchronize(ctx->stream));
   ctx->adjoint[key] = std::move(own);
   return W;
@@ -798,7 +799,7 @@ static AdjointWs* adjoint_ws(otm_context* ctx, int n, int m, int maps) {
 // z = M^+ (source of the records of a kind), every map whose record is active
 static void poisson_rec(otm_context* ctx, AdjointWs* W, int kind) {
   Inst* d = W->rec(kind);
-  const int *L = W->lists.as<int>(), *LC = L + W->rows, *LG = LC + W->cols;
+  const int *L = W->lists, *LC = L + W->rows, *LG = LC + W->cols;
   if (W->fft) {
     if (W->reg)
       dct_reg_run(ctx, W->n, false, d, L, 0, W->rows, LC, 0, W->cols, W->col_warps);
