@@ -14,6 +14,29 @@ void set_error(const std::string& msg) { g_last_error = msg; }
 
 void make_current(otm_context* ctx) { OTM_CUDA(cudaSetDevice(ctx->device)); }
 
+// Stream-ordered allocation comes from a context's own memory pools; the device's default pool is
+// left as it is. keep: freed memory that stays in the pool when the driver synchronises.
+static cudaMemPool_t make_pool(int device, uint64_t keep) {
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.handleTypes = cudaMemHandleTypeNone;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  cudaMemPool_t pool = nullptr;
+  OTM_CUDA(cudaMemPoolCreate(&pool, &props));
+  if (const cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep); e != cudaSuccess) {
+    cudaMemPoolDestroy(pool);
+    OTM_CUDA(e);
+  }
+  return pool;
+}
+
+cudaMemPool_t temp_pool(otm_context* ctx) {
+  // temporaries have no object that owns them: they leave at most 4 GiB behind
+  if (!ctx->temps) ctx->temps = make_pool(ctx->device, uint64_t(4) << 30);
+  return ctx->temps;
+}
+
 void side_stream(otm_context* ctx) {
   if (!ctx->side) OTM_CUDA(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
   if (!ctx->side_ready) OTM_CUDA(cudaEventCreateWithFlags(&ctx->side_ready, cudaEventDisableTiming));
@@ -101,23 +124,10 @@ extern "C" int otm_create(int device, otm_context** out) {
       OTM_CUDA(cudaSetDevice(device));
       OTM_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
       OTM_CUDA(cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device));
-      // Stream-ordered allocation comes from this context's own memory pools; the device's
-      // default pool is left as it is. The per-map buffers' pool keeps what is freed for the
-      // next map instead of returning it to the driver at every synchronisation, without a
-      // limit: the reserved memory that a limit is compared with includes that of the live maps
-      // (with 4 GiB creating and dropping a 16384^2 map took 28 ms, without 2.0). The calls'
-      // temporaries, which have no such owner, leave at most 4 GiB behind.
-      cudaMemPoolProps props = {};
-      props.allocType = cudaMemAllocationTypePinned;
-      props.handleTypes = cudaMemHandleTypeNone;
-      props.location.type = cudaMemLocationTypeDevice;
-      props.location.id = device;
-      auto make_pool = [&](cudaMemPool_t* pool, uint64_t keep) {
-        OTM_CUDA(cudaMemPoolCreate(pool, &props));
-        OTM_CUDA(cudaMemPoolSetAttribute(*pool, cudaMemPoolAttrReleaseThreshold, &keep));
-      };
-      make_pool(&ctx->pool, UINT64_MAX);
-      make_pool(&ctx->temps, uint64_t(4) << 30);
+      // the per-map buffers' pool keeps what is freed for the next map, without a limit: the reserved
+      // memory that a limit is compared with includes that of the live maps (with 4 GiB creating and
+      // dropping a 16384^2 map took 28 ms, without 2.0)
+      ctx->pool = make_pool(device, UINT64_MAX);
     } catch (...) {
       delete ctx;
       throw;

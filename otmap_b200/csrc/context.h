@@ -124,7 +124,7 @@ struct otm_context {
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaMemPool_t pool = nullptr;   // stream-ordered allocations of the per-map buffers
-  cudaMemPool_t temps = nullptr;  // and of the calls' temporaries
+  cudaMemPool_t temps = nullptr;  // and of the calls' temporaries (temp_pool)
   int num_sms = 0;
   long launches = 0;  // kernels launched by this context since creation
   int poisson_mode = 0;  // OTM_POISSON_AUTO / _DENSE / _FFT
@@ -204,6 +204,8 @@ struct otm_map {
 namespace otm {
 // Makes the context's device current; defined in capi.cu.
 void make_current(otm_context* ctx);
+// The pool of the calls' temporaries, created on first use; defined in capi.cu.
+cudaMemPool_t temp_pool(otm_context* ctx);
 // Creates the context's second stream and its event, once; defined in capi.cu.
 void side_stream(otm_context* ctx);
 // Copies `bytes` from src (host or device) into dst (device), on the context stream; pageable

@@ -2103,7 +2103,7 @@ void raster_grid_backward(otm_context* ctx, int n, const double* xy, int rows, i
   const double* value = reinterpret_cast<const double*>(base);
   const int* owner = reinterpret_cast<const int*>(base + al(sizeof(double) * (size_t)(N > 0 ? N : 1)));
   AsyncBuf dA;
-  dA.reserve(sizeof(double) * N, ctx->stream, ctx->temps);
+  dA.reserve(sizeof(double) * N, ctx->stream, temp_pool(ctx));
   MeshRef m{xy, n, N, (n + 1) * (n + 1), nullptr, nullptr};
   launch(ctx, "raster_area_grad", k_raster_area_grad, (N + 255) / 256, 256, m, rows, cols, value, owner, dL_dpix,
          dA.as<double>());
@@ -2122,7 +2122,7 @@ void inverse_grid_backward(otm_context* ctx, int n, const double* fwd, const int
   const size_t b_pg = al(sizeof(InvGrad) * V), b_cnt = al(sizeof(int) * (N + 1)), b_list = al(sizeof(int) * V);
   const size_t b_cs = al(sizeof(double2) * 4 * (size_t)N), b_sums = al(sizeof(int) * ((N + SCAN_B - 1) / SCAN_B + 1));
   AsyncBuf buf;
-  buf.reserve(b_pg + 3 * b_cnt + b_list + b_cs + b_sums, st, ctx->temps);
+  buf.reserve(b_pg + 3 * b_cnt + b_list + b_cs + b_sums, st, temp_pool(ctx));
   char* q = buf.as<char>();
   InvGrad* pg = reinterpret_cast<InvGrad*>(q);
   int* count = reinterpret_cast<int*>(q + b_pg);
@@ -2347,15 +2347,15 @@ static void raster_mesh(otm_context* ctx, const MeshRef& m, const double* densit
     } else {
       int nref = 0;
       OTM_CUDA(cudaMemcpyAsync(&nref, m.start + nf, sizeof(int), cudaMemcpyDeviceToHost, st));
-      vcount.reserve(sizeof(int) * m.nv, st, ctx->temps);
-      vstart.reserve(sizeof(int) * (m.nv + 1), st, ctx->temps);
-      vsums.reserve(sizeof(int) * ((m.nv + SCAN_B - 1) / SCAN_B + 1), st, ctx->temps);
-      inv_area.reserve(sizeof(double) * (size_t)(nf > 0 ? nf : 1), st, ctx->temps);
+      vcount.reserve(sizeof(int) * m.nv, st, temp_pool(ctx));
+      vstart.reserve(sizeof(int) * (m.nv + 1), st, temp_pool(ctx));
+      vsums.reserve(sizeof(int) * ((m.nv + SCAN_B - 1) / SCAN_B + 1), st, temp_pool(ctx));
+      inv_area.reserve(sizeof(double) * (size_t)(nf > 0 ? nf : 1), st, temp_pool(ctx));
       OTM_CUDA(cudaMemsetAsync(vcount.p, 0, sizeof(int) * m.nv, st));
       launch(ctx, "vf_count", k_vf_count, fblocks, 256, m, vcount.as<int>());
       exclusive_scan(st, vcount.as<int>(), vstart.as<int>(), vsums.as<int>(), m.nv);
       OTM_CUDA(cudaStreamSynchronize(st));
-      vfaces.reserve(sizeof(int) * (size_t)(nref > 0 ? nref : 1), st, ctx->temps);
+      vfaces.reserve(sizeof(int) * (size_t)(nref > 0 ? nref : 1), st, temp_pool(ctx));
       OTM_CUDA(cudaMemsetAsync(vcount.p, 0, sizeof(int) * m.nv, st));
       launch(ctx, "vf_fill", k_vf_fill, fblocks, 256, m, (const int*)vstart.as<int>(), vcount.as<int>(),
              vfaces.as<int>(), inv_area.as<double>());
@@ -2405,20 +2405,20 @@ extern "C" int otm_rasterize_mode(otm_context* ctx, int n, const double* xy, con
     AsyncBuf dxy, dden, dimg;
     const double* pxy = xy;
     if (!is_device_ptr(xy)) {
-      dxy.reserve(sizeof(double) * 2 * V, st, ctx->temps);
+      dxy.reserve(sizeof(double) * 2 * V, st, temp_pool(ctx));
       copy_in(ctx, dxy.p, xy, sizeof(double) * 2 * V);
       pxy = dxy.as<double>();
     }
     const double* pden = density;
     if (density && !is_device_ptr(density)) {
-      dden.reserve(sizeof(double) * N, st, ctx->temps);
+      dden.reserve(sizeof(double) * N, st, temp_pool(ctx));
       copy_in(ctx, dden.p, density, sizeof(double) * N);
       pden = dden.as<double>();
     }
     bool idev = is_device_ptr(img);
     double* pimg = img;
     if (!idev) {
-      dimg.reserve(sizeof(double) * pix, st, ctx->temps);
+      dimg.reserve(sizeof(double) * pix, st, temp_pool(ctx));
       pimg = dimg.as<double>();
     }
     raster_grid(ctx, n, pxy, pden, rows, cols, mode, pimg);
@@ -2438,7 +2438,7 @@ extern "C" int otm_rasterize_faces(otm_context* ctx, int n, const double* xy, in
     cudaStream_t st = ctx->stream;
     const size_t V2 = 2 * (size_t)(n + 1) * (n + 1), pix = (size_t)rows * cols;
     AsyncBuf buf;
-    buf.reserve(sizeof(double) * (V2 + pix) + 256, st, ctx->temps);
+    buf.reserve(sizeof(double) * (V2 + pix) + 256, st, temp_pool(ctx));
     const double* pxy = xy;
     if (!is_device_ptr(xy)) {
       copy_in(ctx, buf.p, xy, sizeof(double) * V2);
@@ -2494,27 +2494,27 @@ extern "C" int otm_rasterize_mesh(otm_context* ctx, int nv, const double* xy, in
     AsyncBuf dxy, dden, dimg, dstart, didx;
     const double* pxy = xy;
     if (nv > 0 && !is_device_ptr(xy)) {
-      dxy.reserve(sizeof(double) * 2 * (size_t)nv, st, ctx->temps);
+      dxy.reserve(sizeof(double) * 2 * (size_t)nv, st, temp_pool(ctx));
       copy_in(ctx, dxy.p, xy, sizeof(double) * 2 * (size_t)nv);
       pxy = dxy.as<double>();
     }
     const double* pden = density;
     if (density && !is_device_ptr(density)) {
-      dden.reserve(sizeof(double) * (size_t)cells, st, ctx->temps);
+      dden.reserve(sizeof(double) * (size_t)cells, st, temp_pool(ctx));
       copy_in(ctx, dden.p, density, sizeof(double) * (size_t)cells);
       pden = dden.as<double>();
     }
     bool idev = is_device_ptr(img);
     double* pimg = img;
     if (!idev) {
-      dimg.reserve(sizeof(double) * pix, st, ctx->temps);
+      dimg.reserve(sizeof(double) * pix, st, temp_pool(ctx));
       pimg = dimg.as<double>();
     }
     if (nf == 0) {
       OTM_CUDA(cudaMemsetAsync(pimg, 0, sizeof(double) * pix, st));
     } else {
-      dstart.reserve(sizeof(int) * ((size_t)nf + 1), st, ctx->temps);
-      didx.reserve(sizeof(int) * (size_t)total, st, ctx->temps);
+      dstart.reserve(sizeof(int) * ((size_t)nf + 1), st, temp_pool(ctx));
+      didx.reserve(sizeof(int) * (size_t)total, st, temp_pool(ctx));
       copy_in(ctx, dstart.p, hstart.data(), sizeof(int) * ((size_t)nf + 1));
       copy_in(ctx, didx.p, hidx.data(), sizeof(int) * (size_t)total);
       MeshRef m{pxy, 0, nf, nv, dstart.as<int>(), didx.as<int>()};
@@ -2571,26 +2571,26 @@ extern "C" int otm_sample_image(otm_context* ctx, int nv, const double* xy, int 
     AsyncBuf dxy, dspf, dimg, dstart, didx;
     const double* pxy = xy;
     if (nv > 0 && !is_device_ptr(xy)) {
-      dxy.reserve(sizeof(double) * 2 * (size_t)nv, st, ctx->temps);
+      dxy.reserve(sizeof(double) * 2 * (size_t)nv, st, temp_pool(ctx));
       copy_in(ctx, dxy.p, xy, sizeof(double) * 2 * (size_t)nv);
       pxy = dxy.as<double>();
     }
     const int* pspf = samples_per_face;
     if (nf > 0 && !is_device_ptr(samples_per_face)) {
-      dspf.reserve(sizeof(int) * (size_t)nf, st, ctx->temps);
+      dspf.reserve(sizeof(int) * (size_t)nf, st, temp_pool(ctx));
       copy_in(ctx, dspf.p, samples_per_face, sizeof(int) * (size_t)nf);
       pspf = dspf.as<int>();
     }
     const bool idev = is_device_ptr(img);
     double* pimg = img;
     if (!idev) {
-      dimg.reserve(sizeof(double) * pix, st, ctx->temps);
+      dimg.reserve(sizeof(double) * pix, st, temp_pool(ctx));
       pimg = dimg.as<double>();
     }
     MeshRef m{pxy, grid ? grid_n : 0, nf, nv, nullptr, nullptr};
     if (!grid && nf > 0) {
-      dstart.reserve(sizeof(int) * ((size_t)nf + 1), st, ctx->temps);
-      didx.reserve(sizeof(int) * hidx.size(), st, ctx->temps);
+      dstart.reserve(sizeof(int) * ((size_t)nf + 1), st, temp_pool(ctx));
+      didx.reserve(sizeof(int) * hidx.size(), st, temp_pool(ctx));
       copy_in(ctx, dstart.p, hstart.data(), sizeof(int) * hstart.size());
       copy_in(ctx, didx.p, hidx.data(), sizeof(int) * hidx.size());
       m.start = dstart.as<int>();

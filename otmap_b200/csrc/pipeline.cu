@@ -179,7 +179,7 @@ extern "C" int otm_mesh_blend(otm_context* ctx, int n, int count, const double* 
     cudaStream_t st = ctx->stream;
     const size_t V2 = 2 * (size_t)(n + 1) * (n + 1);
     AsyncBuf buf;
-    buf.reserve(sizeof(double) * (V2 * (count + 1) + count + 8) + sizeof(double*) * count, st, ctx->temps);
+    buf.reserve(sizeof(double) * (V2 * (count + 1) + count + 8) + sizeof(double*) * count, st, temp_pool(ctx));
     double* base = buf.as<double>();
     std::vector<const double*> ptrs = stage_meshes(ctx, meshes, count, V2, base);
     double* d_out = base + V2 * count;
@@ -209,7 +209,7 @@ extern "C" int otm_transport_cost(otm_context* ctx, int n, const double* src_xy,
     const size_t V2 = 2 * (size_t)(n + 1) * (n + 1), N = (size_t)n * n;
     const int nb = 512;
     AsyncBuf buf;
-    buf.reserve(sizeof(double) * (2 * V2 + 2 * N + 2 * nb + 8), st, ctx->temps);
+    buf.reserve(sizeof(double) * (2 * V2 + 2 * N + 2 * nb + 8), st, temp_pool(ctx));
     double* p = buf.as<double>();
     auto in = [&](const double* src, double* tmp, size_t words) -> const double* {
       if (is_device_ptr(src)) return src;
@@ -248,7 +248,7 @@ extern "C" int otm_barycenter(otm_context* ctx, int n, int count, const double* 
     const size_t V2 = 2 * (size_t)(n + 1) * (n + 1), pix = (size_t)rows * cols;
     const int nparts = 512;
     AsyncBuf buf;
-    buf.reserve(sizeof(double) * (V2 * (count + 1) + count + pix + nparts + 16) + sizeof(double*) * count, st, ctx->temps);
+    buf.reserve(sizeof(double) * (V2 * (count + 1) + count + pix + nparts + 16) + sizeof(double*) * count, st, temp_pool(ctx));
     double* base = buf.as<double>();
     std::vector<const double*> ptrs = stage_meshes(ctx, inv_meshes, count, V2, base);
     double* d_mesh = base + V2 * count;
@@ -292,7 +292,7 @@ extern "C" int otm_grid_transport_cost(otm_context* ctx, int n, const double* gr
     const size_t V2 = 2 * (size_t)(n + 1) * (n + 1), N = (size_t)n * n;
     const int nb = 512;
     AsyncBuf buf;
-    buf.reserve(sizeof(double) * (V2 + 2 * N + nb + 8), st, ctx->temps);
+    buf.reserve(sizeof(double) * (V2 + 2 * N + nb + 8), st, temp_pool(ctx));
     double* p = buf.as<double>();
     const double* d_g = grads_xy;
     if (!is_device_ptr(grads_xy)) {
@@ -408,7 +408,7 @@ extern "C" int otm_barycenter_loss(otm_context* ctx, int n, int count, const dou
     // g, partials, scalars, blend pointers and weights
     const size_t per = al(N) * 3 + al(V2) * 3 + al((V + 1) / 2);
     AsyncBuf buf;
-    buf.reserve(sizeof(double) * (per * count + al(V2) * 2 + al(pix) * 3 + al(2 * nparts) + al(64) + al(8) * 2), st, ctx->temps);
+    buf.reserve(sizeof(double) * (per * count + al(V2) * 2 + al(pix) * 3 + al(2 * nparts) + al(64) + al(8) * 2), st, temp_pool(ctx));
     double* p = buf.as<double>();
     auto take = [&](size_t w) {
       double* r = p;
