@@ -3,6 +3,7 @@ call, whatever numbers of maps and sizes came before, and a call's gradient does
 what the others left there."""
 
 import ctypes as C
+import gc
 
 import numpy as np
 import pytest
@@ -39,6 +40,7 @@ def test_memory_is_that_of_the_largest_call():
     from otmap_b200 import native as N
 
     n = 512  # 41 basis vectors and 8 others of 2 MiB for each map
+    gc.collect()  # contexts of other tests
     ctx = N.Context(0)
     _loss(ctx, n, 8)
     torch.cuda.empty_cache()

@@ -2,6 +2,7 @@
 map; of a call's temporaries at most 4 GiB; nothing once it is destroyed."""
 
 import ctypes as C
+import gc
 
 import pytest
 
@@ -31,6 +32,7 @@ def test_map_buffers_are_kept():
     n = 12288
     xy, density = _mesh(n), torch.ones(n * n, dtype=torch.float64, device="cuda")
     size = 8 * (xy.numel() + density.numel())  # 3.6e9: above 4 GiB together with a second map's
+    gc.collect()  # contexts of other tests
     torch.cuda.empty_cache()
     ctx = N.Context(0)
     free = _free()
@@ -61,6 +63,7 @@ def test_temporaries_are_given_back():
     n, count = 8192, 6
     xy = _mesh(n)
     out = torch.empty_like(xy)
+    gc.collect()  # contexts of other tests
     torch.cuda.empty_cache()
     ctx = N.Context(0)
     free = _free()
