@@ -1596,7 +1596,7 @@ __global__ __launch_bounds__(128) void k_raster_stale(MeshRef m, int rows, int c
 // 90 FP64 and 150 other instructions for each of 4.6 tests per face. With one thread per
 // (face, box row) for every face, found by a binary search over 2^20 row counts, and the
 // divisions of bilinear_from_terms in every test, the pass took 148 us at 1024^2 beside 30
-// of boxes, counting and scanning; now 67 us in all (a raster call 222 -> 114 us; the owner
+// of boxes, counting and scanning; now 67 us in all (a raster call 228 -> 105 us; the owner
 // part of a 512^2 barycenter image 83 -> 38 us).
 constexpr int SMALL_BOX = 32, RF_T = 128;
 // Largest box on the first list: a smooth 100^2 mesh drawn at 1400^2 (boxes of 210 to 260 pixels) takes
